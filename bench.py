@@ -7,9 +7,9 @@ same values in separate buffers, d has its own seed).  One step evaluates all
 six contract_enum.h contraction types with Gamma_ij = Gamma_kl = C g5
 (Gamma(5)) for the two projectors (1 +- g4)/2 at zero momentum, i.e. 12
 site-contractions per site, reduced per timeslice.  The headline passes the
-two u buffers, so it evaluates both triangle passes; ``mixed_same_field``
+two u buffers, so it forms all 64 colour wedges of a site; ``mixed_same_field``
 times the same step with one u buffer passed twice, where the library
-evaluates one triangle pass (reported beside the headline, not as it).
+forms half of them (reported beside the headline, not as it).
 
 Metric: GSite/s = site-contractions per second / 1e9 for the mixed form
 (complex64 storage, FP32 arithmetic, FP64 per-timeslice reduction) with the
@@ -46,16 +46,10 @@ GAMMA_CG5 = 5
 N_TYPES = 6
 N_PROJ = 2
 UNITS_PER_SITE = N_TYPES * N_PROJ
-# Complex FMAs per site of the fused kernel's shared-wedge form (16 threads per site, one
-# (i, x) pair each): 4 wedges a ^ P_j[j][n] (36 each), each dotted with the N blocks of
-# both triangle passes for the 2 gamma-basis terms (4 x 9), the loop form's 2 x 9 dots
-# with Q_w, and the projector coefficients 2 x 2 x 2; Q set-up 18 x 3.  8 flops per
-# complex FMA.
-FUSED_CFMA_PER_SITE = 16 * (4 * (36 + 4 * 9) + 2 * 9 + 2 * 2 * 2) + 18 * 3
-# The compiled op behind each tile-shape name of the fused complex64 pass.
-FUSED_KERNELS = {"shared": "BaryonFusedSharedWedgeOp", "merged": "BaryonFusedCliffMergedOp",
-                 "shared_same": "BaryonFusedSharedWedgeSameOp", "same": "BaryonFusedCliffMergedOp (SAMEIJ)",
-                 "cw": "BaryonFusedCliffOp"}
+# Complex FMAs per site of the fused kernel (open-diquark form): 64 colour wedges of 36, then for
+# each of the two triangle passes and the 2 gamma-basis terms 16 colour dots of 9, and the loop's
+# 9 colour entries times 2 terms.  8 flops per complex FMA.
+FUSED_CFMA_PER_SITE = 64 * 36 + 2 * 2 * 16 * 9 + 9 * 2
 WORKLOAD = "baryon_2pt_24c64"
 METRIC = "GSite/s & HBM GB/s: mixed vs FP64 GPU contraction at <=1e-6 rel err/timeslice"
 
@@ -304,8 +298,8 @@ def fused_kernel_name(lib, v):
     tuner's choice, else the default shape)."""
     for key, name, _ in autotune_report(lib):
         if key.startswith("kind=3,prec=1,aux=2,") and f"volume={v}," in key:
-            return f"{FUSED_KERNELS.get(name.split('.')[0], '?')} ({name})"
-    return "BaryonFusedSharedWedgeOp (shared.cw4.tps16.st2.occ3)"
+            return f"BaryonFusedOp ({name})"
+    return "BaryonFusedOp (w12.tps8.occ1)"
 
 
 def run_reference(args, world, rank):

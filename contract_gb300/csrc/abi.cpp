@@ -166,11 +166,12 @@ struct DeviceWorkspace : cgb::Workspace {
 struct StaticWorkspace : cgb::Workspace {
   void *base = nullptr;
   size_t cap = 0;
+  size_t least = 0;  // every request counts as at least this much
   size_t requested = 0;
   void *get(size_t bytes) override
   {
-    requested = bytes;
-    return bytes <= cap ? base : nullptr;
+    requested = std::max(bytes, least);
+    return requested <= cap ? base : nullptr;
   }
 };
 
@@ -608,6 +609,7 @@ void fill_rank(cgb::RankForm<double> &rk, const double *w)
     }
   rk.r = r;
   rk.nnz = nnz;
+  std::memcpy(rk.x, x, sizeof(x));
   // Unit form: within each vector every nonzero entry is the same modulus times
   // a power of i, and the product of a pair's two moduli is the same for every r.
   rk.unit = 1;
@@ -1728,6 +1730,8 @@ int contract_baryon_all_types_noalloc(void *correl, const void *propag_i, const 
   if (!make_job(job, precision, volume, lattice, &s)) return contract_last_error();
   StaticWorkspace ws;
   if (!cuda_ok(cgb::static_scratch(&ws.base, &ws.cap), "static scratch address")) return contract_last_error();
+  // three records per half-timeslice are the entry point's rule (see the header), whatever the tile shape leaves
+  ws.least = (size_t)2 * lattice[3] * 3 * 6 * nproj * 16;
   job.ws = &ws;
   OpParams<double> p {};
   p.in[0] = propag_i;

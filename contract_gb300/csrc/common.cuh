@@ -124,28 +124,43 @@ template <int TPS, class R> __device__ __forceinline__ cx<R> group_sum(cx<R> v)
   return v;
 }
 
-// Sum each of NOUT values over the TPS threads of a site and leave the sum of
-// value o with the thread whose sub == o (o < NOUT <= TPS), by recursive
-// halving: at the step of lane distance h the thread keeps the upper or lower
-// half of its values as (sub & h) says and receives its partner's share of
-// that half, so TPS - 1 shuffles in all instead of NOUT log2(TPS).
-template <int TPS, int NOUT> constexpr bool kScatterSums = NOUT > TPS / 2 && NOUT <= TPS;
-template <int TPS, int NOUT, class R>
-__device__ __forceinline__ cx<R> group_reduce_scatter(const cx<R> (&vals)[NOUT], int sub)
+// Sum each of NVAL values over the TPS threads of a site, leaving the sum of
+// value r with the 2^SH threads whose sub >> SH == r: recursive halving while
+// a thread holds more than one value (at the step of lane distance h it keeps
+// the upper or lower half as (sub & h) says and receives its partner's share of
+// that half), then a butterfly over the threads that share one.
+template <int NVAL> constexpr int values_pow2()
 {
-  static_assert(NOUT <= TPS && (TPS & (TPS - 1)) == 0, "one value per thread, TPS a power of two");
-  cx<R> v[TPS];
+  int p = 1;
+  while (p < NVAL) p *= 2;
+  return p;
+}
+template <int TPS, int NVAL> constexpr int values_shift()
+{
+  int sh = 0;
+  while ((values_pow2<NVAL>() << sh) < TPS) ++sh;
+  return sh;
+}
+template <int TPS, int NVAL, class R>
+__device__ __forceinline__ cx<R> group_reduce_values(const cx<R> (&vals)[NVAL], int sub)
+{
+  constexpr int P = values_pow2<NVAL>();
+  static_assert(P <= TPS, "at most one value per thread");
+  cx<R> v[P];
 #pragma unroll
-  for (int i = 0; i < TPS; ++i) v[i] = i < NOUT ? vals[i] : czero<R>();
+  for (int i = 0; i < P; ++i) v[i] = i < NVAL ? vals[i] : czero<R>();
+  int h = TPS / 2;
 #pragma unroll
-  for (int h = TPS / 2; h > 0; h >>= 1) {
+  for (int m = P / 2; m > 0; m >>= 1, h >>= 1) {
     const bool hi = (sub & h) != 0;
 #pragma unroll
-    for (int i = 0; i < h; ++i) {
-      const cx<R> send = hi ? v[i] : v[h + i], keep = hi ? v[h + i] : v[i];
+    for (int i = 0; i < m; ++i) {
+      const cx<R> send = hi ? v[i] : v[m + i], keep = hi ? v[m + i] : v[i];
       v[i] = cadd(keep, shfl_xor(send, h));
     }
   }
+#pragma unroll
+  for (; h > 0; h >>= 1) v[0] = cadd(v[0], shfl_xor(v[0], h));
   return v[0];
 }
 

@@ -62,8 +62,11 @@ struct TileGeom {
   int withhold_chunk;
 };
 
+// A CTA's walk over its tiles.  The chunk's place is worked out once per chunk;
+// a tile then costs an add (every consumer warp walks).
 template <int SITES> struct TileIter {
   int chunk, k, ntiles;
+  long long first, end;  // first site of the tile, end of its segment
 
   __device__ __forceinline__ void set_chunk(const TileGeom &g, int c)
   {
@@ -71,23 +74,19 @@ template <int SITES> struct TileIter {
     k = 0;
     ntiles = 0;
     if (c < g.total_chunks) {
-      const int cc = c % g.chunks_per_seg;
+      const int seg = c / g.chunks_per_seg, cc = c - seg * g.chunks_per_seg;
       ntiles = min(g.chunk_tiles, g.tiles_per_seg - cc * g.chunk_tiles);
+      first = (long long)seg * g.seg_len + (long long)cc * g.chunk_tiles * SITES;
+      end = (long long)(seg + 1) * g.seg_len;
     }
   }
   __device__ __forceinline__ bool valid(const TileGeom &g) const { return chunk < g.total_chunks; }
   __device__ __forceinline__ bool last_in_chunk() const { return k == ntiles - 1; }
-  __device__ __forceinline__ void next(const TileGeom &g)
+  __device__ __forceinline__ int sites() const { return (int)min((long long)SITES, end - first); }
+  __device__ __forceinline__ void next(const TileGeom &g, int stride)
   {
-    if (++k == ntiles) set_chunk(g, chunk + gridDim.x);
-  }
-  __device__ __forceinline__ void sites(const TileGeom &g, long long &first, int &n) const
-  {
-    const int seg = chunk / g.chunks_per_seg;
-    const int cc = chunk % g.chunks_per_seg;
-    const long long t = (long long)cc * g.chunk_tiles + k;
-    first = (long long)seg * g.seg_len + t * SITES;
-    n = (int)min((long long)SITES, g.seg_len - t * SITES);
+    first += SITES;
+    if (++k == ntiles) set_chunk(g, chunk + stride);
   }
 };
 
@@ -119,7 +118,7 @@ template <class Op> struct OutLayout {
 //   [0, 128)        full[NST], empty[NST] mbarriers, abort flag
 //   stages          NST x NIN x SITES slots
 //   extra           SITES x EXTRA_BYTES (per-site op scratch)
-//   tail            scalar ops: per-warp site values [CW][SPW][NOUT] (cx<R>)
+//   tail            scalar ops of several outputs: per-warp site values [CW][SPW][NOUT] (cx<R>)
 //                   field ops:  per-warp output staging [CW][2][SPW] slots
 template <class Op> struct Smem {
   using L = OpLayout<Op>;
@@ -131,6 +130,7 @@ template <class Op> struct Smem {
   {
     if constexpr (Op::FIELD && Op::DIRECT_OUT) return 0;
     else if constexpr (Op::FIELD) return 2ull * Op::SITES * OutLayout<Op>::SLOT;
+    else if constexpr (Op::NOUT == 1) return 0;
     else return (size_t)Op::SITES * Op::NOUT * 2 * sizeof(typename Op::R);
   }
   static constexpr size_t BYTES = TAIL + tail_bytes();
@@ -224,12 +224,11 @@ __device__ __forceinline__ void produce(const typename Op::Params &p, unsigned c
     }
     if (*abort_flag) return;
     if (it.k == 0 && it.chunk == g.withhold_chunk) {  // test hook: this tile never arrives
-      it.next(g);
+      it.next(g, gridDim.x);
       continue;
     }
-    long long first;
-    int n;
-    it.sites(g, first, n);
+    const long long first = it.first;
+    const int n = it.sites();
     if (lane == 0) mbar_arrive_expect_tx(&full[stage], (uint32_t)n * NIN * L::SITE_BYTES);
     __syncwarp();
     unsigned char *dst = smem + Smem<Op>::STAGES + stage * Smem<Op>::STAGE;
@@ -238,7 +237,7 @@ __device__ __forceinline__ void produce(const typename Op::Params &p, unsigned c
       bulk_g2s(dst + ((size_t)q * SITES + s) * L::SLOT,
                static_cast<const char *>(p.in[q]) + (first + s) * L::SITE_BYTES, L::SITE_BYTES, &full[stage]);
     }
-    it.next(g);
+    it.next(g, gridDim.x);
   }
 }
 
@@ -250,6 +249,20 @@ template <int NST> __device__ void drain(uint64_t *full, int from, unsigned long
 }
 
 // ------------------------------------------------------------ scalar ops --
+// A chunk's sums of a warp: every lane sums the value it holds of its own site
+// (after the site's threads joined theirs), and the warp's sites meet in FP64
+// when the chunk ends.
+template <int TPS, class R> __device__ __forceinline__ double2 warp_chunk_sum(const ChunkSum<R> &acc)
+{
+  double2 v = acc.value();
+#pragma unroll
+  for (int o = 16; o >= TPS; o >>= 1) {
+    v.x += __shfl_xor_sync(0xffffffffu, v.x, o);
+    v.y += __shfl_xor_sync(0xffffffffu, v.y, o);
+  }
+  return v;
+}
+
 template <class Op>
 __global__ void __launch_bounds__(Op::THREADS, min_blocks<Op>()) scalar_kernel(const __grid_constant__ typename Op::Params p)
 {
@@ -286,15 +299,14 @@ __global__ void __launch_bounds__(Op::THREADS, min_blocks<Op>()) scalar_kernel(c
   const int site = w * SPW + local;
   cx<R> *sv = reinterpret_cast<cx<R> *>(smem + Smem<Op>::TAIL) + (size_t)w * SPW * NOUT;  // [SPW][NOUT]
   S *scratch = reinterpret_cast<S *>(smem + Smem<Op>::EXTRA + (size_t)site * Op::EXTRA_BYTES);
-  ChunkSum<R> chunk_acc;  // lane o < NOUT: output o
+  ChunkSum<R> chunk_acc;
 
   TileIter<SITES> it;
   it.set_chunk(g, blockIdx.x);
   for (int u = 0; it.valid(g); ++u) {
     const int stage = u % NST;
-    long long first;
-    int n;
-    it.sites(g, first, n);
+    const long long first = it.first;
+    const int n = it.sites();
     const bool ok = mbar_wait_bounded(&full[stage], (u / NST) & 1, g.wait_ns);
     if (!__all_sync(0xffffffffu, ok) || *abort_flag) {
       if (lane == 0) {
@@ -310,31 +322,6 @@ __global__ void __launch_bounds__(Op::THREADS, min_blocks<Op>()) scalar_kernel(c
     for (int q = 0; q < NIN; ++q) in[q] = reinterpret_cast<const S *>(sb + ((size_t)q * SITES + site) * L::SLOT);
     cx<R> vals[NOUT];
     Op::site(ps, in, scratch, sub, vals);
-    if constexpr (kScatterSums<TPS, NOUT>) {
-      // many outputs: thread sub keeps the site sum of output sub
-      const cx<R> mine = group_reduce_scatter<TPS, NOUT>(vals, sub);
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&empty[stage]);  // inputs consumed; only registers below
-      const bool valid = site < n;
-      if (g.per_site) {
-        if (sub < NOUT && valid)
-          static_cast<double2 *>(p.out[sub])[first + site] = make_double2(double(mine.x), double(mine.y));
-      } else {
-        if (sub < NOUT) sv[local * NOUT + sub] = valid ? mine : czero<R>();
-        __syncwarp();
-        if (lane < NOUT) {
-#pragma unroll
-          for (int s = 0; s < SPW; ++s) chunk_acc.add(sv[s * NOUT + lane]);
-          if (it.last_in_chunk()) {
-            static_cast<double2 *>(p.out[0])[((size_t)it.chunk * CW + w) * NOUT + lane] = chunk_acc.value();
-            chunk_acc.reset();
-          }
-        }
-        __syncwarp();
-      }
-      it.next(g);
-      continue;
-    }
 #pragma unroll
     for (int o = 0; o < NOUT; ++o) vals[o] = group_sum<TPS>(vals[o]);
     __syncwarp();
@@ -345,6 +332,13 @@ __global__ void __launch_bounds__(Op::THREADS, min_blocks<Op>()) scalar_kernel(c
 #pragma unroll
         for (int o = 0; o < NOUT; ++o)
           static_cast<double2 *>(p.out[o])[first + site] = make_double2(double(vals[o].x), double(vals[o].y));
+      }
+    } else if constexpr (NOUT == 1) {
+      chunk_acc.add(valid ? vals[0] : czero<R>());
+      if (it.last_in_chunk()) {
+        const double2 z = warp_chunk_sum<TPS>(chunk_acc);
+        if (lane == 0) static_cast<double2 *>(p.out[0])[(size_t)it.chunk * CW + w] = z;
+        chunk_acc.reset();
       }
     } else {
       if (sub == 0) {
@@ -362,7 +356,7 @@ __global__ void __launch_bounds__(Op::THREADS, min_blocks<Op>()) scalar_kernel(c
       }
       __syncwarp();
     }
-    it.next(g);
+    it.next(g, gridDim.x);
   }
 }
 
@@ -408,9 +402,8 @@ __global__ void __launch_bounds__(Op::THREADS, min_blocks<Op>()) field_kernel(co
   it.set_chunk(g, blockIdx.x);
   for (int u = 0; it.valid(g); ++u) {
     const int stage = u % NST;
-    long long first;
-    int n;
-    it.sites(g, first, n);
+    const long long first = it.first;
+    const int n = it.sites();
     const bool ok = mbar_wait_bounded(&full[stage], (u / NST) & 1, g.wait_ns);
     if (!__all_sync(0xffffffffu, ok) || *abort_flag) {
       if (lane == 0) {
@@ -438,7 +431,7 @@ __global__ void __launch_bounds__(Op::THREADS, min_blocks<Op>()) field_kernel(co
       __syncwarp();
       if (lane == 0) mbar_arrive(&empty[stage]);
       __syncwarp();
-      it.next(g);
+      it.next(g, gridDim.x);
       continue;
     }
     unsigned char *ob = outbuf + (size_t)(u & 1) * SPW * O::SLOT;
@@ -462,7 +455,7 @@ __global__ void __launch_bounds__(Op::THREADS, min_blocks<Op>()) field_kernel(co
       bulk_wait_read<1>();  // the other staging buffer is free again
     }
     __syncwarp();
-    it.next(g);
+    it.next(g, gridDim.x);
   }
   if (lane == 0) bulk_wait<0>();
 }

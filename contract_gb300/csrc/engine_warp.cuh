@@ -1,0 +1,181 @@
+// Tile pipeline of the all-types baryon pass: every warp streams its own tiles.
+//
+// A tile is SPW = 32 / TPS consecutive sites of one reduction segment (a
+// half-timeslice, or the whole volume for per-site outputs); chunks of tiles
+// are dealt to warps, round-robin (ChunkWalk) or from a device queue
+// (QueueWalk, batch.cuh).  A warp owns one shared-memory slot per site and
+// input, filled with cp.async.bulk by its own lanes, and two mbarriers.  Ops
+// work in two steps (Op::first on the inputs before the last one, Op::second on
+// the last), so a slot is refilled as soon as its step is done: P_i and P_j of
+// the next tile arrive while this one's dots run, P_n during the next tile's
+// wedges.  One slot instead of a two-stage ring takes half the shared memory a
+// site, and no warp waits for another.  At 24^3 x 64 in complex64 the pass took
+// 0.740 ms on the shared ring of engine.cuh with its producer warp (12 consumer
+// warps an SM of 2 sites: shared memory full, issue slots 59 % used, dependent
+// instructions the first stall), 0.666 ms here with 20 such warps and 0.590 ms
+// with 12 warps of 4 sites, which hold two blocks a thread (HBM: 0.457 ms).
+//
+// Every wait is bounded in wall time; a warp that times out reports it, waits
+// (bounded) for its copies still in flight and returns.
+//
+// An op yields NVAL values per site and combine() makes its NOUT outputs of
+// them: per site, or per chunk after a compensated sum over the chunk's sites
+// (partial[chunk][NOUT], reduced per timeslice by finalize_kernel).
+#pragma once
+
+#include "engine.cuh"
+
+namespace cgb {
+
+template <class Op> struct WarpSmem {
+  using L = OpLayout<Op>;
+  static constexpr int SPW = 32 / Op::TPS;
+  static constexpr size_t IN = 16;  // the warp's two mbarriers come first
+  static constexpr size_t EXTRA = IN + (size_t)Op::NIN * SPW * L::SLOT;
+  static constexpr size_t WARP = EXTRA + (size_t)SPW * Op::EXTRA_BYTES;
+  static constexpr size_t BYTES = Op::CW * WARP;
+  static_assert(WARP % 16 == 0 && Op::EXTRA_BYTES % 16 == 0, "slots must stay 16-byte aligned");
+};
+
+// A warp's walk over its tiles of one lattice: chunks w, w + (warps of the grid), ...
+template <class Op> struct ChunkWalk {
+  static constexpr int SITES = 32 / Op::TPS;
+  using Params = typename Op::Params;
+  TileIter<SITES> it;
+  int stride;
+
+  __device__ __forceinline__ void start(const Params &p)
+  {
+    stride = gridDim.x * Op::CW;
+    it.set_chunk(p.geom, blockIdx.x * Op::CW + (threadIdx.x >> 5));
+  }
+  __device__ __forceinline__ bool valid(const Params &p) const { return it.valid(p.geom); }
+  __device__ __forceinline__ void next(const Params &p) { it.next(p.geom, stride); }
+  __device__ __forceinline__ bool last_in_chunk() const { return it.last_in_chunk(); }
+  __device__ __forceinline__ long long first() const { return it.first; }
+  __device__ __forceinline__ int sites() const { return it.sites(); }
+  __device__ __forceinline__ int where() const { return it.chunk; }
+  __device__ __forceinline__ bool withheld(const Params &p) const { return it.k == 0 && it.chunk == p.geom.withhold_chunk; }
+  __device__ __forceinline__ const char *in(const Params &p, int q) const { return static_cast<const char *>(p.in[q]); }
+  __device__ __forceinline__ double2 *partial(const Params &p) const
+  {
+    return static_cast<double2 *>(p.out[0]) + (size_t)it.chunk * Op::NOUT;
+  }
+};
+template <class Op> __device__ __forceinline__ const typename Op::Params &op_params(const typename Op::Params &p)
+{
+  return p;
+}
+
+template <class Op, class Walk>
+__global__ void __launch_bounds__(32 * Op::CW, Op::MIN_CTAS) warp_kernel(const __grid_constant__ typename Walk::Params p)
+{
+  using S = typename Op::S;
+  using R = typename Op::R;
+  using L = OpLayout<Op>;
+  constexpr int NIN = Op::NIN, TPS = Op::TPS, SPW = 32 / TPS, NVAL = Op::NVAL, NOUT = Op::NOUT;
+  constexpr int SH = values_shift<TPS, NVAL>();  // value r of a site: thread r << SH
+
+  extern __shared__ __align__(128) unsigned char smem[];
+  __shared__ __align__(16) typename Op::Params ps;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  unsigned char *mine = smem + warp * WarpSmem<Op>::WARP;
+  uint64_t *bars = reinterpret_cast<uint64_t *>(mine);  // [0]: all inputs but the last, [1]: the last
+  if (lane == 0) {
+    mbar_init(&bars[0], 1);
+    mbar_init(&bars[1], 1);
+    fence_barrier_init();
+  }
+  copy_params(ps, op_params<Op>(p));
+  __syncthreads();
+
+  const int local = lane / TPS, sub = lane % TPS;
+  const S *in[NIN];
+#pragma unroll
+  for (int q = 0; q < NIN; ++q)
+    in[q] = reinterpret_cast<const S *>(mine + WarpSmem<Op>::IN + ((size_t)q * SPW + local) * L::SLOT);
+  S *scratch = reinterpret_cast<S *>(mine + WarpSmem<Op>::EXTRA + (size_t)local * Op::EXTRA_BYTES);
+
+  // Issue the copies of a tile's inputs [q0, q1) on barrier b.
+  auto fetch = [&](const Walk &w, int q0, int q1, int b) {
+    if (w.withheld(p)) return;  // test hook: this tile never arrives
+    const int n = w.sites();
+    if (lane == 0) mbar_arrive_expect_tx(&bars[b], (uint32_t)(n * (q1 - q0)) * L::SITE_BYTES);
+    __syncwarp();
+    if (lane < SPW * (q1 - q0)) {
+      const int q = q0 + lane / SPW, s = lane % SPW;
+      if (s < n)
+        bulk_g2s(mine + WarpSmem<Op>::IN + ((size_t)q * SPW + s) * L::SLOT, w.in(p, q) + (w.first() + s) * L::SITE_BYTES,
+                 L::SITE_BYTES, &bars[b]);
+    }
+  };
+  Walk cur;
+  cur.start(p);
+  if (cur.valid(p)) {
+    fetch(cur, 0, NIN - 1, 0);
+    fetch(cur, NIN - 1, NIN, 1);
+  }
+  const unsigned long long wait_ns = ps.geom.wait_ns;
+  // Both barriers complete once per tile.  A warp that gave up waits for what
+  // may still be in flight: this tile's copies on either barrier, and with
+  // `next_too` the next tile's on the first.
+  auto give_up = [&](uint32_t parity, bool next_too) {
+    report(p.status, kDevErrWaitTimeout, (unsigned int)cur.where());
+    if (lane == 0) {
+      mbar_wait_bounded(&bars[0], next_too ? parity ^ 1u : parity, wait_ns / 8);
+      mbar_wait_bounded(&bars[1], parity, wait_ns / 8);
+    }
+  };
+  ChunkSum<R> chunk_acc;
+  for (uint32_t u = 0; cur.valid(p); ++u) {
+    if (!__all_sync(0xffffffffu, mbar_wait_bounded(&bars[0], u & 1u, wait_ns))) {
+      give_up(u & 1u, false);
+      return;
+    }
+    typename Op::State state;
+    Op::first(ps, in, scratch, sub, state);
+    Walk nx = cur;
+    nx.next(p);
+    fence_proxy_async_smem();
+    __syncwarp();
+    if (nx.valid(p)) fetch(nx, 0, NIN - 1, 0);
+    if (!__all_sync(0xffffffffu, mbar_wait_bounded(&bars[1], u & 1u, wait_ns))) {
+      give_up(u & 1u, nx.valid(p));
+      return;
+    }
+    cx<R> vals[NVAL];
+    Op::second(ps, in[NIN - 1], scratch, sub, state, vals);
+    fence_proxy_async_smem();
+    __syncwarp();
+    if (nx.valid(p)) fetch(nx, NIN - 1, NIN, 1);
+    const cx<R> v = group_reduce_values<TPS, NVAL>(vals, sub);
+    const bool ok = local < cur.sites();
+    if (ps.geom.per_site) {
+#pragma unroll
+      for (int o0 = 0; o0 < NOUT; o0 += TPS) {
+        const int o = o0 + sub;
+        const cx<R> z = Op::combine(ps, o < NOUT ? o : 0, v, lane - sub, 1 << SH);
+        if (o < NOUT && ok)
+          static_cast<double2 *>(ps.out[o])[cur.first() + local] = make_double2(double(z.x), double(z.y));
+      }
+    } else {
+      // each lane sums the value it holds of its own site; the warp's sites
+      // meet in FP64 at the end of the chunk
+      chunk_acc.add(ok ? v : czero<R>());
+      if (cur.last_in_chunk()) {
+        double2 c = chunk_acc.value();
+#pragma unroll
+        for (int o = 16; o >= TPS; o >>= 1) {
+          c.x += __shfl_xor_sync(0xffffffffu, c.x, o);
+          c.y += __shfl_xor_sync(0xffffffffu, c.y, o);
+        }
+        const double2 z = Op::combine(ps, lane < NOUT ? lane : 0, c, 0, 1 << SH);
+        if (lane < NOUT) cur.partial(p)[lane] = z;
+        chunk_acc.reset();
+      }
+    }
+    cur = nx;
+  }
+}
+
+} // namespace cgb

@@ -1,8 +1,10 @@
 // Batched all-types baryon contractions: many sources / lattices per launch.
 #include <mutex>
 #include <tuple>
+#include <vector>
 
 #include "batch.cuh"
+#include "ops_fused.cuh"
 #include "launch_impl.cuh"
 #include "batch.hpp"
 #include "momentum.hpp"
@@ -24,8 +26,16 @@ static cudaError_t run_batch(const Job &job, const OpParams<typename Op::R> &op,
   std::lock_guard<std::mutex> lk(mu);
   bp = {};
   bp.op = op;
+  bp.op.geom.wait_ns = job.wait_ns ? job.wait_ns : kWaitLimitNs;
   bp.status = job.status;
   bp.n_items = n;
+  using Walk = QueueWalk<Op>;
+  constexpr size_t smem = WarpSmem<Op>::BYTES;
+  static_assert(smem <= 232448, "op does not fit in shared memory");
+  int bps = 0;
+  cudaError_t e = prepare<Op>(warp_kernel<Op, Walk>, smem, bps, 32 * Op::CW);
+  if (e != cudaSuccess) return e;
+  const int warps = job.num_sms * bps * Op::CW;
   size_t partial_total = 0;
   int chunks = 0;
   long long max_lt = 0;
@@ -37,12 +47,12 @@ static cudaError_t run_batch(const Job &job, const OpParams<typename Op::R> &op,
     ji.half_slice = (long long)specs[i].latt[0] * specs[i].latt[1] * specs[i].latt[2] / 2;
     BatchItem &it = bp.items[i];
     for (int q = 0; q < 3; ++q) it.in[q] = specs[i].in[q];
-    it.geom = make_geom(ji, Op::SITES, job.num_sms, 8);  // the device queue balances the CTAs
+    it.geom = make_geom(ji, Walk::SITES, warps, 3);  // the device queue balances the warps
     it.chunk_begin = chunks;
     it.lt = ji.lt;
     it.out = specs[i].out;
     chunks += it.geom.total_chunks;
-    partial_total += (size_t)it.geom.total_chunks * Op::CW * Op::NOUT;
+    partial_total += (size_t)it.geom.total_chunks * Op::NOUT;
     max_lt = std::max<long long>(max_lt, ji.lt);
   }
   bp.total_chunks = chunks;
@@ -55,16 +65,12 @@ static cudaError_t run_batch(const Job &job, const OpParams<typename Op::R> &op,
   size_t off = 0;
   for (int i = 0; i < n; ++i) {
     bp.items[i].partial = partial + off;
-    off += (size_t)bp.items[i].geom.total_chunks * Op::CW * Op::NOUT;
+    off += (size_t)bp.items[i].geom.total_chunks * Op::NOUT;
   }
-  constexpr size_t smem = engine_smem_bytes<Op>();
-  int bps = 0;
-  cudaError_t e = prepare<Op>(batch_scalar_kernel<Op>, smem, bps);
-  if (e != cudaSuccess) return e;
-  const int grid = (int)std::min<long long>(chunks, (long long)job.num_sms * bps);
+  const int grid = std::min((chunks + Op::CW - 1) / Op::CW, job.num_sms * bps);
   e = cudaMemsetAsync(bp.queue, 0, sizeof(unsigned int), job.stream);
   if (e != cudaSuccess) return e;
-  batch_scalar_kernel<Op><<<grid, Op::THREADS, smem, job.stream>>>(bp);
+  warp_kernel<Op, Walk><<<grid, 32 * Op::CW, smem, job.stream>>>(bp);
   e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   if (fin) {
@@ -76,7 +82,7 @@ static cudaError_t run_batch(const Job &job, const OpParams<typename Op::R> &op,
       f.partial = bp.items[i].partial;
       f.out = bp.items[i].out;
       f.lt = bp.items[i].lt;
-      f.per_seg = bp.items[i].geom.chunks_per_seg * Op::CW;
+      f.per_seg = bp.items[i].geom.chunks_per_seg;
       f.blk_begin = blocks;
       blocks += (Op::NOUT * f.lt + 255) / 256;
     }
@@ -84,24 +90,18 @@ static cudaError_t run_batch(const Job &job, const OpParams<typename Op::R> &op,
     return cudaSuccess;
   }
   const dim3 fg(n, (unsigned)((Op::NOUT * max_lt + 127) / 128));
-  batch_finalize_kernel<R><<<fg, 128, 0, job.stream>>>(bp, Op::NOUT, Op::CW);
+  batch_finalize_kernel<R><<<fg, 128, 0, job.stream>>>(bp, Op::NOUT);
   return cudaGetLastError();
 }
 
 // Tile shapes of the batched launch (the autotuner's choice per batch: one
 // shape serves every item of a launch).
-template <int NW> struct BatchShapes {
-  using Two = std::tuple<BaryonFusedSharedWedgeOp<float, float2, 4, 16, 2, NW, 3>,
-                         BaryonFusedSharedWedgeOp<float, float2, 3, 16, 2, NW, 4>,
-                         BaryonFusedSharedWedgeOp<float, float2, 2, 16, 3, NW, 6>>;
-  using Same = std::tuple<BaryonFusedSharedWedgeSameOp<float, float2, 2, 2, NW, 4>,
-                          BaryonFusedSharedWedgeSameOp<float, float2, 3, 2, NW, 3>,
-                          BaryonFusedSharedWedgeSameOp<float, float2, 4, 2, NW, 2>>;
-};
-static const char *const kBatchShapeNames[] = {"shared.cw4.tps16.st2.occ3", "shared.cw3.tps16.st2.occ4",
-                                               "shared.cw2.tps16.st3.occ6"};
-static const char *const kBatchSameShapeNames[] = {"shared_same.cw2.tps8.st2.occ4", "shared_same.cw3.tps8.st2.occ3",
-                                                   "shared_same.cw4.tps8.st2.occ2"};
+template <int NG, int NW, bool SAME>
+using BatchShapes = std::tuple<BaryonFusedOp<float, float2, 4, 8, NG, NW, SAME, 2>,
+                               BaryonFusedOp<float, float2, 12, 8, NG, NW, SAME, 1>,
+                               BaryonFusedOp<float, float2, 4, 16, NG, NW, SAME, 5>>;
+static const char *const kBatchShapeNames[] = {"w4.tps8.occ2", "w12.tps8.occ1", "w4.tps16.occ5"};
+static const char *const kBatchSameShapeNames[] = {"same.w4.tps8.occ2", "same.w12.tps8.occ1", "same.w4.tps16.occ5"};
 
 template <class Tuple>
 static cudaError_t run_shape(int v, const Job &job, const OpParams<float> &q, const BatchSpec *specs, int n,
@@ -132,41 +132,36 @@ bool batch_rank_form(int nw, const OpParams<double> &p) { return nw == 1 && p.b.
 cudaError_t launch_baryon_fused_batch(const Job &job, int nw, const OpParams<double> &p, const BatchSpec *specs, int n,
                                       BaryonFinParams *fin)
 {
-  // One projector of rank <= 2 that is not one gamma matrix: factored triangles.
-  if (batch_rank_form(nw, p)) {
-    if (job.prec == Prec::C128) return run_batch<BaryonFusedRankOp<double, double2, 3, 16, 2>>(job, p, specs, n, fin);
-    return run_batch<BaryonFusedRankOp<float, float2, 4, 16, 2>>(job, convert_params<float>(p), specs, n, fin);
-  }
-  // Otherwise gamma-basis projectors only (e.g. (1 +- g4)/2): no per-site N' buffers.
-  if (p.b.cl.ng > nw) return cudaErrorInvalidValue;
+  const int ng = p.b.cl.ng, v = job.variant;
+  const bool rank = batch_rank_form(nw, p);
+  if (!rank && ng > nw) return cudaErrorInvalidValue;
+  OpParams<double> d = p;
   if (job.prec == Prec::C128) {
-    return nw == 1 ? run_batch<BaryonFusedCliffOp<double, double2, 4, 16, 2, 1>>(job, p, specs, n, fin)
-                   : run_batch<BaryonFusedCliffOp<double, double2, 4, 16, 2, 2>>(job, p, specs, n, fin);
+    fill_fused_spin(d, false);
+    if (ng == 2) return nw == 1 ? run_batch<BaryonFusedOp<double, double2, 4, 16, 2, 1, false, 2>>(job, d, specs, n, fin)
+                                : run_batch<BaryonFusedOp<double, double2, 4, 16, 2, 2, false, 2>>(job, d, specs, n, fin);
+    if (ng > 2) return p.b.rk.r == 1 ? run_batch<BaryonFusedOp<double, double2, 4, 16, -1, 1, false, 2>>(job, d, specs, n, fin)
+                                     : run_batch<BaryonFusedOp<double, double2, 4, 16, -2, 1, false, 2>>(job, d, specs, n, fin);
+    return nw == 1 ? run_batch<BaryonFusedOp<double, double2, 4, 16, 1, 1, false, 2>>(job, d, specs, n, fin)
+                   : run_batch<BaryonFusedOp<double, double2, 4, 16, 1, 2, false, 2>>(job, d, specs, n, fin);
   }
-  const OpParams<float> q = convert_params<float>(p);
-  bool same = n > 0;
-  for (int i = 0; i < n; ++i) same = same && specs[i].in[0] == specs[i].in[1];
-  // The shared-wedge forms take the Gamma_kl^T variants as a sign (every
-  // Gamma(n) is symmetric or antisymmetric); the one-field form also needs a
-  // Gamma_ij permutation without fixed points (XOR permutations: perm1[0] != 0).
-  const int v = job.variant;
-  if (same && q.b.perm1[0] != 0) {
-    static BatchSpec two[kMaxBatch];  // inputs: the field once, then P_n
-    static std::mutex mu2;
-    std::lock_guard<std::mutex> lk(mu2);
-    if (n > kMaxBatch) return cudaErrorInvalidValue;
-    for (int i = 0; i < n; ++i) {
-      two[i] = specs[i];
-      two[i].in[1] = specs[i].in[2];
-    }
-    return nw == 1 ? run_shape<BatchShapes<1>::Same>(v, job, q, two, n, fin)
-                   : run_shape<BatchShapes<2>::Same>(v, job, q, two, n, fin);
+  OpParams<float> q = convert_params<float>(p);
+  if (ng <= 2 && batch_same_field(p, specs, n)) {
+    fill_fused_spin(q, true);
+    std::vector<BatchSpec> one(specs, specs + n);  // inputs: the field once, then P_n
+    for (BatchSpec &b : one) b.in[1] = b.in[2];
+    if (ng == 2) return nw == 1 ? run_batch<BaryonFusedOp<float, float2, 4, 8, 2, 1, true, 2>>(job, q, one.data(), n, fin)
+                                : run_shape<BatchShapes<2, 2, true>>(v, job, q, one.data(), n, fin);
+    return nw == 1 ? run_shape<BatchShapes<1, 1, true>>(v, job, q, one.data(), n, fin)
+                   : run_batch<BaryonFusedOp<float, float2, 4, 8, 1, 2, true, 2>>(job, q, one.data(), n, fin);
   }
-  if (same)
-    return nw == 1 ? run_batch<BaryonFusedCliffMergedOp<float, float2, 4, 16, 2, 1, 3, true>>(job, q, specs, n, fin)
-                   : run_batch<BaryonFusedCliffMergedOp<float, float2, 4, 16, 2, 2, 3, true>>(job, q, specs, n, fin);
-  return nw == 1 ? run_shape<BatchShapes<1>::Two>(v, job, q, specs, n, fin)
-                 : run_shape<BatchShapes<2>::Two>(v, job, q, specs, n, fin);
+  fill_fused_spin(q, false);
+  if (ng == 2) return nw == 1 ? run_batch<BaryonFusedOp<float, float2, 4, 8, 2, 1, false, 2>>(job, q, specs, n, fin)
+                              : run_shape<BatchShapes<2, 2, false>>(v, job, q, specs, n, fin);
+  if (ng > 2) return p.b.rk.r == 1 ? run_batch<BaryonFusedOp<float, float2, 4, 8, -1, 1, false, 2>>(job, q, specs, n, fin)
+                                   : run_batch<BaryonFusedOp<float, float2, 4, 8, -2, 1, false, 2>>(job, q, specs, n, fin);
+  return nw == 1 ? run_shape<BatchShapes<1, 1, false>>(v, job, q, specs, n, fin)
+                 : run_batch<BaryonFusedOp<float, float2, 4, 8, 1, 2, false, 2>>(job, q, specs, n, fin);
 }
 
 } // namespace cgb

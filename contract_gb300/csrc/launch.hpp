@@ -148,6 +148,9 @@ template <class R> OpParams<R> convert_params(const OpParams<double> &p)
         o.b.rk.c[s][r][k][0] = R(p.b.rk.c[s][r][k][0]);
         o.b.rk.c[s][r][k][1] = R(p.b.rk.c[s][r][k][1]);
       }
+  for (int r = 0; r < 2; ++r)
+    for (int m = 0; m < 4; ++m)
+      for (int k = 0; k < 2; ++k) o.b.rk.x[r][m][k] = R(p.b.rk.x[r][m][k]);
   return o;
 }
 

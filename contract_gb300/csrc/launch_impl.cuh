@@ -49,7 +49,7 @@ template <class K> struct KernelAttr {
   int bps[64] = {};  // resident CTAs per SM, per device ordinal (0 = not yet queried)
 };
 
-template <class Op, class K> cudaError_t prepare(K kernel, size_t smem, int &bps_out)
+template <class Op, class K> cudaError_t prepare(K kernel, size_t smem, int &bps_out, int threads = Op::THREADS)
 {
   static KernelAttr<K> cache;
   int dev = 0;
@@ -62,7 +62,7 @@ template <class Op, class K> cudaError_t prepare(K kernel, size_t smem, int &bps
   e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   int bps = 0;
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, kernel, Op::THREADS, smem);
+  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, kernel, threads, smem);
   if (e != cudaSuccess) return e;
   if (bps < 1) return cudaErrorInvalidConfiguration;
   if (dev < 64) cache.bps[dev] = bps;

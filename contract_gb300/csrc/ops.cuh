@@ -73,6 +73,19 @@ template <class R> struct RankForm {
   int unit;
   uint8_t ph[2][2][4];
   R scale;
+  R x[2][4][2];  // x_r[m], every entry (the all-types pass)
+};
+
+// The all-types pass's spin tables in packed words (fill_fused_spin in
+// ops_fused.cuh): one 16-byte load per site.  Every Gamma(n) is real or
+// imaginary throughout, so its entries are one common power of i, applied to
+// the outputs, times the signs kept here.
+struct alignas(16) FusedSpin {
+  uint32_t s;     // permutation classes: Gamma_ij at bit 0, Gamma_kl at 2, term k at 4 + 2 k
+  uint32_t rows;  // rows of Gamma_ij, negative ones first, at 2 k; number of negative rows at 8
+  uint32_t neg;   // sign bits: c2(l) at bit l, term k at row m at bit 4 + 4 k + m
+  uint32_t out;   // phase of the outputs at 0 (at 8 + 2 k with term k's), of the Gamma_kl^T partners against them
+                  // at 2, of the IM_* group against the IK_JM/IL_JM one (one field) at 4 (the last two 0 or 2)
 };
 
 template <class R> struct BaryonSpin {
@@ -82,6 +95,7 @@ template <class R> struct BaryonSpin {
   ProjOperand<R> proj[2];
   CliffordSet<R> cl;
   RankForm<R> rk;  // proj[0] factored, for the triangle form
+  FusedSpin fu;
 };
 
 template <class R> struct MesonSpin {
@@ -136,30 +150,6 @@ __device__ __forceinline__ void build_q(const BaryonSpin<R> &b, const S *N, S *q
             cfma(s, cx<R> {pw.w[m * 4 + n][0], pw.w[m * 4 + n][1]}, ld<R>(N + (n * 4 + m) * 9 + ad));
     }
     st(q + e, s);
-  }
-}
-
-// Q_w from the gamma-basis form: Q_w = sum_k coef[w][k] sum_m i^ph[k][m] N[perm[k][m]][m].
-template <class R, class S, int TPS, int NW>
-__device__ __forceinline__ void build_q_cliff(const BaryonSpin<R> &b, const S *N, S *q, int sub)
-{
-  // One colour entry ad per thread, all NW projectors at once: each N value is
-  // loaded once and scaled by the precombined coefficients qc.
-  const CliffordSet<R> &cl = b.cl;
-  for (int ad = sub; ad < 9; ad += TPS) {
-    cx<R> s[NW];
-#pragma unroll
-    for (int w = 0; w < NW; ++w) s[w] = czero<R>();
-    for (int k = 0; k < cl.ng; ++k) {
-#pragma unroll
-      for (int m = 0; m < 4; ++m) {
-        const cx<R> n = ld<R>(N + (cl.perm[k][m] * 4 + m) * 9 + ad);
-#pragma unroll
-        for (int w = 0; w < NW; ++w) cfma(s[w], cx<R> {cl.qc[w][k][m][0], cl.qc[w][k][m][1]}, n);
-      }
-    }
-#pragma unroll
-    for (int w = 0; w < NW; ++w) st(q + w * 9 + ad, s[w]);
   }
 }
 
@@ -427,6 +417,27 @@ __device__ __forceinline__ void build_rank(const RankForm<R> &rk, const S *B, co
   }
 }
 
+// Y_r[q] = sum_n y_r[n] N[n][q] at block r*4 + q of y.
+template <class R, class S, int TPS>
+__device__ __forceinline__ void build_rank_y(const RankForm<R> &rk, const S *N, S *y, int sub)
+{
+  for (int e = sub; e < 4 * rk.r; e += TPS) {
+    const int rr = e / 4, q = e % 4;
+    cx<R> o[9];
+#pragma unroll
+    for (int k = 0; k < 9; ++k) o[k] = czero<R>();
+#pragma unroll 1
+    for (int k = 0; k < rk.nnz; ++k) {
+      const S *src = N + (rk.idx[1][rr][k] * 4 + q) * 9;
+      const cx<R> c {rk.c[1][rr][k][0], rk.c[1][rr][k][1]};
+#pragma unroll
+      for (int t = 0; t < 9; ++t) cfma(o[t], c, ld<R>(src + t));
+    }
+#pragma unroll
+    for (int k = 0; k < 9; ++k) st(y + e * 9 + k, o[k]);
+  }
+}
+
 // Triangle values for the NV c2 variants from X_r (block r*4 + j of X) and
 // Y_r (block r*4 + l of Y); c1 from ph1[c1sel].
 template <class R, class S, int TPS, int NV>
@@ -548,408 +559,6 @@ __device__ __forceinline__ void triangle_cliff_site(const BaryonSpin<R> &b, cons
     for (int w = 0; w < NW; ++w) vals[v * NW + w] = mul_phase(acc[v][w], p1);
 }
 
-// One triangle pass of the fused kernel (one (i, l) pair per thread) with the
-// gamma-basis projectors, on the shared-wedge order of triangle_cliff_site.
-// The m loop starts at m = l: with (A, B) = (P_i, P_j) its first wedge
-// A[i][perm2 l] ^ B[perm1 i][l] is the loop form's, so LOOP folds the two loop
-// types (dots with Q_w) into that iteration.  out[v*NW + w] = triangle values,
-// loop[v*NW + w] = loop values.
-template <class R, class S, int NW, bool LOOP>
-__device__ __forceinline__ void fused_triangle_pass(const BaryonSpin<R> &b, const S *A, const S *B, const S *N,
-                                                    const S *q, int i, int l, int c1sel, cx<R> *out, cx<R> *loop)
-{
-  const CliffordSet<R> &cl = b.cl;
-  const int j = b.perm1[i];
-  cx<R> a[9];
-  load9(a, A + (i * 4 + b.perm2[l]) * 9);
-  cx<R> u[NW];
-#pragma unroll
-  for (int w = 0; w < NW; ++w) u[w] = czero<R>();
-  const bool two = cl.ng == 2;
-  cx<R> s0 = czero<R>(), s1 = czero<R>();  // per-term sums when there are two terms
-#pragma unroll 1
-  for (int mm = 0; mm < 4; ++mm) {
-    const int m = (l + mm) & 3;
-    cx<R> e[9];
-    {
-      cx<R> bm[9];
-      load9(bm, B + (j * 4 + m) * 9);
-#pragma unroll
-      for (int k = 0; k < 9; ++k) e[k] = czero<R>();
-      wedge_acc(e, a, bm);
-    }
-    if constexpr (LOOP) {
-      if (mm == 0) {
-#pragma unroll
-        for (int w = 0; w < NW; ++w) {
-          cx<R> qw[9];
-          load9(qw, q + w * 9);
-          const cx<R> sq = dot9(e, qw);
-#pragma unroll
-          for (int v = 0; v < 2; ++v) loop[v * NW + w] = mul_phase(sq, (b.ph1[c1sel][i] + b.ph2[v][l]) & 3u);
-        }
-      }
-    }
-    if (two) {
-      cx<R> nn[9];
-      load9(nn, N + (cl.perm[0][m] * 4 + l) * 9);
-      s0 = cadd(s0, mul_phase(dot9(nn, e), cl.ph[0][m]));
-      load9(nn, N + (cl.perm[1][m] * 4 + l) * 9);
-      s1 = cadd(s1, mul_phase(dot9(nn, e), cl.ph[1][m]));
-    } else {
-#pragma unroll 1
-      for (int k = 0; k < cl.ng; ++k) {
-        cx<R> nn[9];
-        load9(nn, N + (cl.perm[k][m] * 4 + l) * 9);
-        const cx<R> s = mul_phase(dot9(nn, e), cl.ph[k][m]);
-#pragma unroll
-        for (int w = 0; w < NW; ++w) cfma(u[w], cx<R> {cl.coef[w][k][0], cl.coef[w][k][1]}, s);
-      }
-    }
-  }
-  if (two) {
-#pragma unroll
-    for (int w = 0; w < NW; ++w) {
-      cfma(u[w], cx<R> {cl.coef[w][0][0], cl.coef[w][0][1]}, s0);
-      cfma(u[w], cx<R> {cl.coef[w][1][0], cl.coef[w][1][1]}, s1);
-    }
-  }
-  const uint32_t p1 = b.ph1[c1sel][i];
-#pragma unroll
-  for (int w = 0; w < NW; ++w)
-#pragma unroll
-    for (int v = 0; v < 2; ++v) out[v * NW + w] = mul_phase(u[w], (p1 + b.ph2[v][l]) & 3u);
-}
-
-// Both triangle passes of the fused kernel in one m loop: with
-// a1 = P_i[i][perm2 l] and a2 = P_j[i][perm2 l], each N block n_km is loaded
-// once and dotted with both a1 ^ P_j[perm1 i][m] and a2 ^ P_i[perm1 i][m].
-// The loop form is folded into the m = l wedge of the first pass as in
-// fused_triangle_pass.  vals[type * NW + w], types in contract_enum.h order.
-template <class R, class S, int NW, bool SAMEIJ = false>
-__device__ __forceinline__ void fused_merged_site(const BaryonSpin<R> &b, const S *Pi, const S *Pj, const S *N,
-                                                  const S *q, int i, int l, cx<R> *vals)
-{
-  const CliffordSet<R> &cl = b.cl;
-  const int j = b.perm1[i];
-  cx<R> a1[9], a2[9];
-  load9(a1, Pi + (i * 4 + b.perm2[l]) * 9);
-  if constexpr (!SAMEIJ) load9(a2, Pj + (i * 4 + b.perm2[l]) * 9);
-  cx<R> u1[NW], u2[NW];
-  S *lps = const_cast<S *>(q) + 9 * NW + (i * 4 + l) * 2 * NW;  // loop values, parked in shared memory
-#pragma unroll
-  for (int w = 0; w < NW; ++w) u1[w] = u2[w] = czero<R>();
-  const bool two = cl.ng == 2, phased = cl.has_phase[0] || cl.has_phase[1];
-  cx<R> s10 = czero<R>(), s11 = czero<R>(), s20 = czero<R>(), s21 = czero<R>();
-#pragma unroll 1
-  for (int mm = 0; mm < 4; ++mm) {
-    const int m = (l + mm) & 3;
-    cx<R> e1[9], e2[9];
-    {
-      cx<R> bm[9];
-      load9(bm, Pj + (j * 4 + m) * 9);
-#pragma unroll
-      for (int k = 0; k < 9; ++k) e1[k] = czero<R>();
-      wedge_acc(e1, a1, bm);
-      if constexpr (!SAMEIJ) {
-        load9(bm, Pi + (j * 4 + m) * 9);
-#pragma unroll
-        for (int k = 0; k < 9; ++k) e2[k] = czero<R>();
-        wedge_acc(e2, a2, bm);
-      }
-    }
-    if (mm == 0) {
-#pragma unroll
-      for (int w = 0; w < NW; ++w) {
-        cx<R> qw[9];
-        load9(qw, q + w * 9);
-        const cx<R> sq = dot9(e1, qw);
-#pragma unroll
-        for (int v = 0; v < 2; ++v) {
-          const cx<R> lv = mul_phase(sq, (b.ph1[0][i] + b.ph2[v][l]) & 3u);
-          lps[v * NW + w] = S {lv.x, lv.y};
-        }
-      }
-    }
-    if (two && !phased) {  // e.g. (1 +- g4)/2 = (Gamma(0) +- Gamma(8))/2: no phases to apply
-      cx<R> nn[9];
-      load9(nn, N + (cl.perm[0][m] * 4 + l) * 9);
-      s10 = cadd(s10, dot9(nn, e1));
-      if constexpr (!SAMEIJ) s20 = cadd(s20, dot9(nn, e2));
-      load9(nn, N + (cl.perm[1][m] * 4 + l) * 9);
-      s11 = cadd(s11, dot9(nn, e1));
-      if constexpr (!SAMEIJ) s21 = cadd(s21, dot9(nn, e2));
-    } else if (two) {
-      cx<R> nn[9];
-      load9(nn, N + (cl.perm[0][m] * 4 + l) * 9);
-      s10 = cadd(s10, mul_phase(dot9(nn, e1), cl.ph[0][m]));
-      if constexpr (!SAMEIJ) s20 = cadd(s20, mul_phase(dot9(nn, e2), cl.ph[0][m]));
-      load9(nn, N + (cl.perm[1][m] * 4 + l) * 9);
-      s11 = cadd(s11, mul_phase(dot9(nn, e1), cl.ph[1][m]));
-      if constexpr (!SAMEIJ) s21 = cadd(s21, mul_phase(dot9(nn, e2), cl.ph[1][m]));
-    } else {
-#pragma unroll 1
-      for (int k = 0; k < cl.ng; ++k) {
-        cx<R> nn[9];
-        load9(nn, N + (cl.perm[k][m] * 4 + l) * 9);
-        const cx<R> t1 = mul_phase(dot9(nn, e1), cl.ph[k][m]);
-#pragma unroll
-        for (int w = 0; w < NW; ++w) cfma(u1[w], cx<R> {cl.coef[w][k][0], cl.coef[w][k][1]}, t1);
-        if constexpr (!SAMEIJ) {
-          const cx<R> t2 = mul_phase(dot9(nn, e2), cl.ph[k][m]);
-#pragma unroll
-          for (int w = 0; w < NW; ++w) cfma(u2[w], cx<R> {cl.coef[w][k][0], cl.coef[w][k][1]}, t2);
-        }
-      }
-    }
-  }
-  if (two) {
-#pragma unroll
-    for (int w = 0; w < NW; ++w) {
-      const cx<R> c0 {cl.coef[w][0][0], cl.coef[w][0][1]}, c1 {cl.coef[w][1][0], cl.coef[w][1][1]};
-      cfma(u1[w], c0, s10);
-      cfma(u1[w], c1, s11);
-      if constexpr (!SAMEIJ) {
-        cfma(u2[w], c0, s20);
-        cfma(u2[w], c1, s21);
-      }
-    }
-  }
-  if constexpr (SAMEIJ) {  // P_i and P_j are one field: both passes give the same sums
-#pragma unroll
-    for (int w = 0; w < NW; ++w) u2[w] = u1[w];
-  }
-  const uint32_t p1 = b.ph1[0][i], p2 = b.ph1[1][i];
-#pragma unroll
-  for (int w = 0; w < NW; ++w) {
-    vals[0 * NW + w] = cx<R> {lps[0 * NW + w].x, lps[0 * NW + w].y};  // IK_JL_NM
-    vals[2 * NW + w] = cx<R> {lps[1 * NW + w].x, lps[1 * NW + w].y};  // IL_JK_NM
-    vals[1 * NW + w] = mul_phase(u1[w], (p1 + b.ph2[0][l]) & 3u);      // IK_JM_NL
-    vals[3 * NW + w] = mul_phase(u1[w], (p1 + b.ph2[1][l]) & 3u);      // IL_JM_NK
-    vals[4 * NW + w] = mul_phase(u2[w], (p2 + b.ph2[0][l]) & 3u);      // IM_JK_NL
-    vals[5 * NW + w] = mul_phase(u2[w], (p2 + b.ph2[1][l]) & 3u);      // IM_JL_NK
-  }
-}
-
-// Both triangle passes from one set of wedges.  The wedge is symmetric
-// (X ^ Y = Y ^ X) and every gamma permutation is an involution, so the second
-// pass's wedge P_j[i][perm2 l] ^ P_i[perm1 i][m] is the first pass's wedge
-// E[i'][x][n] = P_i[i'][x] ^ P_j[perm1 i'][n] at i' = perm1 i, x = m,
-// n = perm2 l.  Thread (i, x) forms its four wedges E[i][x][n] once and
-// dots each with the N blocks of both passes:
-//   pass 1 (IK_JM_NL, IL_JM_NK; target (i, l = perm2 x), m = n):
-//     N[perm_k n][l], coefficient coef_k i^ph_k(n), output phase fixed per thread;
-//   pass 2 (IM_JK_NL, IM_JL_NK; target (perm1 i, perm2 n), m = x):
-//     N[perm_k x][perm2 n], coefficient coef_k i^ph_k(x) = qc[.][k][x], output
-//     phase i^(ph1[1][perm1 i] + ph2[0][perm2 n]) applied per n.
-// The outputs are summed over the site's 16 threads, so a thread may add
-// terms that belong to another (i, l).  The loop types use the n = l wedge
-// (the loop form's A[i][perm2 l] ^ B[perm1 i][l]) as in fused_merged_site.
-// Every Gamma(n) of the DeGrand-Rossi basis is symmetric or antisymmetric, so
-// the Gamma_kl and Gamma_kl^T variants of each type differ by one sign:
-// IL_JK_NM, IL_JM_NK and IM_JL_NK are i^v1 times IK_JL_NM, IK_JM_NL and
-// IM_JK_NL, v1 = ph2[1] - ph2[0] (0 or 2, the same in every column; the
-// launcher checks it).  Per site: 64 wedges + 256 dots + 32 loop dots (4 898
-// complex FMA with two two-term projectors) instead of 128 wedges + 256 dots
-// + 32 (7 382).
-template <class R, class S, int NW, bool PHASED>
-__device__ __forceinline__ void shared_wedge_loop(const BaryonSpin<R> &b, const cx<R> (&a)[9], const S *Pjj,
-                                                  const S *Nl, const S *const (&Nx)[NW], const S *q, S *lps,
-                                                  int l, uint32_t p2base, cx<R> (&s1)[NW], cx<R> (&s2)[NW])
-{
-  const CliffordSet<R> &cl = b.cl;
-  const int ng = cl.ng;
-#pragma unroll 1
-  for (int mm = 0; mm < 4; ++mm) {
-    const int n = (l + mm) & 3;
-    cx<R> e[9];
-    {
-      cx<R> bn[9];
-      load9(bn, Pjj + n * 9);
-#pragma unroll
-      for (int k = 0; k < 9; ++k) e[k] = czero<R>();
-      wedge_acc(e, a, bn);
-    }
-    if (mm == 0) {  // n = l: the loop form's wedge
-#pragma unroll
-      for (int w = 0; w < NW; ++w) {
-        cx<R> qw[9];
-        load9(qw, q + w * 9);
-        const cx<R> sq = dot9(e, qw);
-        lps[w] = S {sq.x, sq.y};
-      }
-    }
-    const int ln = b.perm2[n];
-    const uint32_t q0 = (p2base + b.ph2[0][ln]) & 3u;
-#pragma unroll
-    for (int k = 0; k < NW; ++k) {
-      if (k < ng) {
-        cx<R> nn[9];
-        load9(nn, Nl + cl.perm[k][n] * 36);  // pass 1
-        const cx<R> d = dot9(e, nn);
-        s1[k] = cadd(s1[k], PHASED ? mul_phase(d, cl.ph[k][n]) : d);
-        load9(nn, Nx[k] + ln * 9);  // pass 2
-        s2[k] = cadd(s2[k], mul_phase(dot9(e, nn), q0));
-      }
-    }
-  }
-}
-
-template <class R, class S, int NW>
-__device__ __forceinline__ void fused_shared_wedge_site(const BaryonSpin<R> &b, const S *Pi, const S *Pj, const S *N,
-                                                        const S *q, int i, int x, cx<R> *vals)
-{
-  const CliffordSet<R> &cl = b.cl;
-  const int j = b.perm1[i];
-  const int l = b.perm2[x];
-  const int ng = cl.ng;  // <= NW gamma-basis terms
-  cx<R> a[9];
-  load9(a, Pi + (i * 4 + x) * 9);
-  S *lps = const_cast<S *>(q) + 9 * NW + (i * 4 + x) * NW;  // loop values, parked in shared memory
-  const S *Nx[NW];
-#pragma unroll
-  for (int k = 0; k < NW; ++k) Nx[k] = N + (k < ng ? cl.perm[k][x] : 0) * 36;
-  cx<R> s1[NW], s2[NW];
-#pragma unroll
-  for (int k = 0; k < NW; ++k) s1[k] = s2[k] = czero<R>();
-  const uint32_t p2base = b.ph1[1][j];
-  if (cl.has_phase[0] || cl.has_phase[1])
-    shared_wedge_loop<R, S, NW, true>(b, a, Pj + j * 36, N + l * 9, Nx, q, lps, l, p2base, s1, s2);
-  else
-    shared_wedge_loop<R, S, NW, false>(b, a, Pj + j * 36, N + l * 9, Nx, q, lps, l, p2base, s1, s2);
-  const uint32_t p1 = (b.ph1[0][i] + b.ph2[0][l]) & 3u, v1 = (b.ph2[1][0] - b.ph2[0][0]) & 3u;
-#pragma unroll
-  for (int w = 0; w < NW; ++w) {
-    cx<R> u1 = czero<R>(), u2 = czero<R>();
-#pragma unroll
-    for (int k = 0; k < NW; ++k) {
-      if (k < ng) {
-        cfma(u1, cx<R> {cl.coef[w][k][0], cl.coef[w][k][1]}, s1[k]);
-        cfma(u2, cx<R> {cl.qc[w][k][x][0], cl.qc[w][k][x][1]}, s2[k]);
-      }
-    }
-    const cx<R> lv = mul_phase(cx<R> {lps[w].x, lps[w].y}, p1);
-    const cx<R> t1 = mul_phase(u1, p1);
-    vals[0 * NW + w] = lv;                  // IK_JL_NM
-    vals[2 * NW + w] = mul_phase(lv, v1);   // IL_JK_NM
-    vals[1 * NW + w] = t1;                  // IK_JM_NL
-    vals[3 * NW + w] = mul_phase(t1, v1);   // IL_JM_NK
-    vals[4 * NW + w] = u2;                  // IM_JK_NL
-    vals[5 * NW + w] = mul_phase(u2, v1);   // IM_JL_NK
-  }
-}
-
-// One field P for P_i and P_j (the proton's two u quarks), with perm1 free of
-// fixed points (Gamma_ij = C g5 and most others): the wedge E[i][x][n] =
-// P[i][x] ^ P[perm1 i][n] is also the wedge of slot (perm1 i, n, x), and with
-// one field the second triangle pass equals the first.  So eight threads per
-// site, thread (i, x) with i < perm1 i, form the 32 distinct wedges once and
-// each wedge serves two slots:
-//   own slot (i, x, n):           target (i, l = perm2 x), m = n  -- as pass 1 above
-//   partner slot (perm1 i, n, x): target (perm1 i, perm2 n), m = x -- the N blocks
-//                                 and coefficients of pass 2 above
-// Both targets feed all four triangle types (IK_JM_NL with the Gamma_ij phase
-// row of P_i first, IM_JK_NL with the transposed row; the Gamma_kl^T variants
-// by the sign i^v1 as above); the n = l wedge gives the loop values of both
-// targets.  Per site: 32 wedges + 128 dots + 16 loop dots (2 592 complex FMA
-// with two two-term projectors) instead of the one-pass form's 64 + 128 + 32
-// (3 744).
-template <class R, class S, int NW, bool PHASED>
-__device__ __forceinline__ void shared_wedge_same_loop(const BaryonSpin<R> &b, const cx<R> (&a)[9], const S *Pjj,
-                                                       const S *Nl, const S *const (&Nx)[NW], const S *q, S *lps,
-                                                       int l, uint32_t lph, cx<R> (&s1)[NW], cx<R> (&s2)[NW])
-{
-  const CliffordSet<R> &cl = b.cl;
-  const int ng = cl.ng;
-#pragma unroll 1
-  for (int mm = 0; mm < 4; ++mm) {
-    const int n = (l + mm) & 3;
-    cx<R> e[9];
-    {
-      cx<R> bn[9];
-      load9(bn, Pjj + n * 9);
-#pragma unroll
-      for (int k = 0; k < 9; ++k) e[k] = czero<R>();
-      wedge_acc(e, a, bn);
-    }
-    if (mm == 0) {  // n = l: the loop wedge of (i, l) and of the partner target (j, x)
-#pragma unroll
-      for (int w = 0; w < NW; ++w) {
-        cx<R> qw[9];
-        load9(qw, q + w * 9);
-        const cx<R> sq = dot9(e, qw);
-        const cx<R> lv = cadd(sq, mul_phase(sq, lph));  // own phase factored out: 1 + i^(partner - own)
-        lps[w] = S {lv.x, lv.y};
-      }
-    }
-    const int ln = b.perm2[n];
-    const uint32_t q0 = b.ph2[0][ln];
-#pragma unroll
-    for (int k = 0; k < NW; ++k) {
-      if (k < ng) {
-        cx<R> nn[9];
-        load9(nn, Nl + cl.perm[k][n] * 36);  // own slot
-        const cx<R> d = dot9(e, nn);
-        s1[k] = cadd(s1[k], PHASED ? mul_phase(d, cl.ph[k][n]) : d);
-        load9(nn, Nx[k] + ln * 9);  // partner slot
-        s2[k] = cadd(s2[k], mul_phase(dot9(e, nn), q0));
-      }
-    }
-  }
-}
-
-template <class R, class S, int NW>
-__device__ __forceinline__ void fused_shared_wedge_same_site(const BaryonSpin<R> &b, const S *P, const S *N,
-                                                             const S *q, int sub, cx<R> *vals)
-{
-  const CliffordSet<R> &cl = b.cl;
-  const int i = (sub >> 2) == 0 ? 0 : (b.perm1[0] == 1 ? 2 : 1);  // the two rows with i < perm1 i
-  const int x = sub & 3;
-  const int j = b.perm1[i];
-  const int l = b.perm2[x];
-  const int ng = cl.ng;
-  cx<R> a[9];
-  load9(a, P + (i * 4 + x) * 9);
-  S *lps = const_cast<S *>(q) + 9 * NW + sub * NW;  // loop values, parked in shared memory
-  const S *Nx[NW];
-#pragma unroll
-  for (int k = 0; k < NW; ++k) Nx[k] = N + (k < ng ? cl.perm[k][x] : 0) * 36;
-  cx<R> s1[NW], s2[NW];
-#pragma unroll
-  for (int k = 0; k < NW; ++k) s1[k] = s2[k] = czero<R>();
-  const uint32_t own = (b.ph1[0][i] + b.ph2[0][l]) & 3u;   // IK_JM_NL / loop phase of target (i, l)
-  const uint32_t part = (b.ph1[0][j] + b.ph2[0][x]) & 3u;  // loop phase of the partner target (j, x)
-  if (cl.has_phase[0] || cl.has_phase[1])
-    shared_wedge_same_loop<R, S, NW, true>(b, a, P + j * 36, N + l * 9, Nx, q, lps, l, (part - own) & 3u, s1, s2);
-  else
-    shared_wedge_same_loop<R, S, NW, false>(b, a, P + j * 36, N + l * 9, Nx, q, lps, l, (part - own) & 3u, s1, s2);
-  // the IM_* group takes the transposed Gamma_ij phase row: a fixed offset per row
-  const uint32_t di = (b.ph1[1][i] - b.ph1[0][i]) & 3u, dj = (b.ph1[1][j] - b.ph1[0][j]) & 3u;
-  const uint32_t v1 = (b.ph2[1][0] - b.ph2[0][0]) & 3u;
-#pragma unroll
-  for (int w = 0; w < NW; ++w) {
-    cx<R> u1 = czero<R>(), u2 = czero<R>();
-#pragma unroll
-    for (int k = 0; k < NW; ++k) {
-      if (k < ng) {
-        cfma(u1, cx<R> {cl.coef[w][k][0], cl.coef[w][k][1]}, s1[k]);
-        cfma(u2, cx<R> {cl.qc[w][k][x][0], cl.qc[w][k][x][1]}, s2[k]);
-      }
-    }
-    const cx<R> o1 = mul_phase(u1, own);   // target (i, l)
-    const cx<R> o2 = mul_phase(u2, b.ph1[0][j]);  // target (j, perm2 n): its column phase is already in s2
-    const cx<R> lv = mul_phase(cx<R> {lps[w].x, lps[w].y}, own);
-    const cx<R> t1 = cadd(o1, o2);
-    const cx<R> t2 = cadd(mul_phase(o1, di), mul_phase(o2, dj));
-    vals[0 * NW + w] = lv;                  // IK_JL_NM
-    vals[2 * NW + w] = mul_phase(lv, v1);   // IL_JK_NM
-    vals[1 * NW + w] = t1;                  // IK_JM_NL
-    vals[3 * NW + w] = mul_phase(t1, v1);   // IL_JM_NK
-    vals[4 * NW + w] = t2;                  // IM_JK_NL
-    vals[5 * NW + w] = mul_phase(t2, v1);   // IM_JL_NK
-  }
-}
-
 // ------------------------------------------------------------------ ops --
 // Common compile-time configuration of an op: CW consumer warps (plus one
 // producer warp), TPS threads per site, NST ring stages.
@@ -1021,152 +630,6 @@ struct BaryonTriCliffOp : OpBase<R, S, CW, TPS, NST> {
   __device__ static void site(const OpParams<R> &p, const S *const *in, S *, int sub, cx<R> *vals)
   {
     triangle_cliff_site<R, S, TPS, 1, 1>(p.b, in[0], in[1], in[2], sub, 0, vals);
-  }
-};
-
-// All six types x NW projectors in one pass over (P_i, P_j, P_n), projectors
-// in the gamma basis (e.g. (1 +- g4)/2 = (Gamma(0) +- Gamma(8))/2).
-// Output o = type * NW + w, types in contract_enum.h order.
-template <class R, class S, int CW, int TPS, int NST, int NW>
-struct BaryonFusedCliffOp : OpBase<R, S, CW, TPS, NST> {
-  static constexpr int NIN = 3, NOUT = 6 * NW, EXTRA_BYTES = cbytes<S>(9 * NW);
-  static constexpr bool FIELD = false;
-  static_assert(TPS == 16, "one (i, l) pair per thread");
-  __device__ static void site(const OpParams<R> &p, const S *const *in, S *scratch, int sub, cx<R> *vals)
-  {
-    build_q_cliff<R, S, TPS, NW>(p.b, in[2], scratch, sub);
-    __syncwarp();
-    const int i = sub >> 2, l = sub & 3;
-    cx<R> t[2 * NW], lp[2 * NW];
-    // IK_JM_NL, IL_JM_NK, with IK_JL_NM, IL_JK_NM folded into the first wedge
-    fused_triangle_pass<R, S, NW, true>(p.b, in[0], in[1], in[2], scratch, i, l, 0, t, lp);
-#pragma unroll
-    for (int w = 0; w < NW; ++w) {
-      vals[0 * NW + w] = lp[0 * NW + w];
-      vals[2 * NW + w] = lp[1 * NW + w];
-      vals[1 * NW + w] = t[0 * NW + w];
-      vals[3 * NW + w] = t[1 * NW + w];
-    }
-    fused_triangle_pass<R, S, NW, false>(p.b, in[1], in[0], in[2], scratch, i, l, 1, t, lp);  // IM_JK_NL, IM_JL_NK
-#pragma unroll
-    for (int w = 0; w < NW; ++w) {
-      vals[4 * NW + w] = t[0 * NW + w];
-      vals[5 * NW + w] = t[1 * NW + w];
-    }
-  }
-};
-
-// The same six types x NW projectors with both triangle passes in one m loop
-// (fused_merged_site): fewer N loads, more live registers.
-template <class R, class S, int CW, int TPS, int NST, int NW, int MINB = 0, bool SAMEIJ = false>
-struct BaryonFusedCliffMergedOp : OpBase<R, S, CW, TPS, NST> {
-  static constexpr int NIN = 3, NOUT = 6 * NW, EXTRA_BYTES = cbytes<S>(9 * NW + 16 * 2 * NW);
-  static constexpr bool FIELD = false;
-  static constexpr int MIN_CTAS = MINB;
-  static_assert(TPS == 16, "one (i, l) pair per thread");
-  __device__ static void site(const OpParams<R> &p, const S *const *in, S *scratch, int sub, cx<R> *vals)
-  {
-    build_q_cliff<R, S, TPS, NW>(p.b, in[2], scratch, sub);
-    __syncwarp();
-    fused_merged_site<R, S, NW, SAMEIJ>(p.b, in[0], in[1], in[2], scratch, sub >> 2, sub & 3, vals);
-  }
-};
-
-// The same six types x NW projectors with every wedge shared by both triangle
-// passes (fused_shared_wedge_site): a third fewer FMAs than the merged form.
-template <class R, class S, int CW, int TPS, int NST, int NW, int MINB = 0>
-struct BaryonFusedSharedWedgeOp : OpBase<R, S, CW, TPS, NST> {
-  static constexpr int NIN = 3, NOUT = 6 * NW, EXTRA_BYTES = cbytes<S>(9 * NW + 16 * NW);
-  static constexpr bool FIELD = false;
-  static constexpr int MIN_CTAS = MINB;
-  static_assert(TPS == 16, "one (i, x) pair per thread");
-  __device__ static void site(const OpParams<R> &p, const S *const *in, S *scratch, int sub, cx<R> *vals)
-  {
-    build_q_cliff<R, S, TPS, NW>(p.b, in[2], scratch, sub);
-    __syncwarp();
-    fused_shared_wedge_site<R, S, NW>(p.b, in[0], in[1], in[2], scratch, sub >> 2, sub & 3, vals);
-  }
-};
-
-// One field for P_i and P_j and perm1 without fixed points: eight threads per
-// site, each wedge serving two slots (fused_shared_wedge_same_site).  Two
-// inputs, in[0] = P and in[1] = P_n: the field is staged once per site.
-template <class R, class S, int CW, int NST, int NW, int MINB = 0>
-struct BaryonFusedSharedWedgeSameOp : OpBase<R, S, CW, 8, NST> {
-  static constexpr int NIN = 2, NOUT = 6 * NW, EXTRA_BYTES = cbytes<S>(9 * NW + 8 * NW);
-  static constexpr bool FIELD = false;
-  // Four sites share a warp here.  Their threads load colour blocks 4 i + x
-  // (x = 0..3, two rows i), 8-byte values at block * 72 bytes: with 1168-byte
-  // slots the next site's blocks land 16 bytes on, in banks the first site's
-  // blocks already use; 1184-byte slots move them 32 bytes on, clear of those.
-  static constexpr int SLOT_PAD = 32;
-  static constexpr int MIN_CTAS = MINB;
-  __device__ static void site(const OpParams<R> &p, const S *const *in, S *scratch, int sub, cx<R> *vals)
-  {
-    build_q_cliff<R, S, 8, NW>(p.b, in[1], scratch, sub);
-    __syncwarp();
-    fused_shared_wedge_same_site<R, S, NW>(p.b, in[0], in[1], scratch, sub, vals);
-  }
-};
-
-// All six types for one projector of rank <= 2 that is not one gamma matrix
-// (e.g. (1 + g4)/2 alone): the loop types through Q, the triangle types through
-// the factored form, with X_r from P_j for the first triangle pass and from P_i
-// for the swapped one, Y_r from P_n shared by both.  Output o = type.
-template <class R, class S, int CW, int TPS, int NST>
-struct BaryonFusedRankOp : OpBase<R, S, CW, TPS, NST> {
-  static constexpr int NIN = 3, NOUT = 6, EXTRA_BYTES = cbytes<S>(216) + cbytes<S>(9);
-  static constexpr bool FIELD = false;
-  __device__ static void site(const OpParams<R> &p, const S *const *in, S *scratch, int sub, cx<R> *vals)
-  {
-    S *q = scratch + 216;  // after the 24 X, Y, X' blocks
-    build_q<R, S, TPS, 1>(p.b, in[2], q, sub);
-    build_rank<R, S, TPS>(p.b.rk, in[1], in[2], in[0], scratch, sub);
-    __syncwarp();
-    cx<R> t[2];
-    loop_site<R, S, TPS, 2, 1>(p.b, in[0], in[1], q, sub, 0, t);  // IK_JL_NM, IL_JK_NM
-    vals[0] = t[0];
-    vals[2] = t[1];
-    triangle_rank_site<R, S, TPS, 2>(p.b, in[0], scratch, scratch + 72, sub, 0, t);  // IK_JM_NL, IL_JM_NK
-    vals[1] = t[0];
-    vals[3] = t[1];
-    triangle_rank_site<R, S, TPS, 2>(p.b, in[1], scratch + 144, scratch + 72, sub, 1, t);  // IM_JK_NL, IM_JL_NK
-    vals[4] = t[0];
-    vals[5] = t[1];
-  }
-};
-
-// All six types x NW projectors with N'_w = W_w N materialised per site
-// (projectors that are not short gamma-basis combinations).
-template <class R, class S, int CW, int TPS, int NST, int NW>
-struct BaryonFusedOp : OpBase<R, S, CW, TPS, NST> {
-  static constexpr int NIN = 3, NOUT = 6 * NW, EXTRA_BYTES = cbytes<S>(144) * NW + cbytes<S>(9 * NW);
-  static constexpr bool FIELD = false;
-  __device__ static void site(const OpParams<R> &p, const S *const *in, S *scratch, int sub, cx<R> *vals)
-  {
-    S *q = reinterpret_cast<S *>(reinterpret_cast<char *>(scratch) + cbytes<S>(144) * NW);
-    build_nprime<R, S, TPS, NW>(p.b, in[2], scratch, sub, p.b.cl.ng <= kNprimeCliffTerms);
-    build_q<R, S, TPS, NW>(p.b, in[2], q, sub);
-    __syncwarp();
-    cx<R> t[2 * NW];
-    loop_site<R, S, TPS, 2, NW>(p.b, in[0], in[1], q, sub, 0, t);  // IK_JL_NM, IL_JK_NM
-#pragma unroll
-    for (int w = 0; w < NW; ++w) {
-      vals[0 * NW + w] = t[0 * NW + w];
-      vals[2 * NW + w] = t[1 * NW + w];
-    }
-    triangle_site<R, S, TPS, 2, NW>(p.b, in[0], in[1], scratch, sub, 0, t);  // IK_JM_NL, IL_JM_NK
-#pragma unroll
-    for (int w = 0; w < NW; ++w) {
-      vals[1 * NW + w] = t[0 * NW + w];
-      vals[3 * NW + w] = t[1 * NW + w];
-    }
-    triangle_site<R, S, TPS, 2, NW>(p.b, in[1], in[0], scratch, sub, 1, t);  // IM_JK_NL, IM_JL_NK
-#pragma unroll
-    for (int w = 0; w < NW; ++w) {
-      vals[4 * NW + w] = t[0 * NW + w];
-      vals[5 * NW + w] = t[1 * NW + w];
-    }
   }
 };
 

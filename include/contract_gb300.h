@@ -213,8 +213,8 @@ void contract_baryon_all_types_host(void *correl, const void *propag_i, const vo
  * a device looks up the array's device address; make it before any stream
  * capture.  A lattice whose partial sums do not fit the array is rejected
  * with CONTRACT_ERROR_INVALID_ARGUMENT and a message naming both sizes (each
- * of the 2 Lt half-timeslices needs at least 1344 bytes with two projectors,
- * so Lt beyond about 6000 never fits; a 48^3 x 96 lattice does).  Returns
+ * of the 2 Lt half-timeslices counts as at least 576 bytes with two projectors,
+ * so Lt beyond 14563 never fits; a 48^3 x 96 lattice does).  Returns
  * CONTRACT_SUCCESS or the error code (errors also follow the error mode, like
  * every other call). */
 int contract_baryon_all_types_noalloc(void *correl, const void *propag_i, const void *propag_j,
