@@ -32,6 +32,7 @@ SOURCES = [
     "kernels_momentum.cu",
     "kernels_momentum_tc.cu",
     "kernels_momentum_fused.cu",
+    "kernels_momentum_rows.cu",
     "kernels_batch.cu",
     "noalloc.cu",
     "kernels_quda.cu",

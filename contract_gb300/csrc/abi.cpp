@@ -1175,7 +1175,7 @@ void run_mixed_batch(const ContractBaryonBatchItem *bitems, int nb, int gamma_ij
   mp->status = job.status;
 
   // per-extent tile shapes
-  int bvar = -1, mvar = -1;
+  int bvar = -1;
   const bool msame = [&] {
     bool same = nm > 0;
     for (int i = 0; i < nm; ++i) same = same && mitems[i].propag_i == mitems[i].propag_j;
@@ -1207,7 +1207,7 @@ void run_mixed_batch(const ContractBaryonBatchItem *bitems, int nb, int gamma_ij
     }, job.stream);
   }
   if (nm > 0) {
-    static const char *const kMomBatchNames[] = {"fused.site8.xy8", "fused.site16.xy8"};
+    static const char *const kMomBatchNames[] = {"rows"};  // one shape: the times are for the report
     std::vector<std::pair<std::string, int>> classes;
     std::vector<int> rep;
     for (int i = 0; i < nm; ++i) {
@@ -1223,7 +1223,7 @@ void run_mixed_batch(const ContractBaryonBatchItem *bitems, int nb, int gamma_ij
     const std::string tag = std::string("batch=meson_momentum,nmom=") + std::to_string(nmom) +
                             ",same=" + (msame ? "1" : "0");
     auto one = std::make_unique<cgb::MomBatchParams>();
-    mvar = tune_batch(tag, 2, kMomBatchNames, classes, [&](int c, int v) {
+    tune_batch(tag, 1, kMomBatchNames, classes, [&](int c, int) {
       // one item of class c alone: its own plane buffer at the workspace start
       *one = *mp;
       one->n_items = 1;
@@ -1236,7 +1236,7 @@ void run_mixed_batch(const ContractBaryonBatchItem *bitems, int nb, int gamma_ij
       float2 *pl = static_cast<float2 *>(ws.get((size_t)l[2] * l[3] * mp->nq * 256 * sizeof(float2)));
       if (!pl) return cudaErrorMemoryAllocation;
       one->items[0].planes = pl;
-      cudaError_t e = cgb::launch_momentum_batch(job, *one, msame, v == 1 ? 16 : 8);
+      cudaError_t e = cgb::launch_momentum_rows(job, *one, msame);
       if (e != cudaSuccess) return e;
       cgb::BaryonFinParams none {};
       return cgb::launch_batch_finalize(job, *one, none);
@@ -1266,7 +1266,7 @@ void run_mixed_batch(const ContractBaryonBatchItem *bitems, int nb, int gamma_ij
       const int *l = mp->items[i].latt;
       off += (size_t)l[2] * l[3] * mp->nq * 256 * sizeof(float2);
     }
-    if (!cuda_ok(cgb::launch_momentum_batch(job, *mp, msame, mvar == 1 ? 16 : 8), what)) return;
+    if (!cuda_ok(cgb::launch_momentum_rows(job, *mp, msame), what)) return;
   }
   cuda_ok(cgb::launch_batch_finalize(job, *mp, *bf), what);
 }

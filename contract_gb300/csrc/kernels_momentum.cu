@@ -11,7 +11,7 @@
 //      H[(nx, ny)][ab], in the form's arithmetic (FP64 planes for complex128,
 //      FP32 planes for the mixed form)
 //   3. momentum_finalize: Z transform and the sum over planes, returned in FP64.
-// The mixed form normally fuses 1 and 2 (kernels_momentum_fused.cu), so the
+// The mixed form normally fuses 1 and 2 (kernels_momentum_rows.cu), so the
 // per-site values never reach HBM.
 // For 32^3 x 64 and 125 momenta that is ~25 GFLOP instead of 537 GFLOP.
 // Phase tables exp(2 pi i k / L) are computed in FP64 on the host from the
@@ -523,7 +523,7 @@ static bool fused_disabled()
   return off;
 }
 
-static const char *const kMomFusedNames[] = {"fused.site8.xy8", "three-kernel", "fused.site16.xy8"};
+static const char *const kMomFusedNames[] = {"rows", "three-kernel", "fused.site16.xy8"};
 static const char *const kMomTcNames[] = {"tc.unit128", "tc.unit64", "tc.unit192"};
 static const int kMomTcSteps[] = {128, 64, 192};
 
@@ -540,15 +540,45 @@ int momentum_variants(Prec prec, int aux, const char *const **names)
   return 1;
 }
 
+// One call's plan as a batch of one item (what the row kernel reads of it).
+static MomBatchParams single_item(const MomPlan &plan, const void *in_i, const void *in_j, float2 *planes,
+                                  DeviceStatus *status)
+{
+  MomBatchParams mp {};
+  mp.status = status;
+  mp.n_items = 1;
+  mp.total_units = plan.latt[2] * plan.latt[3];
+  mp.ngx = plan.ngx;
+  mp.nq = plan.nq;
+  mp.np = plan.np;
+  for (int k = 0; k < plan.ngx; ++k) {
+    mp.gx_k[k] = plan.gx_k[k];
+    mp.gx_plus[k] = plan.gx_plus[k];
+    mp.gx_minus[k] = plan.gx_minus[k];
+  }
+  for (int q = 0; q < plan.nq; ++q) {
+    mp.q_ix[q] = plan.q_ix[q];
+    mp.q_ny[q] = plan.q_ny[q];
+  }
+  MomBatchItem &it = mp.items[0];
+  it.in[0] = static_cast<const char *>(in_i);
+  it.in[1] = static_cast<const char *>(in_j);
+  it.planes = planes;
+  for (int k = 0; k < 4; ++k) it.latt[k] = plan.latt[k];
+  it.ty = 1;
+  for (int k = 0; k < plan.latt[0]; ++k) mp.tab[0][k] = make_float2((float)plan.cosx[k], (float)plan.sinx[k]);
+  for (int k = 0; k < plan.latt[1]; ++k) mp.tab[1][k] = make_float2((float)plan.cosy[k], (float)plan.siny[k]);
+  return mp;
+}
+
 cudaError_t launch_meson_momentum(const Job &job, const OpParams<double> &p, const MomPlan &plan, void *out,
                                   bool tensor_cores)
 {
   if (job.volume == 0) return cudaSuccess;
   if (tensor_cores && job.prec != Prec::C64) return cudaErrorInvalidValue;
-  // job.variant (autotuner): complex64 -- 1 runs the three-kernel form, 2 the
-  // fused kernel with 16 site warps, 0 with 8; tensor cores -- the k-steps per
-  // work unit.  With no variant chosen, two fields take 16 site warps and one
-  // field passed twice 8 (the tuner's choices at 32^3 x 64).
+  // job.variant (autotuner): complex64 -- 0 (the default) runs the row kernel, 1
+  // the three-kernel form, 2 the fused kernel with 16 site warps; tensor cores --
+  // the k-steps per work unit.
   const bool fused = !tensor_cores && job.prec == Prec::C64 && momentum_fused_supported(plan) && !fused_disabled() &&
                      job.variant != 1;
   const size_t elem = job.prec == Prec::C128 ? sizeof(double2) : sizeof(float2);
@@ -566,8 +596,9 @@ cudaError_t launch_meson_momentum(const Job &job, const OpParams<double> &p, con
   float2 *planes_m = reinterpret_cast<float2 *>(ws + c_bytes);   // mixed form
 
   if (fused) {
-    const bool sw16 = job.variant == 2 || (job.variant < 0 && p.in[0] != p.in[1]);
-    cudaError_t e = launch_momentum_fused(job, p.in[0], p.in[1], planes_m, plan, sw16 ? 16 : 8);
+    cudaError_t e;
+    if (job.variant == 2) e = launch_momentum_fused(job, p.in[0], p.in[1], planes_m, plan);
+    else e = launch_momentum_rows(job, single_item(plan, p.in[0], p.in[1], planes_m, job.status), p.in[0] == p.in[1]);
     if (e != cudaSuccess) return e;
     return launch_finalize<float, true>(job, planes_m, static_cast<double2 *>(out), plan);
   }

@@ -52,16 +52,17 @@ size_t tc_partial_bytes(const TcGeom &g);
 cudaError_t launch_momentum_tc(const Job &job, const MomPlan &plan, const TcGeom &g, const void *field,
                                unsigned char *atiles, float *partial, void *out, bool tiles_ready = false);
 
-// Fused site + X/Y transform kernel of the mixed form (kernels_momentum_fused.cu):
-// writes the FP32 planes [Lt][Lz][nq][256] straight from the two complex64
+// Fused site + X/Y transform kernels of the mixed form (kernels_momentum_rows.cu
+// by default, kernels_momentum_fused.cu as the autotuner's alternative): they
+// write the FP32 planes [Lt][Lz][nq][256] straight from the two complex64
 // propagators.  Supported for up to three X groups and kMomQChunk pairs.
 bool momentum_fused_supported(const MomPlan &plan);
 cudaError_t launch_momentum_fused(const Job &job, const void *in_i, const void *in_j, float2 *planes,
-                                  const MomPlan &plan, int site_warps = 8);
+                                  const MomPlan &plan);
 
 // Tile-shape variants of the projection for the autotuner (Kind::Momentum).
 // aux = 2 * tensor_cores + (fused form supported) + 4 * (P_i and P_j one field):
-//   1, 5: complex64 fused with 8 or 16 site warps, or three kernels;
+//   1, 5: complex64 row kernel, three kernels, or fused with 16 site warps;
 //   2, 3: tensor-core unit sizes.
 int momentum_variants(Prec prec, int aux, const char *const **names);
 
@@ -115,9 +116,9 @@ struct BaryonFinParams {
   BaryonFinItem items[kMomBatchMaxItems];
 };
 
-// One persistent launch of the fused site + X/Y kernel over every item's
-// planes (site_warps 8 or 16).
-cudaError_t launch_momentum_batch(const Job &job, const MomBatchParams &p, bool same_field, int site_warps);
+// One persistent launch of the row kernel (kernels_momentum_rows.cu) over every
+// item's planes.
+cudaError_t launch_momentum_rows(const Job &job, const MomBatchParams &p, bool same_field);
 // One launch for the rest: the Z transform and Gamma-pair map of every
 // momentum item, and the per-timeslice sums of every baryon item in bf (n_items
 // may be 0 on either side).
