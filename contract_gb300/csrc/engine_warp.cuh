@@ -90,10 +90,10 @@ __global__ void __launch_bounds__(32 * Op::CW, Op::MIN_CTAS) warp_kernel(const _
   __syncthreads();
 
   const int local = lane / TPS, sub = lane % TPS;
-  const S *in[NIN];
+  S *in[NIN];  // an op may change its inputs in place
 #pragma unroll
   for (int q = 0; q < NIN; ++q)
-    in[q] = reinterpret_cast<const S *>(mine + WarpSmem<Op>::IN + ((size_t)q * SPW + local) * L::SLOT);
+    in[q] = reinterpret_cast<S *>(mine + WarpSmem<Op>::IN + ((size_t)q * SPW + local) * L::SLOT);
   S *scratch = reinterpret_cast<S *>(mine + WarpSmem<Op>::EXTRA + (size_t)local * Op::EXTRA_BYTES);
 
   // Issue the copies of a tile's inputs [q0, q1) on barrier b.
@@ -133,7 +133,7 @@ __global__ void __launch_bounds__(32 * Op::CW, Op::MIN_CTAS) warp_kernel(const _
       return;
     }
     typename Op::State state;
-    Op::first(ps, in, scratch, sub, state);
+    Op::first(ps, in, scratch, sub, local < cur.sites(), state);
     Walk nx = cur;
     nx.next(p);
     fence_proxy_async_smem();
@@ -144,7 +144,7 @@ __global__ void __launch_bounds__(32 * Op::CW, Op::MIN_CTAS) warp_kernel(const _
       return;
     }
     cx<R> vals[NVAL];
-    Op::second(ps, in[NIN - 1], scratch, sub, state, vals);
+    Op::second(ps, in[NIN - 1], scratch, sub, local < cur.sites(), state, vals);
     fence_proxy_async_smem();
     __syncwarp();
     if (nx.valid(p)) fetch(nx, NIN - 1, NIN, 1);

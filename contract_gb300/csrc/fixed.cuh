@@ -1,0 +1,245 @@
+// Colour wedges of complex128 blocks on the integer pipe.
+//
+// The FP64 pipe issues one warp instruction in 64 cycles per scheduler (2 lanes an
+// SM and cycle), IMAD.WIDE (32 x 32 + 64 -> 64 bits) one in about 4.2.  So a wedge,
+// 36 complex products, is summed in 64-bit integers: every value v of a site's
+// field is the fixed-point number (h 2^28 + l) 2^(E - 55), |h| <= 2^28,
+// |l| <= 2^27, E the exponent of the field's largest value at that site, and a
+// real product is three IMAD.WIDE (h h' into one sum, h l' + l h' into another)
+// where it was one DFMA: 13 cycles instead of 64.  The sums of up to 32 products
+// stay below 2^62 and are exact; they join, are rounded and become a double once
+// per result.
+//
+// Scales.  An entry [a][d] of a colour block has the scale 2^(E + r_a + c_d): E the
+// exponent of the field's largest value at the site, r and c of the colour rows
+// and columns, common to both fields (every term of a wedge's entry then has one
+// scale).  Colour rows or columns of very different size so keep their bits.
+//
+// Accuracy.  In units of the operands' scales A and B a value is off by at most
+// 2^-57 A, and the dropped l l' and the last rounding make about half a unit of
+// 2^-56 A B per result.  For entries of one size s (A ~ 4.5 s with the power of
+// two) that is 2^-52 s^2, against 2^-49.8 s^2 for 32 products summed in FP64, where
+// every sum rounds.  A block much smaller than its field keeps fewer bits, so the
+// integer form is taken only if no 3 x 3 block of the site that is not zero lies
+// more than 2 powers of two below the largest, in its scales, if every value is
+// finite and if all exponents leave room for the products; otherwise the warp
+// takes the FP64 form for its sites.  Values below 2^-60 of their scale count as
+// zero.  Measured against extended precision (4096 outputs of all types, two
+// projectors): 1.9e-16 of their norm for Gaussian fields, 2.3e-16 in FP64.
+#pragma once
+
+#include "common.cuh"
+
+namespace cgb {
+
+constexpr int kFixedMinExp = 723, kFixedMaxExp = 1323;  // biased: 2^-300 to 2^300
+constexpr int kFixedSpread = 2;   // powers of two between a block and its field's scale
+constexpr int kFixedColour = 100;  // and between colour rows or columns at most
+
+// The largest of a site's TPS threads' values.
+template <int TPS> __device__ __forceinline__ int group_max(int v)
+{
+#pragma unroll
+  for (int o = TPS / 2; o > 0; o >>= 1) v = max(v, __shfl_xor_sync(0xffffffffu, v, o));
+  return v;
+}
+
+// The scales of one site: entry [a][d] of field f at 2^(E[f] + r[a] + c[d] - 1023).
+struct FixedScales {
+  int E[2], r[3], c[3];
+};
+
+// Scales of the fields whose blocks this thread reads, over the site's TPS
+// threads; false if they do not suit the integer form.
+// blk: NA of the first field, then of the second (none: one field).
+template <int TPS, int NA, int N>
+__device__ __forceinline__ bool fixed_scales(const double2 *const (&blk)[N], FixedScales &f)
+{
+  int e[N][9];  // biased exponents; zeros (and what underflowed) far below
+#pragma unroll
+  for (int n = 0; n < N; ++n)
+#pragma unroll
+    for (int k = 0; k < 9; ++k) {
+      const double2 v = blk[n][k];
+      const int x = max(__double2hiint(v.x) & 0x7fffffff, __double2hiint(v.y) & 0x7fffffff) >> 20;
+      e[n][k] = x ? x : -4096;
+    }
+  f.E[0] = f.E[1] = -4096;
+#pragma unroll
+  for (int n = 0; n < N; ++n)
+#pragma unroll
+    for (int k = 0; k < 9; ++k) f.E[n < NA ? 0 : 1] = max(f.E[n < NA ? 0 : 1], e[n][k]);
+  f.E[0] = group_max<TPS>(f.E[0]);
+  f.E[1] = NA < N ? group_max<TPS>(f.E[1]) : f.E[0];
+  bool ok = min(f.E[0], f.E[1]) >= kFixedMinExp && max(f.E[0], f.E[1]) <= kFixedMaxExp;
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    int m = -8192;
+#pragma unroll
+    for (int n = 0; n < N; ++n)
+#pragma unroll
+      for (int d = 0; d < 3; ++d) m = max(m, e[n][3 * a + d] - f.E[n < NA ? 0 : 1]);
+    f.r[a] = max(group_max<TPS>(m), -kFixedColour);
+  }
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    int m = -8192;
+#pragma unroll
+    for (int n = 0; n < N; ++n)
+#pragma unroll
+      for (int a = 0; a < 3; ++a) m = max(m, e[n][3 * a + d] - f.E[n < NA ? 0 : 1] - f.r[a]);
+    f.c[d] = max(group_max<TPS>(m), -kFixedColour);
+  }
+#pragma unroll
+  for (int n = 0; n < N; ++n) {
+    int m = -8192;
+#pragma unroll
+    for (int k = 0; k < 9; ++k) m = max(m, e[n][k] - f.E[n < NA ? 0 : 1] - f.r[k / 3] - f.c[k % 3]);
+    ok = ok && (m >= -kFixedSpread || m < -2048);
+  }
+  return ok;
+}
+
+// v as h 2^28 + l in units of 2^(E - 55).
+__device__ __forceinline__ int2 to_fixed(double v, int E)
+{
+  const long long bits = __double_as_longlong(v);
+  const int hi = (int)(bits >> 32), e = (hi >> 20) & 0x7ff;
+  const unsigned long long t =
+    ((unsigned long long)(((uint32_t)hi & 0xfffffu) | 0x100000u) << 35) | ((unsigned long long)(uint32_t)bits << 3);
+  const int d = max(E - e, 0);  // below 0 only where the site is not converted for use
+  unsigned long long u = (t + ((1ull << (d & 63)) >> 1)) >> (d & 63);
+  if (d > 60 || e == 0) u = 0;
+  const long long m = hi < 0 ? -(long long)u : (long long)u;
+  const int h = (int)((m + (1ll << 27)) >> 28);
+  return make_int2(h, (int)((uint32_t)m - ((uint32_t)h << 28)));
+}
+
+// A colour block of field `field` to fixed point: (h, l) of re, then of im; dst may be blk.
+__device__ __forceinline__ void block_to_fixed(int4 *dst, const double2 *blk, const FixedScales &f, int field)
+{
+#pragma unroll
+  for (int k = 0; k < 9; ++k) {
+    const double2 v = blk[k];
+    const int E = f.E[field] + f.r[k / 3] + f.c[k % 3];
+    const int2 a = to_fixed(v.x, E), b = to_fixed(v.y, E);
+    dst[k] = make_int4(a.x, a.y, b.x, b.y);
+  }
+}
+
+// Running sums of fixed-point products: high words' products, and the cross ones
+// (2^-28 of a unit of the first).
+struct FixedSum {
+  long long hh, x;
+  __device__ __forceinline__ void mac(int ah, int al, int bh, int bl)
+  {
+    hh += (long long)ah * bh;
+    x += (long long)ah * bl;
+    x += (long long)al * bh;
+  }
+  // In units of 2^(scale + scale - 54); `up` is that power of two.
+  __device__ __forceinline__ double value(int up) const
+  {
+    const long long v = hh + ((x + (1ll << 27)) >> 28);
+    const double d = __ll2double_rn(v);
+    return v == 0 ? 0.0 : __hiloint2double(__double2hiint(d) + (up << 20), __double2loint(d));
+  }
+};
+
+// Row a of a sum of wedges x ^ y of converted blocks (see wedge_acc): three
+// results at a time, so that their sums take 24 registers and not 72.
+struct FixedWedgeRow {
+  FixedSum re[3], im[3];
+  __device__ __forceinline__ void clear()
+  {
+#pragma unroll
+    for (int e = 0; e < 3; ++e) re[e] = im[e] = FixedSum {0, 0};
+  }
+  __device__ __forceinline__ void negate()
+  {
+#pragma unroll
+    for (int e = 0; e < 3; ++e) {
+      re[e] = FixedSum {-re[e].hh, -re[e].x};
+      im[e] = FixedSum {-im[e].hh, -im[e].x};
+    }
+  }
+  __device__ __forceinline__ void add(int a, const int4 *xp, const int4 *yp)
+  {
+    const int a1 = (a + 1) % 3, a2 = (a + 2) % 3;
+    // half 0: x row a1 with y row a2, half 1: x row a2 with y row a1
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+      int4 x[3], y[3];
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        x[k] = xp[3 * (half ? a2 : a1) + k];
+        y[k] = yp[3 * (half ? a1 : a2) + k];
+      }
+#pragma unroll
+      for (int e = 0; e < 3; ++e) {
+        const int e1 = (e + 1) % 3, e2 = (e + 2) % 3;
+        // + x[e1] y[e2] - x[e2] y[e1] in half 0, the signs exchanged in half 1
+        term(e, x[e1], y[e2], half != 0);
+        term(e, x[e2], y[e1], half == 0);
+      }
+    }
+  }
+  __device__ __forceinline__ void term(int e, int4 u, int4 v, bool minus)
+  {
+    const int4 n = make_int4(-u.x, -u.y, -u.z, -u.w);
+    const int4 p = minus ? n : u, q = minus ? u : n;
+    re[e].mac(p.x, p.y, v.x, v.y);
+    re[e].mac(q.z, q.w, v.z, v.w);
+    im[e].mac(p.x, p.y, v.z, v.w);
+    im[e].mac(p.z, p.w, v.x, v.y);
+  }
+  // The sums as doubles: entry [a][e] multiplies the two other rows and columns.
+  __device__ __forceinline__ void get(int a, cx<double> *out, const FixedScales &f) const
+  {
+    const int up = f.E[0] + f.E[1] - 2 * 1023 - 54 + f.r[(a + 1) % 3] + f.r[(a + 2) % 3];
+#pragma unroll
+    for (int e = 0; e < 3; ++e) {
+      const int at = up + f.c[(e + 1) % 3] + f.c[(e + 2) % 3];
+      out[e] = {re[e].value(at), im[e].value(at)};
+    }
+  }
+};
+
+// A block of doubles held for several dots with converted blocks of one field: its
+// entries' scales are the inverse of that field's colour scales, so that all nine
+// products have one.
+struct FixedDotBlock {
+  int4 g[9];
+  int up;
+  __device__ __forceinline__ void set(const cx<double> (&v)[9], const FixedScales &f)
+  {
+    int E = -8192;
+#pragma unroll
+    for (int k = 0; k < 9; ++k) {
+      const int x = max(__double2hiint(v[k].x) & 0x7fffffff, __double2hiint(v[k].y) & 0x7fffffff) >> 20;
+      E = max(E, x ? x + f.r[k / 3] + f.c[k % 3] : -8192);
+    }
+#pragma unroll
+    for (int k = 0; k < 9; ++k) {
+      const int2 a = to_fixed(v[k].x, E - f.r[k / 3] - f.c[k % 3]), b = to_fixed(v[k].y, E - f.r[k / 3] - f.c[k % 3]);
+      g[k] = make_int4(a.x, a.y, b.x, b.y);
+    }
+    up = E + f.E[0] - 2 * 1023 - 54;
+  }
+  __device__ __forceinline__ cx<double> dot(const double2 *blk) const
+  {
+    const int4 *y = reinterpret_cast<const int4 *>(blk);
+    FixedSum re {0, 0}, im {0, 0};
+#pragma unroll
+    for (int k = 0; k < 9; ++k) {
+      const int4 u = g[k], v = y[k];
+      re.mac(u.x, u.y, v.x, v.y);
+      re.mac(-u.z, -u.w, v.z, v.w);
+      im.mac(u.x, u.y, v.z, v.w);
+      im.mac(u.z, u.w, v.x, v.y);
+    }
+    return {re.value(up), im.value(up)};
+  }
+};
+
+} // namespace cgb

@@ -138,12 +138,12 @@ cudaError_t launch_baryon_fused_batch(const Job &job, int nw, const OpParams<dou
   OpParams<double> d = p;
   if (job.prec == Prec::C128) {
     fill_fused_spin(d, false);
-    if (ng == 2) return nw == 1 ? run_batch<BaryonFusedOp<double, double2, 4, 16, 2, 1, false, 2>>(job, d, specs, n, fin)
-                                : run_batch<BaryonFusedOp<double, double2, 4, 16, 2, 2, false, 2>>(job, d, specs, n, fin);
-    if (ng > 2) return p.b.rk.r == 1 ? run_batch<BaryonFusedOp<double, double2, 4, 16, -1, 1, false, 2>>(job, d, specs, n, fin)
-                                     : run_batch<BaryonFusedOp<double, double2, 4, 16, -2, 1, false, 2>>(job, d, specs, n, fin);
-    return nw == 1 ? run_batch<BaryonFusedOp<double, double2, 4, 16, 1, 1, false, 2>>(job, d, specs, n, fin)
-                   : run_batch<BaryonFusedOp<double, double2, 4, 16, 1, 2, false, 2>>(job, d, specs, n, fin);
+    if (ng == 2) return nw == 1 ? run_batch<BaryonFusedOp<double, double2, 4, 16, 2, 1, false, 3>>(job, d, specs, n, fin)
+                                : run_batch<BaryonFusedOp<double, double2, 4, 16, 2, 2, false, 3>>(job, d, specs, n, fin);
+    if (ng > 2) return p.b.rk.r == 1 ? run_batch<BaryonFusedOp<double, double2, 4, 16, -1, 1, false, 3>>(job, d, specs, n, fin)
+                                     : run_batch<BaryonFusedOp<double, double2, 4, 16, -2, 1, false, 3>>(job, d, specs, n, fin);
+    return nw == 1 ? run_batch<BaryonFusedOp<double, double2, 4, 16, 1, 1, false, 3>>(job, d, specs, n, fin)
+                   : run_batch<BaryonFusedOp<double, double2, 4, 16, 1, 2, false, 3>>(job, d, specs, n, fin);
   }
   OpParams<float> q = convert_params<float>(p);
   if (ng <= 2 && batch_same_field(p, specs, n)) {

@@ -30,6 +30,7 @@
 #pragma once
 
 #include "engine_warp.cuh"
+#include "fixed.cuh"
 #include "ops.cuh"
 
 namespace cgb {
@@ -128,6 +129,67 @@ __device__ __forceinline__ void open_diquark(const FusedSpin &f, const S *A, con
   }
 }
 
+// The same in fixed point (fixed.cuh), from blocks that were converted.
+template <int NROW, int NN>
+__device__ __forceinline__ void open_diquark_fixed(const FusedSpin &f, const int4 *A, const int4 *B, int s, int n0,
+                                                   const FixedScales &fs, cx<double> (&g)[NN][9])
+{
+  const int s1 = f.s & 3, turn = (f.rows >> 8) & 7;
+#pragma unroll
+  for (int t = 0; t < NN; ++t)
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      FixedWedgeRow w;
+      w.clear();
+#pragma unroll 1
+      for (int k = 0; k < NROW; ++k) {
+        const int i = two_bits(f.rows, 2 * k);
+        if (k == turn) w.negate();
+        w.add(a, A + (i * 4 + s) * 9, B + ((i ^ s1) * 4 + n0 + t) * 9);
+      }
+      if (turn == NROW) w.negate();
+      w.get(a, g[t] + 3 * a, fs);
+    }
+}
+
+// Converts the site's blocks of P_i and P_j in place, if every site of the warp
+// suits the integer form.
+template <int TPS>
+__device__ __forceinline__ bool fields_to_fixed(double2 *A, double2 *B, int sub, bool live, FixedScales &fs)
+{
+  constexpr int NB = 16 / TPS;
+  const double2 *blk[2 * NB];
+#pragma unroll
+  for (int k = 0; k < NB; ++k) {
+    blk[k] = A + (sub + k * TPS) * 9;
+    blk[NB + k] = B + (sub + k * TPS) * 9;
+  }
+  const bool ok = fixed_scales<TPS, NB>(blk, fs);
+  if (!__all_sync(0xffffffffu, ok || !live)) return false;
+#pragma unroll
+  for (int k = 0; k < NB; ++k) {
+    block_to_fixed(reinterpret_cast<int4 *>(A + (sub + k * TPS) * 9), blk[k], fs, 0);
+    if (A != B) block_to_fixed(reinterpret_cast<int4 *>(B + (sub + k * TPS) * 9), blk[NB + k], fs, 1);
+  }
+  __syncwarp();
+  return true;
+}
+
+// Converts the blocks of P_n in place likewise.
+template <int TPS> __device__ __forceinline__ bool field_to_fixed(double2 *N, int sub, bool live, FixedScales &fs)
+{
+  constexpr int NB = 16 / TPS;
+  const double2 *blk[NB];
+#pragma unroll
+  for (int k = 0; k < NB; ++k) blk[k] = N + (sub + k * TPS) * 9;
+  const bool ok = fixed_scales<TPS, NB>(blk, fs);
+  if (!__all_sync(0xffffffffu, ok || !live)) return false;
+#pragma unroll
+  for (int k = 0; k < NB; ++k) block_to_fixed(reinterpret_cast<int4 *>(N + (sub + k * TPS) * 9), blk[k], fs, 0);
+  __syncwarp();
+  return true;
+}
+
 // A block of G held for several dots.  Complex64: g and its (im, re) swap as
 // FP32 pairs, so that each product pair is one packed FMA on the other block
 // as loaded: P = sum g (.) y, Q = sum swap(g) (.) y, g . y = (P.x - P.y, Q.x + Q.y).
@@ -198,11 +260,20 @@ struct BaryonFusedOp {
 
   // P_i and P_j: the thread's blocks of G, and the loop's blocks G[perm2 l][l]
   // to scratch.
-  __device__ static void first(const OpParams<R> &p, const S *const *in, S *scratch, int sub, State &g)
+  __device__ static void first(const OpParams<R> &p, S *const *in, S *scratch, int sub, bool live, State &g)
   {
     const FusedSpin f = p.b.fu;
     const int s = sub / TPC, n0 = (sub % TPC) * NN, l = s ^ ((f.s >> 2) & 3);
-    open_diquark<SAME ? 2 : 4, NN>(f, in[0], SAME ? in[0] : in[1], s, n0, g);
+    S *A = in[0], *B = SAME ? in[0] : in[1];
+    if constexpr (sizeof(R) == 8) {
+      FixedScales fs;
+      if (fields_to_fixed<TPS>(A, B, sub, live, fs))
+        open_diquark_fixed<SAME ? 2 : 4, NN>(f, reinterpret_cast<const int4 *>(A), reinterpret_cast<const int4 *>(B), s, n0, fs, g);
+      else
+        open_diquark<SAME ? 2 : 4, NN, R, S>(f, A, B, s, n0, g);
+    } else {
+      open_diquark<SAME ? 2 : 4, NN, R, S>(f, A, B, s, n0, g);
+    }
 #pragma unroll
     for (int t = 0; t < NN; ++t)
       if (l == n0 + t) {
@@ -212,7 +283,7 @@ struct BaryonFusedOp {
   }
 
   // P_n: the values of the site (called after a __syncwarp).
-  __device__ static void second(const OpParams<R> &p, const S *N, S *scratch, int sub, const State &g,
+  __device__ static void second(const OpParams<R> &p, S *N, S *scratch, int sub, bool live, const State &g,
                                 cx<R> (&vals)[NVAL])
   {
     const BaryonSpin<R> &b = p.b;
@@ -227,45 +298,6 @@ struct BaryonFusedOp {
     if constexpr (SRC < 0) {
       build_rank_y<R, S, TPS>(b.rk, N, blk, sub);
       __syncwarp();
-    }
-    // passes 1 and 2
-    cx<R> v1[NK], v2[NK];
-#pragma unroll
-    for (int k = 0; k < NK; ++k) v1[k] = v2[k] = czero<R>();
-    DotBlock<R> gb[NN];
-#pragma unroll
-    for (int t = 0; t < NN; ++t) gb[t].set(g[t]);
-#pragma unroll
-    for (int d = 0; d < ND; ++d) {
-      const int k = SRC < 0 ? 0 : d, sk = SRC > 0 ? two_bits(f.s, 4 + 2 * d) : 0;
-#pragma unroll
-      for (int t = 0; t < NN; ++t) {
-        const int n = n0 + t, ln = n ^ s2;
-        const S *e1, *e2;  // the blocks of N' (or of the term, or Y) for passes 1 and 2
-        if constexpr (SRC > 0) {
-          e1 = N + ((n ^ sk) * 4 + l) * 9;
-          e2 = N + ((s ^ sk) * 4 + ln) * 9;
-        } else if constexpr (SRC < 0) {
-          e1 = blk + (d * 4 + l) * 9;
-          e2 = blk + (d * 4 + ln) * 9;
-        } else {
-          e1 = blk + (16 * d + n * 4 + l) * 9;
-          e2 = blk + (16 * d + s * 4 + ln) * 9;
-        }
-        const cx<R> d1 = gb[t].dot(e1), d2 = signed_by(gb[t].dot(e2), f.neg, ln);
-        if constexpr (SRC < 0) {
-          cfma(v1[0], cx<R> {b.rk.x[d][n][0], b.rk.x[d][n][1]}, d1);
-          cfma(v2[0], cx<R> {b.rk.x[d][s][0], b.rk.x[d][s][1]}, d2);
-        } else {
-          v1[k] = cadd(v1[k], SRC > 0 ? signed_by(d1, f.neg, 4 + 4 * d + n) : d1);
-          v2[k] = cadd(v2[k], d2);
-        }
-      }
-    }
-#pragma unroll
-    for (int k = 0; k < NK; ++k) {
-      v1[k] = signed_by(v1[k], f.neg, l);
-      if constexpr (SRC > 0) v2[k] = signed_by(v2[k], f.neg, 4 + 4 * k + s);
     }
     // loop: one colour entry per thread
     cx<R> lp[NK];
@@ -294,6 +326,64 @@ struct BaryonFusedOp {
         }
         cfma(lp[k], r, qk);
       }
+    }
+    // passes 1 and 2
+    cx<R> v1[NK], v2[NK];
+#pragma unroll
+    for (int k = 0; k < NK; ++k) v1[k] = v2[k] = czero<R>();
+    auto dots = [&](const auto (&gb)[NN]) {
+#pragma unroll
+      for (int d = 0; d < ND; ++d) {
+        const int k = SRC < 0 ? 0 : d, sk = SRC > 0 ? two_bits(f.s, 4 + 2 * d) : 0;
+#pragma unroll
+        for (int t = 0; t < NN; ++t) {
+          const int n = n0 + t, ln = n ^ s2;
+          const S *e1, *e2;  // the blocks of N' (or of the term, or Y) for passes 1 and 2
+          if constexpr (SRC > 0) {
+            e1 = N + ((n ^ sk) * 4 + l) * 9;
+            e2 = N + ((s ^ sk) * 4 + ln) * 9;
+          } else if constexpr (SRC < 0) {
+            e1 = blk + (d * 4 + l) * 9;
+            e2 = blk + (d * 4 + ln) * 9;
+          } else {
+            e1 = blk + (16 * d + n * 4 + l) * 9;
+            e2 = blk + (16 * d + s * 4 + ln) * 9;
+          }
+          const cx<R> d1 = gb[t].dot(e1), d2 = signed_by(gb[t].dot(e2), f.neg, ln);
+          if constexpr (SRC < 0) {
+            cfma(v1[0], cx<R> {b.rk.x[d][n][0], b.rk.x[d][n][1]}, d1);
+            cfma(v2[0], cx<R> {b.rk.x[d][s][0], b.rk.x[d][s][1]}, d2);
+          } else {
+            v1[k] = cadd(v1[k], SRC > 0 ? signed_by(d1, f.neg, 4 + 4 * d + n) : d1);
+            v2[k] = cadd(v2[k], d2);
+          }
+        }
+      }
+    };
+    auto plain = [&]() {
+      DotBlock<R> gb[NN];
+#pragma unroll
+      for (int t = 0; t < NN; ++t) gb[t].set(g[t]);
+      dots(gb);
+    };
+    if constexpr (sizeof(R) == 8 && SRC > 0) {
+      __syncwarp();  // the loop above has read P_n
+      FixedScales fs;
+      if (field_to_fixed<TPS>(N, sub, live, fs)) {
+        FixedDotBlock gb[NN];
+#pragma unroll
+        for (int t = 0; t < NN; ++t) gb[t].set(g[t], fs);
+        dots(gb);
+      } else {
+        plain();
+      }
+    } else {
+      plain();
+    }
+#pragma unroll
+    for (int k = 0; k < NK; ++k) {
+      v1[k] = signed_by(v1[k], f.neg, l);
+      if constexpr (SRC > 0) v2[k] = signed_by(v2[k], f.neg, 4 + 4 * k + s);
     }
     if constexpr (SAME) {
       const uint32_t e = f.out >> 5;  // Gamma_ij antisymmetric

@@ -1,0 +1,123 @@
+"""The integer-pipe form of the complex128 contractions (fixed.cuh) over inputs
+that it takes and inputs that it must leave to the FP64 form: Gaussian fields, a
+coherent part, colour rows and spin rows of different size, zero blocks and
+sites, colour-diagonal blocks, very large, very small and denormal values,
+NaN and infinity.
+
+Tolerance: 2e-15 of the norm of a call's outputs.  The results are off by 1.5 to
+3e-16 of that norm (measured against extended precision) in either form and the
+oracle's own FP64 by as much; a dropped low word or a wrong scale is off by 1e-9
+or more."""
+import numpy as np
+import pytest
+
+from oracle import einsum_oracle as eo
+
+pytestmark = pytest.mark.gpu
+LATT = (4, 3, 3, 4)
+V = int(np.prod(LATT))
+TOL = 2e-15
+
+
+def gauss(rng):
+    return rng.standard_normal((V, 4, 4, 3, 3)) + 1j * rng.standard_normal((V, 4, 4, 3, 3))
+
+
+def blocks(rng, kind):
+    p = gauss(rng)
+    if kind == "coherent":
+        p = p + gauss(rng)[:1]
+    elif kind == "colour rows":
+        p = p * np.array([1, 1e-3, 1e-6])[:, None]
+    elif kind == "colour columns":
+        p = p * np.array([1e5, 1, 1e-9])[None, :]
+    elif kind == "spin rows":
+        p = p * np.array([1, 1e-2, 1, 1e-5])[None, :, None, None, None]
+    elif kind == "uneven blocks":
+        p = p * 2.0 ** rng.integers(-6, 7, (V, 4, 4, 1, 1))
+    elif kind == "zeros":
+        p[:, 1, 2] = 0
+        p[:, 3] *= rng.random((V, 4, 1, 1)) < 0.5
+        p[::5] = 0
+    elif kind == "colour diagonal":
+        p = p * np.eye(3)
+    elif kind == "large":
+        p = p * 1e95
+    elif kind == "small":
+        p = p * 1e-95
+    elif kind == "mixed sites":
+        p = p * 10.0 ** rng.integers(-60, 60, (V, 1, 1, 1, 1))
+    elif kind == "denormal":
+        p[:, 0, 0, 1, 1] = 3e-310
+        p[3] = 4e-311 + 5e-312j
+    elif kind == "powers of two":
+        p = np.sign(p.real) * 2.0 ** rng.integers(-1, 2, p.shape) + 0j
+    return p
+
+
+KINDS = ["gauss", "coherent", "colour rows", "colour columns", "spin rows", "uneven blocks", "zeros", "colour diagonal",
+         "large", "small", "mixed sites", "denormal", "powers of two"]
+
+
+@pytest.fixture(scope="module")
+def api():
+    from contract_gb300 import api, build, pycontract
+    build.build()
+    pycontract.init(0)
+    return api
+
+
+def norm(a):
+    m = np.abs(a).max()
+    return m * np.sqrt((np.abs(a / m) ** 2).sum()) if m > 0 else 0.0
+
+
+def close(got, ref, kind):
+    """Per site where sites differ in scale, else over the call."""
+    got, ref = np.asarray(got), np.asarray(ref)
+    assert np.isfinite(got).all(), kind
+    if kind == "mixed sites":
+        scale = np.abs(ref).max(axis=tuple(range(ref.ndim - 1)), keepdims=True)
+        got, ref = got / scale, ref / scale
+    assert norm(got - ref) <= TOL * norm(ref), (kind, norm(got - ref) / norm(ref))
+
+
+def fields(kind, same=False):
+    import torch
+    rng = np.random.default_rng(KINDS.index(kind) + 1)
+    ps = [np.ascontiguousarray(blocks(rng, kind)) for _ in range(3)]
+    if same:
+        ps[1] = ps[0]
+    dev = [torch.from_numpy(p).cuda() for p in ps]
+    if same:
+        dev[1] = dev[0]
+    return ps, dev
+
+
+@pytest.mark.parametrize("same", [False, True])
+@pytest.mark.parametrize("kind", KINDS)
+def test_all_types(api, c_oracle, kind, same):
+    ps, dev = fields(kind, same)
+    pp = api.projector_plus_minus()
+    ref = np.array([[c_oracle.baryon_general_two_point(*ps, t, 5, 5, w) for w in pp] for t in range(6)])
+    got = api.baryon_all_types(*dev, 5, 5, pp).cpu().numpy()
+    if same:  # types that vanish identically are rounding noise on the scale of the others
+        ref, got = ref.reshape(12, V), got.reshape(12, V)
+    close(got, ref, kind)
+
+
+@pytest.mark.parametrize("bad", [np.nan, np.inf, -np.inf])
+def test_not_finite(api, c_oracle, bad):
+    """A value that is not finite spoils its own site and no other."""
+    ps, dev = fields("gauss")
+    pp = api.projector_plus_minus()
+    ref = np.array([[c_oracle.baryon_general_two_point(*ps, t, 5, 5, w) for w in pp] for t in range(6)])
+    for field in range(3):
+        ps2 = [p.copy() for p in ps]
+        ps2[field][7, 1, 2, 0, 1] = bad
+        dev[field].copy_(__import__("torch").from_numpy(ps2[field]))
+        got = api.baryon_all_types(*dev, 5, 5, pp).cpu().numpy()
+        dev[field].copy_(__import__("torch").from_numpy(ps[field]))
+        assert not np.isfinite(got[:, :, 7]).all()
+        keep = np.arange(V) != 7
+        close(got[:, :, keep], ref[:, :, keep], "gauss")
