@@ -1,4 +1,7 @@
-// Site-tile pipeline shared by every contraction kernel.
+// Site-tile pipeline of the field ops (diquark, sequential sources, the all-pair
+// meson field), and what every contraction kernel shares: the cut of the lattice,
+// slot layouts, chunk sums.  Contractions to numbers run on the per-warp pipelines
+// of engine_warp.cuh.
 //
 // Work decomposition
 // ------------------
@@ -29,13 +32,9 @@
 //
 // Outputs
 // -------
-// Scalar ops (mesons, baryons) produce NOUT complex numbers per site: either
-// written per site (the reference's per-site output) or summed per warp and
-// accumulated in FP64 per chunk into `partial[chunk][warp][NOUT]`, which
-// `finalize_kernel` reduces per timeslice in a fixed order (deterministic).
-// Field ops (diquark, sequential sources) produce a propagator-shaped site:
-// lanes write it to a per-warp shared-memory staging slot (double-buffered)
-// and lane 0 stores it with cp.async.bulk shared->global copies.
+// Field ops produce a propagator-shaped site: lanes write it to a per-warp
+// shared-memory staging slot (double-buffered) and lane 0 stores it with
+// cp.async.bulk shared->global copies, or (DIRECT_OUT) the op stores it itself.
 #pragma once
 
 #include <type_traits>
@@ -118,8 +117,7 @@ template <class Op> struct OutLayout {
 //   [0, 128)        full[NST], empty[NST] mbarriers, abort flag
 //   stages          NST x NIN x SITES slots
 //   extra           SITES x EXTRA_BYTES (per-site op scratch)
-//   tail            scalar ops of several outputs: per-warp site values [CW][SPW][NOUT] (cx<R>)
-//                   field ops:  per-warp output staging [CW][2][SPW] slots
+//   tail            per-warp output staging [CW][2][SPW] slots
 template <class Op> struct Smem {
   using L = OpLayout<Op>;
   static constexpr size_t STAGE = (size_t)Op::NIN * Op::SITES * L::SLOT;
@@ -128,10 +126,8 @@ template <class Op> struct Smem {
   static constexpr size_t TAIL = EXTRA + (size_t)Op::EXTRA_BYTES * Op::SITES;
   static constexpr size_t tail_bytes()
   {
-    if constexpr (Op::FIELD && Op::DIRECT_OUT) return 0;
-    else if constexpr (Op::FIELD) return 2ull * Op::SITES * OutLayout<Op>::SLOT;
-    else if constexpr (Op::NOUT == 1) return 0;
-    else return (size_t)Op::SITES * Op::NOUT * 2 * sizeof(typename Op::R);
+    if constexpr (Op::DIRECT_OUT) return 0;
+    else return 2ull * Op::SITES * OutLayout<Op>::SLOT;
   }
   static constexpr size_t BYTES = TAIL + tail_bytes();
   static_assert(2 * Op::NST * 8 + 4 <= 128, "too many stages for the barrier block");
@@ -246,118 +242,6 @@ __device__ __forceinline__ void produce(const typename Op::Params &p, unsigned c
 template <int NST> __device__ void drain(uint64_t *full, int from, unsigned long long wait_ns)
 {
   for (int u = from; u < from + NST; ++u) mbar_wait_bounded(&full[u % NST], (u / NST) & 1, wait_ns / 8);
-}
-
-// ------------------------------------------------------------ scalar ops --
-// A chunk's sums of a warp: every lane sums the value it holds of its own site
-// (after the site's threads joined theirs), and the warp's sites meet in FP64
-// when the chunk ends.
-template <int TPS, class R> __device__ __forceinline__ double2 warp_chunk_sum(const ChunkSum<R> &acc)
-{
-  double2 v = acc.value();
-#pragma unroll
-  for (int o = 16; o >= TPS; o >>= 1) {
-    v.x += __shfl_xor_sync(0xffffffffu, v.x, o);
-    v.y += __shfl_xor_sync(0xffffffffu, v.y, o);
-  }
-  return v;
-}
-
-template <class Op>
-__global__ void __launch_bounds__(Op::THREADS, min_blocks<Op>()) scalar_kernel(const __grid_constant__ typename Op::Params p)
-{
-  using S = typename Op::S;
-  using R = typename Op::R;
-  using L = OpLayout<Op>;
-  constexpr int NIN = Op::NIN, SITES = Op::SITES, TPS = Op::TPS, NST = Op::NST, NOUT = Op::NOUT;
-  constexpr int SPW = 32 / TPS, CW = Op::CW;
-
-  extern __shared__ __align__(128) unsigned char smem[];
-  __shared__ __align__(16) typename Op::Params ps;
-  uint64_t *full = reinterpret_cast<uint64_t *>(smem);
-  uint64_t *empty = full + NST;
-  volatile int *abort_flag = reinterpret_cast<volatile int *>(smem + 120);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (threadIdx.x == 0) {
-    for (int s = 0; s < NST; ++s) {
-      mbar_init(&full[s], 1);
-      mbar_init(&empty[s], CW);
-    }
-    *abort_flag = 0;
-    fence_barrier_init();
-  }
-  copy_params(ps, p);
-  __syncthreads();
-  if (warp == 0) {
-    produce<Op>(p, smem, full, empty, abort_flag);
-    return;
-  }
-
-  const TileGeom &g = p.geom;
-  const int w = warp - 1;
-  const int local = lane / TPS, sub = lane % TPS;
-  const int site = w * SPW + local;
-  cx<R> *sv = reinterpret_cast<cx<R> *>(smem + Smem<Op>::TAIL) + (size_t)w * SPW * NOUT;  // [SPW][NOUT]
-  S *scratch = reinterpret_cast<S *>(smem + Smem<Op>::EXTRA + (size_t)site * Op::EXTRA_BYTES);
-  ChunkSum<R> chunk_acc;
-
-  TileIter<SITES> it;
-  it.set_chunk(g, blockIdx.x);
-  for (int u = 0; it.valid(g); ++u) {
-    const int stage = u % NST;
-    const long long first = it.first;
-    const int n = it.sites();
-    const bool ok = mbar_wait_bounded(&full[stage], (u / NST) & 1, g.wait_ns);
-    if (!__all_sync(0xffffffffu, ok) || *abort_flag) {
-      if (lane == 0) {
-        *abort_flag = 1;
-        report(p.status, kDevErrWaitTimeout, (unsigned int)it.chunk);
-        drain<NST>(full, u, g.wait_ns);
-      }
-      return;
-    }
-    const unsigned char *sb = smem + Smem<Op>::STAGES + stage * Smem<Op>::STAGE;
-    const S *in[NIN];
-#pragma unroll
-    for (int q = 0; q < NIN; ++q) in[q] = reinterpret_cast<const S *>(sb + ((size_t)q * SITES + site) * L::SLOT);
-    cx<R> vals[NOUT];
-    Op::site(ps, in, scratch, sub, vals);
-#pragma unroll
-    for (int o = 0; o < NOUT; ++o) vals[o] = group_sum<TPS>(vals[o]);
-    __syncwarp();
-    if (lane == 0) mbar_arrive(&empty[stage]);  // inputs consumed; only registers below
-    const bool valid = site < n;
-    if (g.per_site) {
-      if (sub == 0 && valid) {
-#pragma unroll
-        for (int o = 0; o < NOUT; ++o)
-          static_cast<double2 *>(p.out[o])[first + site] = make_double2(double(vals[o].x), double(vals[o].y));
-      }
-    } else if constexpr (NOUT == 1) {
-      chunk_acc.add(valid ? vals[0] : czero<R>());
-      if (it.last_in_chunk()) {
-        const double2 z = warp_chunk_sum<TPS>(chunk_acc);
-        if (lane == 0) static_cast<double2 *>(p.out[0])[(size_t)it.chunk * CW + w] = z;
-        chunk_acc.reset();
-      }
-    } else {
-      if (sub == 0) {
-#pragma unroll
-        for (int o = 0; o < NOUT; ++o) sv[local * NOUT + o] = valid ? vals[o] : czero<R>();
-      }
-      __syncwarp();
-      if (lane < NOUT) {
-#pragma unroll
-        for (int s = 0; s < SPW; ++s) chunk_acc.add(sv[s * NOUT + lane]);
-        if (it.last_in_chunk()) {
-          static_cast<double2 *>(p.out[0])[((size_t)it.chunk * CW + w) * NOUT + lane] = chunk_acc.value();
-          chunk_acc.reset();
-        }
-      }
-      __syncwarp();
-    }
-    it.next(g, gridDim.x);
-  }
 }
 
 // ------------------------------------------------------------- field ops --

@@ -178,4 +178,120 @@ __global__ void __launch_bounds__(32 * Op::CW, Op::MIN_CTAS) warp_kernel(const _
   }
 }
 
+// ---------------------------------------------------------------- rings --
+// The same for ops of one step: a warp has an NST-stage ring of whole tiles, and
+// Op::site() yields the site's value -- the sum over its threads is one output
+// (NOUT == 1), or with NOUT > 1 thread sub holds output Op::output(p, sub) complete.
+template <class Op> struct RingSmem {
+  using L = OpLayout<Op>;
+  static constexpr int SPW = 32 / Op::TPS;
+  static constexpr size_t IN = (Op::NST * 8 + 15) / 16 * 16;  // after the warp's mbarriers
+  static constexpr size_t STAGE = (size_t)Op::NIN * SPW * L::SLOT;
+  static constexpr size_t EXTRA = IN + Op::NST * STAGE;
+  static constexpr size_t WARP = EXTRA + (size_t)SPW * Op::EXTRA_BYTES;
+  static constexpr size_t BYTES = Op::CW * WARP;
+  static_assert(Op::EXTRA_BYTES % 16 == 0, "slots must stay 16-byte aligned");
+};
+
+template <class Op, class Walk>
+__global__ void __launch_bounds__(32 * Op::CW, Op::MIN_CTAS) ring_kernel(const __grid_constant__ typename Walk::Params p)
+{
+  using S = typename Op::S;
+  using R = typename Op::R;
+  using L = OpLayout<Op>;
+  using M = RingSmem<Op>;
+  constexpr int NIN = Op::NIN, TPS = Op::TPS, SPW = 32 / TPS, NOUT = Op::NOUT, NST = Op::NST;
+
+  extern __shared__ __align__(128) unsigned char smem[];
+  __shared__ __align__(16) typename Op::Params ps;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  unsigned char *mine = smem + warp * M::WARP;
+  uint64_t *full = reinterpret_cast<uint64_t *>(mine);
+  if (lane == 0) {
+    for (int s = 0; s < NST; ++s) mbar_init(&full[s], 1);
+    fence_barrier_init();
+  }
+  copy_params(ps, op_params<Op>(p));
+  __syncthreads();
+
+  const int local = lane / TPS, sub = lane % TPS;
+  S *scratch = reinterpret_cast<S *>(mine + M::EXTRA + (size_t)local * Op::EXTRA_BYTES);
+  auto fetch = [&](const Walk &w, int stage) {
+    if (w.withheld(p)) return;  // test hook: this tile never arrives
+    const int n = w.sites();
+    if (lane == 0) mbar_arrive_expect_tx(&full[stage], (uint32_t)(n * NIN) * L::SITE_BYTES);
+    __syncwarp();
+    if (lane < SPW * NIN) {
+      const int q = lane / SPW, s = lane % SPW;
+      if (s < n)
+        bulk_g2s(mine + M::IN + stage * M::STAGE + ((size_t)q * SPW + s) * L::SLOT,
+                 w.in(p, q) + (w.first() + s) * L::SITE_BYTES, L::SITE_BYTES, &full[stage]);
+    }
+  };
+  static_assert(SPW * NIN <= 32, "one copy per lane");
+  Walk cur, ahead;
+  cur.start(p);
+  ahead = cur;
+  int issued = 0;
+  for (; issued < NST && ahead.valid(p); ++issued, ahead.next(p)) fetch(ahead, issued);
+  const unsigned long long wait_ns = ps.geom.wait_ns;
+  ChunkSum<R> chunk_acc;
+  for (int u = 0; cur.valid(p); ++u) {
+    const int stage = u % NST;
+    if (!__all_sync(0xffffffffu, mbar_wait_bounded(&full[stage], (u / NST) & 1, wait_ns))) {
+      report(p.status, kDevErrWaitTimeout, (unsigned int)cur.where());
+      if (lane == 0)  // the copies that may still be in flight
+        for (int v = u; v < issued; ++v) mbar_wait_bounded(&full[v % NST], (v / NST) & 1, wait_ns / 8);
+      return;
+    }
+    S *in[NIN];
+#pragma unroll
+    for (int q = 0; q < NIN; ++q)
+      in[q] = reinterpret_cast<S *>(mine + M::IN + stage * M::STAGE + ((size_t)q * SPW + local) * L::SLOT);
+    const bool ok = local < cur.sites();
+    cx<R> v;
+    if constexpr (Op::DIRECT_N) {  // the last field is read from memory by the op
+      const long long at = cur.first() + (ok ? local : 0);
+      v = Op::site(ps, in, reinterpret_cast<const S *>(cur.in(p, NIN) + at * L::SITE_BYTES), scratch, sub, ok);
+    } else {
+      v = Op::site(ps, in, scratch, sub, ok);
+    }
+    if constexpr (Op::CHANGES_INPUT) fence_proxy_async_smem();
+    __syncwarp();  // every lane is done with the stage
+    if (ahead.valid(p)) {
+      fetch(ahead, stage);
+      ++issued;
+      ahead.next(p);
+    }
+    if constexpr (NOUT == 1) v = group_sum<TPS>(v);
+    if (ps.geom.per_site) {
+      if (ok) {
+        if constexpr (NOUT == 1) {
+          if (sub == 0) static_cast<double2 *>(ps.out[0])[cur.first() + local] = make_double2(double(v.x), double(v.y));
+        } else {
+          static_cast<double2 *>(ps.out[Op::output(ps, sub)])[cur.first() + local] = make_double2(double(v.x), double(v.y));
+        }
+      }
+    } else {
+      chunk_acc.add(ok ? v : czero<R>());
+      if (cur.last_in_chunk()) {
+        double2 c = chunk_acc.value();
+#pragma unroll
+        for (int o = 16; o >= TPS; o >>= 1) {
+          c.x += __shfl_xor_sync(0xffffffffu, c.x, o);
+          c.y += __shfl_xor_sync(0xffffffffu, c.y, o);
+        }
+        if constexpr (NOUT == 1) {
+          if (lane == 0) cur.partial(p)[0] = c;
+        } else {
+          static_assert(NOUT == TPS, "one output per thread of a site");
+          if (lane < NOUT) cur.partial(p)[Op::output(ps, lane)] = c;
+        }
+        chunk_acc.reset();
+      }
+    }
+    cur.next(p);
+  }
+}
+
 } // namespace cgb

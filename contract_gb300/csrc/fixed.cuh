@@ -51,8 +51,9 @@ struct FixedScales {
 
 // Scales of the fields whose blocks this thread reads, over the site's TPS
 // threads; false if they do not suit the integer form.
-// blk: NA of the first field, then of the second (none: one field).
-template <int TPS, int NA, int N>
+// blk: NA of the first field, then of the second (none: one field).  Without
+// COLOUR there is one scale per field (contractions that sum over colours).
+template <int TPS, int NA, bool COLOUR = true, int N>
 __device__ __forceinline__ bool fixed_scales(const double2 *const (&blk)[N], FixedScales &f)
 {
   int e[N][9];  // biased exponents; zeros (and what underflowed) far below
@@ -73,22 +74,26 @@ __device__ __forceinline__ bool fixed_scales(const double2 *const (&blk)[N], Fix
   f.E[1] = NA < N ? group_max<TPS>(f.E[1]) : f.E[0];
   bool ok = min(f.E[0], f.E[1]) >= kFixedMinExp && max(f.E[0], f.E[1]) <= kFixedMaxExp;
 #pragma unroll
-  for (int a = 0; a < 3; ++a) {
-    int m = -8192;
+  for (int a = 0; a < 3; ++a) f.r[a] = f.c[a] = 0;
+  if constexpr (COLOUR) {
 #pragma unroll
-    for (int n = 0; n < N; ++n)
+    for (int a = 0; a < 3; ++a) {
+      int m = -8192;
 #pragma unroll
-      for (int d = 0; d < 3; ++d) m = max(m, e[n][3 * a + d] - f.E[n < NA ? 0 : 1]);
-    f.r[a] = max(group_max<TPS>(m), -kFixedColour);
-  }
+      for (int n = 0; n < N; ++n)
 #pragma unroll
-  for (int d = 0; d < 3; ++d) {
-    int m = -8192;
+        for (int d = 0; d < 3; ++d) m = max(m, e[n][3 * a + d] - f.E[n < NA ? 0 : 1]);
+      f.r[a] = max(group_max<TPS>(m), -kFixedColour);
+    }
 #pragma unroll
-    for (int n = 0; n < N; ++n)
+    for (int d = 0; d < 3; ++d) {
+      int m = -8192;
 #pragma unroll
-      for (int a = 0; a < 3; ++a) m = max(m, e[n][3 * a + d] - f.E[n < NA ? 0 : 1] - f.r[a]);
-    f.c[d] = max(group_max<TPS>(m), -kFixedColour);
+      for (int n = 0; n < N; ++n)
+#pragma unroll
+        for (int a = 0; a < 3; ++a) m = max(m, e[n][3 * a + d] - f.E[n < NA ? 0 : 1] - f.r[a]);
+      f.c[d] = max(group_max<TPS>(m), -kFixedColour);
+    }
   }
 #pragma unroll
   for (int n = 0; n < N; ++n) {
@@ -137,6 +142,8 @@ struct FixedSum {
     x += (long long)ah * bl;
     x += (long long)al * bh;
   }
+  // In units of 2^(scale + scale - 53).
+  __device__ __forceinline__ long long half_units() const { return (hh + ((x + (1ll << 27)) >> 28) + 1) >> 1; }
   // In units of 2^(scale + scale - 54); `up` is that power of two.
   __device__ __forceinline__ double value(int up) const
   {
@@ -204,6 +211,87 @@ struct FixedWedgeRow {
     }
   }
 };
+
+// d = sum over k in [k0, k1) of (+-) x_k ^ y_k: pair(k, x, y) gives the converted
+// blocks and returns whether the term is subtracted (the same for every thread).
+template <class Pair>
+__device__ __forceinline__ void fixed_wedge_sum(int k0, int k1, const FixedScales &f, Pair pair, cx<double> (&d)[9])
+{
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    FixedWedgeRow w;
+    w.clear();
+    bool minus = false;  // w holds the negative of the sum so far
+#pragma unroll 1
+    for (int k = k0; k < k1; ++k) {
+      const int4 *x, *y;
+      if (pair(k, x, y) != minus) {
+        w.negate();
+        minus = !minus;
+      }
+      w.add(a, x, y);
+    }
+    if (minus) w.negate();
+    w.get(a, d + 3 * a, f);
+  }
+}
+
+// Sums of nine integer pairs over a site's 16 threads, entry e with thread e (threads
+// 9-15 receive nothing): recursive halving of 16 slots, seven of them empty.
+__device__ __forceinline__ longlong2 group_sum_scatter9(const long long (&re)[9], const long long (&im)[9], int sub)
+{
+  long long a[8], b[8];
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {  // slots k and 8 + k: only slot 8 of the upper half is used
+    const bool up = (sub & 8) != 0;
+    const long long sa = up ? re[k] : (k == 0 ? re[8] : 0), sb = up ? im[k] : (k == 0 ? im[8] : 0);
+    const long long ra = __shfl_xor_sync(0xffffffffu, sa, 8), rb = __shfl_xor_sync(0xffffffffu, sb, 8);
+    a[k] = (up ? (k == 0 ? re[8] : 0) : re[k]) + ra;
+    b[k] = (up ? (k == 0 ? im[8] : 0) : im[k]) + rb;
+  }
+#pragma unroll
+  for (int h = 4; h > 0; h >>= 1) {
+    const bool up = (sub & h) != 0;
+#pragma unroll
+    for (int k = 0; k < h; ++k) {
+      const long long sa = up ? a[k] : a[h + k], sb = up ? b[k] : b[h + k];
+      a[k] = (up ? a[h + k] : a[k]) + __shfl_xor_sync(0xffffffffu, sa, h);
+      b[k] = (up ? b[h + k] : b[k]) + __shfl_xor_sync(0xffffffffu, sb, h);
+    }
+  }
+  return make_longlong2(a[0], b[0]);
+}
+
+// Entry e of a wedge sum held in half units as a double.
+__device__ __forceinline__ cx<double> fixed_entry(longlong2 v, int e, const FixedScales &f)
+{
+  const int a = e / 3, c = e - 3 * a;
+  int rows = 0, cols = 0;  // the two other rows and columns
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    if (k != a) rows += f.r[k];
+    if (k != c) cols += f.c[k];
+  }
+  const int up = f.E[0] + f.E[1] - 2 * 1023 - 53 + rows + cols;
+  const double x = __ll2double_rn(v.x), y = __ll2double_rn(v.y);
+  return {v.x ? __hiloint2double(__double2hiint(x) + (up << 20), __double2loint(x)) : 0.0,
+          v.y ? __hiloint2double(__double2hiint(y) + (up << 20), __double2loint(y)) : 0.0};
+}
+
+// x . conj(y) over two converted blocks of one scale each; up = 2^ of their scales - 54.
+__device__ __forceinline__ cx<double> fixed_conj_dot(const int4 (&x)[9], const int4 *y, int up)
+{
+  FixedSum re {0, 0}, im {0, 0};
+#pragma unroll
+  for (int k = 0; k < 9; ++k) {
+    const int4 u = x[k], v = y[k];
+    re.mac(u.x, u.y, v.x, v.y);
+    re.mac(u.z, u.w, v.z, v.w);
+    im.mac(u.z, u.w, v.x, v.y);
+    im.mac(-u.x, -u.y, v.z, v.w);
+  }
+  return {re.value(up), im.value(up)};
+}
 
 // A block of doubles held for several dots with converted blocks of one field: its
 // entries' scales are the inverse of that field's colour scales, so that all nine

@@ -1,76 +1,83 @@
 // Baryon two-point kernels, one contraction type per launch.
-// Op template arguments: <R, S, consumer warps, threads per site, ring stages>.
+// Op template arguments: <R, S, warps, (threads per site,) ring stages, CTAs per SM>.
 #include "launch_variants.cuh"
+#include "ops_site.cuh"
 
 namespace cgb {
 
-// complex128 (FP64-pipe bound), one (i, l) spin pair per thread: four consumer
-// warps and three ring stages (one CTA per SM: 8 sites x 3 inputs x 2 320 B per
-// stage), or smaller tiles and rings so that two or three CTAs fit.  The
-// default (used with autotuning off) is three consumer warps and two stages,
-// the tuner's choice at 24^3 x 64.
-static const VariantSet<double, 4> kLoopP = {
-  {run_scalar<BaryonLoopOp<double, double2, 4, 16, 3>>, run_scalar<BaryonLoopOp<double, double2, 3, 16, 2>>,
-   run_scalar<BaryonLoopOp<double, double2, 2, 16, 3>>, run_scalar<BaryonLoopOp<double, double2, 2, 16, 2>>},
-  {"cw4.tps16.st3", "cw3.tps16.st2", "cw2.tps16.st3", "cw2.tps16.st2"},
-  1};
-static const VariantSet<double, 4> kTriP = {
-  {run_scalar<BaryonTriOp<double, double2, 4, 16, 3>>, run_scalar<BaryonTriOp<double, double2, 3, 16, 2>>,
-   run_scalar<BaryonTriOp<double, double2, 2, 16, 3>>, run_scalar<BaryonTriOp<double, double2, 2, 16, 2>>},
-  {"cw4.tps16.st3", "cw3.tps16.st2", "cw2.tps16.st3", "cw2.tps16.st2"},
-  1};
-static const VariantSet<double, 4> kTriRankP = {
-  {run_scalar<BaryonTriRankOp<double, double2, 4, 16, 3>>, run_scalar<BaryonTriRankOp<double, double2, 3, 16, 2>>,
-   run_scalar<BaryonTriRankOp<double, double2, 2, 16, 3>>, run_scalar<BaryonTriRankOp<double, double2, 2, 16, 2>>},
-  {"cw4.tps16.st3", "cw3.tps16.st2", "cw2.tps16.st3", "cw2.tps16.st2"},
-  1};
-static const VariantSet<double, 4> kTriCliffP = {
-  {run_scalar<BaryonTriCliffOp<double, double2, 4, 16, 3>>, run_scalar<BaryonTriCliffOp<double, double2, 3, 16, 2>>,
-   run_scalar<BaryonTriCliffOp<double, double2, 2, 16, 3>>, run_scalar<BaryonTriCliffOp<double, double2, 2, 16, 2>>},
-  {"cw4.tps16.st3", "cw3.tps16.st2", "cw2.tps16.st3", "cw2.tps16.st2"},
-  1};
+template <class Op> static cudaError_t run_rank(const Job &job, OpParams<typename Op::R> p)
+{
+  fill_fused_spin(p, false);
+  return run_ring<Op>(job, p);
+}
 
-// complex64 variants: sites per tile x ring depth x CTAs per SM; the default
-// (last field) is the tuner's choice at 24^3 x 64.
-static const VariantSet<float, 4> kLoopM = {
-  {run_scalar<BaryonLoopOp<float, float2, 7, 16, 2>>, run_scalar<BaryonLoopOp<float, float2, 5, 16, 3>>,
-   run_scalar<BaryonLoopOp<float, float2, 4, 8, 3>>, run_scalar<BaryonLoopOp<float, float2, 3, 16, 3>>},
-  {"cw7.tps16.st2", "cw5.tps16.st3", "cw4.tps8.st3", "cw3.tps16.st3"},
-  3};
-// General projector (N' materialised per site).
-static const VariantSet<float, 4> kTriM = {
-  {run_scalar<BaryonTriOp<float, float2, 6, 16, 2>>, run_scalar<BaryonTriOp<float, float2, 7, 16, 3>>,
-   run_scalar<BaryonTriOp<float, float2, 4, 16, 3>>, run_scalar<BaryonTriOp<float, float2, 3, 16, 2>>},
-  {"cw6.tps16.st2", "cw7.tps16.st3", "cw4.tps16.st3", "cw3.tps16.st2"},
-  3};
-// Projector of rank <= 2 (X_r, Y_r blocks per site).
-static const VariantSet<float, 5> kTriRankM = {
-  {run_scalar<BaryonTriRankOp<float, float2, 3, 16, 2>>, run_scalar<BaryonTriRankOp<float, float2, 4, 16, 3>>,
-   run_scalar<BaryonTriRankOp<float, float2, 6, 16, 2>>, run_scalar<BaryonTriRankOp<float, float2, 7, 16, 2>>,
-   run_scalar<BaryonTriRankOp<float, float2, 4, 8, 2>>},
-  {"cw3.tps16.st2", "cw4.tps16.st3", "cw6.tps16.st2", "cw7.tps16.st2", "cw4.tps8.st2"},
+// complex128 on the integer pipe (fixed.cuh): bound by IMAD.WIDE issue and the
+// conversions, so warps in flight count and a second ring stage, which costs warps,
+// does not pay.  24^3 x 32 per site, three different fields, ms (the FP64 kernels
+// that these replaced in brackets): loop 1.17 [2.86 with a projector of two terms],
+// one gamma matrix 2.52, dense projector 3.82, rank 2 1.89 [4.65], rank 1 1.52.
+// The rank form with P_n read from memory: 8 warps an SM, more do not pay (11 warps
+// 1.99, 2 CTAs of 5 2.19: less L1 for P_n and fewer registers).
+static const VariantSet<double, 4> kLoopP = {
+  {run_ring<BaryonLoopOp<double, double2, 4, 16, 1, 3>>, run_ring<BaryonLoopOp<double, double2, 4, 16, 1, 2>>,
+   run_ring<BaryonLoopOp<double, double2, 2, 16, 1, 6>>, run_ring<BaryonLoopOp<double, double2, 13, 16, 1, 1>>},
+  {"w4.st1.occ3", "w4.st1.occ2", "w2.st1.occ6", "w13.st1.occ1"},
   0};
-static const VariantSet<float, 5> kTriCliffM = {
-  {run_scalar<BaryonTriCliffOp<float, float2, 7, 16, 2>>, run_scalar<BaryonTriCliffOp<float, float2, 5, 16, 3>>,
-   run_scalar<BaryonTriCliffOp<float, float2, 4, 8, 2>>, run_scalar<BaryonTriCliffOp<float, float2, 3, 16, 2>>,
-   run_scalar<BaryonTriCliffOp<float, float2, 4, 16, 3>>},
-  {"cw7.tps16.st2", "cw5.tps16.st3", "cw4.tps8.st2", "cw3.tps16.st2", "cw4.tps16.st3"},
-  3};
+static const VariantSet<double, 4> kTriP = {
+  {run_ring<BaryonTriOp<double, double2, 2, 1, 5>>, run_ring<BaryonTriOp<double, double2, 4, 1, 2>>,
+   run_ring<BaryonTriOp<double, double2, 4, 1, 3>>, run_ring<BaryonTriOp<double, double2, 10, 1, 1>>},
+  {"w2.st1.occ5", "w4.st1.occ2", "w4.st1.occ3", "w10.st1.occ1"},
+  0};
+static const VariantSet<double, 4> kTriRankP = {
+  {run_rank<BaryonTriRankOp<double, double2, 8, 1, 1>>, run_rank<BaryonTriRankOp<double, double2, 4, 1, 2>>,
+   run_rank<BaryonTriRankOp<double, double2, 5, 1, 2>>, run_rank<BaryonTriRankOp<double, double2, 3, 1, 3>>},
+  {"w8.st1.occ1", "w4.st1.occ2", "w5.st1.occ2", "w3.st1.occ3"},
+  0};
+static const VariantSet<double, 4> kTriGammaP = {
+  {run_ring<BaryonTriGammaOp<double, double2, 4, 16, 1, 3>>, run_ring<BaryonTriGammaOp<double, double2, 4, 16, 1, 2>>,
+   run_ring<BaryonTriGammaOp<double, double2, 2, 16, 1, 6>>, run_ring<BaryonTriGammaOp<double, double2, 4, 16, 2, 1>>},
+  {"w4.st1.occ3", "w4.st1.occ2", "w2.st1.occ6", "w4.st2.occ1"},
+  0};
+
+// complex64: HBM bound; sites in flight against warps.  24^3 x 64 per timeslice, ms
+// (one producer warp and a CTA-wide ring before, in brackets): loop 0.436 [0.440],
+// one gamma matrix 0.500 [0.565], dense 0.563 [0.655], rank 2 0.445 [0.492],
+// rank 1 0.432; the three fields take 0.457 ms at the copy rate's 6.68 TB/s.
+static const VariantSet<float, 4> kLoopM = {
+  {run_ring<BaryonLoopOp<float, float2, 4, 8, 1, 3>>, run_ring<BaryonLoopOp<float, float2, 4, 16, 1, 6>>,
+   run_ring<BaryonLoopOp<float, float2, 3, 8, 2, 2>>, run_ring<BaryonLoopOp<float, float2, 4, 16, 2, 3>>},
+  {"w4.tps8.st1.occ3", "w4.tps16.st1.occ6", "w3.tps8.st2.occ2", "w4.tps16.st2.occ3"},
+  0};
+static const VariantSet<float, 4> kTriM = {
+  {run_ring<BaryonTriOp<float, float2, 4, 1, 5>>, run_ring<BaryonTriOp<float, float2, 4, 2, 3>>,
+   run_ring<BaryonTriOp<float, float2, 3, 2, 4>>, run_ring<BaryonTriOp<float, float2, 4, 1, 4>>},
+  {"w4.st1.occ5", "w4.st2.occ3", "w3.st2.occ4", "w4.st1.occ4"},
+  0};
+static const VariantSet<float, 4> kTriRankM = {
+  {run_rank<BaryonTriRankOp<float, float2, 4, 1, 3>>, run_rank<BaryonTriRankOp<float, float2, 3, 1, 5>>,
+   run_rank<BaryonTriRankOp<float, float2, 5, 1, 3>>, run_rank<BaryonTriRankOp<float, float2, 8, 1, 2>>},
+  {"w4.st1.occ3", "w3.st1.occ5", "w5.st1.occ3", "w8.st1.occ2"},
+  0};
+static const VariantSet<float, 4> kTriGammaM = {
+  {run_ring<BaryonTriGammaOp<float, float2, 4, 16, 1, 5>>, run_ring<BaryonTriGammaOp<float, float2, 4, 16, 2, 3>>,
+   run_ring<BaryonTriGammaOp<float, float2, 4, 16, 1, 6>>, run_ring<BaryonTriGammaOp<float, float2, 4, 8, 1, 3>>},
+  {"w4.tps16.st1.occ5", "w4.tps16.st2.occ3", "w4.tps16.st1.occ6", "w4.tps8.st1.occ3"},
+  0};
 
 cudaError_t launch_baryon(const Job &job, bool loop, const OpParams<double> &p)
 {
   // A projector that is one gamma matrix (baryon_two_point) needs no N' buffer;
   // one of rank <= 2 takes the factored form.
-  const bool cliff = p.b.cl.ng == 1, rank = !cliff && p.b.rk.r > 0;
+  const bool gamma = p.b.cl.ng == 1, rank = !gamma && p.b.rk.r > 0;
   if (job.prec == Prec::C128) {
     if (loop) return kLoopP.launch(job, p);
     if (rank) return kTriRankP.launch(job, p);
-    return cliff ? kTriCliffP.launch(job, p) : kTriP.launch(job, p);
+    return gamma ? kTriGammaP.launch(job, p) : kTriP.launch(job, p);
   }
   const OpParams<float> q = convert_params<float>(p);
   if (loop) return kLoopM.launch(job, q);
   if (rank) return kTriRankM.launch(job, q);
-  return cliff ? kTriCliffM.launch(job, q) : kTriM.launch(job, q);
+  return gamma ? kTriGammaM.launch(job, q) : kTriM.launch(job, q);
 }
 
 // form: 0 loop, 1 triangle with one gamma, 2 triangle with N' materialised,
@@ -80,11 +87,11 @@ int baryon_variants(Prec prec, int form, const char *const **names)
   if (prec == Prec::C128) {
     if (form == 0) return kLoopP.describe(names);
     if (form == 3) return kTriRankP.describe(names);
-    return form == 1 ? kTriCliffP.describe(names) : kTriP.describe(names);
+    return form == 1 ? kTriGammaP.describe(names) : kTriP.describe(names);
   }
   if (form == 0) return kLoopM.describe(names);
   if (form == 3) return kTriRankM.describe(names);
-  return form == 1 ? kTriCliffM.describe(names) : kTriM.describe(names);
+  return form == 1 ? kTriGammaM.describe(names) : kTriM.describe(names);
 }
 
 } // namespace cgb

@@ -5,34 +5,12 @@
 
 namespace cgb {
 
-template <class Op> static cudaError_t run_warps(const Job &job, OpParams<typename Op::R> p)
+template <class Op> static cudaError_t run_warps(const Job &job, const OpParams<typename Op::R> &p)
 {
   if (job.volume == 0) return cudaSuccess;
-  using Walk = ChunkWalk<Op>;
   constexpr size_t smem = WarpSmem<Op>::BYTES;
   static_assert(smem <= 232448, "op does not fit in shared memory");
-  int bps = 0;
-  cudaError_t e = prepare<Op>(warp_kernel<Op, Walk>, smem, bps, 32 * Op::CW);
-  if (e != cudaSuccess) return e;
-  const int ctas = job.num_sms * bps;
-  p.geom = make_geom(job, Walk::SITES, (long long)ctas * Op::CW, kChunksPerCta);
-  p.status = job.status;
-  OutPtrs user_out {};
-  for (int o = 0; o < Op::NOUT; ++o) user_out.p[o] = static_cast<double2 *>(p.out[o]);
-  double2 *partial = nullptr;
-  if (!job.per_site) {
-    if (!job.ws) return cudaErrorInvalidValue;
-    partial = static_cast<double2 *>(job.ws->get((size_t)p.geom.total_chunks * Op::NOUT * sizeof(double2)));
-    if (!partial) return cudaErrorMemoryAllocation;
-    p.out[0] = partial;
-  }
-  const int grid = std::min((p.geom.total_chunks + Op::CW - 1) / Op::CW, ctas);
-  warp_kernel<Op, Walk><<<grid, 32 * Op::CW, smem, job.stream>>>(p);
-  e = cudaGetLastError();
-  if (e != cudaSuccess || job.per_site) return e;
-  finalize_kernel<<<Op::NOUT * job.lt, kFinThreads, 0, job.stream>>>(partial, user_out, Op::NOUT, job.lt,
-                                                                      p.geom.chunks_per_seg);
-  return cudaGetLastError();
+  return launch_chunks<Op>(job, p, warp_kernel<Op, ChunkWalk<Op>>, smem);
 }
 
 template <class R, class S, int CW, int TPS, int SRC, int NW, bool SAME, int MINB>

@@ -4,6 +4,7 @@
 #include <algorithm>
 #include <mutex>
 
+#include "engine_warp.cuh"
 #include "launch.hpp"
 
 namespace cgb {
@@ -77,16 +78,15 @@ struct OutPtrs {
 constexpr int kFinThreads = 64;  // finalize_kernel's block: the partials of one (output, timeslice)
 __global__ void finalize_kernel(const double2 *__restrict__ partial, OutPtrs out, int nout, int lt, int chunks_per_seg);
 
-template <class Op> cudaError_t run_scalar(const Job &job, OpParams<typename Op::R> p)
+// Launches a kernel of engine_warp.cuh over the job's chunks, dealt to the grid's
+// warps, and reduces the chunk partials if the job sums timeslices.
+template <class Op, class K> cudaError_t launch_chunks(const Job &job, OpParams<typename Op::R> p, K kernel, size_t smem)
 {
-  if (job.volume == 0) return cudaSuccess;
-  constexpr size_t smem = engine_smem_bytes<Op>();
-  static_assert(smem <= 232448, "op does not fit in shared memory");
   int bps = 0;
-  cudaError_t e = prepare<Op>(scalar_kernel<Op>, smem, bps);
+  cudaError_t e = prepare<Op>(kernel, smem, bps, 32 * Op::CW);
   if (e != cudaSuccess) return e;
-  const long long ctas = (long long)job.num_sms * bps;
-  p.geom = make_geom(job, Op::SITES, ctas, kChunksPerCta);
+  const int ctas = job.num_sms * bps;
+  p.geom = make_geom(job, ChunkWalk<Op>::SITES, (long long)ctas * Op::CW, kChunksPerCta);
   p.status = job.status;
   static_assert(Op::NOUT <= 16, "at most 16 outputs per site");
   OutPtrs user_out {};
@@ -94,18 +94,28 @@ template <class Op> cudaError_t run_scalar(const Job &job, OpParams<typename Op:
   double2 *partial = nullptr;
   if (!job.per_site) {
     if (!job.ws) return cudaErrorInvalidValue;
-    partial = static_cast<double2 *>(job.ws->get((size_t)p.geom.total_chunks * Op::CW * Op::NOUT * sizeof(double2)));
+    partial = static_cast<double2 *>(job.ws->get((size_t)p.geom.total_chunks * Op::NOUT * sizeof(double2)));
     if (!partial) return cudaErrorMemoryAllocation;
     p.out[0] = partial;
   }
-  const int grid = (int)std::min<long long>(p.geom.total_chunks, ctas);
-  scalar_kernel<Op><<<grid, Op::THREADS, smem, job.stream>>>(p);
+  const int grid = std::min((p.geom.total_chunks + Op::CW - 1) / Op::CW, ctas);
+  kernel<<<grid, 32 * Op::CW, smem, job.stream>>>(p);
   e = cudaGetLastError();
   if (e != cudaSuccess || job.per_site) return e;
-  // partial is [segment][chunk][consumer warp][NOUT]: fold the warps into the chunk count.
   finalize_kernel<<<Op::NOUT * job.lt, kFinThreads, 0, job.stream>>>(partial, user_out, Op::NOUT, job.lt,
-                                                                      p.geom.chunks_per_seg * Op::CW);
+                                                                      p.geom.chunks_per_seg);
   return cudaGetLastError();
+}
+
+// One launch of a per-call scalar op's ring kernel, then, for per-timeslice sums,
+// the finalisation of its chunk partials.
+template <class Op> cudaError_t run_ring(const Job &job, OpParams<typename Op::R> p)
+{
+  if (job.volume == 0) return cudaSuccess;
+  using Walk = ChunkWalk<Op>;
+  constexpr size_t smem = RingSmem<Op>::BYTES;
+  static_assert(smem <= 232448, "op does not fit in shared memory");
+  return launch_chunks<Op>(job, p, ring_kernel<Op, Walk>, smem);
 }
 
 template <class Op> cudaError_t run_field(const Job &job, OpParams<typename Op::R> p)

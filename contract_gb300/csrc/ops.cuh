@@ -205,215 +205,126 @@ __device__ __forceinline__ void build_nprime(const BaryonSpin<R> &b, const S *N,
   }
 }
 
-// Loop form.  Writes vals[v*NW + w] (partial over this thread's (i, l) pairs).
-template <class R, class S, int TPS, int NV, int NW>
-__device__ __forceinline__ void loop_site(const BaryonSpin<R> &b, const S *A, const S *B, const S *q, int sub, int c1sel,
-                                          cx<R> *vals)
+// Loop form: this thread's share of C (LPT (i, l) pairs).
+template <class R, class S, int TPS>
+__device__ __forceinline__ cx<R> loop_site(const BaryonSpin<R> &b, const S *A, const S *B, const S *q, int sub)
 {
   using Ln = Lanes<TPS>;
   const int i = sub / Ln::TPI, l0 = (sub % Ln::TPI) * Ln::LPT;
   const int j = b.perm1[i];
-  if constexpr (Ln::LPT == 1) {
-    // One (i, l) pair per thread: contract the wedge with Q first and apply
-    // the (i, l) phases to the NV x NW scalars only.
-    cx<R> x[9], y[9], t[9];
-    load9(x, A + (i * 4 + b.perm2[l0]) * 9);
-    load9(y, B + (j * 4 + l0) * 9);
+  cx<R> d[9], qw[9];
 #pragma unroll
-    for (int k = 0; k < 9; ++k) t[k] = czero<R>();
-    wedge_acc(t, x, y);
-#pragma unroll
-    for (int w = 0; w < NW; ++w) {
-      cx<R> qw[9];
-      load9(qw, q + w * 9);
-      const cx<R> s = dot9(t, qw);
-#pragma unroll
-      for (int v = 0; v < NV; ++v) vals[v * NW + w] = mul_phase(s, (b.ph1[c1sel][i] + b.ph2[v][l0]) & 3u);
-    }
-    return;
-  }
-  cx<R> r[NV][9];
-#pragma unroll
-  for (int v = 0; v < NV; ++v)
-#pragma unroll
-    for (int k = 0; k < 9; ++k) r[v][k] = czero<R>();
+  for (int k = 0; k < 9; ++k) d[k] = czero<R>();
 #pragma unroll
   for (int lo = 0; lo < Ln::LPT; ++lo) {
     const int l = l0 + lo;
     cx<R> x[9], y[9];
     load9(x, A + (i * 4 + b.perm2[l]) * 9);
     load9(y, B + (j * 4 + l) * 9);
-    if constexpr (NV == 1) {
-      phase9(x, b.ph2[0][l]);
-      wedge_acc(r[0], x, y);
-    } else {
-      cx<R> t[9];
-#pragma unroll
-      for (int k = 0; k < 9; ++k) t[k] = czero<R>();
-      wedge_acc(t, x, y);
-#pragma unroll
-      for (int v = 0; v < NV; ++v)
-#pragma unroll
-        for (int k = 0; k < 9; ++k) r[v][k] = cadd(r[v][k], mul_phase(t[k], b.ph2[v][l]));
-    }
+    // several pairs meet before Q: their phases relative to the first one's
+    if (lo > 0) phase9(x, (b.ph2[0][l] - b.ph2[0][l0]) & 3u);
+    wedge_acc(d, x, y);
   }
-  const uint32_t p1 = b.ph1[c1sel][i];
-#pragma unroll
-  for (int w = 0; w < NW; ++w) {
-    cx<R> qw[9];
-    load9(qw, q + w * 9);
-#pragma unroll
-    for (int v = 0; v < NV; ++v) vals[v * NW + w] = mul_phase(dot9(r[v], qw), p1);
-  }
+  load9(qw, q);
+  return mul_phase(dot9(d, qw), (b.ph1[0][i] + b.ph2[0][l0]) & 3u);
 }
 
-// Triangle form over N' (NW slots of 144 complex).  Writes vals[v*NW + w].
-// Loop order l -> m -> w: each B block is loaded once and feeds every
-// projector; with two projectors the wedge a ^ B_m is shared between them.
-template <class R, class S, int TPS, int NV, int NW>
-__device__ __forceinline__ void triangle_site(const BaryonSpin<R> &b, const S *A, const S *B, const S *np, int sub,
-                                              int c1sel, cx<R> *vals)
+// Triangle form over N' (16 blocks), one (i, l) pair per thread.
+template <class R, class S>
+__device__ __forceinline__ cx<R> triangle_site(const BaryonSpin<R> &b, const S *A, const S *B, const S *np, int sub)
+{
+  const int i = sub >> 2, l = sub & 3, j = b.perm1[i];
+  cx<R> d[9];
+#pragma unroll
+  for (int k = 0; k < 9; ++k) d[k] = czero<R>();
+  // Not unrolled: keeps one B block and one N' block live (register pressure).
+#pragma unroll 1
+  for (int m = 0; m < 4; ++m) {
+    cx<R> bm[9], nn[9];
+    load9(bm, B + (j * 4 + m) * 9);
+    load9(nn, np + (m * 4 + l) * 9);
+    wedge_acc(d, bm, nn);
+  }
+  cx<R> a[9];
+  load9(a, A + (i * 4 + b.perm2[l]) * 9);
+  return mul_phase(dot9(a, d), (b.ph1[0][i] + b.ph2[0][l]) & 3u);
+}
+
+// Triangle form with W one gamma matrix times a number (always so for
+// baryon_two_point): N'[m][l] = coef i^ph[m] N[perm m][l], no N' buffer.
+// LPT columns l per thread.
+template <class R, class S, int TPS>
+__device__ __forceinline__ cx<R> triangle_gamma_site(const BaryonSpin<R> &b, const S *A, const S *B, const S *N, int sub)
 {
   using Ln = Lanes<TPS>;
+  const CliffordSet<R> &cl = b.cl;
   const int i = sub / Ln::TPI, l0 = (sub % Ln::TPI) * Ln::LPT;
   const int j = b.perm1[i];
-  cx<R> acc[NV][NW];
-#pragma unroll
-  for (int v = 0; v < NV; ++v)
-#pragma unroll
-    for (int w = 0; w < NW; ++w) acc[v][w] = czero<R>();
-
-  constexpr bool kCacheB = Ln::LPT > 1;
-  cx<R> brow[kCacheB ? 4 : 1][9];
-  if constexpr (kCacheB) {
-#pragma unroll
-    for (int m = 0; m < 4; ++m) load9(brow[m], B + (j * 4 + m) * 9);
-  }
+  const bool phased = cl.has_phase[0];
+  cx<R> acc = czero<R>();
 #pragma unroll
   for (int lo = 0; lo < Ln::LPT; ++lo) {
     const int l = l0 + lo;
-    if constexpr (NW >= 2) {
-      // a . (B_m ^ N'_w) = N'_w . (a ^ B_m): one wedge per m shared by the projectors.
-      cx<R> a[9];
-      load9(a, A + (i * 4 + b.perm2[l]) * 9);
-      cx<R> sw[NW];
+    cx<R> d[9];
 #pragma unroll
-      for (int w = 0; w < NW; ++w) sw[w] = czero<R>();
+    for (int e = 0; e < 9; ++e) d[e] = czero<R>();
 #pragma unroll 1
-      for (int m = 0; m < 4; ++m) {
-        cx<R> e[9];
-        {
-          cx<R> bm[9];
-          if constexpr (kCacheB) {
-#pragma unroll
-            for (int k = 0; k < 9; ++k) bm[k] = brow[m][k];
-          } else {
-            load9(bm, B + (j * 4 + m) * 9);
-          }
-#pragma unroll
-          for (int k = 0; k < 9; ++k) e[k] = czero<R>();
-          wedge_acc(e, a, bm);
-        }
-#pragma unroll
-        for (int w = 0; w < NW; ++w) {
-          cx<R> nn[9];
-          load9(nn, np + (size_t)w * 144 + (m * 4 + l) * 9);
-          const cx<R> t = dot9(nn, e);
-          sw[w] = cadd(sw[w], t);
-        }
-      }
-#pragma unroll
-      for (int w = 0; w < NW; ++w)
-#pragma unroll
-        for (int v = 0; v < NV; ++v) acc[v][w] = cadd(acc[v][w], mul_phase(sw[w], b.ph2[v][l]));
-    } else {
-      cx<R> d[NW][9];
-#pragma unroll
-      for (int w = 0; w < NW; ++w)
-#pragma unroll
-        for (int k = 0; k < 9; ++k) d[w][k] = czero<R>();
-      // Not unrolled: keeps one B block and one N' block live (register pressure).
-#pragma unroll 1
-      for (int m = 0; m < 4; ++m) {
-        cx<R> bm[9];
-        if constexpr (kCacheB) {
-#pragma unroll
-          for (int k = 0; k < 9; ++k) bm[k] = brow[m][k];
-        } else {
-          load9(bm, B + (j * 4 + m) * 9);
-        }
-#pragma unroll
-        for (int w = 0; w < NW; ++w) {
-          cx<R> nn[9];
-          load9(nn, np + (size_t)w * 144 + (m * 4 + l) * 9);
-          wedge_acc(d[w], bm, nn);
-        }
-      }
-      cx<R> a[9];
-      load9(a, A + (i * 4 + b.perm2[l]) * 9);
-#pragma unroll
-      for (int w = 0; w < NW; ++w) {
-        const cx<R> s = dot9(a, d[w]);
-#pragma unroll
-        for (int v = 0; v < NV; ++v) acc[v][w] = cadd(acc[v][w], mul_phase(s, b.ph2[v][l]));
-      }
+    for (int m = 0; m < 4; ++m) {
+      cx<R> bm[9], nn[9];
+      load9(bm, B + (j * 4 + m) * 9);
+      load9(nn, N + (cl.perm[0][m] * 4 + l) * 9);
+      if (phased) phase9(nn, cl.ph[0][m]);
+      wedge_acc(d, bm, nn);
     }
+    cx<R> a[9];
+    load9(a, A + (i * 4 + b.perm2[l]) * 9);
+    acc = cadd(acc, mul_phase(dot9(a, d), b.ph2[0][l]));
   }
-  const uint32_t p1 = b.ph1[c1sel][i];
-#pragma unroll
-  for (int v = 0; v < NV; ++v)
-#pragma unroll
-    for (int w = 0; w < NW; ++w) vals[v * NW + w] = mul_phase(acc[v][w], p1);
+  return cmul(cx<R> {cl.coef[0][0][0], cl.coef[0][0][1]}, mul_phase(acc, b.ph1[0][i]));
 }
 
 // Triangle form with a projector of rank r <= 2 (RankForm).  By bilinearity
-// of the wedge,
-//   sum_m B[j][m] ^ N'[m][l] = sum_r X_r[j] ^ Y_r[l],
+// of the wedge, sum_m B[j][m] ^ N'[m][l] = sum_r X_r[j] ^ Y_r[l] with
 //   X_r[j] = sum_m x_r[m] B[j][m],  Y_r[l] = sum_n y_r[n] N[n][l],
-// so each (i, l) pair takes r wedges and one dot where the N' form takes four
-// wedges.  build_rank writes X_r[j] (from B) at block r*4 + j of xy, Y_r[l] at
-// block 8 + r*4 + l and, when B2 is given, X_r[j] from B2 at block 16 + r*4 + j.
-// Whether the factored form runs on unit-modulus phases: complex128 only, where
-// the FP64 pipe bounds the kernels (9.81 -> 9.32 ms for (1 + g4)/2 at
-// 24^3 x 64); the complex64 build, on packed FP32 FMAs, measured 2-4 % slower so.
+// and by the symmetry of the triple product
+//   C = sum_{r,l} c2(l) Y_r[l] . sum_i c1(i) A[i][perm2 l] ^ X_r[perm1 i]:
+// 4 r x 4 wedges and 4 r dots a site (1224 complex FMA for r = 2), where the N'
+// form takes 64 wedges and 16 dots.
+//
+// Whether the factors are applied as unit-modulus phases: complex128 only (an
+// FP64 add each instead of four FMA); the complex64 build, on packed FP32 FMAs,
+// measured 2-4 % slower so.
 template <class R> __device__ __forceinline__ bool rank_unit_form(const RankForm<R> &rk)
 {
   return sizeof(R) == 8 && rk.unit;
 }
 
-template <class R, class S, int TPS>
-__device__ __forceinline__ void build_rank(const RankForm<R> &rk, const S *B, const S *N, const S *B2, S *xy,
-                                           int sub)
+// One combined block: side 0, X_r from a row of B (blocks 9 apart); side 1, Y_r
+// from a column of P_n (blocks 36 apart).
+template <class R, class S>
+__device__ __forceinline__ void rank_block(const RankForm<R> &rk, bool unit, int side, int r, const S *base, int stride,
+                                           cx<R> (&o)[9])
 {
-  const int nb = 4 * rk.r, sides = B2 ? 3 : 2;
-  for (int e = sub; e < sides * nb; e += TPS) {
-    const int side = e / nb, rem = e - side * nb, rr = rem / 4, q = rem % 4;
-    const int ycol = side == 1;  // Y: N[n][q] at block n*4 + q; X: B[q][m] at block q*4 + m
-    const S *base = ycol ? N + q * 9 : (side ? B2 : B) + q * 36;
-    const int stride = ycol ? 36 : 9;
-    cx<R> o[9];
-#pragma unroll
-    for (int k = 0; k < 9; ++k) o[k] = czero<R>();
-    const bool unit = rank_unit_form(rk);
-    if (unit) {
+  if (unit) {
+    load9(o, base + rk.idx[side][r][0] * stride);
+    phase9(o, rk.ph[side][r][0]);
 #pragma unroll 1
-      for (int k = 0; k < rk.nnz; ++k) {
-        const S *src = base + rk.idx[ycol][rr][k] * stride;
-        const uint32_t ph = rk.ph[ycol][rr][k];
+    for (int k = 1; k < rk.nnz; ++k) {
+      const S *src = base + rk.idx[side][r][k] * stride;
+      const uint32_t ph = rk.ph[side][r][k];
 #pragma unroll
-        for (int t = 0; t < 9; ++t) o[t] = cadd(o[t], mul_phase(ld<R>(src + t), ph));
-      }
+      for (int t = 0; t < 9; ++t) o[t] = cadd(o[t], mul_phase(ld<R>(src + t), ph));
     }
+    return;
+  }
+#pragma unroll
+  for (int k = 0; k < 9; ++k) o[k] = czero<R>();
 #pragma unroll 1
-    for (int k = 0; k < (unit ? 0 : rk.nnz); ++k) {
-      const S *src = base + rk.idx[ycol][rr][k] * stride;
-      const cx<R> c {rk.c[ycol][rr][k][0], rk.c[ycol][rr][k][1]};
+  for (int k = 0; k < rk.nnz; ++k) {
+    const S *src = base + rk.idx[side][r][k] * stride;
+    const cx<R> c {rk.c[side][r][k][0], rk.c[side][r][k][1]};
 #pragma unroll
-      for (int t = 0; t < 9; ++t) cfma(o[t], c, ld<R>(src + t));
-    }
-    S *dst = xy + ((side * 2 + rr) * 4 + q) * 9;
-#pragma unroll
-    for (int k = 0; k < 9; ++k) st(dst + k, o[k]);
+    for (int t = 0; t < 9; ++t) cfma(o[t], c, ld<R>(src + t));
   }
 }
 
@@ -422,142 +333,58 @@ template <class R, class S, int TPS>
 __device__ __forceinline__ void build_rank_y(const RankForm<R> &rk, const S *N, S *y, int sub)
 {
   for (int e = sub; e < 4 * rk.r; e += TPS) {
-    const int rr = e / 4, q = e % 4;
     cx<R> o[9];
-#pragma unroll
-    for (int k = 0; k < 9; ++k) o[k] = czero<R>();
-#pragma unroll 1
-    for (int k = 0; k < rk.nnz; ++k) {
-      const S *src = N + (rk.idx[1][rr][k] * 4 + q) * 9;
-      const cx<R> c {rk.c[1][rr][k][0], rk.c[1][rr][k][1]};
-#pragma unroll
-      for (int t = 0; t < 9; ++t) cfma(o[t], c, ld<R>(src + t));
-    }
+    rank_block(rk, false, 1, e / 4, N + (e % 4) * 9, 36, o);
 #pragma unroll
     for (int k = 0; k < 9; ++k) st(y + e * 9 + k, o[k]);
   }
 }
 
-// Triangle values for the NV c2 variants from X_r (block r*4 + j of X) and
-// Y_r (block r*4 + l of Y); c1 from ph1[c1sel].
-template <class R, class S, int TPS, int NV>
-__device__ __forceinline__ void triangle_rank_site(const BaryonSpin<R> &b, const S *A, const S *X, const S *Y, int sub,
-                                                   int c1sel, cx<R> *vals)
+// Gamma classes: the permutation of every Gamma(n) is r -> r ^ s for its class s,
+// and within a class the (g5 Gamma(a))^T row phases factor as
+//   ph(a, r) = beta_s(r) + alpha_a + 2 popcount(h_a & r)  (mod 4)
+// with h_a running over 0..3 (Walsh functions): a sum over spin rows for the four
+// members of a class is one phase per row and a four-point Walsh-Hadamard
+// transform.
+struct ClassWalsh {
+  uint32_t beta;     // 2 bits per (s, r), index 4 s + r
+  uint64_t member;   // 4 bits per (s, h), index 4 s + h
+  uint32_t alpha;    // 2 bits per (s, h)
+  bool ok;
+};
+CGB_HD constexpr ClassWalsh class_walsh()
 {
-  using Ln = Lanes<TPS>;
-  const int i = sub / Ln::TPI, l0 = (sub % Ln::TPI) * Ln::LPT;
-  const int j = b.perm1[i];
-  cx<R> acc[NV];
-#pragma unroll
-  for (int v = 0; v < NV; ++v) acc[v] = czero<R>();
-#pragma unroll
-  for (int lo = 0; lo < Ln::LPT; ++lo) {
-    const int l = l0 + lo;
-    cx<R> d[9];
-#pragma unroll
-    for (int k = 0; k < 9; ++k) d[k] = czero<R>();
-#pragma unroll 1
-    for (int rr = 0; rr < b.rk.r; ++rr) {
-      cx<R> x[9], y[9];
-      load9(x, X + (rr * 4 + j) * 9);
-      load9(y, Y + (rr * 4 + l) * 9);
-      wedge_acc(d, x, y);
-    }
-    cx<R> a[9];
-    load9(a, A + (i * 4 + b.perm2[l]) * 9);
-    const cx<R> t = dot9(a, d);
-#pragma unroll
-    for (int v = 0; v < NV; ++v) acc[v] = cadd(acc[v], mul_phase(t, b.ph2[v][l]));
-  }
-  const R sc = rank_unit_form(b.rk) ? b.rk.scale : R(1);
-#pragma unroll
-  for (int v = 0; v < NV; ++v) {
-    const cx<R> z = mul_phase(acc[v], b.ph1[c1sel][i]);
-    vals[v] = cx<R> {z.x * sc, z.y * sc};
-  }
-}
-
-// Triangle form with the projectors in the gamma basis (CliffordSet):
-//   D_k = sum_m B[perm1 i][m] ^ (i^ph[k][m] N[perm[k][m]][l]),  s_k = A[i][perm2 l] . D_k
-//   vals[v*NW + w] = c1(i) sum_l c2_v(l) sum_k coef[w][k] s_k
-// With two or more basis terms the wedge a ^ B[perm1 i][m] is formed once
-// per m and dotted with each term's N block; with one term the basis term
-// runs outermost so that one D accumulator is live.
-template <class R, class S, int TPS, int NV, int NW>
-__device__ __forceinline__ void triangle_cliff_site(const BaryonSpin<R> &b, const S *A, const S *B, const S *N, int sub,
-                                                    int c1sel, cx<R> *vals)
-{
-  using Ln = Lanes<TPS>;
-  const CliffordSet<R> &cl = b.cl;
-  const int i = sub / Ln::TPI, l0 = (sub % Ln::TPI) * Ln::LPT;
-  const int j = b.perm1[i];
-  cx<R> acc[NV][NW];
-#pragma unroll
-  for (int v = 0; v < NV; ++v)
-#pragma unroll
-    for (int w = 0; w < NW; ++w) acc[v][w] = czero<R>();
-#pragma unroll
-  for (int lo = 0; lo < Ln::LPT; ++lo) {
-    const int l = l0 + lo;
-    cx<R> a[9];
-    load9(a, A + (i * 4 + b.perm2[l]) * 9);
-    cx<R> u[NW];  // sum_k coef[w][k] s_k for this l
-#pragma unroll
-    for (int w = 0; w < NW; ++w) u[w] = czero<R>();
-    if (cl.ng >= 2) {
-      // The triple product a . (b ^ n) is symmetric in a, b, n, so
-      // s_k = sum_m n_km . E_m with E_m = a ^ B[perm1 i][m] shared by every
-      // basis term: 4 wedges + 4 ng dots instead of 4 ng wedges + ng dots.
-#pragma unroll 1
-      for (int m = 0; m < 4; ++m) {
-        cx<R> e[9];
-        {
-          cx<R> bm[9];
-          load9(bm, B + (j * 4 + m) * 9);
-#pragma unroll
-          for (int q = 0; q < 9; ++q) e[q] = czero<R>();
-          wedge_acc(e, a, bm);
-        }
-#pragma unroll 1
-        for (int k = 0; k < cl.ng; ++k) {
-          cx<R> nn[9];
-          load9(nn, N + (cl.perm[k][m] * 4 + l) * 9);
-          const cx<R> s = mul_phase(dot9(nn, e), cl.ph[k][m]);
-#pragma unroll
-          for (int w = 0; w < NW; ++w) cfma(u[w], cx<R> {cl.coef[w][k][0], cl.coef[w][k][1]}, s);
-        }
+  constexpr GammaTables G = build_gamma_tables();
+  ClassWalsh w {0u, 0ull, 0u, true};
+  for (int s = 0; s < 4; ++s) {
+    int base = -1, seen = 0;
+    for (int a = 0; a < 16; ++a) {
+      if (G.perm[a][0] != s) continue;
+      for (int r = 0; r < 4; ++r)
+        if (G.perm[a][r] != (r ^ s)) w.ok = false;
+      if (base < 0) {
+        base = a;
+        for (int r = 0; r < 4; ++r) w.beta |= (uint32_t)G.ph_g5g_t[a][r] << (2 * (4 * s + r));
       }
-    } else {
-#pragma unroll 1
-      for (int k = 0; k < cl.ng; ++k) {
-        cx<R> d[9];
-#pragma unroll
-        for (int e = 0; e < 9; ++e) d[e] = czero<R>();
-        const bool phased = cl.has_phase[k];
-#pragma unroll 1
-        for (int m = 0; m < 4; ++m) {
-          cx<R> bm[9], nn[9];
-          load9(bm, B + (j * 4 + m) * 9);
-          load9(nn, N + (cl.perm[k][m] * 4 + l) * 9);
-          if (phased) phase9(nn, cl.ph[k][m]);
-          wedge_acc(d, bm, nn);
-        }
-        const cx<R> s = dot9(a, d);
-#pragma unroll
-        for (int w = 0; w < NW; ++w) cfma(u[w], cx<R> {cl.coef[w][k][0], cl.coef[w][k][1]}, s);
+      int d[4] = {0, 0, 0, 0};
+      for (int r = 0; r < 4; ++r) d[r] = (G.ph_g5g_t[a][r] - G.ph_g5g_t[base][r] + 4) & 3;
+      const int alpha = d[0];
+      const int h0 = ((d[1] - alpha + 4) & 3) >> 1, h1 = ((d[2] - alpha + 4) & 3) >> 1;
+      for (int r = 0; r < 4; ++r) {
+        const int pc = ((r & 1) & h0) + (((r >> 1) & 1) & h1);
+        if (d[r] != ((alpha + 2 * pc) & 3)) w.ok = false;
       }
+      const int h = h0 | (h1 << 1);
+      if (seen & (1 << h)) w.ok = false;
+      seen |= 1 << h;
+      w.member |= (uint64_t)a << (4 * (4 * s + h));
+      w.alpha |= (uint32_t)alpha << (2 * (4 * s + h));
     }
-#pragma unroll
-    for (int w = 0; w < NW; ++w)
-#pragma unroll
-      for (int v = 0; v < NV; ++v) acc[v][w] = cadd(acc[v][w], mul_phase(u[w], b.ph2[v][l]));
+    if (seen != 15) w.ok = false;
   }
-  const uint32_t p1 = b.ph1[c1sel][i];
-#pragma unroll
-  for (int v = 0; v < NV; ++v)
-#pragma unroll
-    for (int w = 0; w < NW; ++w) vals[v * NW + w] = mul_phase(acc[v][w], p1);
+  return w;
 }
+static_assert(class_walsh().ok, "gamma classes must have the Walsh phase structure");
 
 // ------------------------------------------------------------------ ops --
 // Common compile-time configuration of an op: CW consumer warps (plus one
@@ -579,86 +406,6 @@ template <class R_, class S_, int CW_, int TPS_, int NST_> struct OpBase {
 
 // Bytes of n complex values of storage type S, rounded up to 16.
 template <class S> constexpr int cbytes(int n) { return (int)((n * sizeof(S) + 15) / 16 * 16); }
-
-// One baryon contraction type per launch, loop form (IK_JL_NM, IL_JK_NM).
-template <class R, class S, int CW, int TPS, int NST>
-struct BaryonLoopOp : OpBase<R, S, CW, TPS, NST> {
-  static constexpr int NIN = 3, NOUT = 1, EXTRA_BYTES = cbytes<S>(9);
-  static constexpr bool FIELD = false;
-  __device__ static void site(const OpParams<R> &p, const S *const *in, S *scratch, int sub, cx<R> *vals)
-  {
-    build_q<R, S, TPS, 1>(p.b, in[2], scratch, sub);
-    __syncwarp();
-    loop_site<R, S, TPS, 1, 1>(p.b, in[0], in[1], scratch, sub, 0, vals);
-  }
-};
-
-// One baryon contraction type per launch, triangle form (the other four
-// types), with N' = W N materialised per site (any 4x4 projector).
-template <class R, class S, int CW, int TPS, int NST>
-struct BaryonTriOp : OpBase<R, S, CW, TPS, NST> {
-  static constexpr int NIN = 3, NOUT = 1, EXTRA_BYTES = cbytes<S>(144) + 16;  // +16: bank stagger
-  static constexpr bool FIELD = false;
-  __device__ static void site(const OpParams<R> &p, const S *const *in, S *scratch, int sub, cx<R> *vals)
-  {
-    build_nprime<R, S, TPS, 1>(p.b, in[2], scratch, sub, p.b.cl.ng <= kNprimeCliffTerms);
-    __syncwarp();
-    triangle_site<R, S, TPS, 1, 1>(p.b, in[0], in[1], scratch, sub, 0, vals);
-  }
-};
-
-// Triangle form, one type per launch, with W of rank <= 2 (e.g. (1 +- g4)/2,
-// rank 2; a polarised projector, rank 1): X_r and Y_r blocks in scratch.
-template <class R, class S, int CW, int TPS, int NST>
-struct BaryonTriRankOp : OpBase<R, S, CW, TPS, NST> {
-  static constexpr int NIN = 3, NOUT = 1, EXTRA_BYTES = cbytes<S>(144) + 16;  // +16: bank stagger
-  static constexpr bool FIELD = false;
-  __device__ static void site(const OpParams<R> &p, const S *const *in, S *scratch, int sub, cx<R> *vals)
-  {
-    build_rank<R, S, TPS>(p.b.rk, in[1], in[2], nullptr, scratch, sub);
-    __syncwarp();
-    triangle_rank_site<R, S, TPS, 1>(p.b, in[0], scratch, scratch + 72, sub, 0, vals);
-  }
-};
-
-// Triangle form, one type per launch, with W a combination of few gamma
-// matrices (always one for baryon_two_point): no N' buffer.
-template <class R, class S, int CW, int TPS, int NST>
-struct BaryonTriCliffOp : OpBase<R, S, CW, TPS, NST> {
-  static constexpr int NIN = 3, NOUT = 1, EXTRA_BYTES = 0;
-  static constexpr bool FIELD = false;
-  __device__ static void site(const OpParams<R> &p, const S *const *in, S *, int sub, cx<R> *vals)
-  {
-    triangle_cliff_site<R, S, TPS, 1, 1>(p.b, in[0], in[1], in[2], sub, 0, vals);
-  }
-};
-
-// Meson two-point: C = sum_{i,l} c1(i) c2(l) sum_ad A[i][perm2 l][ad] conj(B[perm1 i][l][ad])
-// with c from (g5 Gamma)^T (include/meson.cuh:33-50).
-template <class R, class S, int CW, int TPS, int NST>
-struct MesonOp : OpBase<R, S, CW, TPS, NST> {
-  static constexpr int NIN = 2, NOUT = 1, EXTRA_BYTES = 0;
-  static constexpr bool FIELD = false;
-  __device__ static void site(const OpParams<R> &p, const S *const *in, S *, int sub, cx<R> *vals)
-  {
-    using Ln = Lanes<TPS>;
-    const MesonSpin<R> &m = p.m;
-    const int i = sub / Ln::TPI, l0 = (sub % Ln::TPI) * Ln::LPT;
-    const int j = m.perm1[i];
-    cx<R> acc = czero<R>();
-#pragma unroll
-    for (int lo = 0; lo < Ln::LPT; ++lo) {
-      const int l = l0 + lo;
-      const S *x = in[0] + (i * 4 + m.perm2[l]) * 9;
-      const S *y = in[1] + (j * 4 + l) * 9;
-      cx<R> t = czero<R>();
-#pragma unroll
-      for (int k = 0; k < 9; ++k) cfma_conj(t, ld<R>(x + k), ld<R>(y + k));
-      acc = cadd(acc, mul_phase(t, m.ph2[l]));
-    }
-    vals[0] = mul_phase(acc, m.ph1[i]);
-  }
-};
 
 // x . conj(y) over a colour block.  Complex64: packed FP32x2 FMAs on two
 // accumulators, A = sum x.re y and B = sum x.im y (y as a pair, x broadcast),
@@ -682,76 +429,6 @@ template <> __device__ __forceinline__ cx<float> conj_dot9<float>(const cx<float
   return {A.x + B.y, B.x - A.y};
 }
 
-template <class R> __device__ __forceinline__ cx<R> pick4(const cx<R> t[4], int k)
-{
-  return k == 0 ? t[0] : (k == 1 ? t[1] : (k == 2 ? t[2] : t[3]));
-}
-
-// meson_all_source_two_point: Gamma_ij fixed (perm1/ph1), all 16 Gamma_kl.
-// Thread = spin row i (TPS = 4); the 4 x 4 colour dots T[k][l] for j = perm1[i]
-// are shared by all 16 outputs (include/meson_all.cuh:53-73 recomputes them per Gamma).
-template <class R, class S, int CW, int NST>
-struct MesonAllSourceOp : OpBase<R, S, CW, 4, NST> {
-  static constexpr int NIN = 2, NOUT = 16, EXTRA_BYTES = 0;
-  static constexpr bool FIELD = false;
-  __device__ static void site(const OpParams<R> &p, const S *const *in, S *, int sub, cx<R> *vals)
-  {
-    constexpr GammaTables G = build_gamma_tables();
-    const int i = sub, j = p.m.perm1[i];
-#pragma unroll
-    for (int g = 0; g < 16; ++g) vals[g] = czero<R>();
-#pragma unroll
-    for (int l = 0; l < 4; ++l) {
-      cx<R> t[4], y[9];
-      if (l & 1) load9p<true>(y, in[1] + (j * 4 + l) * 9);  // block parity = parity of l
-      else load9p<false>(y, in[1] + (j * 4 + l) * 9);
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        cx<R> x[9];
-        if (k & 1) load9p<true>(x, in[0] + (i * 4 + k) * 9);
-        else load9p<false>(x, in[0] + (i * 4 + k) * 9);
-        t[k] = conj_dot9<R>(x, y);
-      }
-#pragma unroll
-      for (int g = 0; g < 16; ++g) vals[g] = cadd(vals[g], mul_phase(pick4(t, G.perm[g][l]), G.ph_g5g_t[g][l]));
-    }
-    const uint32_t p1 = p.m.ph1[i];
-#pragma unroll
-    for (int g = 0; g < 16; ++g) vals[g] = mul_phase(vals[g], p1);
-  }
-};
-
-// meson_all_sink_two_point: Gamma_kl fixed (perm2/ph2), all 16 Gamma_ij.
-// Thread = spin column l (TPS = 4).
-template <class R, class S, int CW, int NST>
-struct MesonAllSinkOp : OpBase<R, S, CW, 4, NST> {
-  static constexpr int NIN = 2, NOUT = 16, EXTRA_BYTES = 0;
-  static constexpr bool FIELD = false;
-  __device__ static void site(const OpParams<R> &p, const S *const *in, S *, int sub, cx<R> *vals)
-  {
-    constexpr GammaTables G = build_gamma_tables();
-    const int l = sub, k = p.m.perm2[l];
-#pragma unroll
-    for (int g = 0; g < 16; ++g) vals[g] = czero<R>();
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      cx<R> t[4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        cx<R> x[9], y[9];
-        load9(x, in[0] + (i * 4 + k) * 9);
-        load9(y, in[1] + (j * 4 + l) * 9);
-        t[j] = conj_dot9<R>(x, y);
-      }
-#pragma unroll
-      for (int g = 0; g < 16; ++g) vals[g] = cadd(vals[g], mul_phase(pick4(t, G.perm[g][i]), G.ph_g5g_t[g][i]));
-    }
-    const uint32_t p2 = p.m.ph2[l];
-#pragma unroll
-    for (int g = 0; g < 16; ++g) vals[g] = mul_phase(vals[g], p2);
-  }
-};
-
 // ----------------------------------------------------------- field ops --
 // Diquark (include/diquark.cuh:33-57):
 //   D[m][l][ad] = g5[m] g5[l] conj( c2(l) sum_i c1(i) (P_i[i][perm2 l] ^ P_j[perm1 i][m])[ad] )
@@ -759,7 +436,6 @@ struct MesonAllSinkOp : OpBase<R, S, CW, 4, NST> {
 template <class R, class S, int CW, int TPS, int NST, bool DIRECT = false>
 struct DiquarkOp : OpBase<R, S, CW, TPS, NST> {
   static constexpr int NIN = 2, EXTRA_BYTES = 0, OUT_ELEMS = 144;
-  static constexpr bool FIELD = true;
   // DIRECT: each thread stores its blocks straight to HBM (72 contiguous bytes
   // a block) instead of staging the site in shared memory for a bulk store.
   static constexpr bool DIRECT_OUT = DIRECT;
@@ -809,7 +485,6 @@ struct DiquarkOp : OpBase<R, S, CW, TPS, NST> {
 template <class R, class S, int CW, int TPS, int NST, bool LOOP, int ROLE>
 struct SequentialOp : OpBase<R, S, CW, TPS, NST> {
   static constexpr int NIN = 2, EXTRA_BYTES = cbytes<S>(144) + 16, OUT_ELEMS = 144;
-  static constexpr bool FIELD = true;
   __device__ static long long out_index(const OpParams<R> &, long long site) { return site; }
   __device__ static S *out_ptr(const OpParams<R> &, long long d, S *base) { return base + d * OUT_ELEMS; }
 
@@ -988,45 +663,6 @@ __device__ __forceinline__ void conj_products_f32x2(cx<float> (&T)[NK][NL], cons
     for (int l = 0; l < NL; ++l) T[k][l] = {acc[k][l].x, acc[k][l].y};
 }
 
-struct ClassWalsh {
-  uint32_t beta;     // 2 bits per (s, r), index 4 s + r
-  uint64_t member;   // 4 bits per (s, h), index 4 s + h
-  uint32_t alpha;    // 2 bits per (s, h)
-  bool ok;
-};
-CGB_HD constexpr ClassWalsh class_walsh()
-{
-  constexpr GammaTables G = build_gamma_tables();
-  ClassWalsh w {0u, 0ull, 0u, true};
-  for (int s = 0; s < 4; ++s) {
-    int base = -1, seen = 0;
-    for (int a = 0; a < 16; ++a) {
-      if (G.perm[a][0] != s) continue;
-      for (int r = 0; r < 4; ++r)
-        if (G.perm[a][r] != (r ^ s)) w.ok = false;
-      if (base < 0) {
-        base = a;
-        for (int r = 0; r < 4; ++r) w.beta |= (uint32_t)G.ph_g5g_t[a][r] << (2 * (4 * s + r));
-      }
-      int d[4] = {0, 0, 0, 0};
-      for (int r = 0; r < 4; ++r) d[r] = (G.ph_g5g_t[a][r] - G.ph_g5g_t[base][r] + 4) & 3;
-      const int alpha = d[0];
-      const int h0 = ((d[1] - alpha + 4) & 3) >> 1, h1 = ((d[2] - alpha + 4) & 3) >> 1;
-      for (int r = 0; r < 4; ++r) {
-        const int pc = ((r & 1) & h0) + (((r >> 1) & 1) & h1);
-        if (d[r] != ((alpha + 2 * pc) & 3)) w.ok = false;
-      }
-      const int h = h0 | (h1 << 1);
-      if (seen & (1 << h)) w.ok = false;
-      seen |= 1 << h;
-      w.member |= (uint64_t)a << (4 * (4 * s + h));
-      w.alpha |= (uint32_t)alpha << (2 * (4 * s + h));
-    }
-    if (seen != 15) w.ok = false;
-  }
-  return w;
-}
-static_assert(class_walsh().ok, "gamma classes must have the Walsh phase structure");
 
 // SPLIT selects the layout [t][pair half][site][128 pairs] (pairs 0-127 and
 // 128-255 of a timeslice in separate planes) that the tensor-core projection
@@ -1040,7 +676,6 @@ static_assert(class_walsh().ok, "gamma classes must have the Walsh phase structu
 template <class R, class S, int CW, int NST, bool SPLIT = false, bool PRODUCTS = false>
 struct MesonAllGammaOp : OpBase<R, S, CW, 16, NST> {
   static constexpr int NIN = 2, EXTRA_BYTES = 0, OUT_ELEMS = 256;
-  static constexpr bool FIELD = true;
   static_assert(!PRODUCTS || sizeof(R) == 4, "the product form is complex64 only");
   // Each thread's 16 outputs are four 32-byte runs: stored straight to HBM.
   static constexpr bool DIRECT_OUT = true;

@@ -137,19 +137,12 @@ __device__ __forceinline__ void open_diquark_fixed(const FusedSpin &f, const int
   const int s1 = f.s & 3, turn = (f.rows >> 8) & 7;
 #pragma unroll
   for (int t = 0; t < NN; ++t)
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-      FixedWedgeRow w;
-      w.clear();
-#pragma unroll 1
-      for (int k = 0; k < NROW; ++k) {
-        const int i = two_bits(f.rows, 2 * k);
-        if (k == turn) w.negate();
-        w.add(a, A + (i * 4 + s) * 9, B + ((i ^ s1) * 4 + n0 + t) * 9);
-      }
-      if (turn == NROW) w.negate();
-      w.get(a, g[t] + 3 * a, fs);
-    }
+    fixed_wedge_sum(0, NROW, fs, [&](int k, const int4 *&x, const int4 *&y) {
+      const int i = two_bits(f.rows, 2 * k);
+      x = A + (i * 4 + s) * 9;
+      y = B + ((i ^ s1) * 4 + n0 + t) * 9;
+      return k < turn;
+    }, g[t]);
 }
 
 // Converts the site's blocks of P_i and P_j in place, if every site of the warp

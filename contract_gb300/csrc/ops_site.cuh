@@ -1,0 +1,319 @@
+// Per-call ops for ring_kernel (engine_warp.cuh): one baryon contraction
+// type, one meson Gamma pair, or all 16 partners of one meson Gamma.
+//
+// Complex128 baryon wedges and the all-partner meson dots run in fixed point on the
+// integer pipe where the site's values allow it (fixed.cuh), in FP64 otherwise;
+// complex64 runs on packed FP32 FMAs.
+#pragma once
+
+#include "ops_fused.cuh"
+
+namespace cgb {
+
+template <class R_, class S_, int CW_, int TPS_, int NST_, int MINB> struct RingOp {
+  using R = R_;
+  using S = S_;
+  using Params = OpParams<R_>;
+  static constexpr int CW = CW_, TPS = TPS_, NST = NST_, MIN_CTAS = MINB;
+  static constexpr int NOUT = 1, EXTRA_BYTES = 0;
+  static constexpr bool CHANGES_INPUT = false;
+  static constexpr bool DIRECT_N = false;  // field NIN is not staged: site() reads it from memory
+};
+
+// Loop form (IK_JL_NM, IL_JK_NM).
+template <class R, class S, int CW, int TPS, int NST, int MINB>
+struct BaryonLoopOp : RingOp<R, S, CW, TPS, NST, MINB> {
+  static constexpr int NIN = 3, EXTRA_BYTES = cbytes<S>(9);
+  static constexpr bool CHANGES_INPUT = sizeof(R) == 8;
+  __device__ static cx<R> site(const OpParams<R> &p, S *const *in, S *scratch, int sub, bool live)
+  {
+    const BaryonSpin<R> &b = p.b;
+    build_q<R, S, TPS, 1>(b, in[2], scratch, sub);
+    __syncwarp();
+    if constexpr (sizeof(R) == 8) {
+      static_assert(TPS == 16, "one (i, l) pair per thread");
+      FixedScales fs;
+      if (fields_to_fixed<TPS>(in[0], in[1], sub, live, fs)) {
+        // all wedges of the site have one scale: they meet as integers, entry e of
+        // the sum with thread e, which multiplies it by Q's
+        const int i = sub >> 2, l = sub & 3;
+        const int4 *x = reinterpret_cast<const int4 *>(in[0]) + (i * 4 + b.perm2[l]) * 9;
+        const int4 *y = reinterpret_cast<const int4 *>(in[1]) + (b.perm1[i] * 4 + l) * 9;
+        // Gamma entries: one common power of i, and signs
+        const uint32_t common = (b.ph1[0][0] & 1u) + (b.ph2[0][0] & 1u);
+        const bool minus = ((b.ph1[0][i] ^ b.ph2[0][l]) & 2u) != 0;
+        long long re[9], im[9];
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+          FixedWedgeRow w;
+          w.clear();
+          w.add(a, x, y);
+#pragma unroll
+          for (int e = 0; e < 3; ++e) {
+            // 16 sums of up to 2^59: half units leave a bit to spare
+            const long long u = w.re[e].half_units(), v = w.im[e].half_units();
+            re[3 * a + e] = minus ? -u : u;
+            im[3 * a + e] = minus ? -v : v;
+          }
+        }
+        const longlong2 d = group_sum_scatter9(re, im, sub);
+        cx<double> v = czero<double>();
+        if (sub < 9) {
+          const cx<double> z = fixed_entry(d, sub, fs);
+          cfma(v, z, ld<double>(scratch + sub));
+        }
+        return mul_phase(v, common);
+      }
+    }
+    return loop_site<R, S, TPS>(b, in[0], in[1], scratch, sub);
+  }
+};
+
+// Triangle form (the other four types), N' = W N materialised (any projector).
+template <class R, class S, int CW, int NST, int MINB>
+struct BaryonTriOp : RingOp<R, S, CW, 16, NST, MINB> {
+  static constexpr int NIN = 3, EXTRA_BYTES = cbytes<S>(144) + 16;  // +16: bank stagger
+  static constexpr bool CHANGES_INPUT = sizeof(R) == 8;
+  __device__ static cx<R> site(const OpParams<R> &p, S *const *in, S *scratch, int sub, bool live)
+  {
+    const BaryonSpin<R> &b = p.b;
+    build_nprime<R, S, 16, 1>(b, in[2], scratch, sub, b.cl.ng <= kNprimeCliffTerms);
+    __syncwarp();
+    if constexpr (sizeof(R) == 8) {
+      FixedScales fs;
+      if (fields_to_fixed<16>(in[1], scratch, sub, live, fs)) {
+        const int4 *B = reinterpret_cast<const int4 *>(in[1]), *np = reinterpret_cast<const int4 *>(scratch);
+        const int i = sub >> 2, l = sub & 3, j = b.perm1[i];
+        cx<double> d[9], a[9];
+        fixed_wedge_sum(0, 4, fs, [&](int m, const int4 *&x, const int4 *&y) {
+          x = B + (j * 4 + m) * 9;
+          y = np + (m * 4 + l) * 9;
+          return false;
+        }, d);
+        load9(a, in[0] + (i * 4 + b.perm2[l]) * 9);
+        return mul_phase(dot9(a, d), (b.ph1[0][i] + b.ph2[0][l]) & 3u);
+      }
+    }
+    return triangle_site<R, S>(b, in[0], in[1], scratch, sub);
+  }
+};
+
+// Triangle form, W a multiple of one gamma matrix.
+template <class R, class S, int CW, int TPS, int NST, int MINB>
+struct BaryonTriGammaOp : RingOp<R, S, CW, TPS, NST, MINB> {
+  static constexpr int NIN = 3;
+  static constexpr bool CHANGES_INPUT = sizeof(R) == 8;
+  __device__ static cx<R> site(const OpParams<R> &p, S *const *in, S *, int sub, bool live)
+  {
+    const BaryonSpin<R> &b = p.b;
+    if constexpr (sizeof(R) == 8) {
+      static_assert(TPS == 16, "one (i, l) pair per thread");
+      const CliffordSet<R> &cl = b.cl;
+      FixedScales fs;
+      if (fields_to_fixed<TPS>(in[1], in[2], sub, live, fs)) {
+        const int4 *B = reinterpret_cast<const int4 *>(in[1]), *N = reinterpret_cast<const int4 *>(in[2]);
+        const int i = sub >> 2, l = sub & 3, j = b.perm1[i];
+        cx<double> d[9], a[9];
+        // the gamma matrix's entries differ by signs
+        fixed_wedge_sum(0, 4, fs, [&](int m, const int4 *&x, const int4 *&y) {
+          x = B + (j * 4 + m) * 9;
+          y = N + (cl.perm[0][m] * 4 + l) * 9;
+          return ((cl.ph[0][m] ^ cl.ph[0][0]) & 2u) != 0;
+        }, d);
+        load9(a, in[0] + (i * 4 + b.perm2[l]) * 9);
+        const cx<R> v = mul_phase(dot9(a, d), (b.ph1[0][i] + b.ph2[0][l] + cl.ph[0][0]) & 3u);
+        return cmul(cx<R> {cl.coef[0][0][0], cl.coef[0][0][1]}, v);
+      }
+    }
+    return triangle_gamma_site<R, S, TPS>(b, in[0], in[1], in[2], sub);
+  }
+};
+
+// Triangle form, W of rank 1 or 2: eight threads a site.  Thread (r, l) with two
+// factors, thread (half of the rows, l) with one: the wedges A[i][perm2 l] ^
+// X_r[perm1 i] over its rows i, then one dot with Y_r[l].  X takes the place of
+// P_j's blocks (X_r[j] at block 4 r + j), and P_n, whose blocks make one Y_r[l] each,
+// is read from memory by the threads that use them: two fields of a site in shared
+// memory let 10 warps of 4 sites share an SM in complex128.
+template <class R, class S, int CW, int NST, int MINB>
+struct BaryonTriRankOp : RingOp<R, S, CW, 8, NST, MINB> {
+  static constexpr bool CHANGES_INPUT = true, DIRECT_N = sizeof(R) == 8;
+  static constexpr int NIN = DIRECT_N ? 2 : 3;
+  __device__ static cx<R> site(const OpParams<R> &p, S *const *in, S *scratch, int sub, bool live)
+  {
+    return site(p, in, in[2], scratch, sub, live);
+  }
+  __device__ static cx<R> site(const OpParams<R> &p, S *const *in, const S *N, S *, int sub, bool live)
+  {
+    const BaryonSpin<R> &b = p.b;
+    const RankForm<R> &rk = b.rk;
+    const FusedSpin f = b.fu;
+    const bool unit = rank_unit_form(rk), two = rk.r == 2;
+    S *X = in[1];
+    {
+      cx<R> o[9];
+      rank_block(rk, unit, 0, two ? sub >> 2 : 0, in[1] + (sub & 3) * 36, 9, o);
+      __syncwarp();  // P_j has been read
+      if (two || sub < 4) {
+#pragma unroll
+        for (int k = 0; k < 9; ++k) st(X + sub * 9 + k, o[k]);
+      }
+    }
+    __syncwarp();
+    const int l = sub & 3, r = two ? sub >> 2 : 0, k0 = two ? 0 : (sub >> 2) * 2, k1 = two ? 4 : k0 + 2;
+    const int s = l ^ ((f.s >> 2) & 3), s1 = f.s & 3, turn = (f.rows >> 8) & 7;
+    cx<R> d[9];
+    bool done = false;
+    if constexpr (sizeof(R) == 8) {
+      FixedScales fs;
+      S *own = X + (two ? sub : sub & 3) * 9;
+      const double2 *blk[3] = {in[0] + sub * 9, in[0] + (sub + 8) * 9, own};
+      const bool ok = fixed_scales<8, 2>(blk, fs);
+      done = __all_sync(0xffffffffu, ok || !live);
+      if (done) {
+        block_to_fixed(reinterpret_cast<int4 *>(in[0] + sub * 9), blk[0], fs, 0);
+        block_to_fixed(reinterpret_cast<int4 *>(in[0] + (sub + 8) * 9), blk[1], fs, 0);
+        if (two || sub < 4) block_to_fixed(reinterpret_cast<int4 *>(own), own, fs, 1);
+        __syncwarp();
+        const int4 *A = reinterpret_cast<const int4 *>(in[0]), *Xf = reinterpret_cast<const int4 *>(X);
+        fixed_wedge_sum(k0, k1, fs, [&](int k, const int4 *&x, const int4 *&y) {
+          const int i = two_bits(f.rows, 2 * k);
+          x = A + (i * 4 + s) * 9;
+          y = Xf + (r * 4 + (i ^ s1)) * 9;
+          return k < turn;
+        }, d);
+      }
+    }
+    if (!done) {
+#pragma unroll
+      for (int k = 0; k < 9; ++k) d[k] = czero<R>();
+      bool minus = false;
+#pragma unroll 1
+      for (int k = k0; k < k1; ++k) {
+        if ((k < turn) != minus) {
+          minus = !minus;
+#pragma unroll
+          for (int e = 0; e < 9; ++e) d[e] = {-d[e].x, -d[e].y};
+        }
+        const int i = two_bits(f.rows, 2 * k);
+        cx<R> x[9], y[9];
+        load9(x, in[0] + (i * 4 + s) * 9);
+        load9(y, X + (r * 4 + (i ^ s1)) * 9);
+        wedge_acc(d, x, y);
+      }
+      if (minus) {
+#pragma unroll
+        for (int e = 0; e < 9; ++e) d[e] = {-d[e].x, -d[e].y};
+      }
+    }
+    cx<R> y[9];
+    rank_block(rk, unit, 1, r, N + l * 9, 36, y);
+    const cx<R> v = mul_phase(signed_by(dot9(d, y), f.neg, l), f.out & 3u);
+    const R sc = unit ? rk.scale : R(1);
+    return {v.x * sc, v.y * sc};
+  }
+};
+
+// Meson two-point: C = sum_{i,l} c1(i) c2(l) sum_ad A[i][perm2 l][ad] conj(B[perm1 i][l][ad])
+// with c from (g5 Gamma)^T (include/meson.cuh:33-50).
+template <class R, class S, int CW, int TPS, int NST, int MINB>
+struct MesonOp : RingOp<R, S, CW, TPS, NST, MINB> {
+  static constexpr int NIN = 2;
+  __device__ static cx<R> site(const OpParams<R> &p, S *const *in, S *, int sub, bool)
+  {
+    using Ln = Lanes<TPS>;
+    const MesonSpin<R> &m = p.m;
+    const int i = sub / Ln::TPI, l0 = (sub % Ln::TPI) * Ln::LPT;
+    const int j = m.perm1[i];
+    cx<R> acc = czero<R>();
+#pragma unroll
+    for (int lo = 0; lo < Ln::LPT; ++lo) {
+      const int l = l0 + lo;
+      const S *x = in[0] + (i * 4 + m.perm2[l]) * 9;
+      const S *y = in[1] + (j * 4 + l) * 9;
+      cx<R> t = czero<R>();
+#pragma unroll
+      for (int k = 0; k < 9; ++k) cfma_conj(t, ld<R>(x + k), ld<R>(y + k));
+      acc = cadd(acc, mul_phase(t, m.ph2[l]));
+    }
+    return mul_phase(acc, m.ph1[i]);
+  }
+};
+
+// meson_all_{source,sink}_two_point: one Gamma fixed, all 16 of the other slot.
+//   source (Gamma_ij fixed): Z[k][l] = sum_i c1(i) A[i][k] . conj(B[perm1 i][l])
+//   sink (Gamma_kl fixed):   Z[i][j] = sum_l c2(l) A[i][perm2 l] . conj(B[j][l])
+//   out_g = sum_r c_g(r) Z[r ^ s][r] (source) or Z[r][r ^ s] (sink), s the class of Gamma_g
+// Thread (a, b) of a site's 16 forms the four dots over the row r for the summed
+// index a and b = k (or j); two halving steps over a leave Z's entry of row r = a
+// and other index b with it, and the four threads of one class s = a ^ b meet in a
+// Walsh-Hadamard transform of two steps, after which each holds one output: 10 FP
+// adds a thread where summing all 16 outputs took 96.
+template <class R, class S, int CW, int NST, int MINB, bool SOURCE>
+struct MesonAllOp : RingOp<R, S, CW, 16, NST, MINB> {
+  static constexpr int NIN = 2, NOUT = 16;
+  static constexpr bool CHANGES_INPUT = sizeof(R) == 8;
+  __device__ static int output(const OpParams<R> &, int sub)
+  {
+    constexpr ClassWalsh W = class_walsh();
+    const int a = sub >> 2, s = a ^ (sub & 3);
+    return (int)((W.member >> (4 * (4 * s + a))) & 15u);
+  }
+  __device__ static cx<R> site(const OpParams<R> &p, S *const *in, S *, int sub, bool live)
+  {
+    constexpr ClassWalsh W = class_walsh();
+    const int a = sub >> 2, b = sub & 3, s = a ^ b;
+    // the fixed block and the four of the other field, `step` blocks apart
+    const int own = SOURCE ? a * 4 + b : b * 4 + a;
+    const int first = SOURCE ? p.m.perm1[a] * 4 : p.m.perm2[a], step = SOURCE ? 1 : 4;
+    cx<R> T[4];
+    bool done = false;
+    if constexpr (sizeof(R) == 8) {
+      FixedScales fs;
+      const double2 *blk[2] = {in[0] + sub * 9, in[1] + sub * 9};
+      const bool ok = fixed_scales<16, 1, false>(blk, fs);
+      done = __all_sync(0xffffffffu, ok || !live);
+      if (done) {
+        block_to_fixed(reinterpret_cast<int4 *>(in[0] + sub * 9), blk[0], fs, 0);
+        block_to_fixed(reinterpret_cast<int4 *>(in[1] + sub * 9), blk[1], fs, 1);
+        __syncwarp();
+        const int up = fs.E[0] + fs.E[1] - 2 * 1023 - 54;
+        const int4 *x = reinterpret_cast<const int4 *>(in[SOURCE ? 0 : 1]) + own * 9;
+        const int4 *y = reinterpret_cast<const int4 *>(in[SOURCE ? 1 : 0]) + first * 9;
+        int4 xv[9];
+#pragma unroll
+        for (int k = 0; k < 9; ++k) xv[k] = x[k];
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+          const cx<double> t = fixed_conj_dot(xv, y + r * step * 9, up);
+          T[r] = SOURCE ? t : conj(t);
+        }
+      }
+    }
+    if (!done) {
+      cx<R> x[9], y[9];
+      load9(x, in[SOURCE ? 0 : 1] + own * 9);
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        load9(y, in[SOURCE ? 1 : 0] + (first + r * step) * 9);
+        T[r] = SOURCE ? conj_dot9<R>(x, y) : conj_dot9<R>(y, x);
+      }
+    }
+    const uint32_t ph = SOURCE ? p.m.ph1[a] : p.m.ph2[a];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) T[r] = mul_phase(T[r], ph);
+    const bool hi = a & 2, odd = a & 1;
+    cx<R> h[2];
+#pragma unroll
+    for (int r = 0; r < 2; ++r) h[r] = cadd(hi ? T[2 + r] : T[r], shfl_xor(hi ? T[r] : T[2 + r], 8));
+    cx<R> u = cadd(odd ? h[1] : h[0], shfl_xor(odd ? h[0] : h[1], 4));  // Z of row r = a
+    u = mul_phase(u, (W.beta >> (2 * (4 * s + a))) & 3u);
+    cx<R> o = shfl_xor(u, 5);  // (a ^ 1, b ^ 1)
+    u = odd ? cx<R> {o.x - u.x, o.y - u.y} : cadd(u, o);
+    o = shfl_xor(u, 10);
+    u = hi ? cx<R> {o.x - u.x, o.y - u.y} : cadd(u, o);
+    return mul_phase(u, (W.alpha >> (2 * (4 * s + a))) & 3u);
+  }
+};
+
+} // namespace cgb

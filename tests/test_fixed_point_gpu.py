@@ -1,4 +1,5 @@
-"""The integer-pipe form of the complex128 contractions (fixed.cuh) over inputs
+"""The contractions of a call (ring_kernel) and of the all-types pass (warp_kernel),
+and the integer-pipe form that complex128 takes there (fixed.cuh), over inputs
 that it takes and inputs that it must leave to the FP64 form: Gaussian fields, a
 coherent part, colour rows and spin rows of different size, zero blocks and
 sites, colour-diagonal blocks, very large, very small and denormal values,
@@ -121,3 +122,83 @@ def test_not_finite(api, c_oracle, bad):
         assert not np.isfinite(got[:, :, 7]).all()
         keep = np.arange(V) != 7
         close(got[:, :, keep], ref[:, :, keep], "gauss")
+
+
+def per_call(api, ps, dev, form):
+    """(result, oracle) of one call of a per-site form."""
+    from contract_gb300 import pycontract as pc
+    rng = np.random.default_rng(11)
+    wd = rng.standard_normal((4, 4)) + 1j * rng.standard_normal((4, 4))
+    pp = api.projector_plus_minus()
+    if form in ("source", "sink"):
+        got = pc._meson_all(dev[0], dev[1], 6, form == "source")
+        ref = (eo.meson_all_source if form == "source" else eo.meson_all_sink)(ps[0], ps[1], 6)
+        return np.array([g.cpu().numpy() for g in got]).reshape(16, V), np.asarray(ref)
+    if form == "meson":
+        return pc.mesonTwoPoint(dev[0], dev[1], 6, 13).cpu().numpy().reshape(V), eo.meson_two_point(ps[0], ps[1], 6, 13)
+    if form == "gamma":
+        return (api.baryon(*dev, 3, 6, 13, gamma_mn=9).cpu().numpy().reshape(V),
+                eo.baryon_two_point(*ps, 3, 6, 13, 9))
+    t, w = {"loop": (0, pp[1]), "dense": (4, wd), "rank 2": (5, pp[0]), "rank 1": (1, np.outer(wd[0], wd[1]))}[form]
+    return api.baryon(*dev, t, 6, 13, project_mn=w).cpu().numpy().reshape(V), eo.baryon_general_two_point(*ps, t, 6, 13, w)
+
+
+FORMS = ["loop", "gamma", "dense", "rank 1", "rank 2", "meson", "source", "sink"]
+
+
+@pytest.mark.parametrize("form", FORMS)
+@pytest.mark.parametrize("kind", KINDS)
+def test_per_call(api, form, kind):
+    ps, dev = fields(kind)
+    got, ref = per_call(api, ps, dev, form)
+    if kind == "mixed sites":  # in units of each site's own values
+        unit = np.prod([np.abs(p).max(axis=(1, 2, 3, 4)) for p in ps[:2 if form in ("meson", "source", "sink") else 3]], axis=0)
+        got, ref, kind = got / unit, ref / unit, "gauss"
+    close(got, ref, kind)
+
+
+@pytest.mark.parametrize("form", FORMS)
+def test_per_call_not_finite(api, form):
+    ps, dev = fields("gauss")
+    ref = per_call(api, ps, dev, form)[1]
+    keep = np.arange(V) != 7
+    for field in range(2 if form in ("meson", "source", "sink") else 3):
+        for bad in (np.nan, np.inf):
+            p = ps[field].copy()
+            p[7] = bad
+            d = list(dev)
+            d[field] = __import__("torch").from_numpy(p).cuda()
+            got = per_call(api, ps, d, form)[0]
+            assert not np.isfinite(got[..., 7]).any()
+            close(got[..., keep], ref[..., keep], "gauss")
+
+
+@pytest.mark.parametrize("latt", [(2, 1, 1, 1), (2, 1, 1, 3), (6, 3, 1, 5), (10, 3, 3, 2)])
+@pytest.mark.parametrize("dtype", ["complex64", "complex128"])
+def test_per_call_edges(api, latt, dtype):
+    """Half-timeslices of 1, 9 and 45 sites: warps with one live site, a last tile
+    part full, fewer tiles than warps."""
+    import torch
+    from contract_gb300 import pycontract as pc
+    rng = np.random.default_rng(sum(latt))
+    n, tol = int(np.prod(latt)), 2e-15 if dtype == "complex128" else 2e-6
+    ps = [(rng.standard_normal((n, 4, 4, 3, 3)) + 1j * rng.standard_normal((n, 4, 4, 3, 3))).astype(dtype) for _ in range(3)]
+    dev = [torch.from_numpy(p).cuda() for p in ps]
+    # the reference in extended precision: a sum of two sites can cancel, and the
+    # oracle's own FP64 rounding is then as large as the bound
+    ps = [p.astype(np.clongdouble) for p in ps]
+    pp = api.projector_plus_minus()
+    wd = rng.standard_normal((4, 4)) + 1j * rng.standard_normal((4, 4))
+    calls = [(t, w) for t, w in ((0, pp[0]), (1, pp[1]), (4, wd), (3, np.outer(wd[0], wd[1])))]
+    pairs = [(api.baryon(*dev, t, 5, 7, project_mn=w, latt=l), eo.baryon_general_two_point(*ps, t, 5, 7, w), l)
+             for t, w in calls for l in (None, latt)]
+    pairs += [(api.baryon(*dev, 1, 5, 7, gamma_mn=8, latt=l), eo.baryon_two_point(*ps, 1, 5, 7, 8), l) for l in (None, latt)]
+    pairs += [(api.meson_timeslice(dev[0], dev[1], latt, 15, 5), eo.meson_two_point(ps[0], ps[1], 15, 5), latt)]
+    for src in (True, False):
+        ref = (eo.meson_all_source if src else eo.meson_all_sink)(ps[0], ps[1], 5)
+        pairs += [(api.meson_all_timeslice(dev[0], dev[1], latt, 5, source=src), ref, latt)]
+    for got, ref, l in pairs:
+        got, ref = got.cpu().numpy(), np.asarray(ref)
+        if l is not None:
+            ref = np.array([eo.timeslice_sum(r, latt) for r in ref.reshape(-1, n)])
+        assert norm(got.ravel() - ref.ravel()) <= tol * norm(ref), (latt, l)
