@@ -850,7 +850,7 @@ bool make_mom_plan(cgb::MomPlan &plan, const int *lattice, const int *moms, int 
     plan.p_q[p] = iq;
     plan.p_nz[p] = nz;
   }
-  // +n / -n groups of the X and Z transforms (see MomPlan).  k = min(m, L - m) for m = n mod L; the sign
+  // +n / -n groups of the X, Y and Z transforms (see MomPlan).  k = min(m, L - m) for m = n mod L; the sign
   // is + when m == k.  A momentum joins an open group of its k and sign slot,
   // else starts one (duplicates get groups of their own).
   auto key = [](int n, int L, bool &plus) {
@@ -878,6 +878,22 @@ bool make_mom_plan(cgb::MomPlan &plan, const int *lattice, const int *moms, int 
       std::swap(plan.gx_plus[0], plan.gx_plus[gi]);
       std::swap(plan.gx_minus[0], plan.gx_minus[gi]);
     }
+  plan.nyg = 0;
+  for (int q = 0; q < plan.nq; ++q) {
+    bool plus;
+    const int k = key(plan.q_ny[q], lattice[1], plus);
+    int gsel = -1;
+    for (int gi = 0; gi < plan.nyg && gsel < 0; ++gi)
+      if (plan.yg_ix[gi] == plan.q_ix[q] && plan.yg_k[gi] == k && (plus ? plan.yg_plus[gi] : plan.yg_minus[gi]) < 0)
+        gsel = gi;
+    if (gsel < 0) {
+      gsel = plan.nyg++;
+      plan.yg_ix[gsel] = plan.q_ix[q];
+      plan.yg_k[gsel] = k;
+      plan.yg_plus[gsel] = plan.yg_minus[gsel] = -1;
+    }
+    (plus ? plan.yg_plus[gsel] : plan.yg_minus[gsel]) = q;
+  }
   int ng = 0;
   for (int q = 0; q < plan.nq; ++q) {
     plan.q_g0[q] = ng;

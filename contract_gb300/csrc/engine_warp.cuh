@@ -182,6 +182,8 @@ __global__ void __launch_bounds__(32 * Op::CW, Op::MIN_CTAS) warp_kernel(const _
 // The same for ops of one step: a warp has an NST-stage ring of whole tiles, and
 // Op::site() yields the site's value -- the sum over its threads is one output
 // (NOUT == 1), or with NOUT > 1 thread sub holds output Op::output(p, sub) complete.
+// NOUT == 0: a field op, site() stores its results at `dst` itself (nullptr: nothing
+// to store).
 template <class Op> struct RingSmem {
   using L = OpLayout<Op>;
   static constexpr int SPW = 32 / Op::TPS;
@@ -250,7 +252,16 @@ __global__ void __launch_bounds__(32 * Op::CW, Op::MIN_CTAS) ring_kernel(const _
       in[q] = reinterpret_cast<S *>(mine + M::IN + stage * M::STAGE + ((size_t)q * SPW + local) * L::SLOT);
     const bool ok = local < cur.sites();
     cx<R> v;
-    if constexpr (Op::DIRECT_N) {  // the last field is read from memory by the op
+    if constexpr (NOUT == 0) {
+      S *dst = nullptr;
+      if (ok) {
+        // checked against the volume, so that a bad layout cannot store out of bounds
+        const long long d = Op::out_index(ps, cur.first() + local);
+        if (d >= 0 && d < ps.geom.volume) dst = static_cast<S *>(p.out[0]) + d * Op::OUT_ELEMS;
+        else if (sub == 0) report(p.status, kDevErrBadWork, (unsigned int)(cur.first() + local));
+      }
+      Op::site(ps, in, scratch, sub, ok, dst);
+    } else if constexpr (Op::DIRECT_N) {  // the last field is read from memory by the op
       const long long at = cur.first() + (ok ? local : 0);
       v = Op::site(ps, in, reinterpret_cast<const S *>(cur.in(p, NIN) + at * L::SITE_BYTES), scratch, sub, ok);
     } else {
@@ -264,7 +275,8 @@ __global__ void __launch_bounds__(32 * Op::CW, Op::MIN_CTAS) ring_kernel(const _
       ahead.next(p);
     }
     if constexpr (NOUT == 1) v = group_sum<TPS>(v);
-    if (ps.geom.per_site) {
+    if constexpr (NOUT == 0) {
+    } else if (ps.geom.per_site) {
       if (ok) {
         if constexpr (NOUT == 1) {
           if (sub == 0) static_cast<double2 *>(ps.out[0])[cur.first() + local] = make_double2(double(v.x), double(v.y));

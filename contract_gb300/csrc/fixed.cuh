@@ -132,6 +132,13 @@ __device__ __forceinline__ void block_to_fixed(int4 *dst, const double2 *blk, co
   }
 }
 
+// v 2^up.
+__device__ __forceinline__ double fixed_value(long long v, int up)
+{
+  const double d = __ll2double_rn(v);
+  return v == 0 ? 0.0 : __hiloint2double(__double2hiint(d) + (up << 20), __double2loint(d));
+}
+
 // Running sums of fixed-point products: high words' products, and the cross ones
 // (2^-28 of a unit of the first).
 struct FixedSum {
@@ -142,14 +149,14 @@ struct FixedSum {
     x += (long long)ah * bl;
     x += (long long)al * bh;
   }
+  // In units of 2^(scale + scale - 54).
+  __device__ __forceinline__ long long units() const { return hh + ((x + (1ll << 27)) >> 28); }
   // In units of 2^(scale + scale - 53).
   __device__ __forceinline__ long long half_units() const { return (hh + ((x + (1ll << 27)) >> 28) + 1) >> 1; }
   // In units of 2^(scale + scale - 54); `up` is that power of two.
   __device__ __forceinline__ double value(int up) const
   {
-    const long long v = hh + ((x + (1ll << 27)) >> 28);
-    const double d = __ll2double_rn(v);
-    return v == 0 ? 0.0 : __hiloint2double(__double2hiint(d) + (up << 20), __double2loint(d));
+    return fixed_value(units(), up);
   }
 };
 
@@ -273,15 +280,12 @@ __device__ __forceinline__ cx<double> fixed_entry(longlong2 v, int e, const Fixe
     if (k != c) cols += f.c[k];
   }
   const int up = f.E[0] + f.E[1] - 2 * 1023 - 53 + rows + cols;
-  const double x = __ll2double_rn(v.x), y = __ll2double_rn(v.y);
-  return {v.x ? __hiloint2double(__double2hiint(x) + (up << 20), __double2loint(x)) : 0.0,
-          v.y ? __hiloint2double(__double2hiint(y) + (up << 20), __double2loint(y)) : 0.0};
+  return {fixed_value(v.x, up), fixed_value(v.y, up)};
 }
 
-// x . conj(y) over two converted blocks of one scale each; up = 2^ of their scales - 54.
-__device__ __forceinline__ cx<double> fixed_conj_dot(const int4 (&x)[9], const int4 *y, int up)
+// re + i im += x . conj(y) over two converted blocks (held in registers or memory).
+template <class X> __device__ __forceinline__ void fixed_conj_mac(FixedSum &re, FixedSum &im, const X &x, const int4 *y)
 {
-  FixedSum re {0, 0}, im {0, 0};
 #pragma unroll
   for (int k = 0; k < 9; ++k) {
     const int4 u = x[k], v = y[k];
@@ -290,6 +294,12 @@ __device__ __forceinline__ cx<double> fixed_conj_dot(const int4 (&x)[9], const i
     im.mac(u.z, u.w, v.x, v.y);
     im.mac(-u.x, -u.y, v.z, v.w);
   }
+}
+// The same as doubles, blocks of one scale each; up = 2^ of their scales - 54.
+__device__ __forceinline__ cx<double> fixed_conj_dot(const int4 (&x)[9], const int4 *y, int up)
+{
+  FixedSum re {0, 0}, im {0, 0};
+  fixed_conj_mac(re, im, x, y);
   return {re.value(up), im.value(up)};
 }
 

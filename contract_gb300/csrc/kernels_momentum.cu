@@ -5,8 +5,8 @@
 // The phase factorises over x, y and z, so instead of one dense
 // [momenta x V3] x [V3 x 256] product per timeslice (8 M N K flop) the
 // projection runs as three short transforms:
-//   1. MesonAllGammaOp (tile engine): C_ab(x) for all 256 pairs, written in
-//      lexicographic site order (HBM-bound: two propagators in, 256 complex out)
+//   1. MesonPairsOp (complex128) or MesonAllGammaOp: C_ab(x) for all 256 pairs,
+//      written in lexicographic site order
 //   2. plane_kernel: per (t, z) plane, X then Y transform of every C_ab into
 //      H[(nx, ny)][ab], in the form's arithmetic (FP64 planes for complex128,
 //      FP32 planes for the mixed form)
@@ -21,150 +21,167 @@
 
 #include "launch_variants.cuh"
 #include "momentum.hpp"
+#include "ops_site.cuh"
 
 namespace cgb {
 
 template <class R> struct Vec2 { using type = double2; };
 template <> struct Vec2<float> { using type = float2; };
 
-using MesonAllGammaP = MesonAllGammaOp<double, double2, 4, 3>;
 using MesonAllGammaM = MesonAllGammaOp<float, float2, 8, 2>;
 // field of the tensor-core path: the spin-colour products, pair halves apart
 using MesonProductsSplitM = MesonAllGammaOp<float, float2, 8, 2, true, true>;
 
-// One CTA per (z, t, chunk of (nx, ny) pairs); one thread per gamma pair.
-// X transform: NG groups of +nx / -nx (C = sum cos * v, S = sum sin * v; the
-// group count is a template argument so that no predicated-off FMA is
-// issued).  Each thread's X values G[nx] go through its own column of shared
-// memory, so the Y step reads G[q_ix[q]] with one load; the Y step runs over
-// QC (>= the chunk's pair count) pairs.
-template <class R> constexpr size_t plane_smem_bytes() { return (size_t)kMomMaxPx * 256 * 2 * sizeof(R); }
+// One CTA per (z, t, chunk of Y groups); one thread per gamma pair.  Sites x and
+// Lx - x have the same cosine and opposite sines, rows y and Ly - y too: their sum
+// and difference make one term of C = sum cos * v and of S = sum sin * v (+k: C + iS,
+// -k: C - iS), half the FMAs of the sites one by one, and the k = 0 transform is a
+// plain sum.  Bound by the FP64 pipe in complex128 (89 % busy): for three X and 15 Y
+// groups 7 instructions a site and pair for X (12 site by site) and 40 / Lx for Y
+// (100 / Lx); 0.83 ms at 18 x 15 x 20 x 28, 125 momenta.
+// Each thread's X sums of a row or of a pair of rows go through its own column of
+// shared memory, so that the Y step finds G[nx] with one load.
+template <class R> constexpr size_t plane_smem_bytes(int npx) { return (size_t)2 * npx * 256 * 2 * sizeof(R); }
 
-template <class R, class S, int NG, int QC>
+template <class R, class S, int NG, int YC>
 __global__ void __launch_bounds__(256) plane_kernel(const S *__restrict__ c, typename Vec2<R>::type *__restrict__ planes,
                                                     const __grid_constant__ MomPlan plan)
 {
-  const int z = blockIdx.x, t = blockIdx.y, q0 = blockIdx.z * kMomQChunk, g = threadIdx.x;
-  const int lx = plan.latt[0], ly = plan.latt[1], lz = plan.latt[2];
-  const int nq = min(kMomQChunk, plan.nq - q0);
-  __shared__ R phx[NG][kMomMaxL][2];
-  __shared__ R phy[QC][kMomMaxL][2];
+  const int z = blockIdx.x, t = blockIdx.y, y0 = blockIdx.z * YC, g = threadIdx.x;
+  const int lx = plan.latt[0], ly = plan.latt[1], lz = plan.latt[2], npx = plan.npx;
+  const int ny = min(YC, plan.nyg - y0);
+  __shared__ R phx[NG][kMomMaxL / 2 + 1][2];
+  __shared__ R phy[YC][kMomMaxL / 2 + 1][2];
+  __shared__ int ygx[YC];
   extern __shared__ __align__(16) unsigned char plane_dyn[];
-  cx<R> *gxs = reinterpret_cast<cx<R> *>(plane_dyn);  // [kMomMaxPx][256]
-  __shared__ int qix[QC];
-  if (g < QC) qix[g] = g < nq ? plan.q_ix[q0 + g] : 0;
-  for (int e = g; e < NG * kMomMaxL; e += blockDim.x) {  // per X group: cos, sin of 2 pi k x / Lx
-    const int gi = e / kMomMaxL, x = e % kMomMaxL;
-    if (x < lx) {
-      const int k = (plan.gx_k[gi] * x) % lx;
-      phx[gi][x][0] = R(plan.cosx[k]);
-      phx[gi][x][1] = R(plan.sinx[k]);
-    }
+  // [2][npx][256]: G of a row and its partner, then their sum and difference
+  cx<R> *gp = reinterpret_cast<cx<R> *>(plane_dyn) + g, *gm = gp + npx * 256;
+  if (g < YC) ygx[g] = g < ny ? plan.yg_ix[y0 + g] : 0;
+  for (int e = g; e < NG * (lx / 2 + 1); e += blockDim.x) {  // per X group: cos, sin of 2 pi k x / Lx
+    const int gi = e / (lx / 2 + 1), x = e % (lx / 2 + 1);
+    const int k = (plan.gx_k[gi] * x) % lx;
+    phx[gi][x][0] = R(plan.cosx[k]);
+    phx[gi][x][1] = R(plan.sinx[k]);
   }
-  for (int e = g; e < QC * kMomMaxL; e += blockDim.x) {
-    const int q = e / kMomMaxL, y = e % kMomMaxL;
-    if (y < ly) {
-      const int k = q < nq ? ((plan.q_ny[q0 + q] * y) % ly + ly) % ly : 0;
-      phy[q][y][0] = q < nq ? R(plan.cosy[k]) : R(0);
-      phy[q][y][1] = q < nq ? R(plan.siny[k]) : R(0);
-    }
+  for (int e = g; e < YC * (ly / 2 + 1); e += blockDim.x) {
+    const int q = e / (ly / 2 + 1), y = e % (ly / 2 + 1);
+    const int k = q < ny ? (plan.yg_k[y0 + q] * y) % ly : 0;
+    phy[q][y][0] = q < ny ? R(plan.cosy[k]) : R(0);
+    phy[q][y][1] = q < ny ? R(plan.siny[k]) : R(0);
   }
   __syncthreads();
-  cx<R> h[QC];
+  const bool zero = plan.gx_k[0] == 0;  // the k = 0 group, if there is one, is the first
+  cx<R> hc[YC], hs[YC];
 #pragma unroll
-  for (int q = 0; q < QC; ++q) h[q] = czero<R>();
-  const S *row = c + ((size_t)(t * lz + z) * ly * lx) * 256 + g;
-  constexpr int XB = 8;  // loads in flight per thread
-  for (int y = 0; y < ly; ++y) {
-    cx<R> gc[NG], gs[NG];
+  for (int q = 0; q < YC; ++q) hc[q] = hs[q] = czero<R>();
+  const S *plane = c + ((size_t)(t * lz + z) * ly * lx) * 256 + g;
+  constexpr int XB = 4;  // pairs of loads in flight per thread
+  for (int y = 0; y <= ly / 2; ++y) {
+    const bool alone = y == 0 || 2 * y == ly;
+    for (int half = 0; half < (alone ? 1 : 2); ++half) {
+      cx<R> gc[NG], gs[NG];
 #pragma unroll
-    for (int gi = 0; gi < NG; ++gi) gc[gi] = gs[gi] = czero<R>();
-    const S *rowy = row + (size_t)y * lx * 256;
-    for (int x0 = 0; x0 < lx; x0 += XB) {
-      cx<R> v[XB];
+      for (int gi = 0; gi < NG; ++gi) gc[gi] = gs[gi] = czero<R>();
+      const S *row = plane + (size_t)(half ? ly - y : y) * lx * 256;
+      for (int x0 = 0; x0 <= lx / 2; x0 += XB) {
+        cx<R> v[XB], w[XB];
 #pragma unroll
-      for (int u = 0; u < XB; ++u) v[u] = (x0 + u < lx) ? ld<R>(rowy + (size_t)(x0 + u) * 256) : czero<R>();
+        for (int u = 0; u < XB; ++u) {
+          const int x = x0 + u;
+          v[u] = x <= lx / 2 ? ld<R>(row + (size_t)x * 256) : czero<R>();
+          w[u] = x > 0 && 2 * x < lx ? ld<R>(row + (size_t)(lx - x) * 256) : czero<R>();
+        }
 #pragma unroll
-      for (int u = 0; u < XB; ++u) {
-        if (x0 + u >= lx) break;
+        for (int u = 0; u < XB; ++u) {
+          if (x0 + u > lx / 2) break;
+          const cx<R> a = cadd(v[u], w[u]), d = {v[u].x - w[u].x, v[u].y - w[u].y};
 #pragma unroll
-        for (int gi = 0; gi < NG; ++gi) {
-          const R cs = phx[gi][x0 + u][0], sn = phx[gi][x0 + u][1];
-          gc[gi].x = fma(cs, v[u].x, gc[gi].x);
-          gc[gi].y = fma(cs, v[u].y, gc[gi].y);
-          gs[gi].x = fma(sn, v[u].x, gs[gi].x);
-          gs[gi].y = fma(sn, v[u].y, gs[gi].y);
+          for (int gi = 0; gi < NG; ++gi) {
+            if (gi == 0 && zero) {
+              gc[0] = cadd(gc[0], a);
+              continue;
+            }
+            const R cs = phx[gi][x0 + u][0], sn = phx[gi][x0 + u][1];
+            gc[gi].x = fma(cs, a.x, gc[gi].x);
+            gc[gi].y = fma(cs, a.y, gc[gi].y);
+            gs[gi].x = fma(sn, d.x, gs[gi].x);
+            gs[gi].y = fma(sn, d.y, gs[gi].y);
+          }
         }
       }
-    }
-    // G(+k) = C + iS, G(-k) = C - iS
+      auto put = [&](int ix, cx<R> v) {
+        if (ix < 0) return;
+        cx<R> *p = gp + ix * 256, *m = gm + ix * 256;
+        if (half) {
+          const cx<R> o = *p;
+          *p = cadd(o, v);
+          *m = {o.x - v.x, o.y - v.y};
+        } else {
+          *p = v;
+          if (alone) *m = v;
+        }
+      };
 #pragma unroll
-    for (int gi = 0; gi < NG; ++gi) {
-      if (plan.gx_plus[gi] >= 0) gxs[plan.gx_plus[gi] * 256 + g] = {gc[gi].x - gs[gi].y, gc[gi].y + gs[gi].x};
-      if (plan.gx_minus[gi] >= 0) gxs[plan.gx_minus[gi] * 256 + g] = {gc[gi].x + gs[gi].y, gc[gi].y - gs[gi].x};
+      for (int gi = 0; gi < NG; ++gi) {  // G(+k) = C + iS, G(-k) = C - iS
+        put(plan.gx_plus[gi], {gc[gi].x - gs[gi].y, gc[gi].y + gs[gi].x});
+        put(plan.gx_minus[gi], {gc[gi].x + gs[gi].y, gc[gi].y - gs[gi].x});
+      }
     }
 #pragma unroll
-    for (int q = 0; q < QC; ++q) cfma(h[q], cx<R> {phy[q][y][0], phy[q][y][1]}, gxs[qix[q] * 256 + g]);
+    for (int q = 0; q < YC; ++q) {
+      const cx<R> a = gp[ygx[q] * 256], d = gm[ygx[q] * 256];
+      const R cs = phy[q][y][0], sn = phy[q][y][1];
+      hc[q].x = fma(cs, a.x, hc[q].x);
+      hc[q].y = fma(cs, a.y, hc[q].y);
+      hs[q].x = fma(sn, d.x, hs[q].x);
+      hs[q].y = fma(sn, d.y, hs[q].y);
+    }
   }
+  const size_t at = ((size_t)(t * lz + z) * plan.nq) * 256 + g;
 #pragma unroll
-  for (int q = 0; q < QC; ++q)
-    if (q < nq)
-      planes[((size_t)(t * lz + z) * plan.nq + q0 + q) * 256 + g] = {h[q].x, h[q].y};
+  for (int q = 0; q < YC; ++q) {
+    if (q >= ny) break;
+    const int qp = plan.yg_plus[y0 + q], qm = plan.yg_minus[y0 + q];
+    if (qp >= 0) planes[at + (size_t)qp * 256] = {hc[q].x - hs[q].y, hc[q].y + hs[q].x};
+    if (qm >= 0) planes[at + (size_t)qm * 256] = {hc[q].x + hs[q].y, hc[q].y - hs[q].x};
+  }
 }
 
-template <int NG> cudaError_t set_plane_smem_attr_ng()
+template <class R, class S, int NG, int YC>
+cudaError_t launch_plane_yc(const Job &job, const S *field, typename Vec2<R>::type *planes, const MomPlan &plan)
 {
-  const int b = (int)plane_smem_bytes<double>();
-  cudaError_t e = cudaFuncSetAttribute(plane_kernel<double, double2, NG, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(plane_kernel<double, double2, NG, 9>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(plane_kernel<double, double2, NG, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(plane_kernel<double, double2, NG, kMomQChunk>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, b);
-  return e;
-}
-
-inline cudaError_t set_plane_smem_attr()
-{
-  cudaError_t e = set_plane_smem_attr_ng<1>();
-  if (e == cudaSuccess) e = set_plane_smem_attr_ng<2>();
-  if (e == cudaSuccess) e = set_plane_smem_attr_ng<3>();
-  if (e == cudaSuccess) e = set_plane_smem_attr_ng<4>();
-  if (e == cudaSuccess) e = set_plane_smem_attr_ng<5>();
-  if (e == cudaSuccess) e = set_plane_smem_attr_ng<6>();
-  if (e == cudaSuccess) e = set_plane_smem_attr_ng<7>();
-  if (e == cudaSuccess) e = set_plane_smem_attr_ng<8>();
-  return e;
-}
-
-template <class R, class S, int NG>
-cudaError_t launch_plane_qc(const Job &job, const S *field, typename Vec2<R>::type *planes, const MomPlan &plan,
-                            dim3 grid)
-{
-  const int qc = plan.nq < kMomQChunk ? plan.nq : kMomQChunk;
-  const size_t smem = plane_smem_bytes<R>();
-  if (qc <= 4) plane_kernel<R, S, NG, 4><<<grid, 256, smem, job.stream>>>(field, planes, plan);
-  else if (qc <= 9) plane_kernel<R, S, NG, 9><<<grid, 256, smem, job.stream>>>(field, planes, plan);
-  else if (qc <= 16) plane_kernel<R, S, NG, 16><<<grid, 256, smem, job.stream>>>(field, planes, plan);
-  else plane_kernel<R, S, NG, kMomQChunk><<<grid, 256, smem, job.stream>>>(field, planes, plan);
+  // complex128 with many nx needs more than the default 48 KB of shared memory
+  const size_t smem = plane_smem_bytes<R>(plan.npx);
+  if (smem > 32768) {
+    const cudaError_t e = cudaFuncSetAttribute(plane_kernel<R, S, NG, YC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               (int)plane_smem_bytes<R>(kMomMaxPx));
+    if (e != cudaSuccess) return e;
+  }
+  const dim3 grid(plan.latt[2], plan.latt[3], (plan.nyg + YC - 1) / YC);
+  plane_kernel<R, S, NG, YC><<<grid, 256, smem, job.stream>>>(field, planes, plan);
   return cudaGetLastError();
+}
+// The groups of one launch: few enough accumulators for the list, or chunks of 15.
+template <class R, class S, int NG>
+cudaError_t launch_plane_ng(const Job &job, const S *field, typename Vec2<R>::type *planes, const MomPlan &plan)
+{
+  if (plan.nyg <= 2) return launch_plane_yc<R, S, NG, 2>(job, field, planes, plan);
+  if (plan.nyg <= 6) return launch_plane_yc<R, S, NG, 6>(job, field, planes, plan);
+  return launch_plane_yc<R, S, NG, kMomYChunk>(job, field, planes, plan);
 }
 
 template <class R, class S>
-cudaError_t launch_plane(const Job &job, const S *field, typename Vec2<R>::type *planes, const MomPlan &plan,
-                         dim3 grid)
+cudaError_t launch_plane(const Job &job, const S *field, typename Vec2<R>::type *planes, const MomPlan &plan)
 {
   switch (plan.ngx) {
-  case 1: return launch_plane_qc<R, S, 1>(job, field, planes, plan, grid);
-  case 2: return launch_plane_qc<R, S, 2>(job, field, planes, plan, grid);
-  case 3: return launch_plane_qc<R, S, 3>(job, field, planes, plan, grid);
-  case 4: return launch_plane_qc<R, S, 4>(job, field, planes, plan, grid);
-  case 5: return launch_plane_qc<R, S, 5>(job, field, planes, plan, grid);
-  case 6: return launch_plane_qc<R, S, 6>(job, field, planes, plan, grid);
-  case 7: return launch_plane_qc<R, S, 7>(job, field, planes, plan, grid);
-  case 8: return launch_plane_qc<R, S, 8>(job, field, planes, plan, grid);
+  case 1: return launch_plane_ng<R, S, 1>(job, field, planes, plan);
+  case 2: return launch_plane_ng<R, S, 2>(job, field, planes, plan);
+  case 3: return launch_plane_ng<R, S, 3>(job, field, planes, plan);
+  case 4: return launch_plane_ng<R, S, 4>(job, field, planes, plan);
+  case 5: return launch_plane_ng<R, S, 5>(job, field, planes, plan);
+  case 6: return launch_plane_ng<R, S, 6>(job, field, planes, plan);
+  case 7: return launch_plane_ng<R, S, 7>(job, field, planes, plan);
+  case 8: return launch_plane_ng<R, S, 8>(job, field, planes, plan);
   default: return cudaErrorInvalidValue;
   }
 }
@@ -371,10 +388,12 @@ __global__ void __launch_bounds__(256) momentum_finalize(const typename Vec2<R>:
           if (pm >= 0) out[((size_t)pm * lt + t) * 256 + g] = o[sg];
         }
       } else {
+        // the complex128 planes are in the order of MesonPairsOp
+        const int at = sizeof(R) == 8 ? pair_of_class(g) : g;
         const double2 c = ca[k].value(), sn = sa[k].value();
         const int pp = plan.gz_plus[base + k], pn = plan.gz_minus[base + k];
-        if (pp >= 0) out[((size_t)pp * lt + t) * 256 + g] = make_double2(c.x - sn.y, c.y + sn.x);
-        if (pn >= 0) out[((size_t)pn * lt + t) * 256 + g] = make_double2(c.x + sn.y, c.y - sn.x);
+        if (pp >= 0) out[((size_t)pp * lt + t) * 256 + at] = make_double2(c.x - sn.y, c.y + sn.x);
+        if (pn >= 0) out[((size_t)pn * lt + t) * 256 + at] = make_double2(c.x + sn.y, c.y - sn.x);
       }
     }
   }
@@ -607,7 +626,7 @@ cudaError_t launch_meson_momentum(const Job &job, const OpParams<double> &p, con
   q.out[0] = ws;
   for (int k = 0; k < 4; ++k) q.latt[k] = plan.latt[k];
   cudaError_t e;
-  if (job.prec == Prec::C128) e = run_field<MesonAllGammaP>(job, q);
+  if (job.prec == Prec::C128) e = run_ring_field<MesonPairsOp<4, 4>>(job, q);
   else if (tensor_cores) e = run_field<MesonProductsSplitM>(job, convert_params<float>(q));
   else e = run_field<MesonAllGammaM>(job, convert_params<float>(q));
   if (e != cudaSuccess) return e;
@@ -623,23 +642,12 @@ cudaError_t launch_meson_momentum(const Job &job, const OpParams<double> &p, con
     return cudaGetLastError();
   }
 
-  const dim3 grid(lz, lt, (plan.nq + kMomQChunk - 1) / kMomQChunk);
   if (job.prec == Prec::C128) {
-    // the complex128 form needs more than the default 48 KB of shared memory
-    static bool attr[64] = {};
-    int dev = 0;
-    e = cudaGetDevice(&dev);
-    if (e != cudaSuccess) return e;
-    if (dev >= 64 || !attr[dev]) {
-      e = set_plane_smem_attr();
-      if (e != cudaSuccess) return e;
-      if (dev < 64) attr[dev] = true;
-    }
-    e = launch_plane<double, double2>(job, reinterpret_cast<const double2 *>(ws), planes, plan, grid);
+    e = launch_plane<double, double2>(job, reinterpret_cast<const double2 *>(ws), planes, plan);
     if (e != cudaSuccess) return e;
     return launch_finalize<double, false>(job, planes, static_cast<double2 *>(out), plan);
   }
-  e = launch_plane<float, float2>(job, reinterpret_cast<const float2 *>(ws), planes_m, plan, grid);
+  e = launch_plane<float, float2>(job, reinterpret_cast<const float2 *>(ws), planes_m, plan);
   if (e != cudaSuccess) return e;
   return launch_finalize<float, false>(job, planes_m, static_cast<double2 *>(out), plan);
 }

@@ -9,7 +9,8 @@ constexpr int kMomMaxL = 64;     // largest spatial extent
 constexpr int kMomMaxPx = 8;     // distinct nx values per call
 constexpr int kMomMaxQ = 128;    // distinct (nx, ny) pairs per call
 constexpr int kMomMaxP = 1024;   // momenta per call
-constexpr int kMomQChunk = 25;   // (nx, ny) pairs per plane-kernel CTA
+constexpr int kMomQChunk = 25;   // (nx, ny) pairs of the fused complex64 kernels
+constexpr int kMomYChunk = 15;   // Y groups per plane-kernel CTA
 
 struct MomPlan {
   int latt[4];
@@ -25,6 +26,8 @@ struct MomPlan {
   // momentum component n (mod L) with -n; an absent partner is -1.
   int ngx;                                                        // X groups
   int gx_k[kMomMaxPx], gx_plus[kMomMaxPx], gx_minus[kMomMaxPx];  // k in [0, Lx/2]; px indices
+  int nyg;                                                        // Y groups (per nx)
+  int yg_ix[kMomMaxQ], yg_k[kMomMaxQ], yg_plus[kMomMaxQ], yg_minus[kMomMaxQ];  // px index, k in [0, Ly/2]; pairs q
   int q_g0[kMomMaxQ + 1];                                // Z groups of pair q: [q_g0[q], q_g0[q+1])
   int gz_k[kMomMaxP], gz_plus[kMomMaxP], gz_minus[kMomMaxP];     // k in [0, Lz/2]; momentum indices
 };

@@ -385,6 +385,31 @@ CGB_HD constexpr ClassWalsh class_walsh()
   return w;
 }
 static_assert(class_walsh().ok, "gamma classes must have the Walsh phase structure");
+// The phases of a class's rows differ by signs only (every Gamma is real or imaginary).
+CGB_HD constexpr bool class_phases_common(const ClassWalsh &w)
+{
+  for (int k = 0; k < 16; ++k)
+    if ((((w.beta >> (2 * k)) ^ (w.beta >> (8 * (k / 4)))) & 1u) != 0) return false;
+  return true;
+}
+
+// Lexicographic index ((t Lz + z) Ly + y) Lx + x of an even/odd-ordered site; -1
+// without a lattice (the engines then skip the site and report it).
+template <class R> __device__ __forceinline__ long long lexicographic(const OpParams<R> &p, long long site)
+{
+  const long long lx = p.latt[0], ly = p.latt[1], lz = p.latt[2], lt = p.latt[3];
+  if (lx < 2 || ly < 1 || lz < 1 || lt < 1) return -1;
+  const long long half = lx / 2;
+  long long r = site / half;
+  const long long xh = site - r * half;
+  const long long y = r % ly;
+  r /= ly;
+  const long long z = r % lz;
+  r /= lz;
+  const long long t = r % lt, par = r / lt;
+  const long long x = 2 * xh + ((par + t + z + y) & 1);
+  return ((t * lz + z) * ly + y) * lx + x;
+}
 
 // ------------------------------------------------------------------ ops --
 // Common compile-time configuration of an op: CW consumer warps (plus one
@@ -667,7 +692,7 @@ __device__ __forceinline__ void conj_products_f32x2(cx<float> (&T)[NK][NL], cons
 // SPLIT selects the layout [t][pair half][site][128 pairs] (pairs 0-127 and
 // 128-255 of a timeslice in separate planes) that the tensor-core projection
 // streams as contiguous 8-site tiles; otherwise [t][site][256 pairs].
-// PRODUCTS (complex64): store the 256 spin-colour products
+// PRODUCTS: store the 256 spin-colour products
 //   T[i][j][k][l] = sum_c S1[i][k][c] conj(S2[j][l][c])
 // instead of the Gamma pairs, product (i, j = i ^ s, k, l) at index
 // (4 k + l) * 16 + 4 s + i.  Each pair is a signed sum of 16 products, the same
@@ -676,7 +701,7 @@ __device__ __forceinline__ void conj_products_f32x2(cx<float> (&T)[NK][NL], cons
 template <class R, class S, int CW, int NST, bool SPLIT = false, bool PRODUCTS = false>
 struct MesonAllGammaOp : OpBase<R, S, CW, 16, NST> {
   static constexpr int NIN = 2, EXTRA_BYTES = 0, OUT_ELEMS = 256;
-  static_assert(!PRODUCTS || sizeof(R) == 4, "the product form is complex64 only");
+  static_assert(sizeof(R) == 4, "complex128: MesonPairsOp (ops_site.cuh)");
   // Each thread's 16 outputs are four 32-byte runs: stored straight to HBM.
   static constexpr bool DIRECT_OUT = true;
 
@@ -697,22 +722,7 @@ struct MesonAllGammaOp : OpBase<R, S, CW, 16, NST> {
     }
   }
 
-  __device__ static long long out_index(const OpParams<R> &p, long long site)
-  {
-    const long long lx = p.latt[0], ly = p.latt[1], lz = p.latt[2], lt = p.latt[3];
-    if (lx < 2 || ly < 1 || lz < 1 || lt < 1) return -1;  // no lattice: the engine skips and reports
-    const long long half = lx / 2;
-    long long r = site / half;
-    const long long xh = site - r * half;
-    const long long y = r % ly;
-    r /= ly;
-    const long long z = r % lz;
-    r /= lz;
-    const long long t = r % lt, par = r / lt;
-    const long long x = 2 * xh + ((par + t + z + y) & 1);
-    return ((t * lz + z) * ly + y) * lx + x;
-  }
-
+  __device__ static long long out_index(const OpParams<R> &p, long long site) { return lexicographic(p, site); }
 
   __device__ static void site(const OpParams<R> &ps_, const S *const *in, S *, int sub, S *out)
   {
@@ -720,41 +730,20 @@ struct MesonAllGammaOp : OpBase<R, S, CW, 16, NST> {
     constexpr ClassWalsh CW8 = class_walsh();
     const int s = sub >> 2, i = sub & 3, j = i ^ s;
     cx<R> T[4][4];
-    if constexpr (sizeof(R) == 4) {
-      conj_products_f32x2(T, in[0] + i * 36, in[1] + j * 36);
-      if constexpr (PRODUCTS) {
-        if (!out) return;
+    conj_products_f32x2(T, in[0] + i * 36, in[1] + j * 36);
+    if constexpr (PRODUCTS) {
+      if (!out) return;
 #pragma unroll
-        for (int k = 0; k < 4; ++k)
-#pragma unroll
-          for (int l = 0; l < 4; ++l) {
-            const int g = (k * 4 + l) * 16 + sub;
-            S *dst;
-            if constexpr (SPLIT) dst = out + (g >> 7) * sites_per_slice(ps_) * 128 + (g & 127);
-            else dst = out + g;
-            *dst = S {T[k][l].x, T[k][l].y};
-          }
-        return;
-      }
-    } else {
-      // Block (i, k) has the parity of k and block (j, l) that of l, so every
-      // colour block loads as 16-byte vectors.
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        cx<R> x[9];
-        if (k & 1) load9p<true>(x, in[0] + (i * 4 + k) * 9);
-        else load9p<false>(x, in[0] + (i * 4 + k) * 9);
+      for (int k = 0; k < 4; ++k)
 #pragma unroll
         for (int l = 0; l < 4; ++l) {
-          cx<R> y[9];
-          if (l & 1) load9p<true>(y, in[1] + (j * 4 + l) * 9);
-          else load9p<false>(y, in[1] + (j * 4 + l) * 9);
-          cx<R> t = czero<R>();
-#pragma unroll
-          for (int e = 0; e < 9; ++e) cfma_conj(t, x[e], y[e]);
-          T[k][l] = t;
+          const int g = (k * 4 + l) * 16 + sub;
+          S *dst;
+          if constexpr (SPLIT) dst = out + (g >> 7) * sites_per_slice(ps_) * 128 + (g & 127);
+          else dst = out + g;
+          *dst = S {T[k][l].x, T[k][l].y};
         }
-      }
+      return;
     }
     // V[b] = i^beta_s(i) sum_l (g5 Gamma(b))^T-phase(l) T[perm_b(l)][l]
     const uint32_t beta = (CW8.beta >> (2 * (4 * s + i))) & 3u;
