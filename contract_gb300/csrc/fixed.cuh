@@ -16,7 +16,7 @@
 // scale).  Colour rows or columns of very different size so keep their bits.
 //
 // Accuracy.  In units of the operands' scales A and B a value is off by at most
-// 2^-57 A, and the dropped l l' and the last rounding make about half a unit of
+// 2^-55 A (cut off; nothing down to A / 8), and the dropped l l' and the last rounding make about half a unit of
 // 2^-56 A B per result.  For entries of one size s (A ~ 4.5 s with the power of
 // two) that is 2^-52 s^2, against 2^-49.8 s^2 for 32 products summed in FP64, where
 // every sum rounds.  A block much smaller than its field keeps fewer bits, so the
@@ -56,68 +56,76 @@ struct FixedScales {
 template <int TPS, int NA, bool COLOUR = true, int N>
 __device__ __forceinline__ bool fixed_scales(const double2 *const (&blk)[N], FixedScales &f)
 {
-  int e[N][9];  // biased exponents; zeros (and what underflowed) far below
+  f.E[0] = f.E[1] = 0;
 #pragma unroll
-  for (int n = 0; n < N; ++n)
+  for (int a = 0; a < 3; ++a) f.r[a] = f.c[a] = 0;
+  int e[N][9], most[N];  // high words without the sign, then biased exponents (0: zero or denormal)
+#pragma unroll
+  for (int n = 0; n < N; ++n) {
+    most[n] = 0;
 #pragma unroll
     for (int k = 0; k < 9; ++k) {
       const double2 v = blk[n][k];
-      const int x = max(__double2hiint(v.x) & 0x7fffffff, __double2hiint(v.y) & 0x7fffffff) >> 20;
-      e[n][k] = x ? x : -4096;
+      e[n][k] = max(__double2hiint(v.x) & 0x7fffffff, __double2hiint(v.y) & 0x7fffffff);
+      most[n] = max(most[n], e[n][k]);
     }
-  f.E[0] = f.E[1] = -4096;
-#pragma unroll
-  for (int n = 0; n < N; ++n)
-#pragma unroll
-    for (int k = 0; k < 9; ++k) f.E[n < NA ? 0 : 1] = max(f.E[n < NA ? 0 : 1], e[n][k]);
+    most[n] >>= 20;
+    f.E[n < NA ? 0 : 1] = max(f.E[n < NA ? 0 : 1], most[n]);
+  }
   f.E[0] = group_max<TPS>(f.E[0]);
   f.E[1] = NA < N ? group_max<TPS>(f.E[1]) : f.E[0];
   bool ok = min(f.E[0], f.E[1]) >= kFixedMinExp && max(f.E[0], f.E[1]) <= kFixedMaxExp;
+  if constexpr (!COLOUR) {
 #pragma unroll
-  for (int a = 0; a < 3; ++a) f.r[a] = f.c[a] = 0;
-  if constexpr (COLOUR) {
+    for (int n = 0; n < N; ++n) ok = ok && (most[n] - f.E[n < NA ? 0 : 1] >= -kFixedSpread || most[n] == 0);
+    return ok;
+  }
+  // Exponents of zeros (0) lie more than kFixedColour below every field's scale.
 #pragma unroll
-    for (int a = 0; a < 3; ++a) {
-      int m = -8192;
+  for (int n = 0; n < N; ++n)
 #pragma unroll
-      for (int n = 0; n < N; ++n)
+    for (int k = 0; k < 9; ++k) e[n][k] >>= 20;
 #pragma unroll
-        for (int d = 0; d < 3; ++d) m = max(m, e[n][3 * a + d] - f.E[n < NA ? 0 : 1]);
-      f.r[a] = max(group_max<TPS>(m), -kFixedColour);
+  for (int a = 0; a < 3; ++a) {
+    int m = -kFixedColour;
+#pragma unroll
+    for (int n = 0; n < N; ++n)
+      m = max(m, max(max(e[n][3 * a], e[n][3 * a + 1]), e[n][3 * a + 2]) - f.E[n < NA ? 0 : 1]);
+    f.r[a] = group_max<TPS>(m);
+  }
+  int col[N][3];  // the columns' largest in the scales of the rows
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    int m = -kFixedColour;
+#pragma unroll
+    for (int n = 0; n < N; ++n) {
+      col[n][d] = max(max(e[n][d] - f.r[0], e[n][3 + d] - f.r[1]), e[n][6 + d] - f.r[2]) - f.E[n < NA ? 0 : 1];
+      m = max(m, col[n][d]);
     }
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-      int m = -8192;
-#pragma unroll
-      for (int n = 0; n < N; ++n)
-#pragma unroll
-        for (int a = 0; a < 3; ++a) m = max(m, e[n][3 * a + d] - f.E[n < NA ? 0 : 1] - f.r[a]);
-      f.c[d] = max(group_max<TPS>(m), -kFixedColour);
-    }
+    f.c[d] = group_max<TPS>(m);
   }
 #pragma unroll
   for (int n = 0; n < N; ++n) {
-    int m = -8192;
-#pragma unroll
-    for (int k = 0; k < 9; ++k) m = max(m, e[n][k] - f.E[n < NA ? 0 : 1] - f.r[k / 3] - f.c[k % 3]);
-    ok = ok && (m >= -kFixedSpread || m < -2048);
+    const int m = max(max(col[n][0] - f.c[0], col[n][1] - f.c[1]), col[n][2] - f.c[2]);
+    ok = ok && (m >= -kFixedSpread || most[n] == 0);
   }
   return ok;
 }
 
-// v as h 2^28 + l in units of 2^(E - 55).
+// v as h 2^28 + l in units of 2^(E - 55).  The 53-bit significand, 3 bits up, goes
+// down by E minus v's exponent (the PTX shift gives 0 from 64 on): exact down to 2^-3
+// of the scale, cut off below; 15 instructions (28 with a rounded shift and clamps).
 __device__ __forceinline__ int2 to_fixed(double v, int E)
 {
   const long long bits = __double_as_longlong(v);
-  const int hi = (int)(bits >> 32), e = (hi >> 20) & 0x7ff;
+  const int hi = (int)(bits >> 32);
+  const uint32_t d = (uint32_t)(E - ((hi >> 20) & 0x7ff));  // negative only where the result is not used
   const unsigned long long t =
     ((unsigned long long)(((uint32_t)hi & 0xfffffu) | 0x100000u) << 35) | ((unsigned long long)(uint32_t)bits << 3);
-  const int d = max(E - e, 0);  // below 0 only where the site is not converted for use
-  unsigned long long u = (t + ((1ull << (d & 63)) >> 1)) >> (d & 63);
-  if (d > 60 || e == 0) u = 0;
-  const long long m = hi < 0 ? -(long long)u : (long long)u;
-  const int h = (int)((m + (1ll << 27)) >> 28);
-  return make_int2(h, (int)((uint32_t)m - ((uint32_t)h << 28)));
+  unsigned long long u;
+  asm("shr.u64 %0, %1, %2;" : "=l"(u) : "l"(t), "r"(d));
+  const int h = (int)((u + (1ull << 27)) >> 28), l = (int)((uint32_t)u - ((uint32_t)h << 28));
+  return hi < 0 ? make_int2(-h, -l) : make_int2(h, l);
 }
 
 // A colour block of field `field` to fixed point: (h, l) of re, then of im; dst may be blk.
@@ -283,23 +291,27 @@ __device__ __forceinline__ cx<double> fixed_entry(longlong2 v, int e, const Fixe
   return {fixed_value(v.x, up), fixed_value(v.y, up)};
 }
 
-// re + i im += x . conj(y) over two converted blocks (held in registers or memory).
-template <class X> __device__ __forceinline__ void fixed_conj_mac(FixedSum &re, FixedSum &im, const X &x, const int4 *y)
+// re + i im = x . conj(y) over two converted blocks (held in registers or memory).
+template <class X> __device__ __forceinline__ void fixed_conj_sums(FixedSum &re, FixedSum &im, const X &x, const int4 *y)
 {
+  FixedSum minus {0, 0};
+  re = im = FixedSum {0, 0};
 #pragma unroll
   for (int k = 0; k < 9; ++k) {
     const int4 u = x[k], v = y[k];
     re.mac(u.x, u.y, v.x, v.y);
     re.mac(u.z, u.w, v.z, v.w);
     im.mac(u.z, u.w, v.x, v.y);
-    im.mac(-u.x, -u.y, v.z, v.w);
+    minus.mac(u.x, u.y, v.z, v.w);
   }
+  im.hh -= minus.hh;
+  im.x -= minus.x;
 }
 // The same as doubles, blocks of one scale each; up = 2^ of their scales - 54.
 __device__ __forceinline__ cx<double> fixed_conj_dot(const int4 (&x)[9], const int4 *y, int up)
 {
-  FixedSum re {0, 0}, im {0, 0};
-  fixed_conj_mac(re, im, x, y);
+  FixedSum re, im;
+  fixed_conj_sums(re, im, x, y);
   return {re.value(up), im.value(up)};
 }
 
@@ -327,15 +339,17 @@ struct FixedDotBlock {
   __device__ __forceinline__ cx<double> dot(const double2 *blk) const
   {
     const int4 *y = reinterpret_cast<const int4 *>(blk);
-    FixedSum re {0, 0}, im {0, 0};
+    FixedSum re {0, 0}, im {0, 0}, minus {0, 0};
 #pragma unroll
     for (int k = 0; k < 9; ++k) {
       const int4 u = g[k], v = y[k];
       re.mac(u.x, u.y, v.x, v.y);
-      re.mac(-u.z, -u.w, v.z, v.w);
+      minus.mac(u.z, u.w, v.z, v.w);
       im.mac(u.x, u.y, v.z, v.w);
       im.mac(u.z, u.w, v.x, v.y);
     }
+    re.hh -= minus.hh;
+    re.x -= minus.x;
     return {re.value(up), im.value(up)};
   }
 };

@@ -14,10 +14,10 @@ template <class Op> static cudaError_t run_rank(const Job &job, OpParams<typenam
 // complex128 on the integer pipe (fixed.cuh): bound by IMAD.WIDE issue and the
 // conversions, so warps in flight count and a second ring stage, which costs warps,
 // does not pay.  24^3 x 32 per site, three different fields, ms (the FP64 kernels
-// that these replaced in brackets): loop 1.17 [2.86 with a projector of two terms],
-// one gamma matrix 2.52, dense projector 3.82, rank 2 1.89 [4.65], rank 1 1.52.
-// The rank form with P_n read from memory: 8 warps an SM, more do not pay (11 warps
-// 1.99, 2 CTAs of 5 2.19: less L1 for P_n and fewer registers).
+// that these replaced in brackets): loop 0.89 [2.86 with a projector of two terms],
+// one gamma matrix 2.34, dense projector 3.51, rank 2 1.73 [4.65], rank 1 1.35.
+// The rank form with P_n read from memory: 8 warps an SM, more do not pay (2 CTAs of
+// 5 1.90, 3 of 3 1.96: less L1 for P_n and fewer registers).
 static const VariantSet<double, 4> kLoopP = {
   {run_ring<BaryonLoopOp<double, double2, 4, 16, 1, 3>>, run_ring<BaryonLoopOp<double, double2, 4, 16, 1, 2>>,
    run_ring<BaryonLoopOp<double, double2, 2, 16, 1, 6>>, run_ring<BaryonLoopOp<double, double2, 13, 16, 1, 1>>},

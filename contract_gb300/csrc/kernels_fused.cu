@@ -37,7 +37,7 @@ template <int SRC, int NW, bool SAME> static VariantSet<float, 7> shapes_m(int d
 static const VariantSet<float, 7> kFused1M = shapes_m<1, 1, false>(0), kFused2M = shapes_m<2, 2, false>(0),
                                   kSame1M = shapes_m<1, 1, true>(1), kSame2M = shapes_m<2, 2, true>(1);
 
-// complex128 (integer pipe, fixed.cuh): 16^3 x 48 with two projectors, 1.76, 1.87 and 2.13 ms in this order (FP64
+// complex128 (integer pipe, fixed.cuh): 16^3 x 48 with two projectors, 1.57 ms; with dearer conversions 1.76, 1.87 and 2.13 in this order (FP64
 // only: 4.24).
 template <int SRC, int NW> static VariantSet<double, 3> shapes_p()
 {

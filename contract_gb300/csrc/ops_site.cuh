@@ -329,10 +329,9 @@ struct MesonAllOp : RingOp<R, S, CW, 16, NST, MINB> {
 // blocks stays below 2^60.2 units, four of them below 2^62.2; they are rounded to
 // quarter units before the four rows meet.
 //
-// 0.86 ms at 18 x 15 x 20 x 28, IMAD.WIDE pipe 67 % busy; the FP64 form with its 4096
-// adds a site for the pairs took 2.9.  The whole projection of 125 momenta 1.77 ms
-// (4.60), of 27 at 24^3 x 16 2.07 (5.66), of one 1.61 (5.10), with errors against
-// extended precision of 3.9e-16 of the norm (4.3e-16).
+// 0.77 ms at 18 x 15 x 20 x 28, bound by the integer pipes.  The whole projection of
+// 125 momenta 1.68 ms (4.60 in FP64), with errors against extended precision of
+// 3.9e-16 of the norm (4.3e-16).
 template <int CW, int MINB> struct MesonPairsOp : RingOp<double, double2, CW, 16, 1, MINB> {
   using P = OpParams<double>;
   static constexpr int NIN = 2, NOUT = 0, OUT_ELEMS = 256;
@@ -415,8 +414,8 @@ template <int CW, int MINB> struct MesonPairsOp : RingOp<double, double2, CW, 16
       const int4 *A = reinterpret_cast<const int4 *>(in[0]), *B = reinterpret_cast<const int4 *>(in[1]);
       long long re[4][4], im[4][4];
       pairs(s, u, re, im, [&](int a, int b, long long &x, long long &y) {
-        FixedSum sx {0, 0}, sy {0, 0};
-        fixed_conj_mac(sx, sy, A + a, B + b);
+        FixedSum sx, sy;
+        fixed_conj_sums(sx, sy, A + a, B + b);
         x = sx.units();
         y = sy.units();
       });
