@@ -461,6 +461,8 @@ void fill_proj(cgb::ProjOperand<double> &w, int gamma_mn, const double *project_
     if (w.w[k][0] != 0.0 || w.w[k][1] != 0.0) {
       w.nzk[w.nnz++] = (uint8_t)k;
       w.nzmask |= 1u << k;
+      w.real |= (uint32_t)(w.w[k][1] == 0.0) << k;
+      w.imag |= (uint32_t)(w.w[k][0] == 0.0) << k;
     }
   }
   // A phased permutation (one entry in {1, i, -1, -i} per row, distinct

@@ -190,6 +190,19 @@ template <> struct ChunkSum<double> {
   __device__ __forceinline__ void reset() { x = y = 0.0; }
 };
 
+// The same for one real component.
+template <class R> struct ChunkPart;
+template <> struct ChunkPart<float> {
+  float h = 0.f, l = 0.f;
+  __device__ __forceinline__ void add(float v) { ChunkSum<float>::two_sum(h, l, v); }
+  __device__ __forceinline__ double value() const { return (double)h + (double)l; }
+};
+template <> struct ChunkPart<double> {
+  double s = 0.0;
+  __device__ __forceinline__ void add(double v) { s += v; }
+  __device__ __forceinline__ double value() const { return s; }
+};
+
 __device__ __forceinline__ void mbar_arrive(uint64_t *bar)
 {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(bar)) : "memory");

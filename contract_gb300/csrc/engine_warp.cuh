@@ -238,6 +238,7 @@ __global__ void __launch_bounds__(32 * Op::CW, Op::MIN_CTAS) ring_kernel(const _
   for (; issued < NST && ahead.valid(p); ++issued, ahead.next(p)) fetch(ahead, issued);
   const unsigned long long wait_ns = ps.geom.wait_ns;
   ChunkSum<R> chunk_acc;
+  ChunkPart<R> chunk_part;
   for (int u = 0; cur.valid(p); ++u) {
     const int stage = u % NST;
     if (!__all_sync(0xffffffffu, mbar_wait_bounded(&full[stage], (u / NST) & 1, wait_ns))) {
@@ -261,9 +262,12 @@ __global__ void __launch_bounds__(32 * Op::CW, Op::MIN_CTAS) ring_kernel(const _
         else if (sub == 0) report(p.status, kDevErrBadWork, (unsigned int)(cur.first() + local));
       }
       Op::site(ps, in, scratch, sub, ok, dst);
-    } else if constexpr (Op::DIRECT_N) {  // the last field is read from memory by the op
-      const long long at = cur.first() + (ok ? local : 0);
-      v = Op::site(ps, in, reinterpret_cast<const S *>(cur.in(p, NIN) + at * L::SITE_BYTES), scratch, sub, ok);
+    } else if constexpr (Op::DIRECT > 0) {  // fields NIN and on are read from memory by the op
+      const long long at = (cur.first() + (ok ? local : 0)) * L::SITE_BYTES;
+      const S *more[Op::DIRECT];
+#pragma unroll
+      for (int q = 0; q < Op::DIRECT; ++q) more[q] = reinterpret_cast<const S *>(cur.in(p, NIN + q) + at);
+      v = Op::site(ps, in, more, scratch, sub, ok);
     } else {
       v = Op::site(ps, in, scratch, sub, ok);
     }
@@ -274,32 +278,42 @@ __global__ void __launch_bounds__(32 * Op::CW, Op::MIN_CTAS) ring_kernel(const _
       ++issued;
       ahead.next(p);
     }
-    if constexpr (NOUT == 1) v = group_sum<TPS>(v);
-    if constexpr (NOUT == 0) {
-    } else if (ps.geom.per_site) {
-      if (ok) {
-        if constexpr (NOUT == 1) {
-          if (sub == 0) static_cast<double2 *>(ps.out[0])[cur.first() + local] = make_double2(double(v.x), double(v.y));
-        } else {
-          static_cast<double2 *>(ps.out[Op::output(ps, sub)])[cur.first() + local] = make_double2(double(v.x), double(v.y));
+    if constexpr (NOUT == 1) {
+      // even threads are left with the site's real part, odd ones with the imaginary:
+      // half the adds of two full sums, which the FP64 pipe feels
+      const bool odd = lane & 1;
+      R part = (odd ? v.y : v.x) + __shfl_xor_sync(0xffffffffu, odd ? v.x : v.y, 1);
+#pragma unroll
+      for (int o = TPS / 2; o > 1; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
+      if (ps.geom.per_site) {
+        if (ok && sub < 2) static_cast<double *>(ps.out[0])[2 * (cur.first() + local) + sub] = double(part);
+      } else {
+        chunk_part.add(ok ? part : R(0));
+        if (cur.last_in_chunk()) {
+          double c = chunk_part.value();
+#pragma unroll
+          for (int o = 16; o >= TPS; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
+          if (lane < 2) reinterpret_cast<double *>(cur.partial(p))[lane] = c;
+          chunk_part = {};
         }
       }
-    } else {
-      chunk_acc.add(ok ? v : czero<R>());
-      if (cur.last_in_chunk()) {
-        double2 c = chunk_acc.value();
+    } else if constexpr (NOUT > 1) {
+      static_assert(NOUT == TPS, "one output per thread of a site");
+      if (ps.geom.per_site) {
+        if (ok)
+          static_cast<double2 *>(ps.out[Op::output(ps, sub)])[cur.first() + local] = make_double2(double(v.x), double(v.y));
+      } else {
+        chunk_acc.add(ok ? v : czero<R>());
+        if (cur.last_in_chunk()) {
+          double2 c = chunk_acc.value();
 #pragma unroll
-        for (int o = 16; o >= TPS; o >>= 1) {
-          c.x += __shfl_xor_sync(0xffffffffu, c.x, o);
-          c.y += __shfl_xor_sync(0xffffffffu, c.y, o);
-        }
-        if constexpr (NOUT == 1) {
-          if (lane == 0) cur.partial(p)[0] = c;
-        } else {
-          static_assert(NOUT == TPS, "one output per thread of a site");
+          for (int o = 16; o >= TPS; o >>= 1) {
+            c.x += __shfl_xor_sync(0xffffffffu, c.x, o);
+            c.y += __shfl_xor_sync(0xffffffffu, c.y, o);
+          }
           if (lane < NOUT) cur.partial(p)[Op::output(ps, lane)] = c;
+          chunk_acc.reset();
         }
-        chunk_acc.reset();
       }
     }
     cur.next(p);

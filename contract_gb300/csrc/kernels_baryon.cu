@@ -15,9 +15,7 @@ template <class Op> static cudaError_t run_rank(const Job &job, OpParams<typenam
 // conversions, so warps in flight count and a second ring stage, which costs warps,
 // does not pay.  24^3 x 32 per site, three different fields, ms (the FP64 kernels
 // that these replaced in brackets): loop 0.89 [2.86 with a projector of two terms],
-// one gamma matrix 2.34, dense projector 3.51, rank 2 1.73 [4.65], rank 1 1.35.
-// The rank form with P_n read from memory: 8 warps an SM, more do not pay (2 CTAs of
-// 5 1.90, 3 of 3 1.96: less L1 for P_n and fewer registers).
+// one gamma matrix 2.32, dense projector 3.50, rank 2 1.52 [4.65], rank 1 1.18.
 static const VariantSet<double, 4> kLoopP = {
   {run_ring<BaryonLoopOp<double, double2, 4, 16, 1, 3>>, run_ring<BaryonLoopOp<double, double2, 4, 16, 1, 2>>,
    run_ring<BaryonLoopOp<double, double2, 2, 16, 1, 6>>, run_ring<BaryonLoopOp<double, double2, 13, 16, 1, 1>>},
@@ -29,9 +27,9 @@ static const VariantSet<double, 4> kTriP = {
   {"w2.st1.occ5", "w4.st1.occ2", "w4.st1.occ3", "w10.st1.occ1"},
   0};
 static const VariantSet<double, 4> kTriRankP = {
-  {run_rank<BaryonTriRankOp<double, double2, 8, 1, 1>>, run_rank<BaryonTriRankOp<double, double2, 4, 1, 2>>,
-   run_rank<BaryonTriRankOp<double, double2, 5, 1, 2>>, run_rank<BaryonTriRankOp<double, double2, 3, 1, 3>>},
-  {"w8.st1.occ1", "w4.st1.occ2", "w5.st1.occ2", "w3.st1.occ3"},
+  {run_rank<BaryonTriRankOp<double, double2, 4, 1, 3>>, run_rank<BaryonTriRankOp<double, double2, 12, 1, 1>>,
+   run_rank<BaryonTriRankOp<double, double2, 4, 1, 2>>, run_rank<BaryonTriRankOp<double, double2, 10, 1, 1>>},
+  {"w4.st1.occ3", "w12.st1.occ1", "w4.st1.occ2", "w10.st1.occ1"},
   0};
 static const VariantSet<double, 4> kTriGammaP = {
   {run_ring<BaryonTriGammaOp<double, double2, 4, 16, 1, 3>>, run_ring<BaryonTriGammaOp<double, double2, 4, 16, 1, 2>>,

@@ -117,6 +117,8 @@ template <class R> OpParams<R> convert_params(const OpParams<double> &p)
     }
     d.is_perm = s.is_perm;
     d.nnz = s.nnz;
+    d.real = s.real;
+    d.imag = s.imag;
     d.nzmask = s.nzmask;
     for (int k = 0; k < 16; ++k) d.nzk[k] = s.nzk[k];
   }

@@ -44,6 +44,7 @@ template <class R> struct ProjOperand {
   uint8_t nzk[16];  // indices m*4 + n of W's nonzero entries, in order
   int nnz;
   uint32_t nzmask;  // bit m*4 + n set where W[m][n] != 0
+  uint32_t real, imag;  // the same where W[m][n] is real, where it is imaginary (and not 0)
 };
 
 // Up to two projectors written in the gamma basis, W_w = sum_k coef[w][k] Gamma(g_k):
@@ -132,12 +133,16 @@ __device__ __forceinline__ void build_q(const BaryonSpin<R> &b, const S *N, S *q
       for (int m = 0; m < 4; ++m) s = cadd(s, mul_phase(ld<R>(N + (pw.perm[m] * 4 + m) * 9 + ad), pw.ph[m]));
     } else if constexpr (sizeof(R) == 8) {
       // complex128: W's nonzero entries from the host's list.  Testing each
-      // entry here takes FP64 compares on the FP64 pipe, which bounds these
-      // kernels (the loop form with (1 + g4)/2: 7.55 ms against 5.72 ms).
+      // entry here takes FP64 compares on the FP64 pipe, half busy in the loop
+      // form; for the same reason a real or imaginary entry takes two FMAs, not
+      // four ((1 + g4)/2: 0.96 ms at 24^3 x 32, one gamma matrix 0.88).
 #pragma unroll 1
       for (int t = 0; t < pw.nnz; ++t) {
         const int k = pw.nzk[t];  // W[m][n], m = k / 4, n = k % 4, times N[n][m]
-        cfma(s, cx<R> {pw.w[k][0], pw.w[k][1]}, ld<R>(N + ((k & 3) * 4 + (k >> 2)) * 9 + ad));
+        const cx<R> n = ld<R>(N + ((k & 3) * 4 + (k >> 2)) * 9 + ad);
+        if ((pw.real >> k) & 1u) s = {fma(pw.w[k][0], n.x, s.x), fma(pw.w[k][0], n.y, s.y)};
+        else if ((pw.imag >> k) & 1u) s = {fma(-pw.w[k][1], n.y, s.x), fma(pw.w[k][1], n.x, s.y)};
+        else cfma(s, cx<R> {pw.w[k][0], pw.w[k][1]}, n);
       }
     } else {
       // complex64: unrolled over W with the host's nonzero mask (a list loop

@@ -17,7 +17,7 @@ template <class R_, class S_, int CW_, int TPS_, int NST_, int MINB> struct Ring
   static constexpr int CW = CW_, TPS = TPS_, NST = NST_, MIN_CTAS = MINB;
   static constexpr int NOUT = 1, EXTRA_BYTES = 0;
   static constexpr bool CHANGES_INPUT = false;
-  static constexpr bool DIRECT_N = false;  // field NIN is not staged: site() reads it from memory
+  static constexpr int DIRECT = 0;  // fields after NIN that are not staged: site() reads them from memory
 };
 
 // Loop form (IK_JL_NM, IL_JK_NM).
@@ -131,29 +131,34 @@ struct BaryonTriGammaOp : RingOp<R, S, CW, TPS, NST, MINB> {
 
 // Triangle form, W of rank 1 or 2: eight threads a site.  Thread (r, l) with two
 // factors, thread (half of the rows, l) with one: the wedges A[i][perm2 l] ^
-// X_r[perm1 i] over its rows i, then one dot with Y_r[l].  X takes the place of
-// P_j's blocks (X_r[j] at block 4 r + j), and P_n, whose blocks make one Y_r[l] each,
-// is read from memory by the threads that use them: two fields of a site in shared
-// memory let 10 warps of 4 sites share an SM in complex128.
+// X_r[perm1 i] over its rows i, then one dot with Y_r[l].  Complex64 writes X over
+// P_j's blocks (X_r[j] at block 4 r + j).  Complex128 reads P_j and P_n, every block of
+// which is used about once, from memory: with one field and X of a site in shared
+// memory 12 warps of 4 sites share an SM, 1.52 ms at 24^3 x 32 with two factors and
+// 1.18 with one (P_j staged too, 8 warps: 1.73 and 1.35).
 template <class R, class S, int CW, int NST, int MINB>
 struct BaryonTriRankOp : RingOp<R, S, CW, 8, NST, MINB> {
-  static constexpr bool CHANGES_INPUT = true, DIRECT_N = sizeof(R) == 8;
-  static constexpr int NIN = DIRECT_N ? 2 : 3;
-  __device__ static cx<R> site(const OpParams<R> &p, S *const *in, S *scratch, int sub, bool live)
+  static constexpr bool CHANGES_INPUT = true;
+  static constexpr int DIRECT = sizeof(R) == 8 ? 2 : 0, NIN = 3 - DIRECT;
+  static constexpr int EXTRA_BYTES = DIRECT ? cbytes<S>(72) + 16 : 0;  // X; +16: bank stagger
+  __device__ static cx<R> site(const OpParams<R> &p, S *const *in, S *, int sub, bool live)
   {
-    return site(p, in, in[2], scratch, sub, live);
+    return contract(p, in[0], in[1], in[2], in[1], sub, live);
   }
-  __device__ static cx<R> site(const OpParams<R> &p, S *const *in, const S *N, S *, int sub, bool live)
+  __device__ static cx<R> site(const OpParams<R> &p, S *const *in, const S *const *more, S *scratch, int sub, bool live)
+  {
+    return contract(p, in[0], more[0], more[1], scratch, sub, live);
+  }
+  __device__ static cx<R> contract(const OpParams<R> &p, S *A, const S *B, const S *N, S *X, int sub, bool live)
   {
     const BaryonSpin<R> &b = p.b;
     const RankForm<R> &rk = b.rk;
     const FusedSpin f = b.fu;
     const bool unit = rank_unit_form(rk), two = rk.r == 2;
-    S *X = in[1];
     {
       cx<R> o[9];
-      rank_block(rk, unit, 0, two ? sub >> 2 : 0, in[1] + (sub & 3) * 36, 9, o);
-      __syncwarp();  // P_j has been read
+      rank_block(rk, unit, 0, two ? sub >> 2 : 0, B + (sub & 3) * 36, 9, o);
+      __syncwarp();  // B, whose place X may take, has been read
       if (two || sub < 4) {
 #pragma unroll
         for (int k = 0; k < 9; ++k) st(X + sub * 9 + k, o[k]);
@@ -167,18 +172,18 @@ struct BaryonTriRankOp : RingOp<R, S, CW, 8, NST, MINB> {
     if constexpr (sizeof(R) == 8) {
       FixedScales fs;
       S *own = X + (two ? sub : sub & 3) * 9;
-      const double2 *blk[3] = {in[0] + sub * 9, in[0] + (sub + 8) * 9, own};
+      const double2 *blk[3] = {A + sub * 9, A + (sub + 8) * 9, own};
       const bool ok = fixed_scales<8, 2>(blk, fs);
       done = __all_sync(0xffffffffu, ok || !live);
       if (done) {
-        block_to_fixed(reinterpret_cast<int4 *>(in[0] + sub * 9), blk[0], fs, 0);
-        block_to_fixed(reinterpret_cast<int4 *>(in[0] + (sub + 8) * 9), blk[1], fs, 0);
+        block_to_fixed(reinterpret_cast<int4 *>(A + sub * 9), blk[0], fs, 0);
+        block_to_fixed(reinterpret_cast<int4 *>(A + (sub + 8) * 9), blk[1], fs, 0);
         if (two || sub < 4) block_to_fixed(reinterpret_cast<int4 *>(own), own, fs, 1);
         __syncwarp();
-        const int4 *A = reinterpret_cast<const int4 *>(in[0]), *Xf = reinterpret_cast<const int4 *>(X);
+        const int4 *Af = reinterpret_cast<const int4 *>(A), *Xf = reinterpret_cast<const int4 *>(X);
         fixed_wedge_sum(k0, k1, fs, [&](int k, const int4 *&x, const int4 *&y) {
           const int i = two_bits(f.rows, 2 * k);
-          x = A + (i * 4 + s) * 9;
+          x = Af + (i * 4 + s) * 9;
           y = Xf + (r * 4 + (i ^ s1)) * 9;
           return k < turn;
         }, d);
@@ -197,7 +202,7 @@ struct BaryonTriRankOp : RingOp<R, S, CW, 8, NST, MINB> {
         }
         const int i = two_bits(f.rows, 2 * k);
         cx<R> x[9], y[9];
-        load9(x, in[0] + (i * 4 + s) * 9);
+        load9(x, A + (i * 4 + s) * 9);
         load9(y, X + (r * 4 + (i ^ s1)) * 9);
         wedge_acc(d, x, y);
       }

@@ -139,11 +139,13 @@ def per_call(api, ps, dev, form):
     if form == "gamma":
         return (api.baryon(*dev, 3, 6, 13, gamma_mn=9).cpu().numpy().reshape(V),
                 eo.baryon_two_point(*ps, 3, 6, 13, 9))
-    t, w = {"loop": (0, pp[1]), "dense": (4, wd), "rank 2": (5, pp[0]), "rank 1": (1, np.outer(wd[0], wd[1]))}[form]
+    t, w = {"loop": (0, pp[1]), "dense": (4, wd), "rank 2": (5, pp[0]), "rank 1": (1, np.outer(wd[0], wd[1])),
+            "rank 2, general": (4, np.outer(wd[0], wd[1]) + np.outer(wd[2], wd[3])),
+            "rank 1, phases": (3, np.outer([1, 0, 1j, 0], [0, 1, 0, -1]))}[form]
     return api.baryon(*dev, t, 6, 13, project_mn=w).cpu().numpy().reshape(V), eo.baryon_general_two_point(*ps, t, 6, 13, w)
 
 
-FORMS = ["loop", "gamma", "dense", "rank 1", "rank 2", "meson", "source", "sink"]
+FORMS = ["loop", "gamma", "dense", "rank 1", "rank 2", "rank 2, general", "rank 1, phases", "meson", "source", "sink"]
 
 
 @pytest.mark.parametrize("form", FORMS)
