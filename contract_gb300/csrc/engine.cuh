@@ -1,7 +1,6 @@
-// Site-tile pipeline of the field ops (diquark, sequential sources, the all-pair
-// meson field), and what every contraction kernel shares: the cut of the lattice,
-// slot layouts, chunk sums.  Contractions to numbers run on the per-warp pipelines
-// of engine_warp.cuh.
+// Site-tile pipeline of the all-pair meson field in complex64, and what every
+// contraction kernel shares: the cut of the lattice, slot layouts, chunk sums.  The
+// other contractions run on the per-warp pipelines of engine_warp.cuh.
 //
 // Work decomposition
 // ------------------
@@ -32,9 +31,7 @@
 //
 // Outputs
 // -------
-// Field ops produce a propagator-shaped site: lanes write it to a per-warp
-// shared-memory staging slot (double-buffered) and lane 0 stores it with
-// cp.async.bulk shared->global copies, or (DIRECT_OUT) the op stores it itself.
+// The op stores its site's results itself.
 #pragma once
 
 #include <type_traits>
@@ -106,30 +103,14 @@ template <class Op> struct SlotPad<Op, std::void_t<decltype(Op::SLOT_PAD)>> {
 };
 template <class Op> using OpLayout = SiteLayout<typename Op::S, SlotPad<Op>::value>;
 
-// Per-site output block of a field op: OUT_ELEMS complex values (a
-// propagator-shaped 144 for diquark/sequential, 256 for the all-gamma meson).
-template <class Op> struct OutLayout {
-  static constexpr uint32_t BYTES = Op::OUT_ELEMS * sizeof(typename Op::S);
-  static constexpr uint32_t SLOT = BYTES + 16;
-};
-
 // Shared-memory map of an engine kernel:
 //   [0, 128)        full[NST], empty[NST] mbarriers, abort flag
 //   stages          NST x NIN x SITES slots
-//   extra           SITES x EXTRA_BYTES (per-site op scratch)
-//   tail            per-warp output staging [CW][2][SPW] slots
 template <class Op> struct Smem {
   using L = OpLayout<Op>;
   static constexpr size_t STAGE = (size_t)Op::NIN * Op::SITES * L::SLOT;
   static constexpr size_t STAGES = 128;
-  static constexpr size_t EXTRA = STAGES + Op::NST * STAGE;
-  static constexpr size_t TAIL = EXTRA + (size_t)Op::EXTRA_BYTES * Op::SITES;
-  static constexpr size_t tail_bytes()
-  {
-    if constexpr (Op::DIRECT_OUT) return 0;
-    else return 2ull * Op::SITES * OutLayout<Op>::SLOT;
-  }
-  static constexpr size_t BYTES = TAIL + tail_bytes();
+  static constexpr size_t BYTES = STAGES + Op::NST * STAGE;
   static_assert(2 * Op::NST * 8 + 4 <= 128, "too many stages for the barrier block");
 };
 
@@ -137,11 +118,9 @@ template <class Op> constexpr size_t engine_smem_bytes() { return Smem<Op>::BYTE
 
 // FP32 ops ask for two CTAs per SM when their shared memory fits (228 KB per
 // SM, 1 KB reserved per CTA), which caps registers at 128 per thread; FP64 ops
-// are bound by the FP64 pipe and keep one CTA with the full register file.  An
-// op may ask for more (MIN_CTAS), trading registers for warps.
+// are bound by the FP64 pipe and keep one CTA with the full register file.
 template <class Op> constexpr int min_blocks()
 {
-  if constexpr (Op::MIN_CTAS > 0) return Op::MIN_CTAS;
   return (sizeof(typename Op::R) == 4 && 2 * (Smem<Op>::BYTES + sizeof(typename Op::Params) + 1024) <= 233472) ? 2
                                                                                                               : 1;
 }
@@ -291,9 +270,6 @@ __global__ void __launch_bounds__(Op::THREADS, min_blocks<Op>()) field_kernel(co
   const int w = warp - 1;
   const int local = lane / TPS, sub = lane % TPS;
   const int site = w * SPW + local;
-  S *scratch = reinterpret_cast<S *>(smem + Smem<Op>::EXTRA + (size_t)site * Op::EXTRA_BYTES);
-  using O = OutLayout<Op>;
-  unsigned char *outbuf = smem + Smem<Op>::TAIL + (size_t)w * 2 * SPW * O::SLOT;  // [2][SPW] slots
 
   TileIter<SITES> it;
   it.set_chunk(g, blockIdx.x);
@@ -307,7 +283,6 @@ __global__ void __launch_bounds__(Op::THREADS, min_blocks<Op>()) field_kernel(co
         *abort_flag = 1;
         report(p.status, kDevErrWaitTimeout, (unsigned int)it.chunk);
         drain<NST>(full, u, g.wait_ns);
-        bulk_wait<0>();
       }
       return;
     }
@@ -315,46 +290,20 @@ __global__ void __launch_bounds__(Op::THREADS, min_blocks<Op>()) field_kernel(co
     const S *in[NIN];
 #pragma unroll
     for (int q = 0; q < NIN; ++q) in[q] = reinterpret_cast<const S *>(sb + ((size_t)q * SITES + site) * L::SLOT);
-    if constexpr (Op::DIRECT_OUT) {
-      // The op stores its outputs itself: pass this site's destination, or
-      // nullptr past the tile's end or for a destination outside the volume.
-      S *dst = nullptr;
-      if (site < n) {
-        const long long d = Op::out_index(ps, first + site);
-        if (d >= 0 && d < g.volume) dst = Op::out_ptr(ps, d, static_cast<S *>(p.out[0]));
-        else if (sub == 0) report(p.status, kDevErrBadWork, (unsigned int)(first + site));
-      }
-      Op::site(ps, in, scratch, sub, dst);
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&empty[stage]);
-      __syncwarp();
-      it.next(g, gridDim.x);
-      continue;
+    // This site's destination, or nullptr past the tile's end or for a destination
+    // outside the volume.
+    S *dst = nullptr;
+    if (site < n) {
+      const long long d = Op::out_index(ps, first + site);
+      if (d >= 0 && d < g.volume) dst = Op::out_ptr(ps, d, static_cast<S *>(p.out[0]));
+      else if (sub == 0) report(p.status, kDevErrBadWork, (unsigned int)(first + site));
     }
-    unsigned char *ob = outbuf + (size_t)(u & 1) * SPW * O::SLOT;
-    Op::site(ps, in, scratch, sub, reinterpret_cast<S *>(ob + (size_t)local * O::SLOT));
-    fence_proxy_async_smem();
+    Op::site(ps, in, sub, dst);
     __syncwarp();
-    if (lane == 0) {
-      mbar_arrive(&empty[stage]);
-      for (int s = 0; s < SPW; ++s) {
-        if (w * SPW + s >= n) continue;
-        // Destination site (identity, or a reordering such as lexicographic):
-        // checked against the volume so a bad layout cannot store out of bounds.
-        const long long dst = Op::out_index(ps, first + w * SPW + s);
-        if (dst < 0 || dst >= g.volume) {
-          report(p.status, kDevErrBadWork, (unsigned int)(first + w * SPW + s));
-          continue;
-        }
-        bulk_s2g(static_cast<char *>(p.out[0]) + dst * O::BYTES, ob + (size_t)s * O::SLOT, O::BYTES);
-      }
-      bulk_commit();
-      bulk_wait_read<1>();  // the other staging buffer is free again
-    }
+    if (lane == 0) mbar_arrive(&empty[stage]);
     __syncwarp();
     it.next(g, gridDim.x);
   }
-  if (lane == 0) bulk_wait<0>();
 }
 
 } // namespace cgb

@@ -320,4 +320,89 @@ __global__ void __launch_bounds__(32 * Op::CW, Op::MIN_CTAS) ring_kernel(const _
   }
 }
 
+// ---------------------------------------------------------------- fields --
+// The same for ops with a propagator-shaped result per site: Op::site() leaves it in
+// the first input's slot, from where lane 0 stores it (cp.async.bulk).  A stage is
+// filled again one tile later than it was used, when its stores have been read:
+// NST - 1 tiles are in flight and no warp waits for its own stores.
+template <class Op, class Walk>
+__global__ void __launch_bounds__(32 * Op::CW, Op::MIN_CTAS)
+  field_ring_kernel(const __grid_constant__ typename Walk::Params p)
+{
+  using S = typename Op::S;
+  using L = OpLayout<Op>;
+  using M = RingSmem<Op>;
+  constexpr int NIN = Op::NIN, TPS = Op::TPS, SPW = 32 / TPS, NST = Op::NST;
+  static_assert(NST >= 2, "a stage rests for one tile");
+  constexpr uint32_t OUT = Op::OUT_ELEMS * sizeof(S);
+  static_assert(OUT <= L::SITE_BYTES, "the result takes the place of an input");
+
+  extern __shared__ __align__(128) unsigned char smem[];
+  __shared__ __align__(16) typename Op::Params ps;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  unsigned char *mine = smem + warp * M::WARP;
+  uint64_t *full = reinterpret_cast<uint64_t *>(mine);
+  if (lane == 0) {
+    for (int s = 0; s < NST; ++s) mbar_init(&full[s], 1);
+    fence_barrier_init();
+  }
+  copy_params(ps, op_params<Op>(p));
+  __syncthreads();
+
+  const int local = lane / TPS, sub = lane % TPS;
+  S *scratch = reinterpret_cast<S *>(mine + M::EXTRA + (size_t)local * Op::EXTRA_BYTES);
+  auto fetch = [&](const Walk &w, int stage) {
+    if (w.withheld(p)) return;  // test hook: this tile never arrives
+    const int n = w.sites();
+    if (lane == 0) mbar_arrive_expect_tx(&full[stage], (uint32_t)(n * NIN) * L::SITE_BYTES);
+    __syncwarp();
+    if (lane < SPW * NIN) {
+      const int q = lane / SPW, s = lane % SPW;
+      if (s < n)
+        bulk_g2s(mine + M::IN + stage * M::STAGE + ((size_t)q * SPW + s) * L::SLOT,
+                 w.in(p, q) + (w.first() + s) * L::SITE_BYTES, L::SITE_BYTES, &full[stage]);
+    }
+  };
+  static_assert(SPW * NIN <= 32, "one copy per lane");
+  Walk cur, ahead;
+  cur.start(p);
+  ahead = cur;
+  int issued = 0;
+  for (; issued < NST - 1 && ahead.valid(p); ++issued, ahead.next(p)) fetch(ahead, issued);
+  const unsigned long long wait_ns = ps.geom.wait_ns;
+  for (int u = 0; cur.valid(p); ++u) {
+    const int stage = u % NST;
+    if (!__all_sync(0xffffffffu, mbar_wait_bounded(&full[stage], (u / NST) & 1, wait_ns))) {
+      report(p.status, kDevErrWaitTimeout, (unsigned int)cur.where());
+      if (lane == 0) {  // the copies that may still be in flight
+        for (int v = u; v < issued; ++v) mbar_wait_bounded(&full[v % NST], (v / NST) & 1, wait_ns / 8);
+        bulk_wait<0>();
+      }
+      return;
+    }
+    unsigned char *sb = mine + M::IN + stage * M::STAGE;
+    S *in[NIN];
+#pragma unroll
+    for (int q = 0; q < NIN; ++q) in[q] = reinterpret_cast<S *>(sb + ((size_t)q * SPW + local) * L::SLOT);
+    const int n = cur.sites();
+    Op::site(ps, in, scratch, sub, local < n);
+    fence_proxy_async_smem();
+    __syncwarp();
+    if (lane == 0) {
+      for (int s = 0; s < n; ++s)
+        bulk_s2g(static_cast<char *>(p.out[0]) + (cur.first() + s) * OUT, sb + (size_t)s * L::SLOT, OUT);
+      bulk_commit();
+      bulk_wait_read<1>();  // the previous tile's stores have left its stage
+    }
+    __syncwarp();
+    if (ahead.valid(p)) {
+      fetch(ahead, issued % NST);
+      ++issued;
+      ahead.next(p);
+    }
+    cur.next(p);
+  }
+  if (lane == 0) bulk_wait<0>();
+}
+
 } // namespace cgb

@@ -251,30 +251,53 @@ __device__ __forceinline__ void fixed_wedge_sum(int k0, int k1, const FixedScale
   }
 }
 
-// Sums of nine integer pairs over a site's 16 threads, entry e with thread e (threads
-// 9-15 receive nothing): recursive halving of 16 slots, seven of them empty.
-__device__ __forceinline__ longlong2 group_sum_scatter9(const long long (&re)[9], const long long (&im)[9], int sub)
+// Sums of nine pairs of numbers over a site's 16 threads, entry e with thread e
+// (threads 9-15 receive nothing): recursive halving of 16 slots, seven of them empty.
+template <class V>
+__device__ __forceinline__ void group_sum_scatter9(const V (&re)[9], const V (&im)[9], int sub, V &x, V &y)
 {
-  long long a[8], b[8];
+  V a[8], b[8];
 #pragma unroll
   for (int k = 0; k < 8; ++k) {  // slots k and 8 + k: only slot 8 of the upper half is used
     const bool up = (sub & 8) != 0;
-    const long long sa = up ? re[k] : (k == 0 ? re[8] : 0), sb = up ? im[k] : (k == 0 ? im[8] : 0);
-    const long long ra = __shfl_xor_sync(0xffffffffu, sa, 8), rb = __shfl_xor_sync(0xffffffffu, sb, 8);
-    a[k] = (up ? (k == 0 ? re[8] : 0) : re[k]) + ra;
-    b[k] = (up ? (k == 0 ? im[8] : 0) : im[k]) + rb;
+    const V sa = up ? re[k] : (k == 0 ? re[8] : V(0)), sb = up ? im[k] : (k == 0 ? im[8] : V(0));
+    a[k] = (up ? (k == 0 ? re[8] : V(0)) : re[k]) + __shfl_xor_sync(0xffffffffu, sa, 8);
+    b[k] = (up ? (k == 0 ? im[8] : V(0)) : im[k]) + __shfl_xor_sync(0xffffffffu, sb, 8);
   }
 #pragma unroll
   for (int h = 4; h > 0; h >>= 1) {
     const bool up = (sub & h) != 0;
 #pragma unroll
     for (int k = 0; k < h; ++k) {
-      const long long sa = up ? a[k] : a[h + k], sb = up ? b[k] : b[h + k];
+      const V sa = up ? a[k] : a[h + k], sb = up ? b[k] : b[h + k];
       a[k] = (up ? a[h + k] : a[k]) + __shfl_xor_sync(0xffffffffu, sa, h);
       b[k] = (up ? b[h + k] : b[k]) + __shfl_xor_sync(0xffffffffu, sb, h);
     }
   }
-  return make_longlong2(a[0], b[0]);
+  x = a[0];
+  y = b[0];
+}
+
+// The wedges x ^ y of a site's 16 threads (one scale), negated where `minus`, summed:
+// entry e with thread e, in half units (16 sums of up to 2^59 leave a bit to spare).
+__device__ __forceinline__ longlong2 fixed_wedge_scatter(const int4 *x, const int4 *y, bool minus, int sub)
+{
+  long long re[9], im[9];
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    FixedWedgeRow w;
+    w.clear();
+    w.add(a, x, y);
+#pragma unroll
+    for (int e = 0; e < 3; ++e) {
+      const long long u = w.re[e].half_units(), v = w.im[e].half_units();
+      re[3 * a + e] = minus ? -u : u;
+      im[3 * a + e] = minus ? -v : v;
+    }
+  }
+  longlong2 d;
+  group_sum_scatter9(re, im, sub, d.x, d.y);
+  return d;
 }
 
 // Entry e of a wedge sum held in half units as a double.

@@ -1,42 +1,49 @@
 // Field-valued kernels: diquark and sequential sources.
-// Op template arguments: <R, S, consumer warps, threads per site, ring stages>.
+// Op template arguments: <R, S, warps, ring stages, CTAs per SM, wedges>.
 #include "launch_variants.cuh"
+#include "ops_field.cuh"
 
 namespace cgb {
 
-template <class R, class S, int CW, int TPS, int NST>
-static cudaError_t seq_dispatch(const Job &job, bool loop, int role, const OpParams<R> &p)
+template <class R, class S, int CW, int NST, int MINB, Wedges KIND>
+static cudaError_t wedges(const Job &job, OpParams<R> p)
 {
-  if (loop) {
-    switch (role) {
-    case 0: return run_field<SequentialOp<R, S, CW, TPS, NST, true, 0>>(job, p);
-    case 1: return run_field<SequentialOp<R, S, CW, TPS, NST, true, 1>>(job, p);
-    default: return run_field<SequentialOp<R, S, CW, TPS, NST, true, 2>>(job, p);
-    }
-  }
-  switch (role) {
-  case 0: return run_field<SequentialOp<R, S, CW, TPS, NST, false, 0>>(job, p);
-  case 1: return run_field<SequentialOp<R, S, CW, TPS, NST, false, 1>>(job, p);
-  default: return run_field<SequentialOp<R, S, CW, TPS, NST, false, 2>>(job, p);
-  }
+  fill_wedges(p, KIND);
+  return run_field_ring<WedgeFieldOp<R, S, CW, NST, MINB, KIND>>(job, p);
 }
 
-// complex64 variants: the two-CTA shapes keep more tiles (and stores) in flight;
-// the default (last field) is the tuner's choice at 24^3 x 64.
-static const VariantSet<float, 6> kDiquarkM = {
-  {run_field<DiquarkOp<float, float2, 6, 16, 2>>, run_field<DiquarkOp<float, float2, 8, 16, 3>>,
-   run_field<DiquarkOp<float, float2, 6, 16, 2, true>>, run_field<DiquarkOp<float, float2, 8, 16, 3, true>>,
-   run_field<DiquarkOp<float, float2, 4, 16, 2, true>>, run_field<DiquarkOp<float, float2, 3, 16, 3, true>>},
-  {"cw6.tps16.st2", "cw8.tps16.st3", "cw6.tps16.st2.direct", "cw8.tps16.st3.direct", "cw4.tps16.st2.direct",
-   "cw3.tps16.st3.direct"},
-  5};
+// complex64: HBM bound; tiles in flight against warps.  32^3 x 48, ms in this order:
+// diquark 0.911, 0.950, 0.918, 1.07, four-wedge sequential sources 0.90 to 0.92,
+// 0.93 to 0.94, 0.90 to 0.92, 1.05, loop ones 0.83 to 0.84, 0.87 to 0.90, 0.83 to 0.85,
+// 0.87 to 0.90 (a CTA-wide ring with a producer warp: 1.00, 1.24, 0.86); the three
+// fields take 0.814 at the copy rate.
+template <Wedges KIND> static VariantSet<float, 4> shapes_m()
+{
+  return {{wedges<float, float2, 4, 2, 5, KIND>, wedges<float, float2, 4, 3, 4, KIND>, wedges<float, float2, 4, 2, 6, KIND>,
+           wedges<float, float2, 4, 4, 3, KIND>},
+          {"w4.st2.occ5", "w4.st3.occ4", "w4.st2.occ6", "w4.st4.occ3"},
+          0};
+}
+// complex128: integer pipe.  24^4, ms in this order: four wedges a block 1.76 to 1.80,
+// 1.85 to 1.87, 1.83 to 1.86 (5.2 to 5.7 in FP64), the closed loop 0.80, 0.88, 0.85
+// (2.29), one wedge a block 1.25, 0.86, 0.86 (1.44).
+template <Wedges KIND> static VariantSet<double, 3> shapes_p()
+{
+  return {{wedges<double, double2, 4, 3, 2, KIND>, wedges<double, double2, 4, 2, 3, KIND>,
+           wedges<double, double2, 4, 2, 2, KIND>},
+          {"w4.st3.occ2", "w4.st2.occ3", "w4.st2.occ2"},
+          KIND == Wedges::LoopA || KIND == Wedges::LoopB ? 1 : 0};
+}
 
-// complex128 (FP64-pipe bound): the first shape is the default.
-static const VariantSet<double, 3> kDiquarkP = {
-  {run_field<DiquarkOp<double, double2, 4, 16, 3>>, run_field<DiquarkOp<double, double2, 3, 16, 2>>,
-   run_field<DiquarkOp<double, double2, 2, 16, 3>>},
-  {"cw4.tps16.st3", "cw3.tps16.st2", "cw2.tps16.st3"},
-  0};
+static const VariantSet<float, 4> kDiquarkM = shapes_m<Wedges::Diquark>();
+static const VariantSet<double, 3> kDiquarkP = shapes_p<Wedges::Diquark>();
+// [loop][role]
+static const VariantSet<float, 4> kSequentialM[2][3] = {
+  {shapes_m<Wedges::TriA>(), shapes_m<Wedges::TriB>(), shapes_m<Wedges::TriN>()},
+  {shapes_m<Wedges::LoopA>(), shapes_m<Wedges::LoopB>(), shapes_m<Wedges::LoopN>()}};
+static const VariantSet<double, 3> kSequentialP[2][3] = {
+  {shapes_p<Wedges::TriA>(), shapes_p<Wedges::TriB>(), shapes_p<Wedges::TriN>()},
+  {shapes_p<Wedges::LoopA>(), shapes_p<Wedges::LoopB>(), shapes_p<Wedges::LoopN>()}};
 
 cudaError_t launch_diquark(const Job &job, const OpParams<double> &p)
 {
@@ -46,30 +53,14 @@ cudaError_t launch_diquark(const Job &job, const OpParams<double> &p)
 
 cudaError_t launch_sequential(const Job &job, bool loop, int role, const OpParams<double> &p)
 {
-  if (job.prec == Prec::C128) {  // default (no variant chosen): three consumer warps, two stages
-    if (job.variant == 0) return seq_dispatch<double, double2, 4, 16, 3>(job, loop, role, p);
-    if (job.variant == 2) return seq_dispatch<double, double2, 2, 16, 3>(job, loop, role, p);
-    return seq_dispatch<double, double2, 3, 16, 2>(job, loop, role, p);
-  }
-  const OpParams<float> q = convert_params<float>(p);
-  if (job.variant == 1) return seq_dispatch<float, float2, 8, 16, 3>(job, loop, role, q);
-  if (job.variant == 2) return seq_dispatch<float, float2, 3, 16, 3>(job, loop, role, q);
-  return seq_dispatch<float, float2, 5, 16, 2>(job, loop, role, q);
+  if (job.prec == Prec::C128) return kSequentialP[loop][role].launch(job, p);
+  return kSequentialM[loop][role].launch(job, convert_params<float>(p));
 }
-
-static const char *const kSequentialNames[3] = {"cw5.tps16.st2", "cw8.tps16.st3", "cw3.tps16.st3"};
-static const char *const kSequentialNamesP[3] = {"cw4.tps16.st3", "cw3.tps16.st2", "cw2.tps16.st3"};
 
 int field_variants(Prec prec, bool sequential, const char *const **names)
 {
-  if (prec == Prec::C128) {
-    if (!sequential) return kDiquarkP.describe(names);
-    if (names) *names = kSequentialNamesP;
-    return 3;
-  }
-  if (!sequential) return kDiquarkM.describe(names);
-  if (names) *names = kSequentialNames;
-  return 3;
+  if (prec == Prec::C128) return (sequential ? kSequentialP[0][0] : kDiquarkP).describe(names);
+  return (sequential ? kSequentialM[0][0] : kDiquarkM).describe(names);
 }
 
 } // namespace cgb

@@ -126,6 +126,17 @@ template <class Op> cudaError_t run_ring_field(const Job &job, OpParams<typename
   return run_ring<Op>(j, p);
 }
 
+// One launch of an op of the field ring kernel.
+template <class Op> cudaError_t run_field_ring(const Job &job, const OpParams<typename Op::R> &p)
+{
+  if (job.volume == 0) return cudaSuccess;
+  Job j = job;
+  j.per_site = true;
+  constexpr size_t smem = RingSmem<Op>::BYTES;
+  static_assert(smem <= 232448, "op does not fit in shared memory");
+  return launch_chunks<Op>(j, p, field_ring_kernel<Op, ChunkWalk<Op>>, smem);
+}
+
 template <class Op> cudaError_t run_field(const Job &job, OpParams<typename Op::R> p)
 {
   if (job.volume == 0) return cudaSuccess;

@@ -426,11 +426,6 @@ template <class R_, class S_, int CW_, int TPS_, int NST_> struct OpBase {
   static constexpr int CW = CW_, TPS = TPS_, NST = NST_;
   static constexpr int SITES = CW_ * (32 / TPS_);
   static constexpr int THREADS = 32 * (CW_ + 1);
-  // Field ops: true when site() stores its outputs to global memory itself
-  // (the engine then passes the destination, or nullptr for a site to skip).
-  static constexpr bool DIRECT_OUT = false;
-  // Resident CTAs per SM that the launch bounds ask for (0: the engine's rule).
-  static constexpr int MIN_CTAS = 0;
   static_assert(32 % TPS_ == 0, "a site's threads must sit in one warp");
 };
 
@@ -458,179 +453,6 @@ template <> __device__ __forceinline__ cx<float> conj_dot9<float>(const cx<float
   }
   return {A.x + B.y, B.x - A.y};
 }
-
-// ----------------------------------------------------------- field ops --
-// Diquark (include/diquark.cuh:33-57):
-//   D[m][l][ad] = g5[m] g5[l] conj( c2(l) sum_i c1(i) (P_i[i][perm2 l] ^ P_j[perm1 i][m])[ad] )
-// with c1 from Gamma_ij, c2 from Gamma_kl^T.  Thread handles 16/TPS blocks (m, l).
-template <class R, class S, int CW, int TPS, int NST, bool DIRECT = false>
-struct DiquarkOp : OpBase<R, S, CW, TPS, NST> {
-  static constexpr int NIN = 2, EXTRA_BYTES = 0, OUT_ELEMS = 144;
-  // DIRECT: each thread stores its blocks straight to HBM (72 contiguous bytes
-  // a block) instead of staging the site in shared memory for a bulk store.
-  static constexpr bool DIRECT_OUT = DIRECT;
-  __device__ static long long out_index(const OpParams<R> &, long long site) { return site; }
-  __device__ static S *out_ptr(const OpParams<R> &, long long d, S *base) { return base + d * OUT_ELEMS; }
-  __device__ static void site(const OpParams<R> &p, const S *const *in, S *, int sub, S *out)
-  {
-    const BaryonSpin<R> &b = p.b;
-    if (!out) return;  // a site past the end of the tile (no cross-thread work below)
-    for (int blk = sub; blk < 16; blk += TPS) {
-      const int m = blk / 4, l = blk % 4, k = b.perm2[l];
-      cx<R> d[9];
-#pragma unroll
-      for (int e = 0; e < 9; ++e) d[e] = czero<R>();
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        cx<R> x[9], y[9];
-        load9(x, in[0] + (i * 4 + k) * 9);
-        load9(y, in[1] + (b.perm1[i] * 4 + m) * 9);
-        phase9(x, b.ph1[0][i]);
-        wedge_acc(d, x, y);
-      }
-      // g5[m] g5[l] = -1 when exactly one of m, l is a lower spin component.
-      const uint32_t sgn = ((m >> 1) ^ (l >> 1)) & 1u;
-      const uint32_t p2 = b.ph2[0][l];
-#pragma unroll
-      for (int e = 0; e < 9; ++e) {
-        cx<R> v = conj(mul_phase(d[e], p2));
-        v.x = flip_sign(v.x, sgn);
-        v.y = flip_sign(v.y, sgn);
-        st(out + blk * 9 + e, v);
-      }
-    }
-  }
-};
-
-// Sequential source: the slot's propagator is overwritten with dC/dP_slot
-// (include/baryon_sequential.cuh:36-163).  With the canonical forms above,
-// A/B/N denote the roles; `role` is which one is differentiated.  Inputs are
-// the two other roles in (A, B, N) order.  W is always a Gamma matrix here.
-//   loop, d/dA[i][perm2 l] = c1 c2 (B[perm1 i][l] ^ Q)
-//   loop, d/dB[perm1 i][l] = c1 c2 (A[i][perm2 l] ^ Q)
-//   loop, d/dN[perm(m)][m] = W[m][perm m] * sum_{i,l} c1 c2 (A ^ B)
-//   tri,  d/dA[i][perm2 l] = c1 c2 sum_m B[perm1 i][m] ^ N'[m][l]
-//   tri,  d/dB[perm1 i][m] = c1 sum_l c2 (A[i][perm2 l] ^ N'[m][l])
-//   tri,  d/dN[perm(m)][l] = W[m][perm m] sum_i c1 c2 (A[i][perm2 l] ^ B[perm1 i][m])
-template <class R, class S, int CW, int TPS, int NST, bool LOOP, int ROLE>
-struct SequentialOp : OpBase<R, S, CW, TPS, NST> {
-  static constexpr int NIN = 2, EXTRA_BYTES = cbytes<S>(144) + 16, OUT_ELEMS = 144;
-  __device__ static long long out_index(const OpParams<R> &, long long site) { return site; }
-  __device__ static S *out_ptr(const OpParams<R> &, long long d, S *base) { return base + d * OUT_ELEMS; }
-
-  __device__ static void site(const OpParams<R> &p, const S *const *in, S *scratch, int sub, S *out)
-  {
-    const BaryonSpin<R> &b = p.b;
-    const ProjOperand<R> &pw = b.proj[0];
-    const S *A = ROLE == 0 ? nullptr : in[0];
-    const S *B = ROLE == 1 ? nullptr : (ROLE == 0 ? in[0] : in[1]);
-    const S *N = ROLE == 2 ? nullptr : in[1];
-    if constexpr (LOOP && ROLE != 2) {
-      build_q<R, S, TPS, 1>(b, N, scratch, sub);
-      __syncwarp();
-    }
-    if constexpr (!LOOP && ROLE != 2) {
-      build_nprime<R, S, TPS, 1>(b, N, scratch, sub);
-      __syncwarp();
-    }
-    if constexpr (LOOP && ROLE == 2) {
-      // R = sum_{i,l} c1 c2 (A ^ B): each thread its (i, l) share, then a group sum.
-      using Ln = Lanes<TPS>;
-      const int i = sub / Ln::TPI, l0 = (sub % Ln::TPI) * Ln::LPT, j = b.perm1[i];
-      cx<R> r[9];
-#pragma unroll
-      for (int e = 0; e < 9; ++e) r[e] = czero<R>();
-#pragma unroll
-      for (int lo = 0; lo < Ln::LPT; ++lo) {
-        const int l = l0 + lo;
-        cx<R> x[9], y[9];
-        load9(x, A + (i * 4 + b.perm2[l]) * 9);
-        load9(y, B + (j * 4 + l) * 9);
-        phase9(x, (b.ph1[0][i] + b.ph2[0][l]) & 3u);
-        wedge_acc(r, x, y);
-      }
-#pragma unroll
-      for (int e = 0; e < 9; ++e) r[e] = group_sum<TPS>(r[e]);
-      // out[n][m] = W[m][n] R for n = perm(m); every other block is zero.
-      for (int blk = sub; blk < 16; blk += TPS) {
-        const int n = blk / 4, m = blk % 4;
-        const bool hit = pw.perm[m] == n;
-        if (!out) continue;  // a site past the end of the tile
-#pragma unroll
-        for (int e = 0; e < 9; ++e) st(out + blk * 9 + e, hit ? mul_phase(r[e], pw.ph[m]) : czero<R>());
-      }
-    } else {
-      field_blocks(b, pw, A, B, scratch, sub, out);
-    }
-  }
-
-  __device__ static void field_blocks(const BaryonSpin<R> &b, const ProjOperand<R> &pw, const S *A, const S *B,
-                                      const S *scratch, int sub, S *out)
-  {
-    if (!out) return;  // a site past the end of the tile (no cross-thread work below)
-    for (int blk = sub; blk < 16; blk += TPS) {
-      cx<R> d[9];
-#pragma unroll
-      for (int e = 0; e < 9; ++e) d[e] = czero<R>();
-      int dst;
-      if constexpr (LOOP) {
-        cx<R> q[9];
-        load9(q, scratch);
-        if constexpr (ROLE == 0) {  // block (i, k), k = perm2 l
-          const int i = blk / 4, k = blk % 4, l = b.perm2[k], j = b.perm1[i];
-          cx<R> y[9];
-          load9(y, B + (j * 4 + l) * 9);
-          phase9(y, (b.ph1[0][i] + b.ph2[0][l]) & 3u);
-          wedge_acc(d, y, q);
-        } else {  // block (j, l), i = perm1 j
-          const int j = blk / 4, l = blk % 4, i = b.perm1[j];
-          cx<R> x[9];
-          load9(x, A + (i * 4 + b.perm2[l]) * 9);
-          phase9(x, (b.ph1[0][i] + b.ph2[0][l]) & 3u);
-          wedge_acc(d, x, q);
-        }
-        dst = blk;
-      } else if constexpr (ROLE == 0) {  // block (i, k)
-        const int i = blk / 4, k = blk % 4, l = b.perm2[k], j = b.perm1[i];
-#pragma unroll
-        for (int m = 0; m < 4; ++m) {
-          cx<R> y[9], nn[9];
-          load9(y, B + (j * 4 + m) * 9);
-          load9(nn, scratch + (m * 4 + l) * 9);
-          wedge_acc(d, y, nn);
-        }
-        phase9(d, (b.ph1[0][i] + b.ph2[0][l]) & 3u);
-        dst = blk;
-      } else if constexpr (ROLE == 1) {  // block (j, m), i = perm1 j
-        const int j = blk / 4, m = blk % 4, i = b.perm1[j];
-#pragma unroll
-        for (int l = 0; l < 4; ++l) {
-          cx<R> x[9], nn[9];
-          load9(x, A + (i * 4 + b.perm2[l]) * 9);
-          phase9(x, b.ph2[0][l]);
-          load9(nn, scratch + (m * 4 + l) * 9);
-          wedge_acc(d, x, nn);
-        }
-        phase9(d, b.ph1[0][i]);
-        dst = blk;
-      } else {  // ROLE 2, triangle: block (n, l), n = perm(m)
-        const int n = blk / 4, l = blk % 4, m = pw.perm[n];  // perm is an involution
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          cx<R> x[9], y[9];
-          load9(x, A + (i * 4 + b.perm2[l]) * 9);
-          load9(y, B + (b.perm1[i] * 4 + m) * 9);
-          phase9(x, b.ph1[0][i]);
-          wedge_acc(d, x, y);
-        }
-        phase9(d, (b.ph2[0][l] + pw.ph[m]) & 3u);
-        dst = blk;
-      }
-#pragma unroll
-      for (int e = 0; e < 9; ++e) st(out + dst * 9 + e, d[e]);
-    }
-  }
-};
 
 // All 16 x 16 meson gamma pairs per site, C[a][b] = meson_two_point(Gamma_a, Gamma_b)
 // (include/meson.cuh:33-50 for every pair), written as a 256-entry block per
@@ -705,11 +527,8 @@ __device__ __forceinline__ void conj_products_f32x2(cx<float> (&T)[NK][NL], cons
 // once from its sums (pair_from_products in kernels_momentum.cu).
 template <class R, class S, int CW, int NST, bool SPLIT = false, bool PRODUCTS = false>
 struct MesonAllGammaOp : OpBase<R, S, CW, 16, NST> {
-  static constexpr int NIN = 2, EXTRA_BYTES = 0, OUT_ELEMS = 256;
+  static constexpr int NIN = 2, OUT_ELEMS = 256;
   static_assert(sizeof(R) == 4, "complex128: MesonPairsOp (ops_site.cuh)");
-  // Each thread's 16 outputs are four 32-byte runs: stored straight to HBM.
-  static constexpr bool DIRECT_OUT = true;
-
   __device__ static long long sites_per_slice(const OpParams<R> &p)
   {
     return (long long)p.latt[0] * p.latt[1] * p.latt[2];
@@ -729,7 +548,7 @@ struct MesonAllGammaOp : OpBase<R, S, CW, 16, NST> {
 
   __device__ static long long out_index(const OpParams<R> &p, long long site) { return lexicographic(p, site); }
 
-  __device__ static void site(const OpParams<R> &ps_, const S *const *in, S *, int sub, S *out)
+  __device__ static void site(const OpParams<R> &ps_, const S *const *in, int sub, S *out)
   {
     constexpr GammaTables G = build_gamma_tables();
     constexpr ClassWalsh CW8 = class_walsh();

@@ -42,21 +42,7 @@ struct BaryonLoopOp : RingOp<R, S, CW, TPS, NST, MINB> {
         // Gamma entries: one common power of i, and signs
         const uint32_t common = (b.ph1[0][0] & 1u) + (b.ph2[0][0] & 1u);
         const bool minus = ((b.ph1[0][i] ^ b.ph2[0][l]) & 2u) != 0;
-        long long re[9], im[9];
-#pragma unroll
-        for (int a = 0; a < 3; ++a) {
-          FixedWedgeRow w;
-          w.clear();
-          w.add(a, x, y);
-#pragma unroll
-          for (int e = 0; e < 3; ++e) {
-            // 16 sums of up to 2^59: half units leave a bit to spare
-            const long long u = w.re[e].half_units(), v = w.im[e].half_units();
-            re[3 * a + e] = minus ? -u : u;
-            im[3 * a + e] = minus ? -v : v;
-          }
-        }
-        const longlong2 d = group_sum_scatter9(re, im, sub);
+        const longlong2 d = fixed_wedge_scatter(x, y, minus, sub);
         cx<double> v = czero<double>();
         if (sub < 9) {
           const cx<double> z = fixed_entry(d, sub, fs);

@@ -175,6 +175,70 @@ def test_per_call_not_finite(api, form):
             close(got[..., keep], ref[..., keep], "gauss")
 
 
+def field_call(ps, dev, form):
+    """(result, oracle) of a propagator-shaped call."""
+    from contract_gb300 import pycontract as pc
+    if form == "diquark":
+        return pc.baryonDiquark(dev[0], dev[1], 6, 13).cpu().numpy().reshape(-1, 144), eo.baryon_diquark(ps[0], ps[1], 6, 13)
+    t, slot = form
+    d = [x.clone() for x in dev]
+    pc.baryonSequentialTwoPoint(*d, t, slot, 6, 13, 9)
+    for k in range(3):
+        assert k == slot or (d[k] == dev[k]).all() or not np.isfinite(ps[k]).all()
+    return d[slot].cpu().numpy().reshape(-1, 144), eo.baryon_sequential(*ps, t, slot, 6, 13, 9)
+
+
+FIELD_FORMS = ["diquark"] + [(t, slot) for t in (0, 2, 1, 5) for slot in range(3)]
+
+
+@pytest.mark.parametrize("form", FIELD_FORMS)
+@pytest.mark.parametrize("kind", KINDS)
+def test_fields(api, form, kind):
+    ps, dev = fields(kind)
+    got, ref = field_call(ps, dev, form)
+    ref = np.asarray(ref).reshape(-1, 144)
+    if kind == "mixed sites":  # in units of each site's own values
+        used = [p for k, p in enumerate(ps) if (k < 2 if form == "diquark" else k != form[1])]
+        unit = np.prod([np.abs(p).max(axis=(1, 2, 3, 4)) for p in used], axis=0)[:, None]
+        got, ref, kind = got / unit, ref / unit, "gauss"
+    close(got, ref, kind)
+
+
+@pytest.mark.parametrize("form", FIELD_FORMS)
+def test_fields_not_finite(api, form):
+    ps, dev = fields("gauss")
+    ref = np.asarray(field_call(ps, dev, form)[1]).reshape(-1, 144)
+    keep = np.arange(V) != 7
+    for field in range(2 if form == "diquark" else 3):
+        if form != "diquark" and field == form[1]:
+            continue
+        p = ps[field].copy()
+        p[7] = np.nan
+        d = list(dev)
+        d[field] = __import__("torch").from_numpy(p).cuda()
+        got = field_call([p if k == field else q for k, q in enumerate(ps)], d, form)[0]
+        bad = ~np.isfinite(got[7])
+        assert bad.all() or (form in ((0, 2), (2, 2)) and bad.sum() == 36)  # four blocks, the others are zero
+        close(got[keep], ref[keep], "gauss")
+
+
+@pytest.mark.parametrize("volume", [1, 2, 3, 31, 1217])
+@pytest.mark.parametrize("dtype", ["complex64", "complex128"])
+def test_field_edges(api, volume, dtype):
+    """One live site in a warp, fewer tiles than warps, stages used once and again."""
+    import torch
+    rng = np.random.default_rng(volume)
+    tol = 2e-15 if dtype == "complex128" else 1e-6
+    ps = [(rng.standard_normal((volume, 4, 4, 3, 3)) + 1j * rng.standard_normal((volume, 4, 4, 3, 3))).astype(dtype)
+          for _ in range(3)]
+    dev = [torch.from_numpy(p).cuda() for p in ps]
+    ps = [p.astype(np.complex128) for p in ps]
+    for form in FIELD_FORMS:
+        got, ref = field_call(ps, dev, form)
+        ref = np.asarray(ref).reshape(-1, 144)
+        assert norm(got - ref) <= tol * norm(ref), form
+
+
 @pytest.mark.parametrize("latt", [(2, 1, 1, 1), (2, 1, 1, 3), (6, 3, 1, 5), (10, 3, 3, 2)])
 @pytest.mark.parametrize("dtype", ["complex64", "complex128"])
 def test_per_call_edges(api, latt, dtype):
