@@ -32,7 +32,7 @@ SOURCES = [
     "kernels_momentum.cu",
     "kernels_momentum_tc.cu",
     "kernels_momentum_fused.cu",
-    "kernels_momentum_rows.cu",
+    "kernels_momentum_rows.cu", "kernels_momentum_c128.cu",
     "kernels_batch.cu",
     "noalloc.cu",
     "kernels_quda.cu",

@@ -182,8 +182,6 @@ __global__ void __launch_bounds__(32 * Op::CW, Op::MIN_CTAS) warp_kernel(const _
 // The same for ops of one step: a warp has an NST-stage ring of whole tiles, and
 // Op::site() yields the site's value -- the sum over its threads is one output
 // (NOUT == 1), or with NOUT > 1 thread sub holds output Op::output(p, sub) complete.
-// NOUT == 0: a field op, site() stores its results at `dst` itself (nullptr: nothing
-// to store).
 template <class Op> struct RingSmem {
   using L = OpLayout<Op>;
   static constexpr int SPW = 32 / Op::TPS;
@@ -253,16 +251,7 @@ __global__ void __launch_bounds__(32 * Op::CW, Op::MIN_CTAS) ring_kernel(const _
       in[q] = reinterpret_cast<S *>(mine + M::IN + stage * M::STAGE + ((size_t)q * SPW + local) * L::SLOT);
     const bool ok = local < cur.sites();
     cx<R> v;
-    if constexpr (NOUT == 0) {
-      S *dst = nullptr;
-      if (ok) {
-        // checked against the volume, so that a bad layout cannot store out of bounds
-        const long long d = Op::out_index(ps, cur.first() + local);
-        if (d >= 0 && d < ps.geom.volume) dst = static_cast<S *>(p.out[0]) + d * Op::OUT_ELEMS;
-        else if (sub == 0) report(p.status, kDevErrBadWork, (unsigned int)(cur.first() + local));
-      }
-      Op::site(ps, in, scratch, sub, ok, dst);
-    } else if constexpr (Op::DIRECT > 0) {  // fields NIN and on are read from memory by the op
+    if constexpr (Op::DIRECT > 0) {  // fields NIN and on are read from memory by the op
       const long long at = (cur.first() + (ok ? local : 0)) * L::SITE_BYTES;
       const S *more[Op::DIRECT];
 #pragma unroll
@@ -297,7 +286,7 @@ __global__ void __launch_bounds__(32 * Op::CW, Op::MIN_CTAS) ring_kernel(const _
           chunk_part = {};
         }
       }
-    } else if constexpr (NOUT > 1) {
+    } else {
       static_assert(NOUT == TPS, "one output per thread of a site");
       if (ps.geom.per_site) {
         if (ok)

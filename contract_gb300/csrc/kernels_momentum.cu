@@ -5,14 +5,14 @@
 // The phase factorises over x, y and z, so instead of one dense
 // [momenta x V3] x [V3 x 256] product per timeslice (8 M N K flop) the
 // projection runs as three short transforms:
-//   1. MesonPairsOp (complex128) or MesonAllGammaOp: C_ab(x) for all 256 pairs,
-//      written in lexicographic site order
+//   1. MesonAllGammaOp: C_ab(x) for all 256 pairs, written in lexicographic site
+//      order
 //   2. plane_kernel: per (t, z) plane, X then Y transform of every C_ab into
-//      H[(nx, ny)][ab], in the form's arithmetic (FP64 planes for complex128,
-//      FP32 planes for the mixed form)
+//      H[(nx, ny)][ab]
 //   3. momentum_finalize: Z transform and the sum over planes, returned in FP64.
-// The mixed form normally fuses 1 and 2 (kernels_momentum_rows.cu), so the
-// per-site values never reach HBM.
+// That is the mixed form's alternative with FP32 planes: normally it fuses 1 and 2
+// (kernels_momentum_rows.cu).  Complex128 has FP64 planes and fuses 1 with the X
+// transform (kernels_momentum_c128.cu).  No per-site value of either reaches HBM.
 // For 32^3 x 64 and 125 momenta that is ~25 GFLOP instead of 537 GFLOP.
 // Phase tables exp(2 pi i k / L) are computed in FP64 on the host from the
 // exact integer index k = (n * x) mod L.
@@ -21,12 +21,8 @@
 
 #include "launch_variants.cuh"
 #include "momentum.hpp"
-#include "ops_site.cuh"
 
 namespace cgb {
-
-template <class R> struct Vec2 { using type = double2; };
-template <> struct Vec2<float> { using type = float2; };
 
 using MesonAllGammaM = MesonAllGammaOp<float, float2, 8, 2>;
 // field of the tensor-core path: the spin-colour products, pair halves apart
@@ -36,72 +32,69 @@ using MesonProductsSplitM = MesonAllGammaOp<float, float2, 8, 2, true, true>;
 // Lx - x have the same cosine and opposite sines, rows y and Ly - y too: their sum
 // and difference make one term of C = sum cos * v and of S = sum sin * v (+k: C + iS,
 // -k: C - iS), half the FMAs of the sites one by one, and the k = 0 transform is a
-// plain sum.  Bound by the FP64 pipe in complex128 (89 % busy): for three X and 15 Y
-// groups 7 instructions a site and pair for X (12 site by site) and 40 / Lx for Y
-// (100 / Lx); 0.83 ms at 18 x 15 x 20 x 28, 125 momenta.
-// Each thread's X sums of a row or of a pair of rows go through its own column of
-// shared memory, so that the Y step finds G[nx] with one load.
-template <class R> constexpr size_t plane_smem_bytes(int npx) { return (size_t)2 * npx * 256 * 2 * sizeof(R); }
+// plain sum.  Each thread's X sums of a row or of a pair of rows go through its own
+// column of shared memory, so that the Y step finds G[nx] with one load.
+constexpr size_t plane_smem_bytes(int npx) { return (size_t)2 * npx * 256 * sizeof(float2); }
 
-template <class R, class S, int NG, int YC>
-__global__ void __launch_bounds__(256) plane_kernel(const S *__restrict__ c, typename Vec2<R>::type *__restrict__ planes,
+template <int NG, int YC>
+__global__ void __launch_bounds__(256) plane_kernel(const float2 *__restrict__ c, float2 *__restrict__ planes,
                                                     const __grid_constant__ MomPlan plan)
 {
   const int z = blockIdx.x, t = blockIdx.y, y0 = blockIdx.z * YC, g = threadIdx.x;
   const int lx = plan.latt[0], ly = plan.latt[1], lz = plan.latt[2], npx = plan.npx;
   const int ny = min(YC, plan.nyg - y0);
-  __shared__ R phx[NG][kMomMaxL / 2 + 1][2];
-  __shared__ R phy[YC][kMomMaxL / 2 + 1][2];
+  __shared__ float phx[NG][kMomMaxL / 2 + 1][2];
+  __shared__ float phy[YC][kMomMaxL / 2 + 1][2];
   __shared__ int ygx[YC];
   extern __shared__ __align__(16) unsigned char plane_dyn[];
   // [2][npx][256]: G of a row and its partner, then their sum and difference
-  cx<R> *gp = reinterpret_cast<cx<R> *>(plane_dyn) + g, *gm = gp + npx * 256;
+  cx<float> *gp = reinterpret_cast<cx<float> *>(plane_dyn) + g, *gm = gp + npx * 256;
   if (g < YC) ygx[g] = g < ny ? plan.yg_ix[y0 + g] : 0;
   for (int e = g; e < NG * (lx / 2 + 1); e += blockDim.x) {  // per X group: cos, sin of 2 pi k x / Lx
     const int gi = e / (lx / 2 + 1), x = e % (lx / 2 + 1);
     const int k = (plan.gx_k[gi] * x) % lx;
-    phx[gi][x][0] = R(plan.cosx[k]);
-    phx[gi][x][1] = R(plan.sinx[k]);
+    phx[gi][x][0] = float(plan.cosx[k]);
+    phx[gi][x][1] = float(plan.sinx[k]);
   }
   for (int e = g; e < YC * (ly / 2 + 1); e += blockDim.x) {
     const int q = e / (ly / 2 + 1), y = e % (ly / 2 + 1);
     const int k = q < ny ? (plan.yg_k[y0 + q] * y) % ly : 0;
-    phy[q][y][0] = q < ny ? R(plan.cosy[k]) : R(0);
-    phy[q][y][1] = q < ny ? R(plan.siny[k]) : R(0);
+    phy[q][y][0] = q < ny ? float(plan.cosy[k]) : float(0);
+    phy[q][y][1] = q < ny ? float(plan.siny[k]) : float(0);
   }
   __syncthreads();
   const bool zero = plan.gx_k[0] == 0;  // the k = 0 group, if there is one, is the first
-  cx<R> hc[YC], hs[YC];
+  cx<float> hc[YC], hs[YC];
 #pragma unroll
-  for (int q = 0; q < YC; ++q) hc[q] = hs[q] = czero<R>();
-  const S *plane = c + ((size_t)(t * lz + z) * ly * lx) * 256 + g;
+  for (int q = 0; q < YC; ++q) hc[q] = hs[q] = czero<float>();
+  const float2 *plane = c + ((size_t)(t * lz + z) * ly * lx) * 256 + g;
   constexpr int XB = 4;  // pairs of loads in flight per thread
   for (int y = 0; y <= ly / 2; ++y) {
     const bool alone = y == 0 || 2 * y == ly;
     for (int half = 0; half < (alone ? 1 : 2); ++half) {
-      cx<R> gc[NG], gs[NG];
+      cx<float> gc[NG], gs[NG];
 #pragma unroll
-      for (int gi = 0; gi < NG; ++gi) gc[gi] = gs[gi] = czero<R>();
-      const S *row = plane + (size_t)(half ? ly - y : y) * lx * 256;
+      for (int gi = 0; gi < NG; ++gi) gc[gi] = gs[gi] = czero<float>();
+      const float2 *row = plane + (size_t)(half ? ly - y : y) * lx * 256;
       for (int x0 = 0; x0 <= lx / 2; x0 += XB) {
-        cx<R> v[XB], w[XB];
+        cx<float> v[XB], w[XB];
 #pragma unroll
         for (int u = 0; u < XB; ++u) {
           const int x = x0 + u;
-          v[u] = x <= lx / 2 ? ld<R>(row + (size_t)x * 256) : czero<R>();
-          w[u] = x > 0 && 2 * x < lx ? ld<R>(row + (size_t)(lx - x) * 256) : czero<R>();
+          v[u] = x <= lx / 2 ? ld<float>(row + (size_t)x * 256) : czero<float>();
+          w[u] = x > 0 && 2 * x < lx ? ld<float>(row + (size_t)(lx - x) * 256) : czero<float>();
         }
 #pragma unroll
         for (int u = 0; u < XB; ++u) {
           if (x0 + u > lx / 2) break;
-          const cx<R> a = cadd(v[u], w[u]), d = {v[u].x - w[u].x, v[u].y - w[u].y};
+          const cx<float> a = cadd(v[u], w[u]), d = {v[u].x - w[u].x, v[u].y - w[u].y};
 #pragma unroll
           for (int gi = 0; gi < NG; ++gi) {
             if (gi == 0 && zero) {
               gc[0] = cadd(gc[0], a);
               continue;
             }
-            const R cs = phx[gi][x0 + u][0], sn = phx[gi][x0 + u][1];
+            const float cs = phx[gi][x0 + u][0], sn = phx[gi][x0 + u][1];
             gc[gi].x = fma(cs, a.x, gc[gi].x);
             gc[gi].y = fma(cs, a.y, gc[gi].y);
             gs[gi].x = fma(sn, d.x, gs[gi].x);
@@ -109,11 +102,11 @@ __global__ void __launch_bounds__(256) plane_kernel(const S *__restrict__ c, typ
           }
         }
       }
-      auto put = [&](int ix, cx<R> v) {
+      auto put = [&](int ix, cx<float> v) {
         if (ix < 0) return;
-        cx<R> *p = gp + ix * 256, *m = gm + ix * 256;
+        cx<float> *p = gp + ix * 256, *m = gm + ix * 256;
         if (half) {
-          const cx<R> o = *p;
+          const cx<float> o = *p;
           *p = cadd(o, v);
           *m = {o.x - v.x, o.y - v.y};
         } else {
@@ -129,8 +122,8 @@ __global__ void __launch_bounds__(256) plane_kernel(const S *__restrict__ c, typ
     }
 #pragma unroll
     for (int q = 0; q < YC; ++q) {
-      const cx<R> a = gp[ygx[q] * 256], d = gm[ygx[q] * 256];
-      const R cs = phy[q][y][0], sn = phy[q][y][1];
+      const cx<float> a = gp[ygx[q] * 256], d = gm[ygx[q] * 256];
+      const float cs = phy[q][y][0], sn = phy[q][y][1];
       hc[q].x = fma(cs, a.x, hc[q].x);
       hc[q].y = fma(cs, a.y, hc[q].y);
       hs[q].x = fma(sn, d.x, hs[q].x);
@@ -147,41 +140,33 @@ __global__ void __launch_bounds__(256) plane_kernel(const S *__restrict__ c, typ
   }
 }
 
-template <class R, class S, int NG, int YC>
-cudaError_t launch_plane_yc(const Job &job, const S *field, typename Vec2<R>::type *planes, const MomPlan &plan)
+template <int NG, int YC>
+cudaError_t launch_plane_yc(const Job &job, const float2 *field, float2 *planes, const MomPlan &plan)
 {
-  // complex128 with many nx needs more than the default 48 KB of shared memory
-  const size_t smem = plane_smem_bytes<R>(plan.npx);
-  if (smem > 32768) {
-    const cudaError_t e = cudaFuncSetAttribute(plane_kernel<R, S, NG, YC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               (int)plane_smem_bytes<R>(kMomMaxPx));
-    if (e != cudaSuccess) return e;
-  }
   const dim3 grid(plan.latt[2], plan.latt[3], (plan.nyg + YC - 1) / YC);
-  plane_kernel<R, S, NG, YC><<<grid, 256, smem, job.stream>>>(field, planes, plan);
+  plane_kernel<NG, YC><<<grid, 256, plane_smem_bytes(plan.npx), job.stream>>>(field, planes, plan);
   return cudaGetLastError();
 }
 // The groups of one launch: few enough accumulators for the list, or chunks of 15.
-template <class R, class S, int NG>
-cudaError_t launch_plane_ng(const Job &job, const S *field, typename Vec2<R>::type *planes, const MomPlan &plan)
+template <int NG>
+cudaError_t launch_plane_ng(const Job &job, const float2 *field, float2 *planes, const MomPlan &plan)
 {
-  if (plan.nyg <= 2) return launch_plane_yc<R, S, NG, 2>(job, field, planes, plan);
-  if (plan.nyg <= 6) return launch_plane_yc<R, S, NG, 6>(job, field, planes, plan);
-  return launch_plane_yc<R, S, NG, kMomYChunk>(job, field, planes, plan);
+  if (plan.nyg <= 2) return launch_plane_yc<NG, 2>(job, field, planes, plan);
+  if (plan.nyg <= 6) return launch_plane_yc<NG, 6>(job, field, planes, plan);
+  return launch_plane_yc<NG, kMomYChunk>(job, field, planes, plan);
 }
 
-template <class R, class S>
-cudaError_t launch_plane(const Job &job, const S *field, typename Vec2<R>::type *planes, const MomPlan &plan)
+inline cudaError_t launch_plane(const Job &job, const float2 *field, float2 *planes, const MomPlan &plan)
 {
   switch (plan.ngx) {
-  case 1: return launch_plane_ng<R, S, 1>(job, field, planes, plan);
-  case 2: return launch_plane_ng<R, S, 2>(job, field, planes, plan);
-  case 3: return launch_plane_ng<R, S, 3>(job, field, planes, plan);
-  case 4: return launch_plane_ng<R, S, 4>(job, field, planes, plan);
-  case 5: return launch_plane_ng<R, S, 5>(job, field, planes, plan);
-  case 6: return launch_plane_ng<R, S, 6>(job, field, planes, plan);
-  case 7: return launch_plane_ng<R, S, 7>(job, field, planes, plan);
-  case 8: return launch_plane_ng<R, S, 8>(job, field, planes, plan);
+  case 1: return launch_plane_ng<1>(job, field, planes, plan);
+  case 2: return launch_plane_ng<2>(job, field, planes, plan);
+  case 3: return launch_plane_ng<3>(job, field, planes, plan);
+  case 4: return launch_plane_ng<4>(job, field, planes, plan);
+  case 5: return launch_plane_ng<5>(job, field, planes, plan);
+  case 6: return launch_plane_ng<6>(job, field, planes, plan);
+  case 7: return launch_plane_ng<7>(job, field, planes, plan);
+  case 8: return launch_plane_ng<8>(job, field, planes, plan);
   default: return cudaErrorInvalidValue;
   }
 }
@@ -190,17 +175,10 @@ cudaError_t launch_plane(const Job &job, const S *field, typename Vec2<R>::type 
 // One CTA per ((nx, ny) pair q, t).  Each plane value is read once per pass
 // and feeds up to CNT Z groups of the pair; a group of +n and -n accumulates
 // C = sum cos * v and S = sum sin * v once for both momenta.
-//   R = double (complex128 planes): FP64 phases and FMAs.
-//   R = float (complex64 planes, whose values are FP32 sums): FP32 phases and
-//     products, summed with a compensated (two-sum) accumulator and returned
-//     in FP64, so the sum over z adds no rounding beyond the products'.  The
-//     FP64 pipe (1/64 of the FP32 rate on this part) would otherwise bound
-//     the kernel.
-__device__ __forceinline__ void zacc(ChunkSum<double> &a, double c, double2 v)
-{
-  a.x = fma(c, v.x, a.x);
-  a.y = fma(c, v.y, a.y);
-}
+// FP32 phases and products (the planes are FP32 sums), summed with a compensated
+// (two-sum) accumulator and returned in FP64, so the sum over z adds no rounding
+// beyond the products'.  The FP64 pipe (1/64 of the FP32 rate on this part) would
+// otherwise bound the kernel.
 __device__ __forceinline__ void zacc(ChunkSum<float> &a, float c, float2 v) { a.add(cx<float> {c * v.x, c * v.y}); }
 
 //   TMAP (planes of the fused kernel, which projects the spin-colour products
@@ -329,34 +307,33 @@ __global__ void __launch_bounds__(256) pair_map_kernel(double2 *__restrict__ row
   }
 }
 
-template <class R, int CNT, bool TMAP>
-__global__ void __launch_bounds__(256) momentum_finalize(const typename Vec2<R>::type *__restrict__ planes,
+template <int CNT, bool TMAP>
+__global__ void __launch_bounds__(256) momentum_finalize(const float2 *__restrict__ planes,
                                                           double2 *__restrict__ out, const __grid_constant__ MomPlan plan)
 {
   const int q = blockIdx.x, t = blockIdx.y, g = threadIdx.x;
   const int lz = plan.latt[2], lt = plan.latt[3];
-  __shared__ R cz[kMomMaxL], sz[kMomMaxL];
+  __shared__ float cz[kMomMaxL], sz[kMomMaxL];
   __shared__ PairSmem<2> ps;  // TMAP: the pair map of one Z group (+n and -n)
   if (TMAP) ps.load_tables(g);
   for (int k = g; k < lz; k += blockDim.x) {
-    cz[k] = R(plan.cosz[k]);
-    sz[k] = R(plan.sinz[k]);
+    cz[k] = float(plan.cosz[k]);
+    sz[k] = float(plan.sinz[k]);
   }
   __syncthreads();
   const int g0 = plan.q_g0[q], g1 = plan.q_g0[q + 1];
   for (int base = g0; base < g1; base += CNT) {
     const int cnt = min(CNT, g1 - base);
-    ChunkSum<R> ca[CNT], sa[CNT];
+    ChunkSum<float> ca[CNT], sa[CNT];
     int kk[CNT], step[CNT];
 #pragma unroll
     for (int k = 0; k < CNT; ++k) {
       kk[k] = 0;
       step[k] = k < cnt ? plan.gz_k[base + k] : 0;
     }
-    using V2 = typename Vec2<R>::type;
     constexpr int ZB = 4;  // plane loads in flight per thread
     for (int z0 = 0; z0 < lz; z0 += ZB) {
-      V2 v[ZB];
+      float2 v[ZB];
 #pragma unroll
       for (int u = 0; u < ZB; ++u)
         if (z0 + u < lz) v[u] = planes[((size_t)(t * lz + z0 + u) * plan.nq + q) * 256 + g];
@@ -388,28 +365,26 @@ __global__ void __launch_bounds__(256) momentum_finalize(const typename Vec2<R>:
           if (pm >= 0) out[((size_t)pm * lt + t) * 256 + g] = o[sg];
         }
       } else {
-        // the complex128 planes are in the order of MesonPairsOp
-        const int at = sizeof(R) == 8 ? pair_of_class(g) : g;
         const double2 c = ca[k].value(), sn = sa[k].value();
         const int pp = plan.gz_plus[base + k], pn = plan.gz_minus[base + k];
-        if (pp >= 0) out[((size_t)pp * lt + t) * 256 + at] = make_double2(c.x - sn.y, c.y + sn.x);
-        if (pn >= 0) out[((size_t)pn * lt + t) * 256 + at] = make_double2(c.x + sn.y, c.y - sn.x);
+        if (pp >= 0) out[((size_t)pp * lt + t) * 256 + g] = make_double2(c.x - sn.y, c.y + sn.x);
+        if (pn >= 0) out[((size_t)pn * lt + t) * 256 + g] = make_double2(c.x + sn.y, c.y - sn.x);
       }
     }
   }
 }
 
-template <class R, bool TMAP>
-cudaError_t launch_finalize(const Job &job, const typename Vec2<R>::type *planes, double2 *out, const MomPlan &plan)
+template <bool TMAP>
+cudaError_t launch_finalize(const Job &job, const float2 *planes, double2 *out, const MomPlan &plan)
 {
   int most = 1;  // Z groups of the pair with the most
   for (int q = 0; q < plan.nq; ++q) most = std::max(most, plan.q_g0[q + 1] - plan.q_g0[q]);
   const dim3 grid(plan.nq, plan.latt[3]);
-  if (most <= 1) momentum_finalize<R, 1, TMAP><<<grid, 256, 0, job.stream>>>(planes, out, plan);
-  else if (most <= 2) momentum_finalize<R, 2, TMAP><<<grid, 256, 0, job.stream>>>(planes, out, plan);
-  else if (most <= 3) momentum_finalize<R, 3, TMAP><<<grid, 256, 0, job.stream>>>(planes, out, plan);
-  else if (most <= 4) momentum_finalize<R, 4, TMAP><<<grid, 256, 0, job.stream>>>(planes, out, plan);
-  else momentum_finalize<R, 8, TMAP><<<grid, 256, 0, job.stream>>>(planes, out, plan);
+  if (most <= 1) momentum_finalize<1, TMAP><<<grid, 256, 0, job.stream>>>(planes, out, plan);
+  else if (most <= 2) momentum_finalize<2, TMAP><<<grid, 256, 0, job.stream>>>(planes, out, plan);
+  else if (most <= 3) momentum_finalize<3, TMAP><<<grid, 256, 0, job.stream>>>(planes, out, plan);
+  else if (most <= 4) momentum_finalize<4, TMAP><<<grid, 256, 0, job.stream>>>(planes, out, plan);
+  else momentum_finalize<8, TMAP><<<grid, 256, 0, job.stream>>>(planes, out, plan);
   return cudaGetLastError();
 }
 
@@ -600,8 +575,9 @@ cudaError_t launch_meson_momentum(const Job &job, const OpParams<double> &p, con
   // the k-steps per work unit.
   const bool fused = !tensor_cores && job.prec == Prec::C64 && momentum_fused_supported(plan) && !fused_disabled() &&
                      job.variant != 1;
-  const size_t elem = job.prec == Prec::C128 ? sizeof(double2) : sizeof(float2);
-  const size_t c_bytes = fused ? 0 : ((size_t)job.volume * 256 * elem + 255) / 256 * 256;
+  const size_t c_bytes = fused                         ? 0
+                         : job.prec == Prec::C128 ? momentum_c128_row_bytes(plan)
+                                                  : ((size_t)job.volume * 256 * sizeof(float2) + 255) / 256 * 256;
   const int lz = plan.latt[2], lt = plan.latt[3];
   const int tcv = tensor_cores && job.variant >= 0 && job.variant < 3 ? job.variant : 0;
   const TcGeom tg = make_tc_geom(plan, kMomTcSteps[tcv]);
@@ -611,23 +587,25 @@ cudaError_t launch_meson_momentum(const Job &job, const OpParams<double> &p, con
                                           : (size_t)lt * lz * plan.nq * 256 * 2 * (job.prec == Prec::C128 ? 8 : 4);
   char *ws = static_cast<char *>(job.ws->get(c_bytes + plane_bytes));
   if (!ws) return cudaErrorMemoryAllocation;
-  double2 *planes = reinterpret_cast<double2 *>(ws + c_bytes);  // complex128 form
-  float2 *planes_m = reinterpret_cast<float2 *>(ws + c_bytes);   // mixed form
+  float2 *planes = reinterpret_cast<float2 *>(ws + c_bytes);  // mixed form
 
   if (fused) {
     cudaError_t e;
-    if (job.variant == 2) e = launch_momentum_fused(job, p.in[0], p.in[1], planes_m, plan);
-    else e = launch_momentum_rows(job, single_item(plan, p.in[0], p.in[1], planes_m, job.status), p.in[0] == p.in[1]);
+    if (job.variant == 2) e = launch_momentum_fused(job, p.in[0], p.in[1], planes, plan);
+    else e = launch_momentum_rows(job, single_item(plan, p.in[0], p.in[1], planes, job.status), p.in[0] == p.in[1]);
     if (e != cudaSuccess) return e;
-    return launch_finalize<float, true>(job, planes_m, static_cast<double2 *>(out), plan);
+    return launch_finalize<true>(job, planes, static_cast<double2 *>(out), plan);
   }
+
+  if (job.prec == Prec::C128)
+    return launch_momentum_c128(job, p.in[0], p.in[1], reinterpret_cast<double2 *>(ws),
+                                reinterpret_cast<double2 *>(ws + c_bytes), static_cast<double2 *>(out), plan);
 
   OpParams<double> q = p;
   q.out[0] = ws;
   for (int k = 0; k < 4; ++k) q.latt[k] = plan.latt[k];
   cudaError_t e;
-  if (job.prec == Prec::C128) e = run_ring_field<MesonPairsOp<4, 4>>(job, q);
-  else if (tensor_cores) e = run_field<MesonProductsSplitM>(job, convert_params<float>(q));
+  if (tensor_cores) e = run_field<MesonProductsSplitM>(job, convert_params<float>(q));
   else e = run_field<MesonAllGammaM>(job, convert_params<float>(q));
   if (e != cudaSuccess) return e;
   if (tensor_cores) {
@@ -642,14 +620,9 @@ cudaError_t launch_meson_momentum(const Job &job, const OpParams<double> &p, con
     return cudaGetLastError();
   }
 
-  if (job.prec == Prec::C128) {
-    e = launch_plane<double, double2>(job, reinterpret_cast<const double2 *>(ws), planes, plan);
-    if (e != cudaSuccess) return e;
-    return launch_finalize<double, false>(job, planes, static_cast<double2 *>(out), plan);
-  }
-  e = launch_plane<float, float2>(job, reinterpret_cast<const float2 *>(ws), planes_m, plan);
+  e = launch_plane(job, reinterpret_cast<const float2 *>(ws), planes, plan);
   if (e != cudaSuccess) return e;
-  return launch_finalize<float, false>(job, planes_m, static_cast<double2 *>(out), plan);
+  return launch_finalize<false>(job, planes, static_cast<double2 *>(out), plan);
 }
 
 } // namespace cgb

@@ -90,7 +90,7 @@ template <class Op, class K> cudaError_t launch_chunks(const Job &job, OpParams<
   p.status = job.status;
   static_assert(Op::NOUT <= 16, "at most 16 outputs per site");
   OutPtrs user_out {};
-  for (int o = 0; o < Op::NOUT; ++o) user_out.p[o] = static_cast<double2 *>(p.out[o]);  // field ops: none
+  for (int o = 0; o < Op::NOUT; ++o) user_out.p[o] = static_cast<double2 *>(p.out[o]);
   double2 *partial = nullptr;
   if (!job.per_site) {
     if (!job.ws) return cudaErrorInvalidValue;
@@ -116,14 +116,6 @@ template <class Op> cudaError_t run_ring(const Job &job, OpParams<typename Op::R
   constexpr size_t smem = RingSmem<Op>::BYTES;
   static_assert(smem <= 232448, "op does not fit in shared memory");
   return launch_chunks<Op>(job, p, ring_kernel<Op, Walk>, smem);
-}
-
-// The same for a field op of the ring kernel.
-template <class Op> cudaError_t run_ring_field(const Job &job, OpParams<typename Op::R> p)
-{
-  Job j = job;
-  j.per_site = true;
-  return run_ring<Op>(j, p);
 }
 
 // One launch of an op of the field ring kernel.

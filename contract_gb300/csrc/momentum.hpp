@@ -10,7 +10,7 @@ constexpr int kMomMaxPx = 8;     // distinct nx values per call
 constexpr int kMomMaxQ = 128;    // distinct (nx, ny) pairs per call
 constexpr int kMomMaxP = 1024;   // momenta per call
 constexpr int kMomQChunk = 25;   // (nx, ny) pairs of the fused complex64 kernels
-constexpr int kMomYChunk = 15;   // Y groups per plane-kernel CTA
+constexpr int kMomYChunk = 15;   // Y groups per CTA of the complex128 Y transform
 
 struct MomPlan {
   int latt[4];
@@ -62,6 +62,13 @@ cudaError_t launch_momentum_tc(const Job &job, const MomPlan &plan, const TcGeom
 bool momentum_fused_supported(const MomPlan &plan);
 cudaError_t launch_momentum_fused(const Job &job, const void *in_i, const void *in_j, float2 *planes,
                                   const MomPlan &plan);
+
+// Complex128: pairs and X transform in one launch, row_sums[Lt][Lz][Ly][npx][256], then
+// the Y transform to planes[Lt][Lz][nq][256], pairs in the order of MesonPairs, then
+// the Z transform (kernels_momentum_c128.cu).
+size_t momentum_c128_row_bytes(const MomPlan &plan);
+cudaError_t launch_momentum_c128(const Job &job, const void *in_i, const void *in_j, double2 *row_sums, double2 *planes,
+                                 double2 *out, const MomPlan &plan);
 
 // Tile-shape variants of the projection for the autotuner (Kind::Momentum).
 // aux = 2 * tensor_cores + (fused form supported) + 4 * (P_i and P_j one field):

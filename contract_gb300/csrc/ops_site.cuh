@@ -307,8 +307,7 @@ struct MesonAllOp : RingOp<R, S, CW, 16, NST, MINB> {
   }
 };
 
-// All 256 meson Gamma pairs of a site in complex128, in lexicographic site order: what
-// the momentum projection sums.
+// All 256 meson Gamma pairs of a site in complex128: what the momentum projection sums.
 //   pair(a, b) = sum_{i,l} c_a(i) c_b(l) A[i][l ^ u] . conj(B[i ^ s][l])
 // for the Gammas a of class s and b of class u.  Thread (s, u) of a site's 16 forms
 // the class's 16 products and turns them into its 16 pairs by Walsh-Hadamard steps
@@ -320,29 +319,33 @@ struct MesonAllOp : RingOp<R, S, CW, 16, NST, MINB> {
 // blocks stays below 2^60.2 units, four of them below 2^62.2; they are rounded to
 // quarter units before the four rows meet.
 //
-// 0.77 ms at 18 x 15 x 20 x 28, bound by the integer pipes.  The whole projection of
-// 125 momenta 1.68 ms (4.60 in FP64), with errors against extended precision of
-// 3.9e-16 of the norm (4.3e-16).
-template <int CW, int MINB> struct MesonPairsOp : RingOp<double, double2, CW, 16, 1, MINB> {
-  using P = OpParams<double>;
-  static constexpr int NIN = 2, NOUT = 0, OUT_ELEMS = 256;
-  static constexpr bool CHANGES_INPUT = true;
-  __device__ static long long out_index(const P &p, long long site) { return lexicographic(p, site); }
-
-  // o[ha][hb] += the Walsh-Hadamard sums over l of row i's four products
-  template <class V> __device__ __forceinline__ static void add_row(V (&o)[4][4], const V (&t)[4], int i)
+// Alone 0.77 ms at 18 x 15 x 20 x 28, bound by the integer pipes.  The projection of 125
+// momenta is off by 3.9e-16 of its norm against extended precision (4.3e-16 in FP64).
+struct MesonPairs {
+  // o[ha][hb] += the Walsh-Hadamard sums w over l of row i's four products
+  template <class V> __device__ __forceinline__ static void add_row(V (&o)[4][4], const V (&w)[4], int i)
   {
-    V a = t[0] + t[1], b = t[0] - t[1], c = t[2] + t[3], d = t[2] - t[3];
-    V w[4] = {a + c, b + d, a - c, b - d};
-    if constexpr (std::is_integral<V>::value) {
-#pragma unroll
-      for (int h = 0; h < 4; ++h) w[h] = (w[h] + 2) >> 2;
-    }
 #pragma unroll
     for (int ha = 0; ha < 4; ++ha) {
       const bool minus = __popc(ha & i) & 1;  // uniform
 #pragma unroll
       for (int h = 0; h < 4; ++h) o[ha][h] = minus ? o[ha][h] - w[h] : o[ha][h] + w[h];
+    }
+  }
+  // w += the sums over l = 2 hi and 2 hi + 1 of products t
+  template <class V> __device__ __forceinline__ static void add_pair(V (&w)[4], const V (&t)[2], int hi)
+  {
+    const V a = t[0] + t[1], b = t[0] - t[1];
+    w[0] += a;
+    w[1] += b;
+    w[2] += hi ? -a : a;
+    w[3] += hi ? -b : b;
+  }
+  template <class V> __device__ __forceinline__ static void quarter(V (&w)[4])
+  {
+    if constexpr (std::is_integral<V>::value) {
+#pragma unroll
+      for (int h = 0; h < 4; ++h) w[h] = (w[h] + 2) >> 2;
     }
   }
   template <class V> __device__ __forceinline__ static V signed_if(V v, bool minus) { return minus ? -v : v; }
@@ -359,20 +362,27 @@ template <int CW, int MINB> struct MesonPairsOp : RingOp<double, double2, CW, 16
 #pragma unroll 1
     for (int i = 0; i < 4; ++i) {
       V x[4], y[4];
+#pragma unroll
+      for (int h = 0; h < 4; ++h) x[h] = y[h] = V(0);
       const uint32_t bs = (W.beta >> (2 * (4 * s + i))) ^ (W.beta >> (8 * s));
 #pragma unroll
-      for (int l = 0; l < 4; ++l) {
-        dot((i * 4 + (l ^ u)) * 9, ((i ^ s) * 4 + l) * 9, x[l], y[l]);
-        const bool minus = ((bs ^ (W.beta >> (2 * (4 * u + l))) ^ (W.beta >> (8 * u))) & 2u) != 0;
-        x[l] = signed_if(x[l], minus);
-        y[l] = signed_if(y[l], minus);
+      for (int hi = 0; hi < 2; ++hi) {  // the products of l = 2 hi, 2 hi + 1
+        V tx[2], ty[2];
+#pragma unroll
+        for (int lo = 0; lo < 2; ++lo) {
+          const int l = 2 * hi + lo;
+          dot((i * 4 + (l ^ u)) * 9, ((i ^ s) * 4 + l) * 9, tx[lo], ty[lo]);
+          const bool minus = ((bs ^ (W.beta >> (2 * (4 * u + l))) ^ (W.beta >> (8 * u))) & 2u) != 0;
+          tx[lo] = signed_if(tx[lo], minus);
+          ty[lo] = signed_if(ty[lo], minus);
+        }
+        add_pair(x, tx, hi);
+        add_pair(y, ty, hi);
       }
-      switch (i) {  // signs known to the compiler
-      case 0: add_row(re, x, 0), add_row(im, y, 0); break;
-      case 1: add_row(re, x, 1), add_row(im, y, 1); break;
-      case 2: add_row(re, x, 2), add_row(im, y, 2); break;
-      default: add_row(re, x, 3), add_row(im, y, 3); break;
-      }
+      quarter(x);
+      quarter(y);
+      add_row(re, x, i);
+      add_row(im, y, i);
     }
   }
 
@@ -392,15 +402,19 @@ template <int CW, int MINB> struct MesonPairsOp : RingOp<double, double2, CW, 16
       }
   }
 
-  __device__ static void site(const P &, double2 *const *in, double2 *, int sub, bool live, double2 *dst)
+  // in: the site's fields, which are changed; ready(): called when they have been read,
+  // before the pairs go to dst.
+  template <class Ready>
+  __device__ static void site(double2 *const (&in)[2], int sub, bool live, double2 *dst, Ready ready)
   {
     const int s = sub >> 2, u = sub & 3;
     FixedScales fs;
     const double2 *blk[2] = {in[0] + sub * 9, in[1] + sub * 9};
     const bool ok = fixed_scales<16, 1, false>(blk, fs);
     if (__all_sync(0xffffffffu, ok || !live)) {
-      block_to_fixed(reinterpret_cast<int4 *>(in[0] + sub * 9), blk[0], fs, 0);
-      block_to_fixed(reinterpret_cast<int4 *>(in[1] + sub * 9), blk[1], fs, 1);
+#pragma unroll 1
+      for (int q = 0; q < 2; ++q)
+        block_to_fixed(reinterpret_cast<int4 *>((q ? in[1] : in[0]) + sub * 9), (q ? in[1] : in[0]) + sub * 9, fs, q);
       __syncwarp();
       const int4 *A = reinterpret_cast<const int4 *>(in[0]), *B = reinterpret_cast<const int4 *>(in[1]);
       long long re[4][4], im[4][4];
@@ -411,7 +425,8 @@ template <int CW, int MINB> struct MesonPairsOp : RingOp<double, double2, CW, 16
         y = sy.units();
       });
       const int up = fs.E[0] + fs.E[1] - 2 * 1023 - 52;
-      if (dst) store(s, u, re, im, dst, [&](long long v) { return fixed_value(v, up); });
+      ready();
+      store(s, u, re, im, dst, [&](long long v) { return fixed_value(v, up); });
     } else {
       double re[4][4], im[4][4];
       pairs(s, u, re, im, [&](int a, int b, double &x, double &y) {
@@ -421,12 +436,13 @@ template <int CW, int MINB> struct MesonPairsOp : RingOp<double, double2, CW, 16
         x = t.x;
         y = t.y;
       });
-      if (dst) store(s, u, re, im, dst, [](double v) { return v; });
+      ready();
+      store(s, u, re, im, dst, [](double v) { return v; });
     }
   }
 };
 
-// The Gamma pair 16 a + b stored at `at` by MesonPairsOp.
+// The Gamma pair 16 a + b stored at `at` by MesonPairs.
 __device__ __forceinline__ int pair_of_class(int at)
 {
   constexpr ClassWalsh W = class_walsh();
