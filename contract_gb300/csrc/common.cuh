@@ -375,6 +375,12 @@ __device__ __forceinline__ bool mbar_wait_bounded_backoff(uint64_t *bar, uint32_
   return false;
 }
 
+// Programmatic dependent launch: the next kernel of the stream, if it was launched
+// that way, may come up while this one runs; its wait returns when this one has ended
+// and its writes are visible.
+__device__ __forceinline__ void grid_dependents_may_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // Global -> shared bulk copy (TMA, non-tensor form).  Both addresses 16-byte
 // aligned, bytes a multiple of 16; completion is signalled on `bar`.
 __device__ __forceinline__ void bulk_g2s(void *sdst, const void *gsrc, uint32_t bytes, uint64_t *bar)

@@ -213,6 +213,7 @@ __global__ void __launch_bounds__(32 * Op::CW, Op::MIN_CTAS) ring_kernel(const _
   }
   copy_params(ps, op_params<Op>(p));
   __syncthreads();
+  grid_dependents_may_launch();
 
   const int local = lane / TPS, sub = lane % TPS;
   S *scratch = reinterpret_cast<S *>(mine + M::EXTRA + (size_t)local * Op::EXTRA_BYTES);

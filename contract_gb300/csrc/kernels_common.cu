@@ -16,13 +16,15 @@ cudaError_t device_status_ptr(DeviceStatus **out) { return cudaGetSymbolAddress(
 // The order is the same on every call, so results are bitwise reproducible.
 // (One thread per (o, t) walking every partial in turn left the sum's latency
 // chain on the critical path: 108 dependent loads per thread for a per-call
-// triangle at 24^3 x 64.)
+// triangle at 24^3 x 64.  One block per t, reading a chunk's outputs together, takes
+// 2 us longer for 12 outputs at 8^3 x 16.)
 __global__ void __launch_bounds__(kFinThreads) finalize_kernel(const double2 *__restrict__ partial, OutPtrs out,
                                                                int nout, int lt, int chunks_per_seg)
 {
   const int o = blockIdx.x / lt, t = blockIdx.x - o * lt;
   const int n = 2 * chunks_per_seg;
   double sx = 0.0, sy = 0.0;
+  grid_dependency_wait();
   for (int k = threadIdx.x; k < n; k += kFinThreads) {
     const int par = k >= chunks_per_seg ? 1 : 0, c = k - par * chunks_per_seg;
     const double2 v = partial[((size_t)(par * lt + t) * chunks_per_seg + c) * nout + o];
@@ -46,6 +48,13 @@ __global__ void __launch_bounds__(kFinThreads) finalize_kernel(const double2 *__
     }
     out.p[o][t] = r;
   }
+}
+
+cudaError_t launch_finalize_chunks(const Job &job, const double2 *partial, const OutPtrs &out, int nout,
+                                   int chunks_per_seg)
+{
+  return launch_overlapped(finalize_kernel, dim3(nout * job.lt), kFinThreads, 0, job.stream, partial, out, nout, job.lt,
+                           chunks_per_seg);
 }
 
 // complex128 <-> complex64, one complex per thread step, grid-stride.

@@ -321,6 +321,7 @@ __global__ void __launch_bounds__(256) momentum_finalize(const float2 *__restric
     sz[k] = float(plan.sinz[k]);
   }
   __syncthreads();
+  grid_dependency_wait();
   const int g0 = plan.q_g0[q], g1 = plan.q_g0[q + 1];
   for (int base = g0; base < g1; base += CNT) {
     const int cnt = min(CNT, g1 - base);
@@ -331,7 +332,7 @@ __global__ void __launch_bounds__(256) momentum_finalize(const float2 *__restric
       kk[k] = 0;
       step[k] = k < cnt ? plan.gz_k[base + k] : 0;
     }
-    constexpr int ZB = 4;  // plane loads in flight per thread
+    constexpr int ZB = 8;  // plane loads in flight per thread
     for (int z0 = 0; z0 < lz; z0 += ZB) {
       float2 v[ZB];
 #pragma unroll
@@ -344,6 +345,7 @@ __global__ void __launch_bounds__(256) momentum_finalize(const float2 *__restric
         for (int k = 0; k < CNT; ++k) {
           if (k < cnt) {
             zacc(ca[k], cz[kk[k]], v[u]);
+            if (step[k] == 0) continue;  // nz = 0: no sine sum
             zacc(sa[k], sz[kk[k]], v[u]);
             if ((kk[k] += step[k]) >= lz) kk[k] -= lz;  // k * z mod Lz
           }
@@ -380,12 +382,12 @@ cudaError_t launch_finalize(const Job &job, const float2 *planes, double2 *out, 
   int most = 1;  // Z groups of the pair with the most
   for (int q = 0; q < plan.nq; ++q) most = std::max(most, plan.q_g0[q + 1] - plan.q_g0[q]);
   const dim3 grid(plan.nq, plan.latt[3]);
-  if (most <= 1) momentum_finalize<1, TMAP><<<grid, 256, 0, job.stream>>>(planes, out, plan);
-  else if (most <= 2) momentum_finalize<2, TMAP><<<grid, 256, 0, job.stream>>>(planes, out, plan);
-  else if (most <= 3) momentum_finalize<3, TMAP><<<grid, 256, 0, job.stream>>>(planes, out, plan);
-  else if (most <= 4) momentum_finalize<4, TMAP><<<grid, 256, 0, job.stream>>>(planes, out, plan);
-  else momentum_finalize<8, TMAP><<<grid, 256, 0, job.stream>>>(planes, out, plan);
-  return cudaGetLastError();
+  auto *const z = most <= 1   ? momentum_finalize<1, TMAP>
+                  : most <= 2 ? momentum_finalize<2, TMAP>
+                  : most <= 3 ? momentum_finalize<3, TMAP>
+                  : most <= 4 ? momentum_finalize<4, TMAP>
+                              : momentum_finalize<8, TMAP>;
+  return launch_overlapped(z, grid, 256, 0, job.stream, planes, out, plan);
 }
 
 // ------------------------------------------------ batched finalisation --
@@ -402,6 +404,7 @@ __global__ void __launch_bounds__(256) batch_finalize_combined(const __grid_cons
                                                                 const __grid_constant__ BaryonFinParams bf)
 {
   const int g = threadIdx.x;
+  grid_dependency_wait();
   if ((int)blockIdx.x < bf.total_blocks) {
     int lo = 0, hi = bf.n_items - 1;
     while (lo < hi) {
@@ -455,7 +458,7 @@ __global__ void __launch_bounds__(256) batch_finalize_combined(const __grid_cons
       kk[k] = 0;
       step[k] = k < cnt ? mp.gz_k[base + k] : 0;
     }
-    constexpr int ZB = 4;  // plane loads in flight per thread
+    constexpr int ZB = 8;  // plane loads in flight per thread
     for (int z0 = 0; z0 < lz; z0 += ZB) {
       float2 v[ZB];
 #pragma unroll
@@ -468,6 +471,7 @@ __global__ void __launch_bounds__(256) batch_finalize_combined(const __grid_cons
         for (int k = 0; k < CNT; ++k) {
           if (k < cnt) {
             zacc(ca[k], cz[kk[k]], v[u]);
+            if (step[k] == 0) continue;  // nz = 0: no sine sum
             zacc(sa[k], sz[kk[k]], v[u]);
             if ((kk[k] += step[k]) >= lz) kk[k] -= lz;
           }
@@ -497,13 +501,12 @@ cudaError_t launch_batch_finalize(const Job &job, const MomBatchParams &mp, cons
   if (blocks <= 0) return cudaSuccess;
   int most = 1;  // Z groups of the pair with the most
   for (int q = 0; q < mp.nq; ++q) most = std::max(most, mp.q_g0[q + 1] - mp.q_g0[q]);
-  const unsigned grid = (unsigned)blocks;
-  if (mp.n_items == 0 || most <= 1) batch_finalize_combined<1><<<grid, 256, 0, job.stream>>>(mp, bf);
-  else if (most <= 2) batch_finalize_combined<2><<<grid, 256, 0, job.stream>>>(mp, bf);
-  else if (most <= 3) batch_finalize_combined<3><<<grid, 256, 0, job.stream>>>(mp, bf);
-  else if (most <= 4) batch_finalize_combined<4><<<grid, 256, 0, job.stream>>>(mp, bf);
-  else batch_finalize_combined<8><<<grid, 256, 0, job.stream>>>(mp, bf);
-  return cudaGetLastError();
+  auto *const f = mp.n_items == 0 || most <= 1 ? batch_finalize_combined<1>
+                  : most <= 2                  ? batch_finalize_combined<2>
+                  : most <= 3                  ? batch_finalize_combined<3>
+                  : most <= 4                  ? batch_finalize_combined<4>
+                                               : batch_finalize_combined<8>;
+  return launch_overlapped(f, dim3((unsigned)blocks), 256, 0, job.stream, mp, bf);
 }
 
 // CONTRACT_MOMENTUM_UNFUSED=1 selects the three-kernel mixed form (site

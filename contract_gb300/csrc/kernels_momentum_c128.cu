@@ -204,6 +204,7 @@ __global__ void __launch_bounds__(256) y_c128_kernel(const double2 *__restrict__
     phy[q][y] = q < ny ? make_double2(plan.cosy[k], plan.siny[k]) : make_double2(0.0, 0.0);
   }
   __syncthreads();
+  grid_dependency_wait();
   cx<double> hc[YC], hs[YC];
 #pragma unroll
   for (int q = 0; q < YC; ++q) hc[q] = hs[q] = czero<double>();
@@ -247,6 +248,7 @@ __global__ void __launch_bounds__(256) z_c128_kernel(const double2 *__restrict__
   __shared__ double2 phz[kMomMaxL];
   for (int k = threadIdx.x; k < lz; k += blockDim.x) phz[k] = make_double2(plan.cosz[k], plan.sinz[k]);
   __syncthreads();
+  grid_dependency_wait();
   const int at = pair_of_class(threadIdx.x), g0 = plan.q_g0[q], g1 = plan.q_g0[q + 1];
   const double2 *col = planes + ((size_t)t * lz * plan.nq + q) * 256 + threadIdx.x;
   const size_t step = (size_t)plan.nq * 256;
@@ -316,8 +318,7 @@ template <int YC> static cudaError_t launch_y(const Job &job, const double2 *g, 
     if (e != cudaSuccess) return e;
   }
   const dim3 grid(plan.latt[2], plan.latt[3], (plan.nyg + YC - 1) / YC);
-  y_c128_kernel<YC><<<grid, 256, smem, job.stream>>>(g, planes, plan);
-  return cudaGetLastError();
+  return launch_overlapped(y_c128_kernel<YC>, grid, 256, smem, job.stream, g, planes, plan);
 }
 
 size_t momentum_c128_row_bytes(const MomPlan &plan)
@@ -357,11 +358,8 @@ cudaError_t launch_momentum_c128(const Job &job, const void *in_i, const void *i
   int most = 1;  // Z groups of the pair with the most
   for (int q = 0; q < plan.nq; ++q) most = std::max(most, plan.q_g0[q + 1] - plan.q_g0[q]);
   const dim3 grid(plan.nq, plan.latt[3]);
-  if (most <= 1) z_c128_kernel<1><<<grid, 256, 0, job.stream>>>(planes, out, plan);
-  else if (most <= 2) z_c128_kernel<2><<<grid, 256, 0, job.stream>>>(planes, out, plan);
-  else if (most <= 3) z_c128_kernel<3><<<grid, 256, 0, job.stream>>>(planes, out, plan);
-  else z_c128_kernel<6><<<grid, 256, 0, job.stream>>>(planes, out, plan);
-  return cudaGetLastError();
+  auto *const z = most <= 1 ? z_c128_kernel<1> : most <= 2 ? z_c128_kernel<2> : most <= 3 ? z_c128_kernel<3> : z_c128_kernel<6>;
+  return launch_overlapped(z, grid, 256, 0, job.stream, planes, out, plan);
 }
 
 } // namespace cgb

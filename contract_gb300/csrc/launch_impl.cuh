@@ -71,12 +71,35 @@ template <class Op, class K> cudaError_t prepare(K kernel, size_t smem, int &bps
   return cudaSuccess;
 }
 
+// Launches a kernel that begins with grid_dependency_wait(): its grid comes up while
+// the kernel before it on the stream drains.  The finalisation of per-timeslice sums
+// this way: 22.7 -> 21.0 us for a call of all types at 8^3 x 16, 299.4 -> 297.3 for one
+// type at 22 x 17 x 25 x 54.
+template <class... Params, class... Args>
+cudaError_t launch_overlapped(void (*kernel)(Params...), dim3 grid, int threads, size_t smem, cudaStream_t stream,
+                              const Args &...args)
+{
+  cudaLaunchAttribute overlap {};
+  overlap.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  overlap.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = &overlap;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
 struct OutPtrs {
   double2 *p[16];
 };
 
 constexpr int kFinThreads = 64;  // finalize_kernel's block: the partials of one (output, timeslice)
-__global__ void finalize_kernel(const double2 *__restrict__ partial, OutPtrs out, int nout, int lt, int chunks_per_seg);
+// Reduces the chunk partials left by the kernel launched before it on the job's stream.
+cudaError_t launch_finalize_chunks(const Job &job, const double2 *partial, const OutPtrs &out, int nout,
+                                   int chunks_per_seg);
 
 // Launches a kernel of engine_warp.cuh over the job's chunks, dealt to the grid's
 // warps, and reduces the chunk partials if the job sums timeslices.
@@ -102,9 +125,7 @@ template <class Op, class K> cudaError_t launch_chunks(const Job &job, OpParams<
   kernel<<<grid, 32 * Op::CW, smem, job.stream>>>(p);
   e = cudaGetLastError();
   if (e != cudaSuccess || job.per_site) return e;
-  finalize_kernel<<<Op::NOUT * job.lt, kFinThreads, 0, job.stream>>>(partial, user_out, Op::NOUT, job.lt,
-                                                                      p.geom.chunks_per_seg);
-  return cudaGetLastError();
+  return launch_finalize_chunks(job, partial, user_out, Op::NOUT, p.geom.chunks_per_seg);
 }
 
 // One launch of a per-call scalar op's ring kernel, then, for per-timeslice sums,
