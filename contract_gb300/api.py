@@ -11,13 +11,10 @@ import ctypes
 import numpy as np
 
 from . import _lib
-from .pycontract import (CONTRACT_C128, CONTRACT_C64, _check, _complex_host, _lib_record, _ptr, _ptr_array, _volume,
-                         decompose_gamma)
+from .pycontract import (CONTRACT_C128, CONTRACT_C64, _check, _complex_host, _lib_record, _ptr, _ptr_array, _torch,
+                         _volume, decompose_gamma)
 
-
-def _torch():
-    import torch
-    return torch
+_Int4 = ctypes.c_int * 4
 
 
 def _prec(p):
@@ -25,8 +22,7 @@ def _prec(p):
 
 
 def _latt(latt):
-    a = (ctypes.c_int * 4)(*[int(x) for x in latt])
-    return a
+    return _Int4(*map(int, latt))
 
 
 def _gamma_int(g):

@@ -206,31 +206,41 @@ def decompose_gamma(g):
 
 # ------------------------------------------------------------ tensor helpers --
 
+_torch_module = None
+
+
 def _torch():
-    import torch
-    return torch
+    global _torch_module
+    if _torch_module is None:
+        import torch
+        _torch_module = torch
+    return _torch_module
 
 
-def _check_prop(p, name):
+def _check_prop(p, k):
+    """Sites of propagator number k, or the error that it makes."""
     torch = _torch()
     if not isinstance(p, torch.Tensor):
-        raise TypeError(f"{name} must be a torch tensor")
+        raise TypeError(f"propag_{k} must be a torch tensor")
     if not p.is_cuda:
-        raise ValueError(f"{name} must live on a CUDA device")
+        raise ValueError(f"propag_{k} must live on a CUDA device")
     if p.dtype not in (torch.complex128, torch.complex64):
-        raise TypeError(f"{name} must be complex128 (or complex64 for the mixed form)")
-    if not p.is_contiguous() or p.numel() % 144:
-        raise ValueError(f"{name} must be contiguous with a multiple of 144 entries per site")
-    return p.numel() // 144
+        raise TypeError(f"propag_{k} must be complex128 (or complex64 for the mixed form)")
+    n = p.numel()
+    if n % 144 or not p.is_contiguous():
+        raise ValueError(f"propag_{k} must be contiguous with a multiple of 144 entries per site")
+    return n // 144
 
 
 def _volume(*props):
-    vols = {_check_prop(p, f"propag_{k}") for k, p in enumerate(props)}
-    if len(vols) != 1:
+    vols = [_check_prop(p, k) for k, p in enumerate(props)]
+    if vols.count(vols[0]) != len(vols):
         raise ValueError("propagators have different volumes")
-    if len({p.dtype for p in props}) != 1:
-        raise ValueError("propagators have different dtypes")
-    return vols.pop()
+    dtype = props[0].dtype
+    for p in props:
+        if p.dtype != dtype:
+            raise ValueError("propagators have different dtypes")
+    return vols[0]
 
 
 def mesonTwoPoint(propag_i, propag_j, gamma_ij, gamma_kl):
