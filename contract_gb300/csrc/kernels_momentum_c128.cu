@@ -321,14 +321,48 @@ template <int YC> static cudaError_t launch_y(const Job &job, const double2 *g, 
   return launch_overlapped(y_c128_kernel<YC>, grid, 256, smem, job.stream, g, planes, plan);
 }
 
-size_t momentum_c128_row_bytes(const MomPlan &plan)
+// The plan with one X sum for all nx that agree modulo Lx: at most Lx a row, so that
+// the row sums never take more room than the pairs of every site would.
+static void merge_nx(MomPlan &plan)
 {
+  const int lx = plan.latt[0];
+  int sum[kMomMaxPx], n = 0;
+  for (int ip = 0; ip < plan.npx; ++ip) {
+    int j = 0;
+    while (j < n && (plan.px[ip] - plan.px[j]) % lx != 0) ++j;
+    if (j == n) plan.px[n++] = plan.px[ip];
+    sum[ip] = j;
+  }
+  if (n == plan.npx) return;
+  plan.npx = n;
+  for (int g = 0; g < plan.nyg; ++g) plan.yg_ix[g] = sum[plan.yg_ix[g]];
+  int groups = 0;  // the groups keep their order, k = 0 first; those of repeated nx go
+  for (int g = 0; g < plan.ngx; ++g) {
+    int seen = 0;
+    while (seen < groups && plan.gx_k[seen] != plan.gx_k[g]) ++seen;
+    const int plus = plan.gx_plus[g] < 0 ? -1 : sum[plan.gx_plus[g]];
+    const int minus = plan.gx_minus[g] < 0 ? -1 : sum[plan.gx_minus[g]];
+    if (seen == groups) {
+      plan.gx_k[groups] = plan.gx_k[g];
+      plan.gx_plus[groups] = plan.gx_minus[groups] = -1;
+      ++groups;
+    }
+    if (plus >= 0) plan.gx_plus[seen] = plus;
+    if (minus >= 0) plan.gx_minus[seen] = minus;
+  }
+  plan.ngx = groups;
+}
+
+size_t momentum_c128_row_bytes(MomPlan plan)
+{
+  merge_nx(plan);
   return (size_t)plan.latt[1] * plan.latt[2] * plan.latt[3] * plan.npx * 256 * sizeof(double2);
 }
 
 cudaError_t launch_momentum_c128(const Job &job, const void *in_i, const void *in_j, double2 *row_sums, double2 *planes,
-                                 double2 *out, const MomPlan &plan)
+                                 double2 *out, MomPlan plan)
 {
+  merge_nx(plan);
   RowsC128 a {};
   a.in[0] = static_cast<const char *>(in_i);
   a.in[1] = static_cast<const char *>(in_j);

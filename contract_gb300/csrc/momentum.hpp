@@ -66,9 +66,9 @@ cudaError_t launch_momentum_fused(const Job &job, const void *in_i, const void *
 // Complex128: pairs and X transform in one launch, row_sums[Lt][Lz][Ly][npx][256], then
 // the Y transform to planes[Lt][Lz][nq][256], pairs in the order of MesonPairs, then
 // the Z transform (kernels_momentum_c128.cu).
-size_t momentum_c128_row_bytes(const MomPlan &plan);
+size_t momentum_c128_row_bytes(MomPlan plan);
 cudaError_t launch_momentum_c128(const Job &job, const void *in_i, const void *in_j, double2 *row_sums, double2 *planes,
-                                 double2 *out, const MomPlan &plan);
+                                 double2 *out, MomPlan plan);
 
 // Tile-shape variants of the projection for the autotuner (Kind::Momentum).
 // aux = 2 * tensor_cores + (fused form supported) + 4 * (P_i and P_j one field):
