@@ -84,8 +84,8 @@ void contract_test_withhold_chunk(int chunk);
 void contract_set_stream(void *stream);
 void *contract_get_stream(void);
 
-/* Tile-shape autotuning (consumer warps, threads per site, ring stages) of
- * the complex64 kernels: when enabled, the first call for a new (op, shape)
+/* Tile-shape autotuning (warps, threads per site, ring stages, CTAs per SM) of
+ * the site kernels: when enabled, the first call for a new (op, shape)
  * times each compiled variant on its own data and keeps the fastest.  Also
  * enabled by CONTRACT_AUTOTUNE=1; CONTRACT_TUNE_CACHE=<file> persists the
  * choices across processes.  Never tunes during stream capture. */
@@ -285,9 +285,10 @@ void contract_batch_mixed(const ContractBaryonBatchItem *baryon_items, int nbary
  * moms: HOST int[nmom][3] = (nx, ny, nz); lattice required, spatial extents
  * <= 64, at most 8 distinct nx and 128 distinct (nx, ny) per call.  correl:
  * device complex128 [nmom][Lt][256].  Uses the per-device workspace for
- * V x 256 site values and the per-plane partial sums (FP64), or with
- * CONTRACT_C64_TC the bf16 phase tiles and the FP32 partials of the
- * tensor-core projection. */
+ * the per-plane partial sums and, in complex128, the X sums of every row (at
+ * most V x 256 values; complex64 with more than three |nx| or 25 (nx, ny): V x
+ * 256 site values), or with CONTRACT_C64_TC the site values, the bf16 phase
+ * tiles and the FP32 partials of the tensor-core projection. */
 void contract_meson_all_gamma_momentum(void *correl, const void *propag_i, const void *propag_j, size_t volume,
                                        const int *lattice, const int *moms, int nmom, int precision);
 
