@@ -392,6 +392,11 @@ __device__ __forceinline__ void bulk_g2s(void *sdst, const void *gsrc, uint32_t 
 }
 
 // Shared -> global bulk copy; tracked by the issuing thread's bulk group.
+// Global memory into L2: address 16-byte aligned, bytes a multiple of 16.
+__device__ __forceinline__ void bulk_prefetch_l2(const void *gsrc, uint32_t bytes)
+{
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(gsrc), "r"(bytes) : "memory");
+}
 __device__ __forceinline__ void bulk_s2g(void *gdst, const void *ssrc, uint32_t bytes)
 {
   asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(gdst), "r"(smem_addr(ssrc)),

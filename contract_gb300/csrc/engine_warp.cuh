@@ -228,6 +228,9 @@ __global__ void __launch_bounds__(32 * Op::CW, Op::MIN_CTAS) ring_kernel(const _
         bulk_g2s(mine + M::IN + stage * M::STAGE + ((size_t)q * SPW + s) * L::SLOT,
                  w.in(p, q) + (w.first() + s) * L::SITE_BYTES, L::SITE_BYTES, &full[stage]);
     }
+    if constexpr (Op::DIRECT > 0) {  // what the op will read from memory is in L2 by then
+      if (lane < Op::DIRECT) bulk_prefetch_l2(w.in(p, NIN + lane) + w.first() * L::SITE_BYTES, (uint32_t)n * L::SITE_BYTES);
+    }
   };
   static_assert(SPW * NIN <= 32, "one copy per lane");
   Walk cur, ahead;

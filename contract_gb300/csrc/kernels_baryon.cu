@@ -15,7 +15,7 @@ template <class Op> static cudaError_t run_rank(const Job &job, OpParams<typenam
 // conversions, so warps in flight count and a second ring stage, which costs warps,
 // does not pay.  24^3 x 32 per site, three different fields, ms (the FP64 kernels
 // that these replaced in brackets): loop 0.89 [2.86 with a projector of two terms],
-// one gamma matrix 2.32, dense projector 3.50, rank 2 1.52 [4.65], rank 1 1.18.
+// one gamma matrix 2.32, dense projector 3.50, rank 2 1.49 [4.65], rank 1 1.15.
 static const VariantSet<double, 4> kLoopP = {
   {run_ring<BaryonLoopOp<double, double2, 4, 16, 1, 3>>, run_ring<BaryonLoopOp<double, double2, 4, 16, 1, 2>>,
    run_ring<BaryonLoopOp<double, double2, 2, 16, 1, 6>>, run_ring<BaryonLoopOp<double, double2, 13, 16, 1, 1>>},
