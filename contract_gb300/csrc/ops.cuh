@@ -524,11 +524,11 @@ __device__ __forceinline__ void conj_products_f32x2(cx<float> (&T)[NK][NL], cons
 // instead of the Gamma pairs, product (i, j = i ^ s, k, l) at index
 // (4 k + l) * 16 + 4 s + i.  Each pair is a signed sum of 16 products, the same
 // at every site, so a linear consumer (the momentum projection) forms the pairs
-// once from its sums (pair_from_products in kernels_momentum.cu).
+// once from its sums (map_pairs in kernels_momentum.cu).
 template <class R, class S, int CW, int NST, bool SPLIT = false, bool PRODUCTS = false>
 struct MesonAllGammaOp : OpBase<R, S, CW, 16, NST> {
   static constexpr int NIN = 2, OUT_ELEMS = 256;
-  static_assert(sizeof(R) == 4, "complex128: MesonPairsOp (ops_site.cuh)");
+  static_assert(sizeof(R) == 4, "complex128: MesonPairs (ops_site.cuh)");
   __device__ static long long sites_per_slice(const OpParams<R> &p)
   {
     return (long long)p.latt[0] * p.latt[1] * p.latt[2];

@@ -1,5 +1,5 @@
 """The complex128 meson momentum projection: pairs of a site in integers or FP64
-(MesonPairsOp), and the plane transform that takes sites x, Lx - x and rows y,
+(MesonPairs), and the plane transform that takes sites x, Lx - x and rows y,
 Ly - y together.  Where it can go wrong: sites and rows without a partner (the
 first, the middle one of an even extent), lists without nx = 0, without the
 partners +n / -n, with one component more than once modulo the extent, more Y
