@@ -35,6 +35,9 @@ namespace cgb {
 constexpr int kFixedMinExp = 723, kFixedMaxExp = 1323;  // biased: 2^-300 to 2^300
 constexpr int kFixedSpread = 2;   // powers of two between a block and its field's scale
 constexpr int kFixedColour = 100;  // and between colour rows or columns at most
+// Powers of two that fixed_value may apply: a sum is 1 to 2^62 units.
+constexpr int kFixedMinUp = -1022, kFixedMaxUp = 960;
+constexpr int kFixedMinDot = 200;  // least biased exponent of a dot block's largest value
 
 // The largest of a site's TPS threads' values.
 template <int TPS> __device__ __forceinline__ int group_max(int v)
@@ -343,21 +346,33 @@ __device__ __forceinline__ cx<double> fixed_conj_dot(const int4 (&x)[9], const i
 // products have one.
 struct FixedDotBlock {
   int4 g[9];
-  int up;
-  __device__ __forceinline__ void set(const cx<double> (&v)[9], const FixedScales &f)
+  int E, up;
+  // The block's scale beside that of the field; false if the block does not suit the
+  // integer form: a value is not finite, all are so small that denormal ones count, or
+  // a dot could leave the exponents of a double (fixed_value tests nothing).  Its values
+  // come from either form of the wedges, so they may be anything.
+  __device__ __forceinline__ bool fits(const cx<double> (&v)[9], const FixedScales &f)
   {
-    int E = -8192;
+    int most = 0;
+    uint32_t any = 0;
+    E = -8192;
 #pragma unroll
     for (int k = 0; k < 9; ++k) {
-      const int x = max(__double2hiint(v[k].x) & 0x7fffffff, __double2hiint(v[k].y) & 0x7fffffff) >> 20;
+      const int hx = __double2hiint(v[k].x) & 0x7fffffff, hy = __double2hiint(v[k].y) & 0x7fffffff, x = max(hx, hy) >> 20;
+      any |= (uint32_t)(hx | hy) | (uint32_t)__double2loint(v[k].x) | (uint32_t)__double2loint(v[k].y);
+      most = max(most, x);
       E = max(E, x ? x + f.r[k / 3] + f.c[k % 3] : -8192);
     }
+    up = E + f.E[0] - 2 * 1023 - 54;
+    return any == 0 || (most < 2047 && most >= kFixedMinDot && up >= kFixedMinUp && up <= kFixedMaxUp);
+  }
+  __device__ __forceinline__ void set(const cx<double> (&v)[9], const FixedScales &f)
+  {
 #pragma unroll
     for (int k = 0; k < 9; ++k) {
       const int2 a = to_fixed(v[k].x, E - f.r[k / 3] - f.c[k % 3]), b = to_fixed(v[k].y, E - f.r[k / 3] - f.c[k % 3]);
       g[k] = make_int4(a.x, a.y, b.x, b.y);
     }
-    up = E + f.E[0] - 2 * 1023 - 54;
   }
   __device__ __forceinline__ cx<double> dot(const double2 *blk) const
   {

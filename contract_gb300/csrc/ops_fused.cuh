@@ -168,17 +168,25 @@ __device__ __forceinline__ bool fields_to_fixed(double2 *A, double2 *B, int sub,
   return true;
 }
 
-// Converts the blocks of P_n in place likewise.
-template <int TPS> __device__ __forceinline__ bool field_to_fixed(double2 *N, int sub, bool live, FixedScales &fs)
+// Converts the blocks of P_n in place likewise, if the thread's blocks g of G, which
+// may come from the FP64 form, suit it as well.
+template <int TPS, int NN>
+__device__ __forceinline__ bool dots_to_fixed(double2 *N, const cx<double> (&g)[NN][9], int sub, bool live,
+                                              FixedDotBlock (&gb)[NN])
 {
   constexpr int NB = 16 / TPS;
+  FixedScales fs;
   const double2 *blk[NB];
 #pragma unroll
   for (int k = 0; k < NB; ++k) blk[k] = N + (sub + k * TPS) * 9;
-  const bool ok = fixed_scales<TPS, NB>(blk, fs);
+  bool ok = fixed_scales<TPS, NB>(blk, fs);
+#pragma unroll
+  for (int t = 0; t < NN; ++t) ok = gb[t].fits(g[t], fs) && ok;
   if (!__all_sync(0xffffffffu, ok || !live)) return false;
 #pragma unroll
   for (int k = 0; k < NB; ++k) block_to_fixed(reinterpret_cast<int4 *>(N + (sub + k * TPS) * 9), blk[k], fs, 0);
+#pragma unroll
+  for (int t = 0; t < NN; ++t) gb[t].set(g[t], fs);
   __syncwarp();
   return true;
 }
@@ -361,15 +369,9 @@ struct BaryonFusedOp {
     };
     if constexpr (sizeof(R) == 8 && SRC > 0) {
       __syncwarp();  // the loop above has read P_n
-      FixedScales fs;
-      if (field_to_fixed<TPS>(N, sub, live, fs)) {
-        FixedDotBlock gb[NN];
-#pragma unroll
-        for (int t = 0; t < NN; ++t) gb[t].set(g[t], fs);
-        dots(gb);
-      } else {
-        plain();
-      }
+      FixedDotBlock gb[NN];
+      if (dots_to_fixed<TPS, NN>(N, g, sub, live, gb)) dots(gb);
+      else plain();
     } else {
       plain();
     }
