@@ -34,9 +34,13 @@ namespace cgb {
 
 constexpr int kFixedMinExp = 723, kFixedMaxExp = 1323;  // biased: 2^-300 to 2^300
 constexpr int kFixedSpread = 2;   // powers of two between a block and its field's scale
-constexpr int kFixedColour = 100;  // and between colour rows or columns at most
+constexpr int kFixedColour = 60;  // and between colour rows or columns at most
 // Powers of two that fixed_value may apply: a sum is 1 to 2^62 units.
 constexpr int kFixedMinUp = -1022, kFixedMaxUp = 960;
+// A wedge's: two fields' scales, two colour rows and two columns (one row and one column have
+// the field's scale).
+static_assert(2 * kFixedMinExp - 2 * 1023 - 54 - 4 * kFixedColour >= kFixedMinUp &&
+              2 * kFixedMaxExp - 2 * 1023 - 54 <= kFixedMaxUp, "a wedge could leave the exponents of a double");
 constexpr int kFixedMinDot = 200;  // least biased exponent of a dot block's largest value
 
 // The largest of a site's TPS threads' values.

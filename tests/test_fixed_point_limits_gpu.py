@@ -98,3 +98,25 @@ def test_overflow_and_underflow(api, c_oracle):
     ps = fields((1e-154, 1e-156, 1e80))  # a diquark of denormal numbers
     got, ref = run(api, ps), oracle(api, c_oracle, ps)
     assert off(got, ref) <= 1e-12
+
+
+def test_wedge_of_small_colour_rows(api):
+    """Two colour rows and columns far below the third, at the least field scale of the
+    integer form, and a wedge's entry that cancels to a few of its units: its exponent
+    must not run out of a double's range.  No entry exceeds the sizes of its products."""
+    import torch
+    from contract_gb300 import pycontract as pc
+    s = 2.0 ** -100
+    x = np.array([[1, s, s], [s, s * s, s * s * (1 + 2.0 ** -40)], [s, 0, 0]]) * 2.0 ** -299
+    y = np.array([[1, s, s], [s, 0, 0], [s, s * s, s * s]]) * 2.0 ** -299
+    rows = np.array([1, 1, 1, 0.5])[:, None, None, None]  # whatever the signs of Gamma_ij, they do not cancel
+    pi = np.broadcast_to(rows * x, (V, 4, 4, 3, 3)).astype(complex, order="C")
+    pj = np.broadcast_to(y, (V, 4, 4, 3, 3)).astype(complex, order="C")
+    got = pc.baryonDiquark(torch.from_numpy(pi).cuda(), torch.from_numpy(pj).cuda(), 5, 5).cpu().numpy()
+    size = np.zeros((3, 3))
+    for a in range(3):
+        for e in range(3):
+            for b, c in ((1, 2), (2, 1)):
+                for f, g in ((1, 2), (2, 1)):
+                    size[a, e] += x[(a + b) % 3, (e + f) % 3] * y[(a + c) % 3, (e + g) % 3]
+    assert (np.abs(got.reshape(V, 4, 4, 3, 3)) <= 4 * size).all()
