@@ -15,17 +15,22 @@
 // and columns, common to both fields (every term of a wedge's entry then has one
 // scale).  Colour rows or columns of very different size so keep their bits.
 //
-// Accuracy.  In units of the operands' scales A and B a value is off by at most
-// 2^-55 A (cut off; nothing down to A / 8), and the dropped l l' and the last rounding make about half a unit of
-// 2^-56 A B per result.  For entries of one size s (A ~ 4.5 s with the power of
-// two) that is 2^-52 s^2, against 2^-49.8 s^2 for 32 products summed in FP64, where
-// every sum rounds.  A block much smaller than its field keeps fewer bits, so the
-// integer form is taken only if no 3 x 3 block of the site that is not zero lies
-// more than 2 powers of two below the largest, in its scales, if every value is
-// finite and if all exponents leave room for the products; otherwise the warp
-// takes the FP64 form for its sites.  Values below 2^-60 of their scale count as
-// zero.  Measured against extended precision (4096 outputs of all types, two
-// projectors): 1.9e-16 of their norm for Gaussian fields, 2.3e-16 in FP64.
+// Accuracy.  A value is off by at most 2^-55 of its scale (cut off; exact down to an
+// eighth of it), and the dropped l l' and the last rounding leave a wedge sum off by
+// about half a unit of 2^-54 of the two scales.  A small result therefore loses bits
+// that FP64 would keep, unless it is made of values near their scales.  So the integer
+// form is taken only where every sum has at least one product of two values that are
+// no more than kFixedNear powers of two below their scales (wedge_cover, pairs_covered,
+// FixedDotBlock::near): then its error, entry by entry and against the sum of the sizes
+// of its products, is below what FP64 leaves.  In exact arithmetic on the host, rms over
+// the sums accepted: Gaussian blocks 1.8e-17 against 6.0e-17 in FP64, blocks near a
+// multiple of the unit matrix with the rest 0.25, 0.06 and 0.001 as large 4.2e-17,
+// 3.3e-17 and 3.4e-17 against 8.5e-17, 1.1e-16 and 1.1e-16; with 3 for kFixedNear the
+// first two come to 8.7e-17 against 8.9e-17, with 1 a quarter of Gaussian sites is
+// refused.  Also every value must be finite and all exponents leave room for the
+// products; otherwise the warp takes the FP64 form for its sites.  Measured against
+// extended precision (4096 outputs of all types, two projectors): 1.9e-16 of their norm
+// for Gaussian fields, 2.3e-16 in FP64.
 #pragma once
 
 #include "common.cuh"
@@ -33,7 +38,7 @@
 namespace cgb {
 
 constexpr int kFixedMinExp = 723, kFixedMaxExp = 1323;  // biased: 2^-300 to 2^300
-constexpr int kFixedSpread = 2;   // powers of two between a block and its field's scale
+constexpr int kFixedNear = 2;     // powers of two between a value that covers a sum and its scale
 constexpr int kFixedColour = 60;  // and between colour rows or columns at most
 // Powers of two that fixed_value may apply: a sum is 1 to 2^62 units.
 constexpr int kFixedMinUp = -1022, kFixedMaxUp = 960;
@@ -51,6 +56,14 @@ template <int TPS> __device__ __forceinline__ int group_max(int v)
   return v;
 }
 
+// The bits of the values of a site's TPS threads.
+template <int TPS> __device__ __forceinline__ uint32_t group_or(uint32_t v)
+{
+#pragma unroll
+  for (int o = TPS / 2; o > 0; o >>= 1) v |= __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
 // The scales of one site: entry [a][d] of field f at 2^(E[f] + r[a] + c[d] - 1023).
 struct FixedScales {
   int E[2], r[3], c[3];
@@ -60,31 +73,34 @@ struct FixedScales {
 // threads; false if they do not suit the integer form.
 // blk: NA of the first field, then of the second (none: one field).  Without
 // COLOUR there is one scale per field (contractions that sum over colours).
+// near: the entries of each block near their scale, a bit each.
 template <int TPS, int NA, bool COLOUR = true, int N>
-__device__ __forceinline__ bool fixed_scales(const double2 *const (&blk)[N], FixedScales &f)
+__device__ __forceinline__ bool fixed_scales(const double2 *const (&blk)[N], FixedScales &f, uint32_t (&near)[N])
 {
   f.E[0] = f.E[1] = 0;
 #pragma unroll
   for (int a = 0; a < 3; ++a) f.r[a] = f.c[a] = 0;
-  int e[N][9], most[N];  // high words without the sign, then biased exponents (0: zero or denormal)
+  int e[N][9];  // high words without the sign, then biased exponents (0: zero or denormal)
 #pragma unroll
   for (int n = 0; n < N; ++n) {
-    most[n] = 0;
+    int most = 0;
 #pragma unroll
     for (int k = 0; k < 9; ++k) {
       const double2 v = blk[n][k];
       e[n][k] = max(__double2hiint(v.x) & 0x7fffffff, __double2hiint(v.y) & 0x7fffffff);
-      most[n] = max(most[n], e[n][k]);
+      most = max(most, e[n][k]);
     }
-    most[n] >>= 20;
-    f.E[n < NA ? 0 : 1] = max(f.E[n < NA ? 0 : 1], most[n]);
+    near[n] = 0;
+    f.E[n < NA ? 0 : 1] = max(f.E[n < NA ? 0 : 1], most >> 20);
   }
   f.E[0] = group_max<TPS>(f.E[0]);
   f.E[1] = NA < N ? group_max<TPS>(f.E[1]) : f.E[0];
-  bool ok = min(f.E[0], f.E[1]) >= kFixedMinExp && max(f.E[0], f.E[1]) <= kFixedMaxExp;
+  const bool ok = min(f.E[0], f.E[1]) >= kFixedMinExp && max(f.E[0], f.E[1]) <= kFixedMaxExp;
   if constexpr (!COLOUR) {
 #pragma unroll
-    for (int n = 0; n < N; ++n) ok = ok && (most[n] - f.E[n < NA ? 0 : 1] >= -kFixedSpread || most[n] == 0);
+    for (int n = 0; n < N; ++n)
+#pragma unroll
+      for (int k = 0; k < 9; ++k) near[n] |= (uint32_t)(e[n][k] >= (f.E[n < NA ? 0 : 1] - kFixedNear) << 20) << k;
     return ok;
   }
   // Exponents of zeros (0) lie more than kFixedColour below every field's scale.
@@ -100,21 +116,56 @@ __device__ __forceinline__ bool fixed_scales(const double2 *const (&blk)[N], Fix
       m = max(m, max(max(e[n][3 * a], e[n][3 * a + 1]), e[n][3 * a + 2]) - f.E[n < NA ? 0 : 1]);
     f.r[a] = group_max<TPS>(m);
   }
-  int col[N][3];  // the columns' largest in the scales of the rows
 #pragma unroll
-  for (int d = 0; d < 3; ++d) {
+  for (int d = 0; d < 3; ++d) {  // the columns' largest in the scales of the rows
     int m = -kFixedColour;
 #pragma unroll
-    for (int n = 0; n < N; ++n) {
-      col[n][d] = max(max(e[n][d] - f.r[0], e[n][3 + d] - f.r[1]), e[n][6 + d] - f.r[2]) - f.E[n < NA ? 0 : 1];
-      m = max(m, col[n][d]);
-    }
+    for (int n = 0; n < N; ++n)
+      m = max(m, max(max(e[n][d] - f.r[0], e[n][3 + d] - f.r[1]), e[n][6 + d] - f.r[2]) - f.E[n < NA ? 0 : 1]);
     f.c[d] = group_max<TPS>(m);
   }
 #pragma unroll
-  for (int n = 0; n < N; ++n) {
-    const int m = max(max(col[n][0] - f.c[0], col[n][1] - f.c[1]), col[n][2] - f.c[2]);
-    ok = ok && (m >= -kFixedSpread || most[n] == 0);
+  for (int k = 0; k < 9; ++k) {
+    const int scale = f.r[k / 3] + f.c[k % 3] - kFixedNear;
+#pragma unroll
+    for (int n = 0; n < N; ++n) near[n] |= (uint32_t)(e[n][k] >= f.E[n < NA ? 0 : 1] + scale) << k;
+  }
+  return ok;
+}
+
+// What of block w's nine colour entries is near its scale, by the thread of the site's
+// 16 that holds the block.
+__device__ __forceinline__ uint32_t block_word(uint32_t w, int block) { return __shfl_sync(0xffffffffu, w, block, 16); }
+
+// A block's near bits for wedge_cover: the columns rotated by one in the lower half and
+// by two in the upper one, rows 0 to 2 and again 0 and 1.
+__device__ __forceinline__ uint32_t cover_word(uint32_t near)
+{
+  const uint32_t c1 = ((near >> 1) & 0333u) | ((near & 0111u) << 2), c2 = ((near >> 2) & 0111u) | ((near & 0333u) << 1);
+  return ((c1 | c1 << 9) & 0x7fffu) | ((c2 | c2 << 9) & 0x7fffu) << 16;
+}
+// Which entries [a][d] of x ^ y have a product of two near values, x[a + r][d + c] and
+// y[a + 2 r][d + 2 c], r, c = 1 or 2: bit 3 a + d of either half (c = 1 and c = 2).
+__device__ __forceinline__ uint32_t wedge_cover(uint32_t x, uint32_t y)
+{
+  const uint32_t z = __byte_perm(y, 0, 0x1032);
+  return ((x >> 3) & (z >> 6)) | ((x >> 6) & (z >> 3));
+}
+// Whether the covers of a sum's wedges, or-ed, leave no entry out.
+__device__ __forceinline__ bool wedges_covered(uint32_t c) { return ((c | c >> 16) & 0x1ffu) == 0x1ffu; }
+
+// Whether the 16 products of colour blocks that a class of meson pairs sums, one block
+// of either field each in some order, hold two near values at one colour entry: so it
+// is if more than 16 of the site's 32 blocks are near there.  Usually the first entry
+// shows it.
+__device__ __forceinline__ bool pairs_covered(uint32_t a, uint32_t b, bool live)
+{
+  const uint32_t site = 0xffffu << (threadIdx.x & 16u);
+  bool ok = !live;
+#pragma unroll 1
+  for (int k = 0; k < 9 && !__all_sync(0xffffffffu, ok); ++k) {
+    const uint32_t x = __ballot_sync(0xffffffffu, (a >> k) & 1u), y = __ballot_sync(0xffffffffu, (b >> k) & 1u);
+    ok = ok || __popc(x & site) + __popc(y & site) > 16;
   }
   return ok;
 }
@@ -351,6 +402,7 @@ __device__ __forceinline__ cx<double> fixed_conj_dot(const int4 (&x)[9], const i
 struct FixedDotBlock {
   int4 g[9];
   int E, up;
+  uint32_t near;  // the entries near the scale; all of a block of zeros, whose dots are exact
   // The block's scale beside that of the field; false if the block does not suit the
   // integer form: a value is not finite, all are so small that denormal ones count, or
   // a dot could leave the exponents of a double (fixed_value tests nothing).  Its values
@@ -366,6 +418,12 @@ struct FixedDotBlock {
       any |= (uint32_t)(hx | hy) | (uint32_t)__double2loint(v[k].x) | (uint32_t)__double2loint(v[k].y);
       most = max(most, x);
       E = max(E, x ? x + f.r[k / 3] + f.c[k % 3] : -8192);
+    }
+    near = any ? 0u : 0x1ffu;
+#pragma unroll
+    for (int k = 0; k < 9; ++k) {
+      const int x = max(__double2hiint(v[k].x) & 0x7fffffff, __double2hiint(v[k].y) & 0x7fffffff) >> 20;
+      near |= (uint32_t)(x + f.r[k / 3] + f.c[k % 3] >= E - kFixedNear) << k;
     }
     up = E + f.E[0] - 2 * 1023 - 54;
     return any == 0 || (most < 2047 && most >= kFixedMinDot && up >= kFixedMinUp && up <= kFixedMaxUp);

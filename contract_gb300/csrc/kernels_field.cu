@@ -26,7 +26,8 @@ template <Wedges KIND> static VariantSet<float, 4> shapes_m()
 }
 // complex128: integer pipe.  24^4, ms in this order: four wedges a block 1.76 to 1.80,
 // 1.85 to 1.87, 1.83 to 1.86 (5.2 to 5.7 in FP64), the closed loop 0.80, 0.88, 0.85
-// (2.29), one wedge a block 1.25, 0.86, 0.86 (1.44).
+// (2.29).  One wedge a block runs in FP64 (WedgeFieldOp::with_q): 0.94 at 24^3 x 16 in the second shape (0.98 on a
+// CTA-wide ring).
 template <Wedges KIND> static VariantSet<double, 3> shapes_p()
 {
   return {{wedges<double, double2, 4, 3, 2, KIND>, wedges<double, double2, 4, 2, 3, KIND>,

@@ -85,7 +85,16 @@ struct WedgeFieldOp : RingOp<R, S, CW, 16, NST, MINB> {
     const int r = sub >> 2, c = sub & 3, turn = (f.rows >> 8) & 7;
     if constexpr (sizeof(R) == 8) {
       FixedScales fs;
-      if (fields_to_fixed<16>(X, Y, sub, live, fs)) {
+      if (fields_to_fixed(X, Y, sub, live, fs, [&](uint32_t x, uint32_t y) {
+            uint32_t cover = 0;
+#pragma unroll
+            for (int t = 0; t < 4; ++t) {
+              int xb, yb;
+              term(f, r, c, t, xb, yb);
+              cover |= wedge_cover(block_word(x, xb), block_word(y, yb));
+            }
+            return cover;
+          })) {
         fixed_wedge_sum(0, 4, fs, [&](int k, const int4 *&x, const int4 *&y) {
           int xb, yb;
           term(f, r, c, two_bits(f.rows, 2 * k), xb, yb);
@@ -117,30 +126,14 @@ struct WedgeFieldOp : RingOp<R, S, CW, 16, NST, MINB> {
     }
   }
 
-  // One wedge a block, with Q (in q) of the field N.
-  __device__ __forceinline__ static void with_q(const BaryonSpin<R> &b, S *X, const S *N, S *q, int sub, bool live,
-                                                cx<R> (&d)[9])
+  // One wedge a block, with Q (in q) of the field N.  FP64 in complex128: the four products
+  // of an entry are too few for one of them to be near its scale as a rule.
+  __device__ __forceinline__ static void with_q(const BaryonSpin<R> &b, S *X, const S *N, S *q, int sub, cx<R> (&d)[9])
   {
     const FusedSpin f = b.fu;
     const int xb = sub ^ (f.s & 3) << 2 ^ ((f.s >> 2) & 3);  // block (r ^ s1, c ^ s2)
     build_q<R, S, 16, 1>(b, N, q, sub);
     __syncwarp();
-    if constexpr (sizeof(R) == 8) {
-      FixedScales fs;
-      const double2 *blk[2] = {X + sub * 9, q};
-      const bool ok = fixed_scales<16, 1>(blk, fs);
-      if (__all_sync(0xffffffffu, ok || !live)) {
-        block_to_fixed(reinterpret_cast<int4 *>(X + sub * 9), blk[0], fs, 0);
-        if (sub == 0) block_to_fixed(reinterpret_cast<int4 *>(q), q, fs, 1);
-        __syncwarp();
-        fixed_wedge_sum(0, 1, fs, [&](int, const int4 *&x, const int4 *&y) {
-          x = reinterpret_cast<const int4 *>(X) + xb * 9;
-          y = reinterpret_cast<const int4 *>(q);
-          return false;
-        }, d);
-        return;
-      }
-    }
     cx<R> x[9], y[9];
 #pragma unroll
     for (int e = 0; e < 9; ++e) d[e] = czero<R>();
@@ -156,7 +149,9 @@ struct WedgeFieldOp : RingOp<R, S, CW, 16, NST, MINB> {
     const uint32_t ph = (b.ph1[0][i] + b.ph2[0][l]) & 3u;
     if constexpr (sizeof(R) == 8) {
       FixedScales fs;
-      if (fields_to_fixed<16>(A, B, sub, live, fs)) {
+      if (fields_to_fixed(A, B, sub, live, fs, [&](uint32_t x, uint32_t y) {
+            return group_or<16>(wedge_cover(block_word(x, xb), block_word(y, yb)));
+          })) {
         const uint32_t common = (b.ph1[0][0] & 1u) + (b.ph2[0][0] & 1u);
         const longlong2 d = fixed_wedge_scatter(reinterpret_cast<const int4 *>(A) + xb * 9,
                                                 reinterpret_cast<const int4 *>(B) + yb * 9, ((ph - common) & 2u) != 0, sub);
@@ -200,7 +195,7 @@ struct WedgeFieldOp : RingOp<R, S, CW, 16, NST, MINB> {
       }
     } else {
       cx<R> d[9];
-      if constexpr (LOOP) with_q(b, in[0], in[1], scratch, sub, live, d);
+      if constexpr (LOOP) with_q(b, in[0], in[1], scratch, sub, d);
       else sums(b, in[0], in[1], sub, live, d);
       phase9(d, phase(b, r, c) & 3u);
       if constexpr (KIND == Wedges::Diquark) {

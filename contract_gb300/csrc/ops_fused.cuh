@@ -145,46 +145,59 @@ __device__ __forceinline__ void open_diquark_fixed(const FusedSpin &f, const int
     }, g[t]);
 }
 
-// Converts the site's blocks of P_i and P_j in place, if every site of the warp
-// suits the integer form.
-template <int TPS>
-__device__ __forceinline__ bool fields_to_fixed(double2 *A, double2 *B, int sub, bool live, FixedScales &fs)
+// What open_diquark_fixed's sum for thread (s, n0) covers.  One field: G[s][n] is H[s][n]
+// with H[n][s], the other thread's.
+template <int NROW>
+__device__ __forceinline__ uint32_t open_diquark_cover(const FusedSpin &f, uint32_t x, uint32_t y, int s, int n0)
 {
-  constexpr int NB = 16 / TPS;
-  const double2 *blk[2 * NB];
+  uint32_t c = 0;
 #pragma unroll
-  for (int k = 0; k < NB; ++k) {
-    blk[k] = A + (sub + k * TPS) * 9;
-    blk[NB + k] = B + (sub + k * TPS) * 9;
+  for (int k = 0; k < NROW; ++k) {
+    const int i = two_bits(f.rows, 2 * k);
+    c |= wedge_cover(block_word(x, i * 4 + s), block_word(y, (i ^ (f.s & 3)) * 4 + n0));
   }
-  const bool ok = fixed_scales<TPS, NB>(blk, fs);
+  return NROW == 4 ? c : c | block_word(c, n0 * 4 + s);
+}
+
+// Converts the site's blocks of two fields, one of each per thread, in place, if every
+// site of the warp suits the integer form.  cover(x, y): what the thread's sum of wedges
+// covers, from its own blocks' words.
+template <class Cover>
+__device__ __forceinline__ bool fields_to_fixed(double2 *A, double2 *B, int sub, bool live, FixedScales &fs, Cover cover)
+{
+  const double2 *blk[2] = {A + sub * 9, B + sub * 9};
+  uint32_t near[2];
+  const bool scaled = fixed_scales<16, 1>(blk, fs, near);
+  const bool ok = wedges_covered(cover(cover_word(near[0]), cover_word(near[1]))) && scaled;
   if (!__all_sync(0xffffffffu, ok || !live)) return false;
-#pragma unroll
-  for (int k = 0; k < NB; ++k) {
-    block_to_fixed(reinterpret_cast<int4 *>(A + (sub + k * TPS) * 9), blk[k], fs, 0);
-    if (A != B) block_to_fixed(reinterpret_cast<int4 *>(B + (sub + k * TPS) * 9), blk[NB + k], fs, 1);
-  }
+  block_to_fixed(reinterpret_cast<int4 *>(A + sub * 9), blk[0], fs, 0);
+  if (A != B) block_to_fixed(reinterpret_cast<int4 *>(B + sub * 9), blk[1], fs, 1);
   __syncwarp();
   return true;
 }
 
 // Converts the blocks of P_n in place likewise, if the thread's blocks g of G, which
-// may come from the FP64 form, suit it as well.
-template <int TPS, int NN>
+// may come from the FP64 form, suit it as well.  covered(near): whether all of the
+// thread's dots are, from its own block's near bits.
+template <int NN, class Covered>
 __device__ __forceinline__ bool dots_to_fixed(double2 *N, const cx<double> (&g)[NN][9], int sub, bool live,
-                                              FixedDotBlock (&gb)[NN])
+                                              FixedDotBlock (&gb)[NN], Covered covered)
 {
-  constexpr int NB = 16 / TPS;
   FixedScales fs;
-  const double2 *blk[NB];
+  const double2 *blk[1] = {N + sub * 9};
+  uint32_t near[1];
+  bool ok = fixed_scales<16, 1>(blk, fs, near);
+  uint32_t any = 0;  // dots with a block of zeros are exact
 #pragma unroll
-  for (int k = 0; k < NB; ++k) blk[k] = N + (sub + k * TPS) * 9;
-  bool ok = fixed_scales<TPS, NB>(blk, fs);
+  for (int k = 0; k < 9; ++k) {
+    const int4 v = reinterpret_cast<const int4 *>(blk[0])[k];
+    any |= (uint32_t)(v.x | v.z) | ((uint32_t)(v.y | v.w) & 0x7fffffffu);
+  }
 #pragma unroll
   for (int t = 0; t < NN; ++t) ok = gb[t].fits(g[t], fs) && ok;
+  ok = covered(any ? near[0] : 0x1ffu) && ok;
   if (!__all_sync(0xffffffffu, ok || !live)) return false;
-#pragma unroll
-  for (int k = 0; k < NB; ++k) block_to_fixed(reinterpret_cast<int4 *>(N + (sub + k * TPS) * 9), blk[k], fs, 0);
+  block_to_fixed(reinterpret_cast<int4 *>(N + sub * 9), blk[0], fs, 0);
 #pragma unroll
   for (int t = 0; t < NN; ++t) gb[t].set(g[t], fs);
   __syncwarp();
@@ -268,7 +281,10 @@ struct BaryonFusedOp {
     S *A = in[0], *B = SAME ? in[0] : in[1];
     if constexpr (sizeof(R) == 8) {
       FixedScales fs;
-      if (fields_to_fixed<TPS>(A, B, sub, live, fs))
+      static_assert(TPS == 16, "one block of G per thread");
+      if (fields_to_fixed(A, B, sub, live, fs, [&](uint32_t x, uint32_t y) {
+            return open_diquark_cover<SAME ? 2 : 4>(f, x, y, s, n0);
+          }))
         open_diquark_fixed<SAME ? 2 : 4, NN>(f, reinterpret_cast<const int4 *>(A), reinterpret_cast<const int4 *>(B), s, n0, fs, g);
       else
         open_diquark<SAME ? 2 : 4, NN, R, S>(f, A, B, s, n0, g);
@@ -370,7 +386,21 @@ struct BaryonFusedOp {
     if constexpr (sizeof(R) == 8 && SRC > 0) {
       __syncwarp();  // the loop above has read P_n
       FixedDotBlock gb[NN];
-      if (dots_to_fixed<TPS, NN>(N, g, sub, live, gb)) dots(gb);
+      const auto covered = [&](uint32_t near) {
+        bool ok = true;
+#pragma unroll
+        for (int d = 0; d < ND; ++d) {
+          const int sk = two_bits(f.s, 4 + 2 * d);
+#pragma unroll
+          for (int t = 0; t < NN; ++t) {
+            const int n = n0 + t;
+            ok = (gb[t].near & block_word(near, (n ^ sk) * 4 + l)) != 0 && ok;
+            ok = (gb[t].near & block_word(near, (s ^ sk) * 4 + (n ^ s2))) != 0 && ok;
+          }
+        }
+        return ok;
+      };
+      if (dots_to_fixed(N, g, sub, live, gb, covered)) dots(gb);
       else plain();
     } else {
       plain();

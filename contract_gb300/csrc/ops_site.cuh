@@ -33,12 +33,14 @@ struct BaryonLoopOp : RingOp<R, S, CW, TPS, NST, MINB> {
     if constexpr (sizeof(R) == 8) {
       static_assert(TPS == 16, "one (i, l) pair per thread");
       FixedScales fs;
-      if (fields_to_fixed<TPS>(in[0], in[1], sub, live, fs)) {
+      const int i = sub >> 2, l = sub & 3, xb = i * 4 + b.perm2[l], yb = b.perm1[i] * 4 + l;
+      if (fields_to_fixed(in[0], in[1], sub, live, fs, [&](uint32_t x, uint32_t y) {
+            return group_or<16>(wedge_cover(block_word(x, xb), block_word(y, yb)));
+          })) {
         // all wedges of the site have one scale: they meet as integers, entry e of
         // the sum with thread e, which multiplies it by Q's
-        const int i = sub >> 2, l = sub & 3;
-        const int4 *x = reinterpret_cast<const int4 *>(in[0]) + (i * 4 + b.perm2[l]) * 9;
-        const int4 *y = reinterpret_cast<const int4 *>(in[1]) + (b.perm1[i] * 4 + l) * 9;
+        const int4 *x = reinterpret_cast<const int4 *>(in[0]) + xb * 9;
+        const int4 *y = reinterpret_cast<const int4 *>(in[1]) + yb * 9;
         // Gamma entries: one common power of i, and signs
         const uint32_t common = (b.ph1[0][0] & 1u) + (b.ph2[0][0] & 1u);
         const bool minus = ((b.ph1[0][i] ^ b.ph2[0][l]) & 2u) != 0;
@@ -67,9 +69,14 @@ struct BaryonTriOp : RingOp<R, S, CW, 16, NST, MINB> {
     __syncwarp();
     if constexpr (sizeof(R) == 8) {
       FixedScales fs;
-      if (fields_to_fixed<16>(in[1], scratch, sub, live, fs)) {
+      const int i = sub >> 2, l = sub & 3, j = b.perm1[i];
+      if (fields_to_fixed(in[1], scratch, sub, live, fs, [&](uint32_t x, uint32_t y) {
+            uint32_t c = 0;
+#pragma unroll
+            for (int m = 0; m < 4; ++m) c |= wedge_cover(block_word(x, j * 4 + m), block_word(y, m * 4 + l));
+            return c;
+          })) {
         const int4 *B = reinterpret_cast<const int4 *>(in[1]), *np = reinterpret_cast<const int4 *>(scratch);
-        const int i = sub >> 2, l = sub & 3, j = b.perm1[i];
         cx<double> d[9], a[9];
         fixed_wedge_sum(0, 4, fs, [&](int m, const int4 *&x, const int4 *&y) {
           x = B + (j * 4 + m) * 9;
@@ -96,9 +103,15 @@ struct BaryonTriGammaOp : RingOp<R, S, CW, TPS, NST, MINB> {
       static_assert(TPS == 16, "one (i, l) pair per thread");
       const CliffordSet<R> &cl = b.cl;
       FixedScales fs;
-      if (fields_to_fixed<TPS>(in[1], in[2], sub, live, fs)) {
+      const int i = sub >> 2, l = sub & 3, j = b.perm1[i];
+      if (fields_to_fixed(in[1], in[2], sub, live, fs, [&](uint32_t x, uint32_t y) {
+            uint32_t c = 0;
+#pragma unroll
+            for (int m = 0; m < 4; ++m)
+              c |= wedge_cover(block_word(x, j * 4 + m), block_word(y, cl.perm[0][m] * 4 + l));
+            return c;
+          })) {
         const int4 *B = reinterpret_cast<const int4 *>(in[1]), *N = reinterpret_cast<const int4 *>(in[2]);
-        const int i = sub >> 2, l = sub & 3, j = b.perm1[i];
         cx<double> d[9], a[9];
         // the gamma matrix's entries differ by signs
         fixed_wedge_sum(0, 4, fs, [&](int m, const int4 *&x, const int4 *&y) {
@@ -160,7 +173,18 @@ struct BaryonTriRankOp : RingOp<R, S, CW, 8, NST, MINB> {
       FixedScales fs;
       S *own = X + (two ? sub : sub & 3) * 9;
       const double2 *blk[3] = {A + sub * 9, A + (sub + 8) * 9, own};
-      const bool ok = fixed_scales<8, 2>(blk, fs);
+      uint32_t near[3];
+      bool ok = fixed_scales<8, 2>(blk, fs, near);
+      const uint32_t w0 = cover_word(near[0]), w1 = cover_word(near[1]), wx = cover_word(near[2]);
+      uint32_t c = 0;
+#pragma unroll 2
+      for (int k = k0; k < k1; ++k) {
+        const int i = two_bits(f.rows, 2 * k), xb = i * 4 + s;
+        const uint32_t lo = __shfl_sync(0xffffffffu, w0, xb & 7, 8), hi = __shfl_sync(0xffffffffu, w1, xb & 7, 8);
+        c |= wedge_cover(xb & 8 ? hi : lo, __shfl_sync(0xffffffffu, wx, r * 4 + (i ^ s1), 8));
+      }
+      if (!two) c |= __shfl_xor_sync(0xffffffffu, c, 4);  // the two halves of the rows meet in the dot with Y
+      ok = wedges_covered(c) && ok;
       done = __all_sync(0xffffffffu, ok || !live);
       if (done) {
         block_to_fixed(reinterpret_cast<int4 *>(A + sub * 9), blk[0], fs, 0);
@@ -263,7 +287,8 @@ struct MesonAllOp : RingOp<R, S, CW, 16, NST, MINB> {
     if constexpr (sizeof(R) == 8) {
       FixedScales fs;
       const double2 *blk[2] = {in[0] + sub * 9, in[1] + sub * 9};
-      const bool ok = fixed_scales<16, 1, false>(blk, fs);
+      uint32_t near[2];
+      const bool scaled = fixed_scales<16, 1, false>(blk, fs, near), ok = pairs_covered(near[0], near[1], live) && scaled;
       done = __all_sync(0xffffffffu, ok || !live);
       if (done) {
         block_to_fixed(reinterpret_cast<int4 *>(in[0] + sub * 9), blk[0], fs, 0);
@@ -411,7 +436,8 @@ struct MesonPairs {
     const int s = sub >> 2, u = sub & 3;
     FixedScales fs;
     const double2 *blk[2] = {in[0] + sub * 9, in[1] + sub * 9};
-    const bool ok = fixed_scales<16, 1, false>(blk, fs);
+    uint32_t near[2];
+    const bool scaled = fixed_scales<16, 1, false>(blk, fs, near), ok = pairs_covered(near[0], near[1], live) && scaled;
     if (__all_sync(0xffffffffu, ok || !live)) {
 #pragma unroll 1
       for (int q = 0; q < 2; ++q)
