@@ -348,9 +348,20 @@ struct MesonAllOp : RingOp<R, S, CW, 16, NST, MINB> {
 // Alone 0.77 ms at 18 x 15 x 20 x 28, bound by the integer pipes.  The projection of 125
 // momenta is off by 3.9e-16 of its norm against extended precision (4.3e-16 in FP64).
 struct MesonPairs {
-  // o[ha][hb] += the Walsh-Hadamard sums w over l of row i's four products
+  // o[ha][hb] += the Walsh-Hadamard sums w over l of row i's four products.  In FP64 row 0
+  // begins the sums instead of being added to zero, and so does the first pair of a row: 64
+  // adds of 224 less on the pipe that bounds it (integers: a branch costs more).
   template <class V> __device__ __forceinline__ static void add_row(V (&o)[4][4], const V (&w)[4], int i)
   {
+    if constexpr (std::is_floating_point<V>::value) {
+      if (i == 0) {  // uniform
+#pragma unroll
+        for (int ha = 0; ha < 4; ++ha)
+#pragma unroll
+          for (int h = 0; h < 4; ++h) o[ha][h] = w[h];
+        return;
+      }
+    }
 #pragma unroll
     for (int ha = 0; ha < 4; ++ha) {
       const bool minus = __popc(ha & i) & 1;  // uniform
@@ -362,6 +373,11 @@ struct MesonPairs {
   template <class V> __device__ __forceinline__ static void add_pair(V (&w)[4], const V (&t)[2], int hi)
   {
     const V a = t[0] + t[1], b = t[0] - t[1];
+    if (std::is_floating_point<V>::value && hi == 0) {
+      w[0] = w[2] = a;
+      w[1] = w[3] = b;
+      return;
+    }
     w[0] += a;
     w[1] += b;
     w[2] += hi ? -a : a;
