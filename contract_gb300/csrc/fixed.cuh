@@ -28,9 +28,9 @@
 // 3.3e-17 and 3.4e-17 against 8.5e-17, 1.1e-16 and 1.1e-16; with 3 for kFixedNear the
 // first two come to 8.7e-17 against 8.9e-17, with 1 a quarter of Gaussian sites is
 // refused.  Also every value must be finite and all exponents leave room for the
-// products; otherwise the warp takes the FP64 form for its sites.  Measured against
-// extended precision (4096 outputs of all types, two projectors): 1.9e-16 of their norm
-// for Gaussian fields, 2.3e-16 in FP64.
+// products; otherwise the warp takes the FP64 form for its sites.  In the norm, against
+// extended precision (test_extended_precision_gpu.py): all types 1.5e-16, one call a type
+// 1.8e-16, all partners of a meson Gamma 1.2e-16, in FP64 2.2e-16, 2.3e-16 and 1.8e-16.
 #pragma once
 
 #include "common.cuh"

@@ -346,7 +346,8 @@ struct MesonAllOp : RingOp<R, S, CW, 16, NST, MINB> {
 // quarter units before the four rows meet.
 //
 // Alone 0.77 ms at 18 x 15 x 20 x 28, bound by the integer pipes.  The projection of 125
-// momenta is off by 3.9e-16 of its norm against extended precision (4.3e-16 in FP64).
+// momenta is off by 2.5e-16 of its norm against extended precision at 18 x 15 x 20 x 2 (3.2e-16 in FP64;
+// test_extended_precision_gpu.py).
 struct MesonPairs {
   // o[ha][hb] += the Walsh-Hadamard sums w over l of row i's four products.  In FP64 row 0
   // begins the sums instead of being added to zero, and so does the first pair of a row: 64
