@@ -1105,7 +1105,6 @@ bool meson_batch_setup(cgb::MomBatchParams &mp, size_t &plane_floats, const Cont
     b.out = static_cast<double2 *>(it.correl);
     for (int k = 0; k < 4; ++k) b.latt[k] = l[k];
     b.unit_begin = units;
-    b.tpp = (l[0] * l[1] + 15) / 16;
     b.fin_begin = fin;
     const int ex = ext_index(l[0]), ey = ext_index(l[1]), ez = ext_index(l[2]);
     if ((int)ext.size() > cgb::kMomBatchMaxExt)

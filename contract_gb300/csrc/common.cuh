@@ -116,14 +116,6 @@ template <class R> __device__ __forceinline__ cx<R> shfl_xor(cx<R> v, int lane_m
   return {__shfl_xor_sync(0xffffffffu, v.x, lane_mask), __shfl_xor_sync(0xffffffffu, v.y, lane_mask)};
 }
 
-// Sum v over the TPS consecutive lanes of a group (TPS a power of two <= 32).
-template <int TPS, class R> __device__ __forceinline__ cx<R> group_sum(cx<R> v)
-{
-#pragma unroll
-  for (int o = TPS / 2; o > 0; o >>= 1) v = cadd(v, shfl_xor(v, o));
-  return v;
-}
-
 // Sum each of NVAL values over the TPS threads of a site, leaving the sum of
 // value r with the 2^SH threads whose sub >> SH == r: recursive halving while
 // a thread holds more than one value (at the step of lane distance h it keeps
@@ -391,12 +383,12 @@ __device__ __forceinline__ void bulk_g2s(void *sdst, const void *gsrc, uint32_t 
                : "memory");
 }
 
-// Shared -> global bulk copy; tracked by the issuing thread's bulk group.
 // Global memory into L2: address 16-byte aligned, bytes a multiple of 16.
 __device__ __forceinline__ void bulk_prefetch_l2(const void *gsrc, uint32_t bytes)
 {
   asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(gsrc), "r"(bytes) : "memory");
 }
+// Shared -> global bulk copy; tracked by the issuing thread's bulk group.
 __device__ __forceinline__ void bulk_s2g(void *gdst, const void *ssrc, uint32_t bytes)
 {
   asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(gdst), "r"(smem_addr(ssrc)),

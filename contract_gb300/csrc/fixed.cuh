@@ -25,8 +25,8 @@
 // of its products, is below what FP64 leaves.  In exact arithmetic on the host, rms over
 // the sums accepted: Gaussian blocks 1.8e-17 against 6.0e-17 in FP64, blocks near a
 // multiple of the unit matrix with the rest 0.25, 0.06 and 0.001 as large 4.2e-17,
-// 3.3e-17 and 3.4e-17 against 8.5e-17, 1.1e-16 and 1.1e-16; with 3 for kFixedNear the
-// first two come to 8.7e-17 against 8.9e-17, with 1 a quarter of Gaussian sites is
+// 3.3e-17 and 3.4e-17 against 8.5e-17, 1.1e-16 and 1.1e-16; with 3 for kFixedNear an
+// eighth as large gives 8.7e-17 against 8.9e-17, with 1 a quarter of Gaussian sites is
 // refused.  Also every value must be finite and all exponents leave room for the
 // products; otherwise the warp takes the FP64 form for its sites.  In the norm, against
 // extended precision (test_extended_precision_gpu.py): all types 1.5e-16, one call a type

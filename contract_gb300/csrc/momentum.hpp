@@ -95,7 +95,6 @@ struct MomBatchItem {
   double2 *out;         // [np][Lt][256] complex128 correlators
   int latt[4];
   int unit_begin;       // first (t, z) plane of this item in the batch's unit space
-  int tpp;              // tiles of 16 sites per plane
   int fin_begin;        // first finalisation block of this item (nq * Lt blocks)
   uint8_t tx, ty, tz;   // phase table of the x, y and z extents
 };
