@@ -207,7 +207,7 @@ template <int UNROLL> struct LaneProducts<true, UNROLL> {
 // UNROLL: colours of a product in flight.
 template <int Z, int NS, bool SAME, int W, int UNROLL>
 __global__ void __launch_bounds__(32 * W, 1)
-  momentum_rows_kernel(const __grid_constant__ MomBatchParams p, const int nst, const unsigned long long wait_ns)
+  momentum_rows_kernel(const __grid_constant__ MomBatchParams p, const int nst)
 {
   using LP = LaneProducts<SAME, UNROLL>;
   constexpr int NP = LP::NP, PX = Z + 2 * NS;  // PX rows of 256: nx = 0, then +-k of each group
@@ -299,7 +299,7 @@ __global__ void __launch_bounds__(32 * W, 1)
       *abort_flag = 1;
       report(p.status, kDevErrWaitTimeout, (unsigned int)fc.unit);
       for (int s = cstage, n = 0, ps = cphase; n < in_flight; ++n) {
-        mbar_wait_bounded(&full[s], ps, wait_ns / 8);
+        mbar_wait_bounded(&full[s], ps, kWaitLimitNs / 8);
         if (++s == nst) {
           s = 0;
           ps ^= 1u;
@@ -309,7 +309,7 @@ __global__ void __launch_bounds__(32 * W, 1)
   };
   auto wait_all = [&](uint64_t *bar, uint32_t parity) -> bool {
     if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
-    const bool ok = mbar_wait_bounded(bar, parity, wait_ns);
+    const bool ok = mbar_wait_bounded(bar, parity, kWaitLimitNs);
     return __all_sync(0xffffffffu, ok) && !*abort_flag;
   };
 
@@ -528,8 +528,7 @@ template <int Z, int NS, bool SAME> cudaError_t launch_rows(const Job &job, cons
     if (dev < 64) attr_set[dev] = 1;
   }
   const int grid = std::min(p.total_units, job.num_sms);
-  momentum_rows_kernel<Z, NS, SAME, W, UNROLL><<<grid, 32 * W, smem, job.stream>>>(p, stages,
-                                                                                    job.wait_ns ? job.wait_ns : kWaitLimitNs);
+  momentum_rows_kernel<Z, NS, SAME, W, UNROLL><<<grid, 32 * W, smem, job.stream>>>(p, stages);
   return cudaGetLastError();
 }
 

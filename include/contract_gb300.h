@@ -69,7 +69,9 @@ int contract_check_device(void);
 /* Wall-time limit, in nanoseconds, of every wait of the site kernels on their
  * own copies (0 = the default, 2 s).  A wait that runs out sets the timeout
  * bit that contract_check_device() reports; the kernel then waits (bounded)
- * for its copies still in flight and returns, so the context stays usable. */
+ * for its copies still in flight and returns, so the context stays usable.
+ * The complex64 momentum projections keep the default: a limit that is not a
+ * constant costs them up to 4 % of their time. */
 void contract_set_wait_limit(unsigned long long ns);
 /* Test hook for the timeout path: in the next call only, the site kernel's
  * producer never issues (nor announces) the copies of the first tile of work
