@@ -20,14 +20,16 @@
 // about half a unit of 2^-54 of the two scales.  A small result therefore loses bits
 // that FP64 would keep, unless it is made of values near their scales.  So the integer
 // form is taken only where every sum has at least one product of two values that are
-// no more than kFixedNear powers of two below their scales (wedge_cover, pairs_covered,
+// no more than kFixedNear powers of two below their scales (wedge_cover, fixed_pair_scales,
 // FixedDotBlock::near): then its error, entry by entry and against the sum of the sizes
-// of its products, is below what FP64 leaves.  In exact arithmetic on the host, rms over
-// the sums accepted: Gaussian blocks 1.8e-17 against 6.0e-17 in FP64, blocks near a
-// multiple of the unit matrix with the rest 0.25, 0.06 and 0.001 as large 4.2e-17,
-// 3.3e-17 and 3.4e-17 against 8.5e-17, 1.1e-16 and 1.1e-16; with 3 for kFixedNear an
-// eighth as large gives 8.7e-17 against 8.9e-17, with 1 a quarter of Gaussian sites is
-// refused.  Also every value must be finite and all exponents leave room for the
+// of its products, is no larger than what FP64 leaves.  In exact arithmetic on the host,
+// rms over the sites accepted, sums of four wedges (of two): Gaussian blocks 1.9e-17
+// (2.8e-17) against 6.0e-17 in FP64; blocks near a multiple of the unit matrix, the rest
+// 0.35, 0.25 and 0.18 as large, 3.6e-17, 4.6e-17 and 5.5e-17 (5.5e-17, 6.4e-17 and
+// 6.9e-17) against 7.5e-17, 8.0e-17 and 8.3e-17 (7.1e-17, 7.4e-17 and 7.7e-17); with
+// 0.09 no site is accepted.  With 2 for kFixedNear 4 to 5 % of Gaussian sites have a sum
+// of two wedges that is refused, with 3 none of 3000.
+// Also every value must be finite and all exponents leave room for the
 // products; otherwise the warp takes the FP64 form for its sites.  In the norm, against
 // extended precision (test_extended_precision_gpu.py): all types 1.5e-16, one call a type
 // 1.8e-16, all partners of a meson Gamma 1.2e-16, in FP64 2.2e-16, 2.3e-16 and 1.8e-16.
@@ -38,7 +40,7 @@
 namespace cgb {
 
 constexpr int kFixedMinExp = 723, kFixedMaxExp = 1323;  // biased: 2^-300 to 2^300
-constexpr int kFixedNear = 2;     // powers of two between a value that covers a sum and its scale
+constexpr int kFixedNear = 3;     // powers of two between a value that covers a sum and its scale
 constexpr int kFixedColour = 60;  // and between colour rows or columns at most
 // Powers of two that fixed_value may apply: a sum is 1 to 2^62 units.
 constexpr int kFixedMinUp = -1022, kFixedMaxUp = 960;
@@ -71,15 +73,12 @@ struct FixedScales {
 
 // Scales of the fields whose blocks this thread reads, over the site's TPS
 // threads; false if they do not suit the integer form.
-// blk: NA of the first field, then of the second (none: one field).  Without
-// COLOUR there is one scale per field (contractions that sum over colours).
+// blk: NA of the first field, then of the second (none: one field).
 // near: the entries of each block near their scale, a bit each.
-template <int TPS, int NA, bool COLOUR = true, int N>
+template <int TPS, int NA, int N>
 __device__ __forceinline__ bool fixed_scales(const double2 *const (&blk)[N], FixedScales &f, uint32_t (&near)[N])
 {
   f.E[0] = f.E[1] = 0;
-#pragma unroll
-  for (int a = 0; a < 3; ++a) f.r[a] = f.c[a] = 0;
   int e[N][9];  // high words without the sign, then biased exponents (0: zero or denormal)
 #pragma unroll
   for (int n = 0; n < N; ++n) {
@@ -96,13 +95,6 @@ __device__ __forceinline__ bool fixed_scales(const double2 *const (&blk)[N], Fix
   f.E[0] = group_max<TPS>(f.E[0]);
   f.E[1] = NA < N ? group_max<TPS>(f.E[1]) : f.E[0];
   const bool ok = min(f.E[0], f.E[1]) >= kFixedMinExp && max(f.E[0], f.E[1]) <= kFixedMaxExp;
-  if constexpr (!COLOUR) {
-#pragma unroll
-    for (int n = 0; n < N; ++n)
-#pragma unroll
-      for (int k = 0; k < 9; ++k) near[n] |= (uint32_t)(e[n][k] >= (f.E[n < NA ? 0 : 1] - kFixedNear) << 20) << k;
-    return ok;
-  }
   // Exponents of zeros (0) lie more than kFixedColour below every field's scale.
 #pragma unroll
   for (int n = 0; n < N; ++n)
@@ -154,20 +146,38 @@ __device__ __forceinline__ uint32_t wedge_cover(uint32_t x, uint32_t y)
 // Whether the covers of a sum's wedges, or-ed, leave no entry out.
 __device__ __forceinline__ bool wedges_covered(uint32_t c) { return ((c | c >> 16) & 0x1ffu) == 0x1ffu; }
 
-// Whether the 16 products of colour blocks that a class of meson pairs sums, one block
-// of either field each in some order, hold two near values at one colour entry: so it
-// is if more than 16 of the site's 32 blocks are near there.  Usually the first entry
-// shows it.
-__device__ __forceinline__ bool pairs_covered(uint32_t a, uint32_t b, bool live)
+// Scales for dots of the blocks of two fields, one of each per thread of a site's 16: one
+// scale per field, colours being summed over.  False if they do not suit the integer form.
+// A class of meson pairs sums 16 products of blocks, every block of either field once, so
+// two near values meet at a colour entry if more than 16 of the site's 32 blocks are near
+// there; usually the first entry shows it.
+__device__ __forceinline__ bool fixed_pair_scales(const double2 *x, const double2 *y, bool live, FixedScales &f)
 {
-  const uint32_t site = 0xffffu << (threadIdx.x & 16u);
-  bool ok = !live;
-#pragma unroll 1
-  for (int k = 0; k < 9 && !__all_sync(0xffffffffu, ok); ++k) {
-    const uint32_t x = __ballot_sync(0xffffffffu, (a >> k) & 1u), y = __ballot_sync(0xffffffffu, (b >> k) & 1u);
-    ok = ok || __popc(x & site) + __popc(y & site) > 16;
+  int e[2][9];  // high words without the sign
+#pragma unroll
+  for (int n = 0; n < 2; ++n) {
+    int most = 0;
+#pragma unroll
+    for (int k = 0; k < 9; ++k) {
+      const double2 v = n ? y[k] : x[k];
+      e[n][k] = max(__double2hiint(v.x) & 0x7fffffff, __double2hiint(v.y) & 0x7fffffff);
+      most = max(most, e[n][k]);
+    }
+    f.E[n] = group_max<16>(most >> 20);
   }
-  return ok;
+#pragma unroll
+  for (int a = 0; a < 3; ++a) f.r[a] = f.c[a] = 0;
+  const bool fits = min(f.E[0], f.E[1]) >= kFixedMinExp && max(f.E[0], f.E[1]) <= kFixedMaxExp;
+  const uint32_t site = 0xffffu << (threadIdx.x & 16u);
+  bool covered = false;
+#pragma unroll
+  for (int k = 0; k < 9; ++k) {
+    if (__all_sync(0xffffffffu, covered || !fits || !live)) break;
+    const uint32_t a = __ballot_sync(0xffffffffu, e[0][k] >= (f.E[0] - kFixedNear) << 20);
+    const uint32_t b = __ballot_sync(0xffffffffu, e[1][k] >= (f.E[1] - kFixedNear) << 20);
+    covered = covered || __popc(a & site) + __popc(b & site) > 16;
+  }
+  return fits && covered;
 }
 
 // v as h 2^28 + l in units of 2^(E - 55).  The 53-bit significand, 3 bits up, goes

@@ -287,8 +287,7 @@ struct MesonAllOp : RingOp<R, S, CW, 16, NST, MINB> {
     if constexpr (sizeof(R) == 8) {
       FixedScales fs;
       const double2 *blk[2] = {in[0] + sub * 9, in[1] + sub * 9};
-      uint32_t near[2];
-      const bool scaled = fixed_scales<16, 1, false>(blk, fs, near), ok = pairs_covered(near[0], near[1], live) && scaled;
+      const bool ok = fixed_pair_scales(blk[0], blk[1], live, fs);
       done = __all_sync(0xffffffffu, ok || !live);
       if (done) {
         block_to_fixed(reinterpret_cast<int4 *>(in[0] + sub * 9), blk[0], fs, 0);
@@ -452,9 +451,7 @@ struct MesonPairs {
   {
     const int s = sub >> 2, u = sub & 3;
     FixedScales fs;
-    const double2 *blk[2] = {in[0] + sub * 9, in[1] + sub * 9};
-    uint32_t near[2];
-    const bool scaled = fixed_scales<16, 1, false>(blk, fs, near), ok = pairs_covered(near[0], near[1], live) && scaled;
+    const bool ok = fixed_pair_scales(in[0] + sub * 9, in[1] + sub * 9, live, fs);
     if (__all_sync(0xffffffffu, ok || !live)) {
 #pragma unroll 1
       for (int q = 0; q < 2; ++q)
