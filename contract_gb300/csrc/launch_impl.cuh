@@ -121,7 +121,7 @@ template <class Op, class K> cudaError_t launch_chunks(const Job &job, OpParams<
     if (!partial) return cudaErrorMemoryAllocation;
     p.out[0] = partial;
   }
-  const int grid = std::min((p.geom.total_chunks + Op::CW - 1) / Op::CW, ctas);
+  const int grid = std::min(ChunkWalk<Op>::ctas_for(p.geom.total_chunks), ctas);
   kernel<<<grid, 32 * Op::CW, smem, job.stream>>>(p);
   e = cudaGetLastError();
   if (e != cudaSuccess || job.per_site) return e;
