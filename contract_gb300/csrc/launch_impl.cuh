@@ -2,6 +2,7 @@
 #pragma once
 
 #include <algorithm>
+#include <climits>
 #include <mutex>
 
 #include "engine_warp.cuh"
@@ -9,12 +10,14 @@
 
 namespace cgb {
 
-// Tile geometry for an op with `sites` sites per tile, its chunks dealt
-// round-robin to `ctas` persistent CTAs.  About `chunks_per_cta` chunks per
-// CTA keeps the round-robin tail (CTAs that draw one chunk more than others)
-// near 1/chunks_per_cta of a CTA's work; chunks never span segments and hold
-// at most 64 tiles.
-inline TileGeom make_geom(const Job &job, int sites, long long ctas, int chunks_per_cta)
+// Tile geometry for an op with `sites` sites per tile, its chunks dealt round-robin to
+// `warps` persistent warps (or CTAs).  About `chunks_per_warp` chunks each keep the tail
+// of the round-robin (warps that draw one chunk more than others) near
+// 1/chunks_per_warp of a warp's work; chunks never span segments and hold at most 64
+// tiles.  `level`: where that makes chunks of four tiles or fewer, of these lengths and
+// longer ones the one that takes least time if all warps run alike and the end of a chunk
+// costs half a tile.
+inline TileGeom make_geom(const Job &job, int sites, long long warps, int chunks_per_warp, bool level = false)
 {
   TileGeom g {};
   g.volume = job.volume;
@@ -29,9 +32,20 @@ inline TileGeom make_geom(const Job &job, int sites, long long ctas, int chunks_
   }
   g.tiles_per_seg = (int)((g.seg_len + sites - 1) / sites);
   const long long tiles = (long long)g.tiles_per_seg * g.num_segs;
-  long long ct = tiles / (std::max(1LL, ctas) * chunks_per_cta);
-  g.chunk_tiles = (int)std::max(1LL, std::min(ct, 64LL));
-  g.chunk_tiles = std::min(g.chunk_tiles, g.tiles_per_seg);
+  warps = std::max(1LL, warps);
+  const int most = std::min(64, g.tiles_per_seg);
+  g.chunk_tiles = (int)std::max(1LL, std::min<long long>(tiles / (warps * chunks_per_warp), most));
+  if (level && g.chunk_tiles <= 4) {
+    long long best = LLONG_MAX;
+    for (int n = g.chunk_tiles; n <= most; ++n) {
+      const long long chunks = (long long)((g.tiles_per_seg + n - 1) / n) * g.num_segs;
+      const long long cost = (chunks + warps - 1) / warps * (2 * n + 1);
+      if (cost < best) {
+        best = cost;
+        g.chunk_tiles = n;
+      }
+    }
+  }
   g.chunks_per_seg = (g.tiles_per_seg + g.chunk_tiles - 1) / g.chunk_tiles;
   g.total_chunks = g.chunks_per_seg * g.num_segs;
   g.wait_ns = job.wait_ns ? job.wait_ns : kWaitLimitNs;
@@ -39,12 +53,16 @@ inline TileGeom make_geom(const Job &job, int sites, long long ctas, int chunks_
   return g;
 }
 
-// Chunks per resident CTA of the per-call kernels.  Measured at 24^3 x 64
-// (fused, triangle, loop, meson, diquark kernels): 8 chunks per SM (one to
-// three per CTA) left 3-10 % of the time in the round-robin tail; 24 to 96
-// per SM ran 3-10 % faster, the chunk partials' extra finalisation costing
-// no more than a few microseconds.
-constexpr int kChunksPerCta = 12;
+// Chunks per warp of the kernels of engine_warp.cuh (per CTA of field_kernel).  Sums in
+// complex64 then level the rounds: with one tile a chunk, as middle sizes had, the ends of
+// the chunks and the partials that they leave took a fifth of the time.  us before and
+// after, 12^3 x 24, 16 x 15 x 16 x 32 and 20^3 x 36: all types 47.7, 113.8, 210.6 and
+// 40.0, 93.5, 192.6; all partners of a Gamma 32.7, 55.4 and 23.6, 49.2 (the last alike);
+// one meson at the last two 53.5, 116.1 and 48.2, 103.9.  Longer chunks gain nothing
+// (loop at 28^3 x 56: 595, 621 with level rounds of 25 tiles).  Per-site results end a chunk
+// for nothing, and in complex128 fewer warps at work cost more than the ends: both keep
+// the plain rule (all types at 8^3 x 16 in complex128 79 us, 95 with level rounds).
+constexpr int kChunksPerWarp = 12;
 
 template <class K> struct KernelAttr {
   int bps[64] = {};  // resident CTAs per SM, per device ordinal (0 = not yet queried)
@@ -109,7 +127,8 @@ template <class Op, class K> cudaError_t launch_chunks(const Job &job, OpParams<
   cudaError_t e = prepare<Op>(kernel, smem, bps, 32 * Op::CW);
   if (e != cudaSuccess) return e;
   const int ctas = job.num_sms * bps;
-  p.geom = make_geom(job, ChunkWalk<Op>::SITES, (long long)ctas * Op::CW, kChunksPerCta);
+  p.geom = make_geom(job, ChunkWalk<Op>::SITES, (long long)ctas * Op::CW, kChunksPerWarp,
+                     sizeof(typename Op::R) == 4 && !job.per_site);
   p.status = job.status;
   static_assert(Op::NOUT <= 16, "at most 16 outputs per site");
   OutPtrs user_out {};
@@ -161,7 +180,7 @@ template <class Op> cudaError_t run_field(const Job &job, OpParams<typename Op::
   cudaError_t e = prepare<Op>(field_kernel<Op>, smem, bps);
   if (e != cudaSuccess) return e;
   const long long ctas = (long long)job.num_sms * bps;
-  p.geom = make_geom(j, Op::SITES, ctas, kChunksPerCta);
+  p.geom = make_geom(j, Op::SITES, ctas, kChunksPerWarp);
   p.status = job.status;
   const int grid = (int)std::min<long long>(p.geom.total_chunks, ctas);
   field_kernel<Op><<<grid, Op::THREADS, smem, job.stream>>>(p);
