@@ -1141,6 +1141,8 @@ bool meson_batch_setup(cgb::MomBatchParams &mp, size_t &plane_floats, const Cont
     mp.gz_plus[g] = first.gz_plus[g];
     mp.gz_minus[g] = first.gz_minus[g];
   }
+  mp.n_ext = (int)ext.size();
+  cgb::order_pairs(mp);
   return true;
 }
 

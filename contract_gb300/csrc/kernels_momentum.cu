@@ -563,8 +563,10 @@ static MomBatchParams single_item(const MomPlan &plan, const void *in_i, const v
   it.planes = planes;
   for (int k = 0; k < 4; ++k) it.latt[k] = plan.latt[k];
   it.ty = 1;
+  mp.n_ext = 2;
   for (int k = 0; k < plan.latt[0]; ++k) mp.tab[0][k] = make_float2((float)plan.cosx[k], (float)plan.sinx[k]);
   for (int k = 0; k < plan.latt[1]; ++k) mp.tab[1][k] = make_float2((float)plan.cosy[k], (float)plan.siny[k]);
+  order_pairs(mp);
   return mp;
 }
 

@@ -220,40 +220,21 @@ __global__ void __launch_bounds__(32 * W, 1)
   volatile int *abort_flag = reinterpret_cast<volatile int *>(smem + 504);
   float2 *tab = reinterpret_cast<float2 *>(smem + kRowTab);
   float4 *ph = reinterpret_cast<float4 *>(smem + kRowPh);
-  uint8_t *qlist = smem + kRowQ, *qstart = qlist + 32, *qslot = qlist + 64;  // pairs in the order of their slot
+  const uint8_t *qlist = reinterpret_cast<const PairOrder *>(smem + kRowQ)->list;
+  const uint8_t *qstart = reinterpret_cast<const PairOrder *>(smem + kRowQ)->start;
   float2 *G = reinterpret_cast<float2 *>(smem + kRowG);  // [warp][PX][256]
   unsigned char *ring = reinterpret_cast<unsigned char *>(G + (size_t)W * PX * 256) + (size_t)warp * nst * kStage;
 
-  if (threadIdx.x == 0) {
-    for (int s = 0; s < W * nst; ++s) mbar_init(&bars[s], 1);
-    mbar_init(ready, W);
-    mbar_init(consumed, W);
-    *abort_flag = 0;
+  if (lane == 0) {
+    for (int s = 0; s < nst; ++s) mbar_init(&full[s], 1);
+    if (warp == 0) {
+      mbar_init(ready, W);
+      mbar_init(consumed, W);
+      *abort_flag = 0;
+    }
     fence_barrier_init();
   }
-  if (threadIdx.x < p.nq) {  // pair q = this thread's: its slot
-    int sl = 0;
-    for (; sl < PX - 1; ++sl) {
-      const int gi = sl < Z ? 0 : Z + (sl - Z) / 2;
-      const int px = sl < Z ? max(p.gx_plus[0], p.gx_minus[0]) : ((sl - Z) & 1 ? p.gx_minus[gi] : p.gx_plus[gi]);
-      if (px == p.q_ix[threadIdx.x]) break;
-    }
-    qslot[threadIdx.x] = (uint8_t)sl;
-  }
-  for (int e = threadIdx.x; e < kMomBatchMaxExt * kMomMaxL; e += 32 * W) tab[e] = p.tab[e / kMomMaxL][e % kMomMaxL];
-  for (int e = threadIdx.x; e < kMomQChunk * kRowMax; e += 32 * W) ph[e] = make_float4(0.f, 0.f, 0.f, 0.f);
-  __syncthreads();
-  if (threadIdx.x < 32) {  // the pairs in the order of their slots, and each slot's first
-    int before = 0, first = 0;
-    for (int q = 0; q < p.nq; ++q) {
-      const int sl = qslot[q];
-      if (threadIdx.x < p.nq) before += sl < qslot[threadIdx.x] || (sl == qslot[threadIdx.x] && q < (int)threadIdx.x);
-      first += sl < (int)threadIdx.x;
-    }
-    if (threadIdx.x < p.nq) qlist[before] = (uint8_t)threadIdx.x;
-    if (threadIdx.x <= PX) qstart[threadIdx.x] = (uint8_t)first;
-  }
-  __syncthreads();
+  __syncwarp();
 
   const int hw = SAME ? lane >> 4 : 0;  // SAME: the half-warp's parity
   LP lp;
@@ -289,6 +270,12 @@ __global__ void __launch_bounds__(32 * W, 1)
   };
   int in_flight = 0;
   for (; in_flight < nst && fc.valid(p); ++in_flight) fetch();
+  // while they come: the tables that all warps read
+  for (int e = threadIdx.x; e < p.n_ext * kMomMaxL; e += 32 * W) tab[e] = p.tab[e / kMomMaxL][e % kMomMaxL];
+  for (int e = threadIdx.x; e < kMomQChunk * kRowMax; e += 32 * W) ph[e] = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (threadIdx.x < sizeof(p.pairs) / 4)
+    reinterpret_cast<uint32_t *>(smem + kRowQ)[threadIdx.x] = reinterpret_cast<const uint32_t *>(&p.pairs)[threadIdx.x];
+  __syncthreads();
 
   int cstage = 0;
   uint32_t cphase = 0;
@@ -511,7 +498,7 @@ template <int Z, int NS, bool SAME> cudaError_t launch_rows(const Job &job, cons
   // sums a lane and spills there (0.649 ms at 32^3 x 32, 0.541 with eight warps).
   // Two fields and up to three slots leave room to unroll the products' colour
   // loop (one slot 0.543 -> 0.474 ms, three 0.627 -> 0.595; five 0.758 -> 0.830).
-  constexpr int W = SAME && NS >= 2 ? 8 : 12, UNROLL = !SAME && NS <= 1 ? 9 : 3;
+  constexpr int W = SAME && NS >= 2 ? 8 : 12, UNROLL = NS == 0 || (!SAME && NS == 1) ? 9 : 3;
   constexpr size_t kMax = 232448;
   constexpr size_t stage = (size_t)W * 2 * kSiteBytes, fixed = kRowG + sizeof(float2) * 256 * W * (Z + 2 * NS);
   constexpr int stages = std::min<int>(kRowMaxStages, (kMax - fixed) / stage);
@@ -547,6 +534,23 @@ template <bool SAME> cudaError_t launch_rows_groups(const Job &job, const MomBat
 }
 
 } // namespace
+
+void order_pairs(MomBatchParams &p)
+{
+  const int zero = p.gx_k[0] == 0 ? 1 : 0, slots = zero + 2 * (p.ngx - zero);
+  auto px = [&](int slot) {  // the nx of a slot; -1: none (a group without its partner)
+    if (slot < zero) return std::max(p.gx_plus[0], p.gx_minus[0]);
+    const int group = zero + (slot - zero) / 2;
+    return (slot - zero) & 1 ? p.gx_minus[group] : p.gx_plus[group];
+  };
+  int n = 0;
+  for (int slot = 0; slot < slots; ++slot) {
+    p.pairs.start[slot] = (uint8_t)n;
+    for (int q = 0; q < p.nq; ++q)
+      if (p.q_ix[q] == px(slot)) p.pairs.list[n++] = (uint8_t)q;
+  }
+  p.pairs.start[slots] = (uint8_t)n;
+}
 
 cudaError_t launch_momentum_rows(const Job &job, const MomBatchParams &p, bool same_field)
 {

@@ -99,9 +99,18 @@ struct MomBatchItem {
   uint8_t tx, ty, tz;   // phase table of the x, y and z extents
 };
 
+// The (nx, ny) pairs in the order of the X sums that they use: list[start[s]] up to
+// list[start[s + 1]] are those of slot s (nx = 0 if there is one, then +k and -k of each
+// other X group).
+struct PairOrder {
+  uint8_t list[28], start[8];
+};
+
 struct MomBatchParams {
   DeviceStatus *status;
   int n_items, total_units, total_fin;
+  int n_ext;        // distinct extents with a table
+  PairOrder pairs;  // set by order_pairs
   int ngx, nq, np;
   int gx_k[kMomMaxPx], gx_plus[kMomMaxPx], gx_minus[kMomMaxPx];
   int q_ix[kMomQChunk], q_ny[kMomQChunk];
@@ -125,6 +134,8 @@ struct BaryonFinParams {
   BaryonFinItem items[kMomBatchMaxItems];
 };
 
+// Fills p.pairs from the X groups and pairs.
+void order_pairs(MomBatchParams &p);
 // One persistent launch of the row kernel (kernels_momentum_rows.cu) over every
 // item's planes.
 cudaError_t launch_momentum_rows(const Job &job, const MomBatchParams &p, bool same_field);
