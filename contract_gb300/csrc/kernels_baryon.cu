@@ -5,10 +5,12 @@
 
 namespace cgb {
 
-template <class Op> static cudaError_t run_rank(const Job &job, OpParams<typename Op::R> p)
+// One or two factors: kernels of their own, each with the registers that its sums need.
+template <class R, class S, int CW, int NST, int MINB> static cudaError_t run_rank(const Job &job, OpParams<R> p)
 {
   fill_fused_spin(p, false);
-  return run_ring<Op>(job, p);
+  return p.b.rk.r == 2 ? run_ring<BaryonTriRankOp<R, S, CW, NST, MINB, true>>(job, p)
+                       : run_ring<BaryonTriRankOp<R, S, CW, NST, MINB, false>>(job, p);
 }
 
 // complex128 on the integer pipe (fixed.cuh): bound by IMAD.WIDE issue and the
@@ -29,8 +31,8 @@ static const VariantSet<double, 4> kTriP = {
   {"w12.st1.occ1", "w2.st1.occ5", "w4.st1.occ2", "w10.st1.occ1"},
   0};
 static const VariantSet<double, 4> kTriRankP = {
-  {run_rank<BaryonTriRankOp<double, double2, 4, 1, 3>>, run_rank<BaryonTriRankOp<double, double2, 12, 1, 1>>,
-   run_rank<BaryonTriRankOp<double, double2, 4, 1, 2>>, run_rank<BaryonTriRankOp<double, double2, 10, 1, 1>>},
+  {run_rank<double, double2, 4, 1, 3>, run_rank<double, double2, 12, 1, 1>,
+   run_rank<double, double2, 4, 1, 2>, run_rank<double, double2, 10, 1, 1>},
   {"w4.st1.occ3", "w12.st1.occ1", "w4.st1.occ2", "w10.st1.occ1"},
   0};
 static const VariantSet<double, 4> kTriGammaP = {
@@ -54,8 +56,8 @@ static const VariantSet<float, 4> kTriM = {
   {"w4.st1.occ5", "w4.st2.occ3", "w3.st2.occ4", "w4.st1.occ4"},
   0};
 static const VariantSet<float, 4> kTriRankM = {
-  {run_rank<BaryonTriRankOp<float, float2, 4, 1, 3>>, run_rank<BaryonTriRankOp<float, float2, 3, 1, 5>>,
-   run_rank<BaryonTriRankOp<float, float2, 5, 1, 3>>, run_rank<BaryonTriRankOp<float, float2, 8, 1, 2>>},
+  {run_rank<float, float2, 4, 1, 3>, run_rank<float, float2, 3, 1, 5>,
+   run_rank<float, float2, 5, 1, 3>, run_rank<float, float2, 8, 1, 2>},
   {"w4.st1.occ3", "w3.st1.occ5", "w5.st1.occ3", "w8.st1.occ2"},
   0};
 static const VariantSet<float, 4> kTriGammaM = {

@@ -304,33 +304,44 @@ template <class R> __device__ __forceinline__ bool rank_unit_form(const RankForm
   return sizeof(R) == 8 && rk.unit;
 }
 
-// One combined block: side 0, X_r from a row of B (blocks 9 apart); side 1, Y_r
-// from a column of P_n (blocks 36 apart).
-template <class R, class S>
-__device__ __forceinline__ void rank_block(const RankForm<R> &rk, bool unit, int side, int r, const S *base, int stride,
-                                           cx<R> (&o)[9])
+// N colour entries of one combined block from entry `first` on (past the ninth: the ninth
+// again): side 0, X_r from a row of B (blocks 9 apart); side 1, Y_r from a column of P_n
+// (blocks 36 apart).  Part of a block: two terms' loads are in flight.
+template <int N, class R, class S>
+__device__ __forceinline__ void rank_entries(const RankForm<R> &rk, bool unit, int side, int r, const S *base, int stride,
+                                             int first, cx<R> (&o)[N])
 {
+  int at[N];
+#pragma unroll
+  for (int t = 0; t < N; ++t) at[t] = N == 9 ? t : min(first + t, 8);
   if (unit) {
-    load9(o, base + rk.idx[side][r][0] * stride);
-    phase9(o, rk.ph[side][r][0]);
+    const S *src = base + rk.idx[side][r][0] * stride;
+#pragma unroll
+    for (int t = 0; t < N; ++t) o[t] = mul_phase(ld<R>(src + at[t]), rk.ph[side][r][0]);
 #pragma unroll 1
     for (int k = 1; k < rk.nnz; ++k) {
-      const S *src = base + rk.idx[side][r][k] * stride;
+      src = base + rk.idx[side][r][k] * stride;
       const uint32_t ph = rk.ph[side][r][k];
 #pragma unroll
-      for (int t = 0; t < 9; ++t) o[t] = cadd(o[t], mul_phase(ld<R>(src + t), ph));
+      for (int t = 0; t < N; ++t) o[t] = cadd(o[t], mul_phase(ld<R>(src + at[t]), ph));
     }
     return;
   }
 #pragma unroll
-  for (int k = 0; k < 9; ++k) o[k] = czero<R>();
-#pragma unroll 1
+  for (int t = 0; t < N; ++t) o[t] = czero<R>();
+#pragma unroll (N < 9 ? 2 : 1)
   for (int k = 0; k < rk.nnz; ++k) {
     const S *src = base + rk.idx[side][r][k] * stride;
     const cx<R> c {rk.c[side][r][k][0], rk.c[side][r][k][1]};
 #pragma unroll
-    for (int t = 0; t < 9; ++t) cfma(o[t], c, ld<R>(src + t));
+    for (int t = 0; t < N; ++t) cfma(o[t], c, ld<R>(src + at[t]));
   }
+}
+template <class R, class S>
+__device__ __forceinline__ void rank_block(const RankForm<R> &rk, bool unit, int side, int r, const S *base, int stride,
+                                           cx<R> (&o)[9])
+{
+  rank_entries<9>(rk, unit, side, r, base, stride, 0, o);
 }
 
 // Y_r[q] = sum_n y_r[n] N[n][q] at block r*4 + q of y.

@@ -136,7 +136,7 @@ struct BaryonTriGammaOp : RingOp<R, S, CW, TPS, NST, MINB> {
 // memory 12 warps of 4 sites share an SM, 1.49 ms at 24^3 x 32 with two factors and
 // 1.15 with one (without the L2 prefetch of the two 1.52 and 1.18; P_j staged too, 8
 // warps: 1.73 and 1.35).
-template <class R, class S, int CW, int NST, int MINB>
+template <class R, class S, int CW, int NST, int MINB, bool TWO>
 struct BaryonTriRankOp : RingOp<R, S, CW, 8, NST, MINB> {
   static constexpr bool CHANGES_INPUT = true;
   static constexpr int DIRECT = sizeof(R) == 8 ? 2 : 0, NIN = 3 - DIRECT;
@@ -154,24 +154,37 @@ struct BaryonTriRankOp : RingOp<R, S, CW, 8, NST, MINB> {
     const BaryonSpin<R> &b = p.b;
     const RankForm<R> &rk = b.rk;
     const FusedSpin f = b.fu;
-    const bool unit = rank_unit_form(rk), two = rk.r == 2;
+    const bool unit = rank_unit_form(rk);
+    // One factor, from memory: threads sub and sub + 4 form five entries of X[sub] and Y[sub]
+    // each (the ninth twice in effect), half the loads and FP64 adds.
+    constexpr int NE = 5;
+    const int e0 = (sub >> 2) * NE;
     {
-      cx<R> o[9];
-      rank_block(rk, unit, 0, two ? sub >> 2 : 0, B + (sub & 3) * 36, 9, o);
-      __syncwarp();  // B, whose place X may take, has been read
-      if (two || sub < 4) {
+      const S *row = B + (sub & 3) * 36;
+      if constexpr (DIRECT && !TWO) {  // two threads share a block
+        cx<R> o[NE];
+        rank_entries<NE>(rk, unit, 0, 0, row, 9, e0, o);
 #pragma unroll
-        for (int k = 0; k < 9; ++k) st(X + sub * 9 + k, o[k]);
+        for (int k = 0; k < NE; ++k)
+          if (e0 + k < 9) st(X + (sub & 3) * 9 + e0 + k, o[k]);
+      } else {
+        cx<R> o[9];
+        rank_block(rk, unit, 0, TWO ? sub >> 2 : 0, row, 9, o);
+        __syncwarp();  // B, whose place X may take, has been read
+        if (TWO || sub < 4) {
+#pragma unroll
+          for (int k = 0; k < 9; ++k) st(X + sub * 9 + k, o[k]);
+        }
       }
     }
     __syncwarp();
-    const int l = sub & 3, r = two ? sub >> 2 : 0, k0 = two ? 0 : (sub >> 2) * 2, k1 = two ? 4 : k0 + 2;
+    const int l = sub & 3, r = TWO ? sub >> 2 : 0, k0 = TWO ? 0 : (sub >> 2) * 2, k1 = TWO ? 4 : k0 + 2;
     const int s = l ^ ((f.s >> 2) & 3), s1 = f.s & 3, turn = (f.rows >> 8) & 7;
     cx<R> d[9];
     bool done = false;
     if constexpr (sizeof(R) == 8) {
       FixedScales fs;
-      S *own = X + (two ? sub : sub & 3) * 9;
+      S *own = X + (TWO ? sub : sub & 3) * 9;
       const double2 *blk[3] = {A + sub * 9, A + (sub + 8) * 9, own};
       uint32_t near[3];
       bool ok = fixed_scales<8, 2>(blk, fs, near);
@@ -183,13 +196,13 @@ struct BaryonTriRankOp : RingOp<R, S, CW, 8, NST, MINB> {
         const uint32_t lo = __shfl_sync(0xffffffffu, w0, xb & 7, 8), hi = __shfl_sync(0xffffffffu, w1, xb & 7, 8);
         c |= wedge_cover(xb & 8 ? hi : lo, __shfl_sync(0xffffffffu, wx, r * 4 + (i ^ s1), 8));
       }
-      if (!two) c |= __shfl_xor_sync(0xffffffffu, c, 4);  // the two halves of the rows meet in the dot with Y
+      if constexpr (!TWO) c |= __shfl_xor_sync(0xffffffffu, c, 4);  // the two halves of the rows meet in the dot with Y
       ok = wedges_covered(c) && ok;
       done = __all_sync(0xffffffffu, ok || !live);
       if (done) {
         block_to_fixed(reinterpret_cast<int4 *>(A + sub * 9), blk[0], fs, 0);
         block_to_fixed(reinterpret_cast<int4 *>(A + (sub + 8) * 9), blk[1], fs, 0);
-        if (two || sub < 4) block_to_fixed(reinterpret_cast<int4 *>(own), own, fs, 1);
+        if (TWO || sub < 4) block_to_fixed(reinterpret_cast<int4 *>(own), own, fs, 1);
         __syncwarp();
         const int4 *Af = reinterpret_cast<const int4 *>(A), *Xf = reinterpret_cast<const int4 *>(X);
         fixed_wedge_sum(k0, k1, fs, [&](int k, const int4 *&x, const int4 *&y) {
@@ -223,7 +236,18 @@ struct BaryonTriRankOp : RingOp<R, S, CW, 8, NST, MINB> {
       }
     }
     cx<R> y[9];
-    rank_block(rk, unit, 1, r, N + l * 9, 36, y);
+    if constexpr (DIRECT && !TWO) {
+      cx<R> o[NE];
+      rank_entries<NE>(rk, unit, 1, 0, N + l * 9, 36, e0, o);
+#pragma unroll
+      for (int k = 0; k < NE; ++k) {
+        const cx<R> p = shfl_xor(o[k], 4);
+        y[k] = sub & 4 ? p : o[k];
+        if (NE + k < 9) y[NE + k < 9 ? NE + k : 0] = sub & 4 ? o[k] : p;
+      }
+    } else {
+      rank_block(rk, unit, 1, r, N + l * 9, 36, y);
+    }
     const cx<R> v = mul_phase(signed_by(dot9(d, y), f.neg, l), f.out & 3u);
     const R sc = unit ? rk.scale : R(1);
     return {v.x * sc, v.y * sc};
