@@ -58,12 +58,14 @@ template <int TPS> __device__ __forceinline__ int group_max(int v)
   return v;
 }
 
-// The bits of the values of a site's TPS threads.
-template <int TPS> __device__ __forceinline__ uint32_t group_or(uint32_t v)
+// The same for two values of 16 bits at a time.
+template <int TPS> __device__ __forceinline__ void group_max(int &lo, int &hi)
 {
+  unsigned int v = ((unsigned int)lo & 0xffffu) | (unsigned int)hi << 16;
 #pragma unroll
-  for (int o = TPS / 2; o > 0; o >>= 1) v |= __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
+  for (int o = TPS / 2; o > 0; o >>= 1) v = __vmaxs2(v, __shfl_xor_sync(0xffffffffu, v, o));
+  lo = (short)v;
+  hi = (int)v >> 16;
 }
 
 // The scales of one site: entry [a][d] of field f at 2^(E[f] + r[a] + c[d] - 1023).
@@ -79,48 +81,54 @@ template <int TPS, int NA, int N>
 __device__ __forceinline__ bool fixed_scales(const double2 *const (&blk)[N], FixedScales &f, uint32_t (&near)[N])
 {
   f.E[0] = f.E[1] = 0;
-  int e[N][9];  // high words without the sign, then biased exponents (0: zero or denormal)
+  // High words without the sign: biased exponent from bit 20 on.  Differences of them
+  // wrap only where the values are refused anyway.
+  unsigned int e[N][9];
 #pragma unroll
   for (int n = 0; n < N; ++n) {
-    int most = 0;
+    unsigned int most = 0;
 #pragma unroll
     for (int k = 0; k < 9; ++k) {
       const double2 v = blk[n][k];
-      e[n][k] = max(__double2hiint(v.x) & 0x7fffffff, __double2hiint(v.y) & 0x7fffffff);
+      e[n][k] = max((unsigned int)__double2hiint(v.x) & 0x7fffffffu, (unsigned int)__double2hiint(v.y) & 0x7fffffffu);
       most = max(most, e[n][k]);
     }
-    near[n] = 0;
-    f.E[n < NA ? 0 : 1] = max(f.E[n < NA ? 0 : 1], most >> 20);
+    f.E[n < NA ? 0 : 1] = max(f.E[n < NA ? 0 : 1], (int)(most >> 20));
   }
-  f.E[0] = group_max<TPS>(f.E[0]);
-  f.E[1] = NA < N ? group_max<TPS>(f.E[1]) : f.E[0];
+  group_max<TPS>(f.E[0], f.E[1]);
+  if (NA == N) f.E[1] = f.E[0];
   const bool ok = min(f.E[0], f.E[1]) >= kFixedMinExp && max(f.E[0], f.E[1]) <= kFixedMaxExp;
-  // Exponents of zeros (0) lie more than kFixedColour below every field's scale.
+  // Rows, then columns in the scales of the rows.  Zeros (0) lie more than kFixedColour
+  // below every scale.
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    f.r[a] = -kFixedColour;
+#pragma unroll
+    for (int n = 0; n < N; ++n)
+      f.r[a] = max(f.r[a], (int)(max(max(e[n][3 * a], e[n][3 * a + 1]), e[n][3 * a + 2]) >> 20) - f.E[n < NA ? 0 : 1]);
+  }
+  group_max<TPS>(f.r[0], f.r[1]);
+  f.r[2] = group_max<TPS>(f.r[2]);
 #pragma unroll
   for (int n = 0; n < N; ++n)
 #pragma unroll
-    for (int k = 0; k < 9; ++k) e[n][k] >>= 20;
+    for (int k = 0; k < 9; ++k) e[n][k] -= (unsigned int)f.r[k / 3] << 20;
 #pragma unroll
-  for (int a = 0; a < 3; ++a) {
-    int m = -kFixedColour;
-#pragma unroll
-    for (int n = 0; n < N; ++n)
-      m = max(m, max(max(e[n][3 * a], e[n][3 * a + 1]), e[n][3 * a + 2]) - f.E[n < NA ? 0 : 1]);
-    f.r[a] = group_max<TPS>(m);
-  }
-#pragma unroll
-  for (int d = 0; d < 3; ++d) {  // the columns' largest in the scales of the rows
-    int m = -kFixedColour;
+  for (int d = 0; d < 3; ++d) {
+    f.c[d] = -kFixedColour;
 #pragma unroll
     for (int n = 0; n < N; ++n)
-      m = max(m, max(max(e[n][d] - f.r[0], e[n][3 + d] - f.r[1]), e[n][6 + d] - f.r[2]) - f.E[n < NA ? 0 : 1]);
-    f.c[d] = group_max<TPS>(m);
+      f.c[d] = max(f.c[d], (int)(max(max(e[n][d], e[n][3 + d]), e[n][6 + d]) >> 20) - f.E[n < NA ? 0 : 1]);
   }
+  group_max<TPS>(f.c[0], f.c[1]);
+  f.c[2] = group_max<TPS>(f.c[2]);
 #pragma unroll
-  for (int k = 0; k < 9; ++k) {
-    const int scale = f.r[k / 3] + f.c[k % 3] - kFixedNear;
+  for (int n = 0; n < N; ++n) {
+    unsigned int far = 0;  // the sign of what an entry lies above the limit, entry by entry
 #pragma unroll
-    for (int n = 0; n < N; ++n) near[n] |= (uint32_t)(e[n][k] >= f.E[n < NA ? 0 : 1] + scale) << k;
+    for (int k = 8; k >= 0; --k)
+      far = __funnelshift_l(e[n][k] - ((unsigned int)(f.E[n < NA ? 0 : 1] + f.c[k % 3] - kFixedNear) << 20), far, 1);
+    near[n] = ~far & 0x1ffu;
   }
   return ok;
 }
@@ -142,6 +150,12 @@ __device__ __forceinline__ uint32_t wedge_cover(uint32_t x, uint32_t y)
 {
   const uint32_t z = __byte_perm(y, 0, 0x1032);
   return ((x >> 3) & (z >> 6)) | ((x >> 6) & (z >> 3));
+}
+// The covers of a site's 16 threads, or-ed (both sites of the warp at once).
+__device__ __forceinline__ uint32_t site_cover(uint32_t c)
+{
+  const uint32_t at = threadIdx.x & 16u;
+  return __reduce_or_sync(0xffffffffu, ((c | c >> 16) & 0x1ffu) << at) >> at;
 }
 // Whether the covers of a sum's wedges, or-ed, leave no entry out.
 __device__ __forceinline__ bool wedges_covered(uint32_t c) { return ((c | c >> 16) & 0x1ffu) == 0x1ffu; }

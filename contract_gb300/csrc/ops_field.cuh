@@ -150,7 +150,7 @@ struct WedgeFieldOp : RingOp<R, S, CW, 16, NST, MINB> {
     if constexpr (sizeof(R) == 8) {
       FixedScales fs;
       if (fields_to_fixed(A, B, sub, live, fs, [&](uint32_t x, uint32_t y) {
-            return group_or<16>(wedge_cover(block_word(x, xb), block_word(y, yb)));
+            return site_cover(wedge_cover(block_word(x, xb), block_word(y, yb)));
           })) {
         const uint32_t common = (b.ph1[0][0] & 1u) + (b.ph2[0][0] & 1u);
         const longlong2 d = fixed_wedge_scatter(reinterpret_cast<const int4 *>(A) + xb * 9,

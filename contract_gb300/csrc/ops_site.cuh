@@ -35,7 +35,7 @@ struct BaryonLoopOp : RingOp<R, S, CW, TPS, NST, MINB> {
       FixedScales fs;
       const int i = sub >> 2, l = sub & 3, xb = i * 4 + b.perm2[l], yb = b.perm1[i] * 4 + l;
       if (fields_to_fixed(in[0], in[1], sub, live, fs, [&](uint32_t x, uint32_t y) {
-            return group_or<16>(wedge_cover(block_word(x, xb), block_word(y, yb)));
+            return site_cover(wedge_cover(block_word(x, xb), block_word(y, yb)));
           })) {
         // all wedges of the site have one scale: they meet as integers, entry e of
         // the sum with thread e, which multiplies it by Q's
