@@ -1,4 +1,6 @@
-// Tile pipeline of the all-types baryon pass: every warp streams its own tiles.
+// Tile pipelines in which every warp streams its own tiles: warp_kernel for the all-types
+// baryon pass, ring_kernel for the per-call contractions, field_ring_kernel for diquark
+// and sequential sources.  First the all-types pass.
 //
 // A tile is SPW = 32 / TPS consecutive sites of one reduction segment (a
 // half-timeslice, or the whole volume for per-site outputs); chunks of tiles

@@ -16,8 +16,12 @@ template <class R, class S, int CW, int NST, int MINB> static cudaError_t run_ra
 // complex128 on the integer pipe (fixed.cuh): bound by IMAD.WIDE issue and the
 // conversions, so warps in flight count and a second ring stage, which costs warps,
 // does not pay.  24^3 x 32 per site, three different fields, ms (the FP64 kernels
-// that these replaced in brackets): loop 0.89 [2.86 with a projector of two terms],
-// one gamma matrix 2.32, dense projector 3.50, rank 2 1.49 [4.65], rank 1 1.15.
+// that these replaced in brackets): loop 0.91 [2.86 with a projector of two terms],
+// one gamma matrix 2.33, dense projector 3.43, rank 2 1.45 [4.65], a polarised projector
+// (rank 1) 1.02, four terms a vector 1.69.  On fields that the integer form refuses, at
+// 24^3 x 16 (replaced kernels in brackets; accepted in parentheses): loop 1.26 [1.46]
+// (0.54), gamma 3.70 [3.78] (1.19), dense 4.46 to 4.70 [4.65] (1.78), rank 2 2.15 [2.35]
+// (0.78), rank 1 1.25 to 1.65 [1.52 to 2.09] (0.55 to 0.88).
 static const VariantSet<double, 4> kLoopP = {
   {run_ring<BaryonLoopOp<double, double2, 4, 16, 1, 3>>, run_ring<BaryonLoopOp<double, double2, 4, 16, 1, 2>>,
    run_ring<BaryonLoopOp<double, double2, 2, 16, 1, 6>>, run_ring<BaryonLoopOp<double, double2, 13, 16, 1, 1>>},

@@ -24,10 +24,10 @@ template <Wedges KIND> static VariantSet<float, 4> shapes_m()
           {"w4.st2.occ5", "w4.st3.occ4", "w4.st2.occ6", "w4.st4.occ3"},
           0};
 }
-// complex128: integer pipe.  24^4, ms in this order: four wedges a block 1.76 to 1.80,
-// 1.85 to 1.87, 1.83 to 1.86 (5.2 to 5.7 in FP64), the closed loop 0.80, 0.88, 0.85
-// (2.29).  One wedge a block runs in FP64 (WedgeFieldOp::with_q): 0.94 at 24^3 x 16 in the second shape (0.98 on a
-// CTA-wide ring).
+// complex128: integer pipe.  24^4, ms in this order: four wedges a block 1.83 to 1.88,
+// 1.90 to 1.93, 1.88 to 1.90 (5.2 to 5.7 in FP64 on a CTA-wide ring; where the fields refuse the
+// integer form 5.3), the closed loop 0.75, 0.86, 0.82 (2.29).  One wedge a block runs in
+// FP64 (WedgeFieldOp::with_q): 1.71, 1.44, 1.44.
 template <Wedges KIND> static VariantSet<double, 3> shapes_p()
 {
   return {{wedges<double, double2, 4, 3, 2, KIND>, wedges<double, double2, 4, 2, 3, KIND>,

@@ -23,7 +23,7 @@ static cudaError_t fused(const Job &job, OpParams<R> q)
 
 // complex64 tile shapes: 16 threads a site (one block of G each) or 8 (two blocks of G each, which share the
 // loads of one P_i block and take half the reduction).  At 24^3 x 64 with two projectors, two fields / one field:
-// w12.tps8 0.590 / 0.428 ms, w4.tps8.occ2 0.604 / 0.418, w4.tps8.occ3 0.611 / 0.425, w4.tps16.occ5 0.666 / 0.462.
+// in this order 0.588 / 0.426 ms, 0.613 / 0.421, 0.622 / 0.429, 0.624 / 0.430, 0.636 / 0.437 and 0.675 / 0.473.
 template <int SRC, int NW, bool SAME> static VariantSet<float, 7> shapes_m(int def)
 {
   return {{fused<float, float2, 12, 8, SRC, NW, SAME, 1>, fused<float, float2, 4, 8, SRC, NW, SAME, 2>,
@@ -37,8 +37,8 @@ template <int SRC, int NW, bool SAME> static VariantSet<float, 7> shapes_m(int d
 static const VariantSet<float, 7> kFused1M = shapes_m<1, 1, false>(0), kFused2M = shapes_m<2, 2, false>(0),
                                   kSame1M = shapes_m<1, 1, true>(1), kSame2M = shapes_m<2, 2, true>(1);
 
-// complex128 (integer pipe, fixed.cuh): 16^3 x 48 with two projectors, 1.57 ms; with dearer conversions 1.76, 1.87 and 2.13 in this order (FP64
-// only: 4.24).
+// complex128 (integer pipe, fixed.cuh): 16^3 x 48 with two projectors, ms in this order, 1.59, 1.80 and 1.64
+// (in FP64 only 4.24; the shared-wedge FP64 kernel before it 7.28).
 template <int SRC, int NW> static VariantSet<double, 3> shapes_p()
 {
   return {{fused<double, double2, 4, 16, SRC, NW, false, 3>, fused<double, double2, 4, 16, SRC, NW, false, 2>,

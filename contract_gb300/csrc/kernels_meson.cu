@@ -6,7 +6,7 @@
 namespace cgb {
 
 // One Gamma pair.  complex128: FP64 pipe and HBM within a third of each other;
-// 0.515 ms at 24^3 x 32 per site, 0.305 of it the two fields at the copy rate.
+// 0.51 ms at 24^3 x 32 per site, 0.305 of it the two fields at the copy rate.
 static const VariantSet<double, 4> kMesonP = {
   {run_ring<MesonOp<double, double2, 4, 8, 1, 3>>, run_ring<MesonOp<double, double2, 2, 8, 2, 3>>,
    run_ring<MesonOp<double, double2, 4, 16, 1, 5>>, run_ring<MesonOp<double, double2, 4, 16, 2, 2>>},

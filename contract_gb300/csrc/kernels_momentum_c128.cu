@@ -8,9 +8,10 @@
 // Lx - x of a row (0 and Lx / 2 together), leaves their 2 x 256 pairs in its slot of
 // shared memory and goes on to its next sites while the X warps, a thread per 4 or 8
 // pairs, add the slots up in the order of x.  Only the X sums of a row leave the chip.
-// 1.29 ms (both pipes about 60 % busy) where pairs, X and Y transform in two launches
-// took 1.68 and the FP64 form 4.60; 24^3 x 16: one momentum 1.15 (1.60), 27 momenta 1.32
-// (2.06), 125 momenta 1.72 (2.49).  Twelve pair warps make as many pairs as 16 did with
+// 1.23 ms (both pipes about 60 % busy) where pairs, X and Y transform in two launches
+// took 1.68 and the FP64 form 4.60; 24^3 x 16: one momentum 1.15 (1.60), 27 momenta 1.30
+// (2.06), 125 momenta 1.68 (2.49), and 27 momenta where the fields refuse the integer form
+// 5.52 (5.67 in the FP64 form).  Twelve pair warps make as many pairs as 16 did with
 // an SM of their own.
 #include "launch_variants.cuh"
 #include "momentum.hpp"

@@ -29,7 +29,7 @@
 // hand-off per product.  Before and after, with the finalisation, at 32^3 x 64:
 //   momenta            125 two fields   27 two    27 one    125 one   zero alone
 //   hand-off           1.784 ms         1.637     1.495     1.699     1.596
-//   this kernel        1.632 ms         1.218     0.867     1.186     0.956
+//   this kernel        1.598 ms         1.178     0.852     1.159     0.931
 // A 4 x 4 tile of 16 lanes a site reads less shared memory but takes 255 registers
 // (two warps a scheduler) and was slower: 0.94 ms against 0.76 at 32^3 x 32.
 //
@@ -496,8 +496,9 @@ template <int Z, int NS, bool SAME> cudaError_t launch_rows(const Job &job, cons
 {
   // Twelve warps have 168 registers; the one-field form of five slots holds 90
   // sums a lane and spills there (0.649 ms at 32^3 x 32, 0.541 with eight warps).
-  // Two fields and up to three slots leave room to unroll the products' colour
-  // loop (one slot 0.543 -> 0.474 ms, three 0.627 -> 0.595; five 0.758 -> 0.830).
+  // Two fields and up to three slots, and one field and one slot, leave room to unroll the
+  // products' colour loop (0.543 -> 0.474 ms, 0.627 -> 0.595 and 0.369 -> 0.359; two fields
+  // and five slots 0.758 -> 0.830).
   constexpr int W = SAME && NS >= 2 ? 8 : 12, UNROLL = NS == 0 || (!SAME && NS == 1) ? 9 : 3;
   constexpr size_t kMax = 232448;
   constexpr size_t stage = (size_t)W * 2 * kSiteBytes, fixed = kRowG + sizeof(float2) * 256 * W * (Z + 2 * NS);

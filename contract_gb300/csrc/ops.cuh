@@ -135,7 +135,7 @@ __device__ __forceinline__ void build_q(const BaryonSpin<R> &b, const S *N, S *q
       // complex128: W's nonzero entries from the host's list.  Testing each
       // entry here takes FP64 compares on the FP64 pipe, half busy in the loop
       // form; for the same reason a real or imaginary entry takes two FMAs, not
-      // four ((1 + g4)/2: 0.96 ms at 24^3 x 32, one gamma matrix 0.88).
+      // four ((1 + g4)/2: 0.99 ms at 24^3 x 32, one gamma matrix 0.91).
 #pragma unroll 1
       for (int t = 0; t < pw.nnz; ++t) {
         const int k = pw.nzk[t];  // W[m][n], m = k / 4, n = k % 4, times N[n][m]

@@ -17,8 +17,9 @@
 // (include/baryon_sequential.cuh:36-163).  The summed index runs over the negative
 // terms first, so that the signs cost one negation of the sum.
 //
-// Complex64 is HBM bound, two fields in and one out.  Complex128 takes its wedges on
-// the integer pipe where a site allows it (fixed.cuh), else in FP64.
+// Complex64 is HBM bound, two fields in and one out.  Complex128 takes its sums of wedges
+// on the integer pipe where a site allows it (fixed.cuh), else, and for one wedge a block,
+// in FP64.
 #pragma once
 
 #include "ops_site.cuh"

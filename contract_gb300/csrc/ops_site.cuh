@@ -133,9 +133,10 @@ struct BaryonTriGammaOp : RingOp<R, S, CW, TPS, NST, MINB> {
 // X_r[perm1 i] over its rows i, then one dot with Y_r[l].  Complex64 writes X over
 // P_j's blocks (X_r[j] at block 4 r + j).  Complex128 reads P_j and P_n, every block of
 // which is used about once, from memory: with one field and X of a site in shared
-// memory 12 warps of 4 sites share an SM, 1.49 ms at 24^3 x 32 with two factors and
-// 1.15 with one (without the L2 prefetch of the two 1.52 and 1.18; P_j staged too, 8
-// warps: 1.73 and 1.35).
+// memory 12 warps of 4 sites share an SM, 1.45 ms at 24^3 x 32 with two factors, 1.02
+// with one of two terms a vector, 1.69 with one of four.  Before the two had kernels of
+// their own it was 1.49 with two; without the L2 prefetch of the fields read from memory
+// 1.52; with P_j staged too, 8 warps, 1.73.
 template <class R, class S, int CW, int NST, int MINB, bool TWO>
 struct BaryonTriRankOp : RingOp<R, S, CW, 8, NST, MINB> {
   static constexpr bool CHANGES_INPUT = true;

@@ -5,6 +5,10 @@
  * callers otherwise do themselves (per-timeslice sums, many contraction types
  * per pass, precision choice) plus error reporting and stream control.
  *
+ * Complex128 calls (drop-in ones included) form sums of products in 64-bit
+ * fixed point where a site's values suit it and in FP64 elsewhere; every entry
+ * of a result is as exact as FP64 makes it.
+ *
  * Shared conventions (see also contract.h):
  *  - precision: CONTRACT_C128 propagators are complex128 (the drop-in format);
  *    CONTRACT_C64 propagators are complex64 and the arithmetic is FP32 with
